@@ -8,6 +8,7 @@
 #include <stdexcept>
 
 #include "kdtree_build.h"
+#include "quad_build.h"
 #include "trace_launch.h"
 #include "wr_context.h"
 
@@ -178,6 +179,7 @@ int wr_scene_upload(wr_ctx* ctx, const wr_scene_desc* d, wr_scene_id* out) {
     HostTree ht = build_reference_tree(d->vertices, d->num_vertices, gtris.data(), nt, 0);
     DeviceLayout L = layout_for_device(ht, d->vertices, d->num_vertices, gtris.data(), sc->tri_obj.data(),
                                        sc->tri_local.data());
+    QuadLayout Q = build_quads(ht, 0);
     auto t1 = std::chrono::steady_clock::now();
     WR_CUDA(ctx, cudaSetDevice(ctx->device));
     const size_t pb = sizeof(NodePair) * (L.pairs.size() ? L.pairs.size() : 1);
@@ -188,6 +190,18 @@ int wr_scene_upload(wr_ctx* ctx, const wr_scene_desc* d, wr_scene_id* out) {
         WR_CUDA(ctx, cudaMemcpy(sc->pairs.p, L.pairs.data(), sizeof(NodePair) * L.pairs.size(), cudaMemcpyHostToDevice));
     if (!L.slots.empty())
         WR_CUDA(ctx, cudaMemcpy(sc->tris.p, L.slots.data(), sizeof(TriRec) * L.slots.size(), cudaMemcpyHostToDevice));
+    const size_t qb = sizeof(QuadNode) * Q.quads.size();
+    const size_t ub = sizeof(uint32_t) * (Q.leaf_up.size() + Q.pair_up.size());
+    WR_CUDA(ctx, sc->quads.reserve(qb ? qb : 1));
+    WR_CUDA(ctx, sc->leaf_up.reserve(sizeof(uint32_t) * std::max<size_t>(1, Q.leaf_up.size())));
+    WR_CUDA(ctx, sc->pair_up.reserve(sizeof(uint32_t) * std::max<size_t>(1, Q.pair_up.size())));
+    if (qb) WR_CUDA(ctx, cudaMemcpy(sc->quads.p, Q.quads.data(), qb, cudaMemcpyHostToDevice));
+    if (!Q.leaf_up.empty())
+        WR_CUDA(ctx, cudaMemcpy(sc->leaf_up.p, Q.leaf_up.data(), sizeof(uint32_t) * Q.leaf_up.size(),
+                                cudaMemcpyHostToDevice));
+    if (!Q.pair_up.empty())
+        WR_CUDA(ctx, cudaMemcpy(sc->pair_up.p, Q.pair_up.data(), sizeof(uint32_t) * Q.pair_up.size(),
+                                cudaMemcpyHostToDevice));
     DevTree& T = sc->tree;
     T.pairs = sc->pairs.as<NodePair>();
     T.tris = sc->tris.as<TriRec>();
@@ -201,11 +215,15 @@ int wr_scene_upload(wr_ctx* ctx, const wr_scene_desc* d, wr_scene_id* out) {
     T.max_depth = ht.max_depth;
     T.num_pairs = (uint32_t)L.pairs.size();
     T.num_slots = (uint32_t)L.slots.size();
+    T.quads = qb ? sc->quads.as<QuadNode>() : nullptr;
+    T.leaf_up = sc->leaf_up.as<uint32_t>();
+    T.pair_up = sc->pair_up.as<uint32_t>();
+    T.quad_stack = Q.stack;
     sc->info.num_triangles = nt;
     sc->info.num_nodes = ht.num_nodes();
     sc->info.num_leaves = ht.num_leaves;
     sc->info.max_depth = ht.max_depth;
-    sc->info.device_bytes = pb + tb;
+    sc->info.device_bytes = pb + tb + qb + ub;
     sc->info.build_seconds = std::chrono::duration<double>(t1 - t0).count();
     sc->id = ctx->next_scene++;
     *out = sc->id;

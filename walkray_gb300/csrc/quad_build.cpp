@@ -1,0 +1,428 @@
+// quad_build.cpp — the four-wide tree over the reference tree's leaves.
+//
+// The reference's median-split tree decides which triangles a ray may hit, but
+// it is a poor order to search them in: on the 512,006-triangle mixed-material
+// scene a bounce ray visits 52 of its nodes, 17 of this tree's.  A leaf here is
+// a reference leaf with its box unchanged and a node's box is the union of
+// leaf boxes, so every triangle the reference tests is under boxes that
+// contain its leaf's: the search sees a superset of the reference's
+// candidates, and wr_quad.cuh checks the winner against the reference's own
+// boxes.
+//
+// Binned surface-area heuristic, in two levels so that it runs in parallel:
+// the reference's subtrees of at most CLUSTER leaves are the units of the
+// upper tree, and each is built over its own leaves by one thread.  The binary
+// tree is then cut into four-wide nodes by the cut of least summed area
+// (dynamic programming over the number of slots a subtree may take: Wald,
+// Benthin, Boulos 2008; Ylitie, Karras, Laine 2017).
+#include "quad_build.h"
+
+#include <algorithm>
+#include <cmath>
+#include <cstring>
+#ifdef _OPENMP
+#include <omp.h>
+#endif
+
+namespace wr {
+namespace {
+
+constexpr int BINS = 16;
+constexpr uint32_t CLUSTER = 64;
+// bin of a centre (a box of a vertex that is not finite: the first)
+int bin_of(float c, float base, float scale) {
+    const float x = (c - base) * scale;
+    return x > 0.f ? (x < (float)BINS ? (int)x : BINS - 1) : 0;
+}
+
+constexpr float NODE_COST = 1.0f, TRI_COST = 0.6f;  // one four-wide node against one triangle test
+
+struct QBox {
+    float lo[3], hi[3];
+    void clear() {
+        for (int k = 0; k < 3; k++) {
+            lo[k] = INFINITY;
+            hi[k] = -INFINITY;
+        }
+    }
+    void add(const QBox& b) {
+        for (int k = 0; k < 3; k++) {
+            lo[k] = std::min(lo[k], b.lo[k]);
+            hi[k] = std::max(hi[k], b.hi[k]);
+        }
+    }
+    float area() const {
+        const float x = hi[0] - lo[0], y = hi[1] - lo[1], z = hi[2] - lo[2];
+        return x < 0.f ? 0.f : x * y + y * z + z * x;
+    }
+};
+
+// a unit of a build: a leaf (or a cluster) with its box and triangle count
+struct Item {
+    QBox box;
+    uint32_t word;   // child word of a leaf, index of a cluster
+    uint32_t count;  // triangles
+};
+
+struct BinNode {
+    QBox box;
+    uint32_t word;       // items: Item::word
+    int32_t l, r;        // -1: an item
+    float cost[3];       // least cost in at most 1, 2, 3 slots
+    uint8_t split[2];    // slots of the left child when given 2, 3 (0: one slot fewer)
+    uint8_t split4;      // the same when given 4 (a node of its own)
+};
+
+// binary SAH tree over items[0, n); nodes appended to `out`, the root's index returned
+int32_t build_binary(Item* items, size_t n, std::vector<BinNode>& out) {
+    struct Job {
+        Item* a;
+        size_t n;
+        int32_t at;
+    };
+    const int32_t root = (int32_t)out.size();
+    out.emplace_back();
+    std::vector<Job> jobs{{items, n, root}};
+    while (!jobs.empty()) {
+        const Job j = jobs.back();
+        jobs.pop_back();
+        QBox box, cen;
+        box.clear();
+        cen.clear();
+        for (size_t i = 0; i < j.n; i++) {
+            box.add(j.a[i].box);
+            for (int k = 0; k < 3; k++) {
+                const float c = j.a[i].box.lo[k] + j.a[i].box.hi[k];
+                cen.lo[k] = std::min(cen.lo[k], c);
+                cen.hi[k] = std::max(cen.hi[k], c);
+            }
+        }
+        out[j.at].box = box;
+        if (j.n == 1) {
+            out[j.at].word = j.a[0].word;
+            out[j.at].l = out[j.at].r = -1;
+            out[j.at].cost[0] = (float)j.a[0].count;  // times area and TRI_COST below
+            continue;
+        }
+        float best = INFINITY;
+        int best_d = -1, best_s = 0;
+        float best_scale = 0.f;
+        for (int d = 0; d < 3; d++) {
+            const float w = cen.hi[d] - cen.lo[d];
+            if (!(w > 0.f)) continue;
+            const float scale = (float)BINS / w;
+            if (!(scale < INFINITY)) continue;
+            QBox bb[BINS];
+            uint32_t bc[BINS] = {};
+            for (QBox& b : bb) b.clear();
+            for (size_t i = 0; i < j.n; i++) {
+                const Item& it = j.a[i];
+                const int k = bin_of(it.box.lo[d] + it.box.hi[d], cen.lo[d], scale);
+                bb[k].add(it.box);
+                bc[k] += it.count;
+            }
+            float ra[BINS];
+            uint32_t rc[BINS], c = 0;
+            QBox acc;
+            acc.clear();
+            for (int k = BINS - 1; k > 0; k--) {
+                acc.add(bb[k]);
+                c += bc[k];
+                ra[k] = acc.area();
+                rc[k] = c;
+            }
+            acc.clear();
+            c = 0;
+            for (int k = 0; k + 1 < BINS; k++) {
+                acc.add(bb[k]);
+                c += bc[k];
+                if (!c || !rc[k + 1]) continue;
+                const float cost = acc.area() * (float)c + ra[k + 1] * (float)rc[k + 1];
+                if (cost < best) {
+                    best = cost;
+                    best_d = d;
+                    best_s = k;
+                    best_scale = scale;
+                }
+            }
+        }
+        size_t m = 0;
+        if (best_d >= 0) {
+            const float base = cen.lo[best_d];
+            m = (size_t)(std::partition(j.a, j.a + j.n, [&](const Item& it) {
+                             return bin_of(it.box.lo[best_d] + it.box.hi[best_d], base, best_scale) <= best_s;
+                         }) -
+                         j.a);
+        }
+        if (m == 0 || m == j.n) m = j.n / 2;  // equal centres: halves, in the order they have
+        const int32_t l = (int32_t)out.size();
+        out.emplace_back();
+        out.emplace_back();
+        out[j.at].l = l;
+        out[j.at].r = l + 1;
+        jobs.push_back({j.a, m, l});
+        jobs.push_back({j.a + m, j.n - m, l + 1});
+    }
+    return root;
+}
+
+// least costs of nodes [first, end) (children come after their parents).
+// `cluster_cost` (may be null): the cost of the tree below each item.
+void cut_costs(std::vector<BinNode>& nodes, int32_t first, const std::vector<float>* cluster_cost) {
+    for (int32_t i = (int32_t)nodes.size() - 1; i >= first; i--) {
+        BinNode& n = nodes[i];
+        const float a = n.box.area();
+        if (n.l < 0) {
+            const float c = cluster_cost ? (*cluster_cost)[n.word] : n.cost[0] * a * TRI_COST;
+            n.cost[0] = n.cost[1] = n.cost[2] = c;
+            continue;
+        }
+        const BinNode &l = nodes[n.l], &r = nodes[n.r];
+        const float c2 = l.cost[0] + r.cost[0];
+        const float c3a = l.cost[0] + r.cost[1], c3b = l.cost[1] + r.cost[0];
+        const float c4[3] = {l.cost[0] + r.cost[2], l.cost[1] + r.cost[1], l.cost[2] + r.cost[0]};
+        int s4 = 0;
+        for (int k = 1; k < 3; k++)
+            if (c4[k] < c4[s4]) s4 = k;
+        n.split4 = (uint8_t)(s4 + 1);
+        n.cost[0] = c4[s4] + a * NODE_COST;  // a node of its own with four slots
+        n.cost[1] = n.cost[0];
+        n.split[0] = 0;
+        if (c2 < n.cost[1]) {
+            n.cost[1] = c2;
+            n.split[0] = 1;
+        }
+        n.cost[2] = n.cost[1];
+        n.split[1] = 0;
+        if (std::min(c3a, c3b) < n.cost[2]) {
+            n.cost[2] = std::min(c3a, c3b);
+            n.split[1] = c3a <= c3b ? 1 : 2;
+        }
+    }
+}
+
+// the subtrees that fill the slots of a cut: node i with at most `slots` of them
+void cut(const std::vector<BinNode>& nodes, int32_t i, int slots, int32_t* out, int* n) {
+    const BinNode& b = nodes[i];
+    if (b.l >= 0)
+        for (; slots > 1; slots--)
+            if (b.split[slots - 2]) {
+                cut(nodes, b.l, b.split[slots - 2], out, n);
+                cut(nodes, b.r, slots - b.split[slots - 2], out, n);
+                return;
+            }
+    out[(*n)++] = i;
+}
+
+void set_child(QuadNode& q, int k, const QBox* b, uint32_t word) {
+    // an unused slot: a box that no ray meets
+    const float none_lo = 1e30f, none_hi = -1e30f;
+    (&q.lox.x)[k] = b ? b->lo[0] : none_lo;
+    (&q.loy.x)[k] = b ? b->lo[1] : none_lo;
+    (&q.loz.x)[k] = b ? b->lo[2] : none_lo;
+    (&q.hix.x)[k] = b ? b->hi[0] : none_hi;
+    (&q.hiy.x)[k] = b ? b->hi[1] : none_hi;
+    (&q.hiz.x)[k] = b ? b->hi[2] : none_hi;
+    (&q.child.x)[k] = word;
+}
+
+// the four-wide nodes of the binary tree at `root`, breadth first from
+// out[0].  Items become `word_of(item word)`; nodes' child words are indices
+// into `out`.
+template <class WordOf>
+void emit(const std::vector<BinNode>& nodes, int32_t root, std::vector<QuadNode>& out, WordOf word_of) {
+    std::vector<std::pair<int32_t, uint32_t>> todo{{root, 0u}};
+    out.emplace_back();
+    for (size_t at = 0; at < todo.size(); at++) {
+        const auto [i, q] = todo[at];
+        int32_t ch[4];
+        int n = 0;
+        if (nodes[i].l < 0) {
+            ch[n++] = i;  // a tree of one item
+        } else {
+            cut(nodes, nodes[i].l, nodes[i].split4, ch, &n);
+            cut(nodes, nodes[i].r, 4 - nodes[i].split4, ch, &n);
+        }
+        for (int k = 0; k < 4; k++) {
+            if (k >= n) {
+                set_child(out[q], k, nullptr, QUAD_HOLE);
+                continue;
+            }
+            const BinNode& c = nodes[ch[k]];
+            uint32_t word;
+            if (c.l < 0) {
+                word = word_of(c.word);
+            } else {
+                word = (uint32_t)out.size();
+                out.emplace_back();
+                todo.push_back({ch[k], word});
+            }
+            set_child(out[q], k, &c.box, word);
+        }
+    }
+}
+
+}  // namespace
+
+// the deepest walk's stack: at every node all children but the one walked into
+// wait on it
+static uint32_t stack_need(const std::vector<QuadNode>& q) {
+    std::vector<uint32_t> need(q.size(), 0u);  // entries waiting when the node is entered (parents come first)
+    uint32_t most = 0;
+    for (size_t i = 0; i < q.size(); i++) {
+        uint32_t n = 0;
+        for (int k = 0; k < 4; k++) n += (&q[i].child.x)[k] != QUAD_HOLE;
+        const uint32_t below = need[i] + (n ? n - 1 : 0);
+        most = std::max(most, below);
+        for (int k = 0; k < 4; k++) {
+            const uint32_t w = (&q[i].child.x)[k];
+            if (!(w & QUAD_LEAF)) need[w] = below;
+        }
+    }
+    return most;
+}
+
+QuadLayout build_quads(const HostTree& t, int threads) {
+    QuadLayout L;
+    const uint32_t N = t.num_nodes();
+#ifdef _OPENMP
+    if (threads <= 0) threads = omp_get_max_threads();
+#endif
+    (void)threads;
+    // parent links of the reference tree, in the device layout's numbering
+    // (pairs in pre-order, slots leaf by leaf)
+    std::vector<uint32_t> up(N, UP_ROOT), leaves_below(N, 0u);
+    L.leaf_up.resize(t.leaf_tris.size());
+    uint32_t np = 0;
+    size_t slot = 0;
+    std::vector<Item> items;
+    items.reserve(t.num_leaves);
+    std::vector<uint32_t> node_item(N, 0u);  // first item at or after each node
+    const bool fits = t.leaf_tris.size() <= QUAD_MAX_SLOTS;
+    for (uint32_t n = 0; n < N; n++) {
+        node_item[n] = (uint32_t)items.size();
+        if (t.left[n] >= 0) {
+            up[t.left[n]] = np << 1;
+            up[t.right[n]] = np << 1 | 1u;
+            L.pair_up.push_back(up[n]);
+            np++;
+            continue;
+        }
+        for (uint32_t k = 0; k < t.leaf_count[n]; k += QUAD_LEAF_MAX) {  // a longer leaf: several items, one box
+            Item it;
+            std::memcpy(it.box.lo, &t.box[6 * (size_t)n], 12);
+            std::memcpy(it.box.hi, &t.box[6 * (size_t)n + 3], 12);
+            it.count = std::min(QUAD_LEAF_MAX, t.leaf_count[n] - k);
+            it.word = QUAD_LEAF | it.count << QUAD_COUNT_AT | (uint32_t)(slot + k);
+            items.push_back(it);
+        }
+        for (uint32_t k = 0; k < t.leaf_count[n]; k++) L.leaf_up[slot + k] = up[n];
+        slot += t.leaf_count[n];
+    }
+    if (!fits) return L;
+    if (items.empty()) {  // no triangles: a root of holes
+        L.quads.emplace_back();
+        for (int k = 0; k < 4; k++) set_child(L.quads[0], k, nullptr, QUAD_HOLE);
+        return L;
+    }
+    // clusters: the reference's largest subtrees of at most CLUSTER items
+    // (a subtree's leaves are consecutive in pre-order)
+    std::vector<std::pair<uint32_t, uint32_t>> range;  // item ranges
+    {
+        std::vector<std::pair<uint32_t, uint32_t>> todo{{0u, (uint32_t)items.size()}};  // node, end of its items
+        while (!todo.empty()) {
+            const auto [n, end] = todo.back();
+            todo.pop_back();
+            const uint32_t a = node_item[n];
+            if (a == end) continue;
+            bool unit = t.left[n] < 0;
+            if (!unit && end - a <= CLUSTER) {  // compact: no gap between what the reference's plane put together
+                float sum = 0.f;
+                for (uint32_t i = a; i < end; i++) sum += items[i].box.area();
+                QBox b;
+                std::memcpy(b.lo, &t.box[6 * (size_t)n], 12);
+                std::memcpy(b.hi, &t.box[6 * (size_t)n + 3], 12);
+                unit = b.area() <= sum;
+            }
+            if (unit) {
+                range.push_back({a, end});
+                continue;
+            }
+            const uint32_t mid = node_item[t.right[n]];
+            todo.push_back({(uint32_t)t.right[n], end});
+            todo.push_back({(uint32_t)t.left[n], mid});
+        }
+    }
+    const size_t nc = range.size();
+    std::vector<std::vector<QuadNode>> sub(nc);
+    std::vector<Item> top(nc);
+    std::vector<float> sub_cost(nc);
+#ifdef _OPENMP
+#pragma omp parallel num_threads(threads)
+#endif
+    {
+        std::vector<BinNode> bin;
+#ifdef _OPENMP
+#pragma omp for schedule(dynamic, 16)
+#endif
+        for (size_t c = 0; c < nc; c++) {
+            bin.clear();
+            const uint32_t a = range[c].first, e = range[c].second;
+            top[c].word = (uint32_t)c;
+            top[c].count = 0;
+            for (uint32_t i = a; i < e; i++) top[c].count += items[i].count;
+            build_binary(&items[a], e - a, bin);
+            cut_costs(bin, 0, nullptr);
+            top[c].box = bin[0].box;
+            sub_cost[c] = bin[0].cost[0];
+            if (e - a > 1 || nc == 1) emit(bin, 0, sub[c], [](uint32_t w) { return w; });
+        }
+    }
+    if (nc == 1) {
+        L.quads.swap(sub[0]);
+        L.stack = stack_need(L.quads);
+        return L;
+    }
+    std::vector<BinNode> bin;
+    build_binary(top.data(), nc, bin);
+    cut_costs(bin, 0, &sub_cost);
+    // the upper tree, its clusters marked by the leaf bit for now; the
+    // clusters' nodes follow it in the order it reaches them
+    std::vector<QuadNode> upper;
+    std::vector<size_t> base(nc, 0);
+    std::vector<uint32_t> order;
+    emit(bin, 0, upper, [&](uint32_t c) {
+        order.push_back(c);
+        return c | QUAD_LEAF;
+    });
+    size_t total = upper.size();
+    for (uint32_t c : order) {
+        base[c] = total;
+        total += sub[c].size();
+    }
+    for (QuadNode& q : upper)
+        for (int k = 0; k < 4; k++) {
+            uint32_t& w = (&q.child.x)[k];
+            if (w == QUAD_HOLE || !(w & QUAD_LEAF)) continue;
+            const uint32_t c = w & ~QUAD_LEAF;
+            w = sub[c].empty() ? items[range[c].first].word : (uint32_t)base[c];
+        }
+    L.quads.resize(total);
+    std::memcpy(L.quads.data(), upper.data(), sizeof(QuadNode) * upper.size());
+#ifdef _OPENMP
+#pragma omp parallel for num_threads(threads) schedule(dynamic, 64)
+#endif
+    for (size_t c = 0; c < nc; c++)
+        for (size_t k = 0; k < sub[c].size(); k++) {
+            QuadNode q = sub[c][k];
+            for (int j = 0; j < 4; j++) {
+                uint32_t& w = (&q.child.x)[j];
+                if (!(w & QUAD_LEAF)) w += (uint32_t)base[c];
+            }
+            L.quads[base[c] + k] = q;
+        }
+    L.stack = stack_need(L.quads);
+    return L;
+}
+
+}  // namespace wr

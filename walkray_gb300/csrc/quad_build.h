@@ -1,0 +1,26 @@
+// quad_build.h — host construction of the four-wide tree that the closest-hit
+// kernels walk (QuadNode, wr_device.cuh).
+#pragma once
+
+#include <cstdint>
+#include <vector>
+
+#include "kdtree_build.h"
+#include "wr_device.cuh"
+
+namespace wr {
+
+// what the device needs beside the reference tree's own records
+struct QuadLayout {
+    std::vector<QuadNode> quads;     // [0] is the root
+    std::vector<uint32_t> leaf_up;   // per triangle slot: (pair << 1 | side) of its leaf, UP_ROOT if the root is that leaf
+    std::vector<uint32_t> pair_up;   // per pair: (parent pair << 1 | side), UP_ROOT for the root's
+    uint32_t stack = 0;              // entries that the deepest walk can need (a node's other children, all the way down)
+};
+
+// Four-wide tree over the reference tree's leaves (their own boxes, bit for
+// bit) by the surface-area heuristic, and the reference tree's parent links.
+// A scene of more than QUAD_MAX_SLOTS triangles gets an empty `quads`.
+QuadLayout build_quads(const HostTree& t, int threads);
+
+}  // namespace wr

@@ -1,10 +1,15 @@
 // trace.cu — k_trace_closest: closest hits for a batch of rays
 // (KDTree::intersect / Scene::intersect, kdtree.cpp:349-353, scene.cpp:102-113).
 //
-// Persistent warps (the loop of wr_warp_trace.cuh): the grid is sized to fill
-// every SM once; lanes refill from a global ray counter.  Per-thread
-// traversal stacks live in shared memory, column-major (entry k of thread t
-// at k * blockDim.x + t) so a warp's pushes hit 32 distinct banks.
+// Persistent warps (the loop of wr_quad_trace.cuh): the grid is sized to fill
+// every SM once; warps take rays from a global counter.  Per-thread stacks live
+// in shared memory, column-major (entry k of thread t at k * blockDim.x + t) so
+// a warp's pushes hit 32 distinct banks.
+//
+// Bound by the latency of the tree's nodes in L2 and by issue (2^24 incoherent
+// rays on the 1,310,720-triangle icosphere: 3.38 ms walking the reference's
+// tree with both of its slab tests per box, 2.30 ms here; 93 -> 61 warp
+// instructions a ray).
 #include <cuda_runtime.h>
 
 #include <algorithm>
@@ -24,61 +29,96 @@ struct BatchSrc {
     wr_hit* __restrict__ hits;
     bool filtered;
 
-    __device__ __forceinline__ void load(uint64_t id, TraceLane& L, uint32_t* stack, int stride) {
+    __device__ __forceinline__ void fetch(uint64_t id, TraceRay& a) const {
         const float* r = rays + 6 * id;
-        L.pairs = T.pairs;
-        L.tris = T.tris;
-        L.q = make_rayq(mk(r[0], r[1], r[2]), mk(r[3], r[4], r[5]), T.scene_mag);
-        L.filt = filtered;
-        L.inside = filtered ? inside[id] : -1;
-        L.contact = filtered ? contact[id] : -1;
-        lane_start(L, root_box(T), T.root_w0, T.root_w1, stack, stride);
+        a.T = &T;
+        a.o = mk(r[0], r[1], r[2]);
+        a.d = mk(r[3], r[4], r[5]);
+        a.pf = 1.001f;
+        a.filt = filtered;
+        a.inside = filtered ? inside[id] : -1;
+        a.contact = filtered ? contact[id] : -1;
     }
-    __device__ __forceinline__ void store(uint64_t id, const TraceLane& L) {
+    __device__ __forceinline__ void put(uint64_t id, const TraceRay& a, const Hit& h) const {
         uint4 out = make_uint4(WR_NO_HIT, __float_as_uint(-1.f), 0u, 0u);
-        if (L.h.slot >= 0) {
+        if (h.slot >= 0) {
             float u1, u2;
             uint32_t gid;
-            hit_barycentrics(T, L.h.slot, L.q, L.h.t, &u1, &u2, &gid);
-            out = make_uint4(gid, __float_as_uint(L.h.t), __float_as_uint(u1), __float_as_uint(u2));
+            hit_barycentrics(T, h.slot, a.o, a.d, h.t, &u1, &u2, &gid);
+            out = make_uint4(gid, __float_as_uint(h.t), __float_as_uint(u1), __float_as_uint(u2));
         }
         reinterpret_cast<uint4*>(hits)[id] = out;
+    }
+    __device__ __forceinline__ const TriRec* tris_of(const TriRec*, int) const { return T.tris; }
+    // the same for the walk that visits every box the reference visits (warp_trace)
+    __device__ __forceinline__ void load(uint64_t id, TraceLane& L, uint32_t* stack, int stride) const {
+        TraceRay a;
+        fetch(id, a);
+        load_lane(a, L, stack, stride);
+    }
+    __device__ __forceinline__ void store(uint64_t id, const TraceLane& L) const {
+        TraceRay a;
+        a.o = L.q.o;
+        a.d = L.q.d;
+        put(id, a, L.h);
     }
 };
 
 // MINB > 0: compiled for at least MINB resident CTAs per SM (a register cap)
-template <bool PRUNE, int MINB>
-__global__ void __launch_bounds__(128, MINB > 0 ? MINB : 1) k_trace_closest(DevTree T, const float* __restrict__ rays, uint64_t n,
-                                                         const int32_t* __restrict__ inside,
-                                                         const int32_t* __restrict__ contact, wr_hit* __restrict__ hits,
-                                                         unsigned long long* __restrict__ counter, int stack_cap,
-                                                         TraceTune tune, unsigned int* __restrict__ err) {
-    extern __shared__ uint32_t s_stack[];
+template <int MINB>
+__global__ void __launch_bounds__(128, MINB > 0 ? MINB : 1)
+    k_trace_closest(const __grid_constant__ DevTree T, const float* __restrict__ rays, uint64_t n,
+                    const int32_t* __restrict__ inside, const int32_t* __restrict__ contact,
+                    wr_hit* __restrict__ hits, unsigned long long* __restrict__ counter, int stack_cap, TraceTune tune,
+                    unsigned int* __restrict__ err) {
+    extern __shared__ __align__(16) uint32_t s_stack[];
     BatchSrc src{T, rays, inside, contact, hits, inside != nullptr};
-    warp_trace<PRUNE, false>(src, n, counter, tune, s_stack + threadIdx.x, blockDim.x, stack_cap, err);
+    TraceWork work;
+    quad_trace<false>(src, (uint32_t)n, reinterpret_cast<unsigned int*>(counter), tune, s_stack + threadIdx.x, blockDim.x, stack_cap,
+                      warp_queues(s_stack, stack_cap), work);
+}
+
+// WR_CTX_EXACT_TRAVERSAL: every box the reference visits, without pruning by distance
+__global__ void __launch_bounds__(128, 7)
+    k_trace_closest_exact(const __grid_constant__ DevTree T, const float* __restrict__ rays, uint64_t n,
+                          const int32_t* __restrict__ inside, const int32_t* __restrict__ contact,
+                          wr_hit* __restrict__ hits, unsigned long long* __restrict__ counter, int stack_cap,
+                          TraceTune tune, unsigned int* __restrict__ err) {
+    extern __shared__ __align__(16) uint32_t s_stack[];
+    BatchSrc src{T, rays, inside, contact, hits, inside != nullptr};
+    warp_trace<false, false>(src, n, counter, tune, s_stack + threadIdx.x, blockDim.x, stack_cap, err);
 }
 
 cudaError_t launch_trace_closest(const DevTree& T, const float* d_rays, uint64_t n, const int32_t* d_inside,
                                  const int32_t* d_contact, wr_hit* d_hits, unsigned long long* d_counter,
                                  unsigned int* d_err, int num_sms, bool prune, cudaStream_t stream,
                                  int* launched_blocks, const TraceTune* tune, int ctas_per_sm) {
+    constexpr uint64_t MOST = 1ull << 31;  // rays of a launch (32-bit ray ids)
+    for (; n > MOST; n -= MOST) {
+        const cudaError_t e = launch_trace_closest(T, d_rays, MOST, d_inside, d_contact, d_hits, d_counter, d_err,
+                                                   num_sms, prune, stream, launched_blocks, tune, ctas_per_sm);
+        if (e != cudaSuccess) return e;
+        d_rays += 6 * MOST;
+        d_hits += MOST;
+        if (d_inside) d_inside += MOST, d_contact += MOST;
+    }
     const int block = 128;
-    const int stack_cap = (int)T.max_depth + 3;
-    const size_t smem = (size_t)stack_cap * block * sizeof(uint32_t);
-    if (smem > 200 * 1024) return cudaErrorInvalidValue;
+    const int ref_cap = (int)T.max_depth + 3;  // stack of the reference's own walk
+    if ((size_t)ref_cap * block * sizeof(uint32_t) > 200 * 1024) return cudaErrorInvalidValue;
+    const int stack_cap = prune ? quad_stack_cap(T) : ref_cap;
+    const size_t smem = prune ? quad_smem(stack_cap, block) : (size_t)stack_cap * block * sizeof(uint32_t);
     cudaError_t e = cudaMemsetAsync(d_counter, 0, sizeof(unsigned long long), stream);
     if (e != cudaSuccess) return e;
     // blocks per SM from the occupancy calculator for this stack size
     int per_sm = 1;
-    // default: the 7-CTA variant (72 registers), fastest on the kd workload (six steps per
-    // turn: 4810 Mrays/s against 4691 with 8 CTAs and 4775 with 6)
+    // 0: the 7-CTA variant (72 registers; 2^24 rays: 2.31 ms, 2.30 with 6, 2.38 with 5, 2.49 with 8)
     const int variant = ctas_per_sm ? ctas_per_sm : 7;
     void (*kern)(DevTree, const float*, uint64_t, const int32_t*, const int32_t*, wr_hit*, unsigned long long*, int,
-                 TraceTune, unsigned int*) =
-        variant >= 8   ? (prune ? k_trace_closest<true, 8> : k_trace_closest<false, 8>)
-        : variant >= 7 ? (prune ? k_trace_closest<true, 7> : k_trace_closest<false, 7>)
-        : variant >= 6 ? (prune ? k_trace_closest<true, 6> : k_trace_closest<false, 6>)
-                           : (prune ? k_trace_closest<true, 0> : k_trace_closest<false, 0>);
+                 TraceTune, unsigned int*) = !prune         ? k_trace_closest_exact
+                                             : variant >= 8 ? k_trace_closest<8>
+                                             : variant >= 7 ? k_trace_closest<7>
+                                             : variant >= 6 ? k_trace_closest<6>
+                                                            : k_trace_closest<0>;
     if (smem > 48 * 1024) {
         e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
         if (e != cudaSuccess) return e;

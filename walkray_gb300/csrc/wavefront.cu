@@ -235,29 +235,38 @@ struct ExtendSrc {
     const WfJob* __restrict__ jobs;
     WfSide X;
     int2* __restrict__ hits;
-    unsigned long long n_rays, n_box, n_tri;  // this thread's work counts (profiling launches)
+    TraceWork work;  // this thread's counts of the exact walk (profiling launches)
 
-    __device__ __forceinline__ void load(uint64_t id, TraceLane& L, uint32_t* stack, int stride) {
+    __device__ __forceinline__ void fetch(uint64_t id, TraceRay& a) const {
         const float4* r = X.rec + (size_t)WF_REC * id;
         const float4 a0 = r[WF_O], a1 = r[WF_D];
         const int4 ids = as_i4(r[WF_IDS]);
         const WfJob& J = jobs[ids.z];
-        const DevTree& T = scenes[J.scene].tree;
-        L.pairs = T.pairs;
-        L.tris = T.tris;
-        L.q = make_rayq(mk(a0.x, a0.y, a0.z), mk(a1.x, a1.y, a1.z), T.scene_mag);
-        L.q.pf = prune_factor(J.flags);
-        L.inside = ids.x;
-        L.contact = ids.y;
-        L.filt = ids.y != CAMERA_OBJ;
-        const Box root{T.root_lo[0], T.root_lo[1], T.root_lo[2], T.root_hi[0], T.root_hi[1], T.root_hi[2]};
-        lane_start(L, root, T.root_w0, T.root_w1, stack, stride);
+        a.T = &scenes[J.scene].tree;
+        a.o = mk(a0.x, a0.y, a0.z);
+        a.d = mk(a1.x, a1.y, a1.z);
+        a.pf = prune_factor(J.flags);
+        a.filt = ids.y != CAMERA_OBJ;
+        a.inside = ids.x;
+        a.contact = ids.y;
+    }
+    __device__ __forceinline__ void put(uint64_t id, const TraceRay&, const Hit& h) const {
+        hits[id] = make_int2(h.slot, __float_as_int(h.t));
+    }
+    // rays of several scenes share the queue
+    __device__ __forceinline__ const TriRec* tris_of(const TriRec* tris, int from) const {
+        return shfl_ptr(tris, from);
+    }
+    __device__ __forceinline__ void load(uint64_t id, TraceLane& L, uint32_t* stack, int stride) const {
+        TraceRay a;
+        fetch(id, a);
+        load_lane(a, L, stack, stride);
     }
     __device__ __forceinline__ void store(uint64_t id, const TraceLane& L) {
         hits[id] = make_int2(L.h.slot, __float_as_int(L.h.t));
-        n_rays += 1;
-        n_box += L.n_box;
-        n_tri += L.n_tri;
+        work.rays += 1;
+        work.boxes += L.n_box;
+        work.tris += L.n_tri;
     }
 };
 
@@ -271,20 +280,26 @@ __device__ __forceinline__ void warp_add(unsigned long long* dst, unsigned long 
 // (a register cap), chosen by the configuration's ctas_per_sm
 #define WR_EXTEND_BOUNDS(MINB) __launch_bounds__(128, (MINB) > 0 ? (MINB) : 1)
 
-template <bool STATS, int MINB>
+// EXACT: every box the reference visits (launched while a job with
+// WR_RENDER_EXACT_TRAVERSAL is in the table; its counts are the reference's)
+template <bool STATS, bool EXACT, int MINB>
 __global__ void WR_EXTEND_BOUNDS(MINB) k_wf_extend(const RenderScene* __restrict__ scenes,
                                                      const WfJob* __restrict__ jobs, WfSide X, int2* __restrict__ hits,
                                                      unsigned long long* __restrict__ work, int stack_cap,
                                                      TraceTune tune, unsigned int* __restrict__ err,
                                                      unsigned long long* __restrict__ stats) {
-    extern __shared__ uint32_t s_stack[];
+    extern __shared__ __align__(16) uint32_t s_stack[];
     const uint64_t n = (uint64_t)X.counts[0] + X.counts[1];
-    ExtendSrc src{scenes, jobs, X, hits, 0ull, 0ull, 0ull};
-    warp_trace<true, STATS>(src, n, work, tune, s_stack + threadIdx.x, blockDim.x, stack_cap, err);
+    ExtendSrc src{scenes, jobs, X, hits, TraceWork{0ull, 0ull, 0ull}};
+    if (EXACT)
+        warp_trace<true, STATS>(src, n, work, tune, s_stack + threadIdx.x, blockDim.x, stack_cap, err);
+    else
+        quad_trace<STATS>(src, (uint32_t)n, reinterpret_cast<unsigned int*>(work), tune, s_stack + threadIdx.x, blockDim.x, stack_cap,
+                          warp_queues(s_stack, stack_cap), src.work);
     if (STATS) {
-        warp_add(stats + 0, src.n_rays);
-        warp_add(stats + 1, src.n_box);
-        warp_add(stats + 2, src.n_tri);
+        warp_add(stats + 0, src.work.rays);
+        warp_add(stats + 1, src.work.boxes);
+        warp_add(stats + 2, src.work.tris);
     }
 }
 
@@ -300,23 +315,24 @@ struct ShadowSrc {
     WfShadow Q;
     int2* __restrict__ hits;
 
-    __device__ __forceinline__ void load(uint64_t id, TraceLane& L, uint32_t* stack, int stride) {
+    __device__ __forceinline__ void fetch(uint64_t id, TraceRay& a) const {
         const float4 o = Q.o[id], d = Q.d[id];
         const int4 ids = Q.ids[id];
         const WfJob& J = jobs[ids.z];
-        const DevTree& T = scenes[J.scene].tree;
-        L.pairs = T.pairs;
-        L.tris = T.tris;
-        L.q = make_rayq(mk(o.x, o.y, o.z), mk(d.x, d.y, d.z), T.scene_mag);
-        L.q.pf = prune_factor(J.flags);
-        L.inside = ids.x;
-        L.contact = ids.y;
-        L.filt = true;
-        const Box root{T.root_lo[0], T.root_lo[1], T.root_lo[2], T.root_hi[0], T.root_hi[1], T.root_hi[2]};
-        lane_start(L, root, T.root_w0, T.root_w1, stack, stride);
+        a.T = &scenes[J.scene].tree;
+        a.o = mk(o.x, o.y, o.z);
+        a.d = mk(d.x, d.y, d.z);
+        a.pf = prune_factor(J.flags);
+        a.filt = true;
+        a.inside = ids.x;
+        a.contact = ids.y;
     }
-    __device__ __forceinline__ void store(uint64_t id, const TraceLane& L) {
-        hits[id] = make_int2(L.h.slot, __float_as_int(L.h.t));
+    __device__ __forceinline__ void put(uint64_t id, const TraceRay&, const Hit& h) const {
+        hits[id] = make_int2(h.slot, __float_as_int(h.t));
+    }
+    // rays of several scenes share the queue
+    __device__ __forceinline__ const TriRec* tris_of(const TriRec* tris, int from) const {
+        return shfl_ptr(tris, from);
     }
 };
 
@@ -325,10 +341,12 @@ __global__ void WR_EXTEND_BOUNDS(MINB)
     k_wf_shadow_trace(const RenderScene* __restrict__ scenes, const WfJob* __restrict__ jobs, WfShadow Q,
                       int2* __restrict__ hits, unsigned long long* __restrict__ work, int stack_cap, TraceTune tune,
                       unsigned int* __restrict__ err) {
-    extern __shared__ uint32_t s_stack[];
+    extern __shared__ __align__(16) uint32_t s_stack[];
     const uint64_t n = *Q.count;
     ShadowSrc src{scenes, jobs, Q, hits};
-    warp_trace<true, false>(src, n, work, tune, s_stack + threadIdx.x, blockDim.x, stack_cap, err);
+    TraceWork none;
+    quad_trace<false>(src, (uint32_t)n, reinterpret_cast<unsigned int*>(work), tune, s_stack + threadIdx.x, blockDim.x, stack_cap,
+                      warp_queues(s_stack, stack_cap), none);
 }
 
 using ShadowTraceKernel = void (*)(const RenderScene*, const WfJob*, WfShadow, int2*, unsigned long long*, int,
@@ -336,7 +354,7 @@ using ShadowTraceKernel = void (*)(const RenderScene*, const WfJob*, WfShadow, i
 
 // the shadow traversal for a configuration: the extend stage's register cap
 static ShadowTraceKernel shadow_trace_kernel(int ctas_per_sm) {
-    if (ctas_per_sm == 0) ctas_per_sm = 6;
+    if (ctas_per_sm == 0) ctas_per_sm = 7;
     if (ctas_per_sm >= 8) return k_wf_shadow_trace<8>;
     if (ctas_per_sm >= 7) return k_wf_shadow_trace<7>;
     if (ctas_per_sm >= 6) return k_wf_shadow_trace<6>;
@@ -344,13 +362,14 @@ static ShadowTraceKernel shadow_trace_kernel(int ctas_per_sm) {
 }
 
 // the extend kernel for a configuration: register cap from ctas_per_sm
-// (0 = the 6-CTA variant, fastest on the mixed-material scene)
-static ExtendKernel extend_kernel(int ctas_per_sm, bool stats) {
-    if (ctas_per_sm == 0) ctas_per_sm = 6;
-    if (ctas_per_sm >= 8) return stats ? k_wf_extend<true, 8> : k_wf_extend<false, 8>;
-    if (ctas_per_sm >= 7) return stats ? k_wf_extend<true, 7> : k_wf_extend<false, 7>;
-    if (ctas_per_sm >= 6) return stats ? k_wf_extend<true, 6> : k_wf_extend<false, 6>;
-    return stats ? k_wf_extend<true, 0> : k_wf_extend<false, 0>;
+// (0 = the 7-CTA variant: mixed-material scene 1024^2 x 32 spp 35.3 ms, 35.6 with 6, 37.4 with 8)
+static ExtendKernel extend_kernel(int ctas_per_sm, bool stats, bool exact) {
+    if (exact) return stats ? k_wf_extend<true, true, 6> : k_wf_extend<false, true, 6>;
+    if (ctas_per_sm == 0) ctas_per_sm = 7;
+    if (ctas_per_sm >= 8) return stats ? k_wf_extend<true, false, 8> : k_wf_extend<false, false, 8>;
+    if (ctas_per_sm >= 7) return stats ? k_wf_extend<true, false, 7> : k_wf_extend<false, false, 7>;
+    if (ctas_per_sm >= 6) return stats ? k_wf_extend<true, false, 6> : k_wf_extend<false, false, 6>;
+    return stats ? k_wf_extend<true, false, 0> : k_wf_extend<false, false, 0>;
 }
 
 // shade: one bounce per path; survivors compacted into Y, finished paths to
@@ -714,12 +733,14 @@ struct WfEngine {
     std::vector<RenderScene> scene_tab;
     std::vector<WfJob> job_tab;               // host mirror of the job slots
     std::vector<int> order_host;               // [n, slot...]
-    int stack_cap = 0;
-    int grid_extend = 0, grid_shade = 0, grid_gen = 0;
-    size_t smem_extend = 0;
+    int stack_cap = 0;       // the reference walk's stack (tree depth + 3)
+    int quad_cap = 0;        // the search's stack
+    int grid_extend = 0, grid_exact = 0, grid_shade = 0, grid_gen = 0;
+    size_t smem_extend = 0, smem_exact = 0;
     cudaGraphExec_t graph = nullptr;
     int graph_stack = -1;
     bool mis_any = false;  // a job in the table has WR_RENDER_NEE_MIS: the shade stage with that code
+    bool exact_any = false;  // a job in the table has WR_RENDER_EXACT_TRAVERSAL: the extend stage of that walk
     bool conn_any = true;  // a job in the table connects to lights (NEE or MIS): the shadow stage is in the loop
     int launches_per_iteration() const { return conn_any ? 8 : 6; }
     WfJobCounters* host_counters = nullptr;  // pinned
@@ -902,7 +923,7 @@ int wf_update_jobs(wr_ctx* ctx, WfEngine* E, const std::vector<WfSlotUpdate>& up
     }
     if (scenes_changed) {
         E->scene_tab.resize(E->scene_of.size());
-        int cap = 8;
+        int cap = 8, quad_cap = 8;
         for (size_t k = 0; k < E->scene_of.size(); k++) {
             if (!E->scene_of[k]) {
                 std::memset(&E->scene_tab[k], 0, sizeof(RenderScene));
@@ -910,40 +931,46 @@ int wf_update_jobs(wr_ctx* ctx, WfEngine* E, const std::vector<WfSlotUpdate>& up
             }
             E->scene_tab[k] = RenderDataView::scene(E->scene_of[k]);
             cap = std::max(cap, (int)E->scene_tab[k].tree.max_depth + 3);
+            quad_cap = std::max(quad_cap, quad_stack_cap(E->scene_tab[k].tree));
         }
         WR_CUDA(ctx, cudaMemcpyAsync(E->scenes.p, E->scene_tab.data(), sizeof(RenderScene) * E->scene_tab.size(),
                                      cudaMemcpyHostToDevice, s));
-        if (cap > E->stack_cap) {
-            E->stack_cap = cap;
-            E->smem_extend = (size_t)cap * E->cfg.extend_block * sizeof(uint32_t);
-            if (E->smem_extend > 200 * 1024) return set_error(ctx, WR_ERR_UNSUPPORTED, "tree too deep for the stack");
-            if (E->smem_extend > 48 * 1024) {
+        if (cap > E->stack_cap || quad_cap > E->quad_cap) {
+            const int block = E->cfg.extend_block;
+            E->stack_cap = std::max(cap, E->stack_cap);
+            E->quad_cap = std::max(quad_cap, E->quad_cap);
+            E->smem_exact = (size_t)E->stack_cap * block * sizeof(uint32_t);
+            E->smem_extend = quad_smem(E->quad_cap, block);
+            if (E->smem_exact > 200 * 1024) return set_error(ctx, WR_ERR_UNSUPPORTED, "tree too deep for the stack");
+            if (E->smem_exact > 48 * 1024)
                 for (bool st : {false, true})
-                    WR_CUDA(ctx, cudaFuncSetAttribute(extend_kernel(E->cfg.ctas_per_sm, st),
+                    WR_CUDA(ctx, cudaFuncSetAttribute(extend_kernel(E->cfg.ctas_per_sm, st, true),
                                                       cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                                      (int)E->smem_extend));
-            }
+                                                      (int)E->smem_exact));
             int per_sm = 0;
             WR_CUDA(ctx, cudaOccupancyMaxActiveBlocksPerMultiprocessor(
-                             &per_sm, extend_kernel(E->cfg.ctas_per_sm, false), E->cfg.extend_block, E->smem_extend));
+                             &per_sm, extend_kernel(E->cfg.ctas_per_sm, false, false), block, E->smem_extend));
             if (E->cfg.ctas_per_sm > 0) per_sm = std::min(per_sm, E->cfg.ctas_per_sm);
             E->grid_extend = ctx->num_sms * std::max(1, per_sm);
-            if (E->smem_extend > 48 * 1024)
-                WR_CUDA(ctx, cudaFuncSetAttribute(shadow_trace_kernel(E->cfg.ctas_per_sm),
-                                                  cudaFuncAttributeMaxDynamicSharedMemorySize, (int)E->smem_extend));
+            WR_CUDA(ctx, cudaOccupancyMaxActiveBlocksPerMultiprocessor(
+                             &per_sm, extend_kernel(E->cfg.ctas_per_sm, false, true), block, E->smem_exact));
+            if (E->cfg.ctas_per_sm > 0) per_sm = std::min(per_sm, E->cfg.ctas_per_sm);
+            E->grid_exact = ctx->num_sms * std::max(1, per_sm);
             WR_CUDA(ctx, cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_wf_shadow, 128, 0));
             E->grid_shadow = ctx->num_sms * std::max(1, per_sm);
         }
     }
     // the shade stage compiled with the light-connection code only while a job needs it
     // and the shadow stage only while a job can queue a connection
-    bool mis_any = false, conn_any = false;
+    bool mis_any = false, conn_any = false, exact_any = false;
     for (int slot : order) {
         if (!E->job_tab[slot].active) continue;
         if (E->job_tab[slot].flags & WR_RENDER_NEE_MIS) mis_any = true;
+        if (E->job_tab[slot].flags & WR_RENDER_EXACT_TRAVERSAL) exact_any = true;
         if (E->job_tab[slot].flags & (WR_RENDER_NEE | WR_RENDER_NEE_MIS)) conn_any = true;
     }
-    if (mis_any != E->mis_any || conn_any != E->conn_any) {
+    if (mis_any != E->mis_any || conn_any != E->conn_any || exact_any != E->exact_any) {
+        E->exact_any = exact_any;
         E->mis_any = mis_any;
         E->conn_any = conn_any;
         if (E->graph) {
@@ -970,9 +997,11 @@ static void enqueue_iteration(WfEngine* E, int x, cudaStream_t s, cudaEvent_t* e
     WfJobCounters* cnt = E->counters.as<WfJobCounters>();
     k_wf_reset<<<1, 1, 0, s>>>(E->side[y], E->work.as<unsigned long long>(), E->shadow.count, E->sort);
     if (ev) cudaEventRecord(ev[0], s);
-    extend_kernel(E->cfg.ctas_per_sm, stats != nullptr)<<<E->grid_extend, E->cfg.extend_block, E->smem_extend, s>>>(
-        scenes, jobs, E->side[x], E->hits.as<int2>(), E->work.as<unsigned long long>(), E->stack_cap, E->cfg.trace,
-        E->err_word.as<unsigned int>(), stats);
+    extend_kernel(E->cfg.ctas_per_sm, stats != nullptr, E->exact_any)
+        <<<E->exact_any ? E->grid_exact : E->grid_extend, E->cfg.extend_block,
+           E->exact_any ? E->smem_exact : E->smem_extend, s>>>(
+            scenes, jobs, E->side[x], E->hits.as<int2>(), E->work.as<unsigned long long>(),
+            E->exact_any ? E->stack_cap : E->quad_cap, E->cfg.trace, E->err_word.as<unsigned int>(), stats);
     if (ev) cudaEventRecord(ev[1], s);
     k_wf_sort<<<E->grid_sort, 256, 0, s>>>(scenes, jobs, E->side[x], E->hits.as<int2>(), E->sort, E->cfg.capacity);
     (E->mis_any ? k_wf_shade<true> : k_wf_shade<false>)<<<E->grid_shade, E->cfg.shade_block, 0, s>>>(scenes, jobs, cnt, E->side[x], E->hits.as<int2>(),
@@ -980,7 +1009,7 @@ static void enqueue_iteration(WfEngine* E, int x, cudaStream_t s, cudaEvent_t* e
     if (ev) cudaEventRecord(ev[2], s);
     if (E->conn_any) {  // the connections' closest hits go into E->hits, which shade has read
         shadow_trace_kernel(E->cfg.ctas_per_sm)<<<E->grid_extend, E->cfg.extend_block, E->smem_extend, s>>>(
-            scenes, jobs, E->shadow, E->hits.as<int2>(), E->work.as<unsigned long long>() + 1, E->stack_cap,
+            scenes, jobs, E->shadow, E->hits.as<int2>(), E->work.as<unsigned long long>() + 1, E->quad_cap,
             E->cfg.trace, E->err_word.as<unsigned int>());
         k_wf_shadow<<<E->grid_shadow, 128, 0, s>>>(scenes, jobs, E->shadow, E->hits.as<int2>(), E->side[y]);
     }
@@ -1086,7 +1115,8 @@ int profile_wavefront(wr_ctx* ctx, RenderData& rd, const RenderParams& P, uint32
 
 int wf_launch(wr_ctx* ctx, WfEngine* E, cudaStream_t s) {
     if (E->stack_cap == 0) return set_error(ctx, WR_ERR_INTERNAL, "wavefront launched without a scene");
-    if (!E->graph || E->graph_stack != E->stack_cap) {
+    const int caps = E->stack_cap << 8 | E->quad_cap;
+    if (!E->graph || E->graph_stack != caps) {
         if (E->graph) {
             cudaGraphExecDestroy(E->graph);
             E->graph = nullptr;
@@ -1107,7 +1137,7 @@ int wf_launch(wr_ctx* ctx, WfEngine* E, cudaStream_t s) {
         e = cudaGraphInstantiate(&E->graph, g, 0);
         cudaGraphDestroy(g);
         if (e != cudaSuccess) return cuda_error(ctx, e, "instantiating the bounce loop");
-        E->graph_stack = E->stack_cap;
+        E->graph_stack = caps;
     }
     WR_CUDA(ctx, cudaGraphLaunch(E->graph, s));
     // reset, extend, sort, shade, [shadow trace, shadow,] plan, generate

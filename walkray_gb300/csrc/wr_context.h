@@ -46,7 +46,7 @@ struct DeviceBuffer {
 struct SceneGPU {
     uint32_t id = 0;
     DevTree tree{};
-    DeviceBuffer pairs, tris;
+    DeviceBuffer pairs, tris, quads, leaf_up, pair_up;
     wr_scene_info info{};
     // scene description kept on the host for rendering set-up
     std::vector<wr_object_desc> objects;

@@ -43,6 +43,25 @@ struct __align__(16) TriRec {
 };
 static_assert(sizeof(TriRec) == 48, "TriRec must be 48 bytes");
 
+// Four children of the tree the closest-hit search walks (quad_build.cpp):
+// their boxes by axis, so that a ray takes the four near planes and the four
+// far planes of an axis as one 16-byte load each, chosen by the sign of its
+// direction.  112 bytes: an odd multiple of 16 spreads the lanes of a warp,
+// each at its own node, over all shared-memory banks of the L1 cache (random
+// records read in 16-byte pieces: 64- and 128-byte strides take 0.61 and 0.99
+// cycles a piece on an SM, 48- and 80-byte strides 0.34).
+struct __align__(16) QuadNode {
+    float4 lox, loy, loz, hix, hiy, hiz;
+    uint4 child;  // node index, QUAD_LEAF | count << QUAD_COUNT_AT | first slot, or QUAD_HOLE
+};
+static_assert(sizeof(QuadNode) == 112, "QuadNode must be 112 bytes");
+constexpr uint32_t QUAD_LEAF = 0x80000000u;
+constexpr uint32_t QUAD_HOLE = 0xffffffffu;  // an unused child: its box meets no ray
+constexpr uint32_t QUAD_COUNT_AT = 28u;      // leaf words: first slot below this bit, triangle count above it
+constexpr uint32_t QUAD_LEAF_MAX = 7u;       // triangles of one leaf word
+constexpr uint32_t QUAD_MAX_SLOTS = (1u << QUAD_COUNT_AT) - 8u;
+constexpr uint32_t UP_ROOT = 0xffffffffu;    // leaf_up / pair_up of the root
+
 struct DevTree {
     const NodePair* pairs;
     const TriRec* tris;
@@ -51,6 +70,12 @@ struct DevTree {
     float scene_mag;            // max |coordinate| over all vertices
     uint32_t max_depth;
     uint32_t num_pairs, num_slots;
+    // the four-wide tree the search walks (nullptr: more than QUAD_MAX_SLOTS
+    // triangles) and the reference tree's parent links, (pair << 1 | side)
+    const QuadNode* quads;
+    const uint32_t* leaf_up;  // per triangle slot
+    const uint32_t* pair_up;  // per pair
+    uint32_t quad_stack;      // stack entries that the deepest walk of `quads` can need
 };
 
 // Knobs of the warp-persistent traversal loop (wr_warp_trace.cuh)

@@ -358,12 +358,12 @@ __device__ __forceinline__ Hit trace_closest(const DevTree& T, const RayQ& q0, i
 }
 
 // barycentric weights of v1, v2 at the hit point (mesh.h:67-73)
-__device__ __forceinline__ void hit_barycentrics(const DevTree& T, int slot, const RayQ& q, float t, float* u1,
-                                                 float* u2, uint32_t* gid) {
+__device__ __forceinline__ void hit_barycentrics(const DevTree& T, int slot, f3 o, f3 d, float t, float* u1, float* u2,
+                                                 uint32_t* gid) {
     const TriRec* tr = T.tris + slot;
     const float4 a = ldg4(&tr->v0), b = ldg4(&tr->v1), c = ldg4(&tr->v2);
     const f3 v0 = xyz(a), b1 = xyz(b) - v0, b2 = xyz(c) - v0;
-    const f3 v = (q.o + q.d * t) - v0;
+    const f3 v = (o + d * t) - v0;
     const float d12 = dot(b1, b2), l1 = length(b1), l2 = length(b2);
     const float vb1 = dot(v, b1), vb2 = dot(v, b2);
     const float w2 = (vb1 * d12 - vb2 * l1 * l1) / (d12 * d12 - l1 * l1 * l2 * l2);

@@ -1,5 +1,8 @@
-// wr_warp_trace.cuh — the warp-persistent closest-hit loop shared by the
-// batch kernel (k_trace_closest) and the wavefront extend stage.
+// wr_warp_trace.cuh — the warp-persistent walk of the reference's own tree: the
+// exact forms of the batch kernel and of the wavefront's extend stage
+// (WR_CTX_EXACT_TRAVERSAL, WR_RENDER_EXACT_TRAVERSAL), which visit every box
+// the reference visits and count them.  wr_quad_trace.cuh is the search that
+// everything else runs.
 //
 // Same result as trace_closest() (wr_traverse.cuh): the same box predicate
 // decides every descent and the winner is order-free ("smallest t, then
@@ -21,7 +24,7 @@
 // result.
 #pragma once
 
-#include "wr_traverse.cuh"
+#include "wr_quad_trace.cuh"
 
 namespace wr {
 
@@ -58,6 +61,19 @@ __device__ __forceinline__ void lane_start(TraceLane& L, const Box& root, uint32
             stack[(L.sp++) * stride] = w0;
         }
     }
+}
+
+// a ray's lane, started
+__device__ __forceinline__ void load_lane(const TraceRay& a, TraceLane& L, uint32_t* stack, int stride) {
+    const DevTree& T = *a.T;
+    L.pairs = T.pairs;
+    L.tris = T.tris;
+    L.q = make_rayq(a.o, a.d, T.scene_mag);
+    L.q.pf = a.pf;
+    L.filt = a.filt;
+    L.inside = a.inside;
+    L.contact = a.contact;
+    lane_start(L, root_box(T), T.root_w0, T.root_w1, stack, stride);
 }
 
 // One traversal step of a searching lane (npend == 0, sp > 0): pop a pair,
