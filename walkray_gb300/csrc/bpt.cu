@@ -44,6 +44,7 @@
 
 namespace wr {
 
+constexpr int BPT_BLOCK = 128;  // threads per CTA of the kernels that trace rays
 constexpr uint32_t BPT_LIGHT_DIM0 = 0x40000000u;
 constexpr int BPT_MAX_RECORDS = 32;  // records per sub-path: max_path_len + 2
 constexpr double INV_PI_D = 0.31830988618379067153776752674503;
@@ -129,7 +130,6 @@ struct BptParams {
     // nslots + slot of the same arrays; their point entries carry bit 31
     bool vol_grid;
     uint32_t nslots;      // slots (iterations) of the batch
-    unsigned int* err;    // error bits of the traversals inside the weights (heterogeneous media)
 };
 
 // the weight's technique set for a sample of this batch
@@ -166,8 +166,9 @@ __device__ __forceinline__ void warp_append(bool ok, uint2 item, uint2* list, un
 // ray unfiltered (camera.cpp:52), which a filter with no inside and no
 // contact object is, the emitted ray with NoSelfCondition).
 template <bool HM>
-__global__ void __launch_bounds__(128) k_bpt_subpaths(RenderScene S, BptParams P, unsigned int* __restrict__ err) {
+__global__ void __launch_bounds__(128) k_bpt_subpaths(RenderScene S, BptParams P) {
     constexpr unsigned FULL = 0xffffffffu;
+    __shared__ uint8_t s_item[BPT_BLOCK / 32][LEAF_ITEMS];
     extern __shared__ uint32_t s_stack[];
     uint32_t* stack = s_stack + threadIdx.x;
     const int stride = blockDim.x;
@@ -263,16 +264,8 @@ __global__ void __launch_bounds__(128) k_bpt_subpaths(RenderScene S, BptParams P
             }
         }
         // every ray of the turn at one call site
-        Hit h;
-        h.t = __int_as_float(0x7f800000);
-        h.slot = -1;
-        if (has_ray) {
-            RayQ q = make_rayq(ray.o, ray.d, S.tree.scene_mag);
-            q.pf = P.pf;
-            const bool filt = !(fresh && !light);
-            h = trace_closest<true, true>(S.tree, q, filt ? ray.inside : -1, filt ? ray.contact : -1, stack, stride,
-                                          P.stack_cap, err);
-        }
+        const Hit h = search_warp(S.tree, has_ray, ray.o, ray.d, P.pf, !(fresh && !light), ray.inside, ray.contact,
+                                  stack, stride, P.stack_cap, s_item[threadIdx.x >> 5]);
         if (active && fresh) {  // the sub-path's first record, its hit set
             if (light) {
                 if (has_ray && h.slot >= 0 && h.t > 0.f) set_hit(S, ray, h);  // `if(dist > 0)`
@@ -368,25 +361,19 @@ __device__ __forceinline__ f3 bpt_eval_bsdf(const RenderScene& S, f3 in_d, const
 // distance (homogeneousVolume.cpp:209-214, homogeneousVolume.h:40-53) it is
 // ---- heterogeneous media in the weights: the reference's ray-marched
 // integrals (HeterogeneousVolume.cpp:171-248) -------------------------------
-constexpr int HV_STACK = 96;  // traversal stack of these helpers (thread-local memory)
+constexpr int HV_STACK = 28;  // stack of these helpers' searches (thread-local memory)
 
 struct HvCtx {  // what their own traversal needs
     float pf;
-    int cap;
-    unsigned int* err;
 };
-__device__ __forceinline__ HvCtx hv_ctx(const BptParams& P) {
-    return HvCtx{P.pf, P.stack_cap < HV_STACK ? P.stack_cap : HV_STACK, P.err};
-}
+__device__ __forceinline__ HvCtx hv_ctx(const BptParams& P) { return HvCtx{P.pf}; }
 
 // HeterogeneousVolume::check (:171-185) of a record inside the medium (its
 // origin is inside the mesh by the record's inside object): the first hit of
 // the record's ray under its NoSelfCondition
 __device__ __forceinline__ bool hv_first_hit(const RenderScene& S, const PRay& r, const HvCtx& hc, float& idist) {
     uint32_t stack[HV_STACK];
-    RayQ q = make_rayq(r.o, r.d, S.tree.scene_mag);
-    q.pf = hc.pf;
-    const Hit h = trace_closest<true, true>(S.tree, q, r.inside, r.contact, stack, 1, hc.cap, hc.err);
+    const Hit h = search_closest(S.tree, r.o, r.d, hc.pf, true, r.inside, r.contact, stack, 1, HV_STACK);
     if (h.slot < 0 || !(h.t > 0.f)) return false;
     idist = h.t;
     return true;
@@ -747,7 +734,8 @@ __device__ __forceinline__ void bpt_connect_edge(const RenderScene& S, const Bpt
 // MCRenderer::visibilityTest (mcRenderer.cpp:59-65) of every candidate, from
 // the eye vertex towards the light vertex; the visible ones join the list of
 // contributing connections.  Persistent: the grid strides over the list.
-__global__ void __launch_bounds__(128) k_bpt_visible(RenderScene S, BptParams P, unsigned int* __restrict__ err) {
+__global__ void __launch_bounds__(128) k_bpt_visible(RenderScene S, BptParams P) {
+    __shared__ uint8_t s_item[BPT_BLOCK / 32][LEAF_ITEMS];
     extern __shared__ uint32_t s_stack[];
     uint32_t* stack = s_stack + threadIdx.x;
     const int stride = blockDim.x;
@@ -759,15 +747,14 @@ __global__ void __launch_bounds__(128) k_bpt_visible(RenderScene S, BptParams P,
         const unsigned long long i = t * step + (unsigned long long)blockIdx.x * blockDim.x + threadIdx.x;
         bool ok = false;
         uint2 c = make_uint2(0, 0);
+        PRay lc = ray_default(), ec = ray_default();
         if (i < total) {
             c = P.cand[i];
-            PRay lc, ec;
             bpt_connect_edge(S, P, c.x, (int)(c.y & 0xffu), (int)(c.y >> 8), lc, ec);
-            RayQ q = make_rayq(ec.o, ec.d, S.tree.scene_mag);
-            q.pf = P.pf;
-            const Hit h = trace_closest<true, true>(S.tree, q, ec.inside, ec.contact, stack, stride, P.stack_cap, err);
-            ok = h.slot < 0 || (double)(h.t - length(ec.o - lc.o)) >= -EPS_D;
         }
+        const Hit h = search_warp(S.tree, i < total, ec.o, ec.d, P.pf, true, ec.inside, ec.contact, stack, stride,
+                                  P.stack_cap, s_item[threadIdx.x >> 5]);
+        if (i < total) ok = h.slot < 0 || (double)(h.t - length(ec.o - lc.o)) >= -EPS_D;
         warp_append(ok, c, P.vis, P.ncand + 1);
     }
 }
@@ -1354,7 +1341,7 @@ struct PpmSeg {
 // inside a medium before the estimate ray-marched against the volume photons
 // (photonMap.cpp:306-367): color = Tr * surface + volume.
 template <bool MEDIA, bool HM>
-__global__ void __launch_bounds__(128) k_ppm_eye(RenderScene S, BptParams P, unsigned int* __restrict__ err) {
+__global__ void __launch_bounds__(128) k_ppm_eye(RenderScene S, BptParams P) {
     extern __shared__ uint32_t s_stack[];
     uint32_t* stack = s_stack + threadIdx.x;
     const int stride = blockDim.x;
@@ -1366,9 +1353,7 @@ __global__ void __launch_bounds__(128) k_ppm_eye(RenderScene S, BptParams P, uns
     const PRay cam = camera_ray(S.cam, pixel, g);
     PRay prev = cam;
     {
-        RayQ q = make_rayq(cam.o, cam.d, S.tree.scene_mag);
-        q.pf = P.pf;
-        const Hit h = trace_closest<false, true>(S.tree, q, -1, -1, stack, stride, P.stack_cap, err);
+        const Hit h = search_closest(S.tree, cam.o, cam.d, P.pf, false, -1, -1, stack, stride, P.stack_cap);
         set_hit(S, prev, h);
     }
     InsideStack st;
@@ -1398,10 +1383,8 @@ __global__ void __launch_bounds__(128) k_ppm_eye(RenderScene S, BptParams P, uns
                 // (or on it as the record's contact), then the first hit
                 float chk = 0.f;
                 if (cur.contact == self || inside_mesh(S, self, cur.o)) {
-                    RayQ q = make_rayq(cur.o, cur.d, S.tree.scene_mag);
-                    q.pf = P.pf;
-                    const Hit h =
-                        trace_closest<true, true>(S.tree, q, cur.inside, cur.contact, stack, stride, P.stack_cap, err);
+                    const Hit h = search_closest(S.tree, cur.o, cur.d, P.pf, true, cur.inside, cur.contact, stack,
+                                                 stride, P.stack_cap);
                     if (h.slot >= 0 && h.t > 0.f) chk = h.t;
                 }
                 bool del = false;
@@ -1448,9 +1431,8 @@ __global__ void __launch_bounds__(128) k_ppm_eye(RenderScene S, BptParams P, uns
         }
         if (ended) break;
         st.set_top(next.inside);
-        RayQ q = make_rayq(next.o, next.d, S.tree.scene_mag);
-        q.pf = P.pf;
-        const Hit h = trace_closest<true, true>(S.tree, q, next.inside, next.contact, stack, stride, P.stack_cap, err);
+        const Hit h = search_closest(S.tree, next.o, next.d, P.pf, true, next.inside, next.contact, stack, stride,
+                                     P.stack_cap);
         if (h.slot < 0) break;  // `next` was the last record and is checked above
         pdir = prev.d;
         prev = next;
@@ -1541,7 +1523,7 @@ float vcm_radius(float base, uint32_t s) {
 }
 
 int render_bidirectional(wr_ctx* ctx, const RenderScene& S, const RenderParams& RP, uint32_t spp_offset,
-                         uint32_t spp, float* d_sum, float* d_sumsq, unsigned int* err, cudaStream_t stream,
+                         uint32_t spp, float* d_sum, float* d_sumsq, cudaStream_t stream,
                          int kind, float base_radius, bool hetero, bool media) {
     if (RP.max_path_len + 2 > (uint32_t)BPT_MAX_RECORDS)
         return set_error(ctx, WR_ERR_INVALID_ARGUMENT, "bidirectional mode: max_path_len is limited to 30");
@@ -1584,7 +1566,6 @@ int render_bidirectional(wr_ctx* ctx, const RenderScene& S, const RenderParams& 
     P.max_path_len = RP.max_path_len;
     P.pf = prune_factor(RP.flags);
     P.stack_cap = RP.stack_cap;
-    P.err = err;
     P.eye.base = st.eye.as<float4>();
     P.light.base = st.light.as<float4>();
     P.counts = st.counts.as<uint32_t>();
@@ -1627,7 +1608,7 @@ int render_bidirectional(wr_ctx* ctx, const RenderScene& S, const RenderParams& 
     const auto k_eval = hetero ? k_vcm_eval<true> : k_vcm_eval<false>;
     const auto k_tput = hetero ? k_ppm_tput<true> : k_ppm_tput<false>;
     const auto k_eye = !media ? k_ppm_eye<false, false> : hetero ? k_ppm_eye<true, true> : k_ppm_eye<true, false>;
-    const int block = 128;
+    const int block = BPT_BLOCK;
     const size_t smem = (size_t)RP.stack_cap * block * sizeof(uint32_t);
     if (smem > 48 * 1024) {
         WR_CUDA(ctx, cudaFuncSetAttribute(k_subpaths, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
@@ -1650,7 +1631,7 @@ int render_bidirectional(wr_ctx* ctx, const RenderScene& S, const RenderParams& 
         P.eye.nsamp = P.light.nsamp = P.nsamp;
         const int grid = (int)((P.nsamp + block - 1) / block);
         WR_CUDA(ctx, cudaMemsetAsync(P.ncand, 0, 5 * sizeof(unsigned long long), stream));
-        k_subpaths<<<subpath_grid, block, smem, stream>>>(S, P, err);
+        k_subpaths<<<subpath_grid, block, smem, stream>>>(S, P);
         WR_CUDA(ctx, cudaGetLastError());
         if (grid_on) {  // the batch's hash grids: one per slot (iteration), a second one for volume photons
             P.nslots = b;
@@ -1669,13 +1650,13 @@ int render_bidirectional(wr_ctx* ctx, const RenderScene& S, const RenderParams& 
         if (ppm) {
             k_tput<<<stride_grid, 256, 0, stream>>>(S, P);
             WR_CUDA(ctx, cudaGetLastError());
-            k_eye<<<grid, block, smem, stream>>>(S, P, err);
+            k_eye<<<grid, block, smem, stream>>>(S, P);
             WR_CUDA(ctx, cudaGetLastError());
             ctx->kernel_launches += 2;
         } else {
             k_bpt_enum<<<grid, block, 0, stream>>>(S, P);
             WR_CUDA(ctx, cudaGetLastError());
-            k_bpt_visible<<<visible_grid, block, smem, stream>>>(S, P, err);
+            k_bpt_visible<<<visible_grid, block, smem, stream>>>(S, P);
             WR_CUDA(ctx, cudaGetLastError());
             k_connect<<<connect_grid, block, 0, stream>>>(S, P);
             WR_CUDA(ctx, cudaGetLastError());

@@ -239,12 +239,11 @@ int wr_render_device(wr_ctx* ctx, wr_scene_id id, const wr_render_desc* desc, fl
         if (!rd->unsupported.empty()) return set_error(ctx, WR_ERR_UNSUPPORTED, rd->unsupported);
         if (desc->spp == 0) return WR_OK;
         cudaStream_t s = stream ? static_cast<cudaStream_t>(stream) : ctx->stream;
-        unsigned int* err = reinterpret_cast<unsigned int*>(ctx->scratch_words.as<unsigned long long>() + 1);
         RenderParams P{};
         P.seed = desc->seed;
         P.max_path_len = desc->max_path_len;
         P.flags = desc->flags;
-        P.stack_cap = (int)sc->tree.max_depth + 3;
+        P.stack_cap = quad_stack_cap(sc->tree);
         const uint64_t npix = (uint64_t)rd->S.cam.width * rd->S.cam.height;
         if (desc->mode == WR_MODE_BIDIRECTIONAL || desc->mode == WR_MODE_VCM || desc->mode == WR_MODE_PHOTON_MAP) {
             if (desc->mode == WR_MODE_PHOTON_MAP && rd->has_media)  // the march step of each medium's segments
@@ -257,7 +256,7 @@ int wr_render_device(wr_ctx* ctx, wr_scene_id id, const wr_render_desc* desc, fl
                 return set_error(ctx, WR_ERR_INVALID_ARGUMENT, "bidirectional / VCM / photon-mapping mode has no NEE switch");
             const int kind = desc->mode == WR_MODE_VCM ? BIDIR_VCM
                            : desc->mode == WR_MODE_PHOTON_MAP ? BIDIR_PHOTON_MAP : BIDIR_BPT;
-            return render_bidirectional(ctx, rd->S, P, desc->spp_offset, desc->spp, d_sum, d_sumsq, err, s, kind,
+            return render_bidirectional(ctx, rd->S, P, desc->spp_offset, desc->spp, d_sum, d_sumsq, s, kind,
                                         desc->radius > 0.f ? desc->radius : 0.01f, rd->has_hetero, rd->has_media);
         }
         if (desc->mode == WR_MODE_WAVEFRONT) {
@@ -269,7 +268,7 @@ int wr_render_device(wr_ctx* ctx, wr_scene_id id, const wr_render_desc* desc, fl
         for (uint64_t s0 = 0; s0 < desc->spp; s0 += per_launch) {
             P.s0 = (uint32_t)(desc->spp_offset + s0);
             P.s1 = (uint32_t)(desc->spp_offset + std::min<uint64_t>(desc->spp, s0 + per_launch));
-            WR_CUDA(ctx, launch_megakernel(rd->S, P, d_sum, d_sumsq, err, s));
+            WR_CUDA(ctx, launch_megakernel(rd->S, P, d_sum, d_sumsq, s));
             ctx->kernel_launches++;
         }
         return WR_OK;
@@ -412,6 +411,6 @@ extern "C" int wr_profile_render(wr_ctx* ctx, wr_scene_id id, const wr_render_de
     P.seed = desc->seed;
     P.max_path_len = desc->max_path_len;
     P.flags = desc->flags;
-    P.stack_cap = (int)sc->tree.max_depth + 3;
+    P.stack_cap = quad_stack_cap(sc->tree);
     return profile_wavefront(ctx, *rd, P, desc->spp_offset, desc->spp, d_sum, out);
 }

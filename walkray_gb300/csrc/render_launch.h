@@ -34,13 +34,13 @@ struct RenderParams {
     uint32_t s0, s1;          // sample range [s0, s1)
     uint32_t max_path_len;    // MCRenderer maxPathLen
     uint32_t flags;
-    int stack_cap;            // traversal stack entries per thread (tree depth + 3)
+    int stack_cap;            // the search's stack entries per thread (quad_stack_cap)
 };
 
 // plain megakernel: film[3*p+c] += sum over samples of the pixel colour
 // (film2 != NULL: also the sum of squares)
 cudaError_t launch_megakernel(const RenderScene& S, const RenderParams& P, float* film, float* film2,
-                              unsigned int* err, cudaStream_t stream);
+                              cudaStream_t stream);
 
 // WR_MODE_BIDIRECTIONAL, WR_MODE_VCM and WR_MODE_PHOTON_MAP (bpt.cu): adds
 // samples [spp_offset, spp_offset + spp) of every pixel to d_sum (and their
@@ -50,7 +50,7 @@ cudaError_t launch_megakernel(const RenderScene& S, const RenderParams& P, float
 // participating medium (photon mapping's volume photons and marched segments)
 enum : int { BIDIR_BPT = 0, BIDIR_VCM = 1, BIDIR_PHOTON_MAP = 2 };
 int render_bidirectional(wr_ctx* ctx, const RenderScene& S, const RenderParams& P, uint32_t spp_offset, uint32_t spp,
-                         float* d_sum, float* d_sumsq, unsigned int* err, cudaStream_t stream, int kind = BIDIR_BPT,
+                         float* d_sum, float* d_sumsq, cudaStream_t stream, int kind = BIDIR_BPT,
                          float base_radius = 0.01f, bool hetero = false, bool media = false);
 
 }  // namespace wr

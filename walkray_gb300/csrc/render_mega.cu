@@ -8,69 +8,86 @@
 
 namespace wr {
 
+constexpr int MEGA_BLOCK = 128;
+
+// The lanes of a warp stay together: each takes one ray of its own path per
+// turn (search_warp) and goes on to its pixel's next sample as soon as a path
+// ends, so that a warp waits for the lane with the most rays in all, not for
+// the longest path of every sample.
 template <bool STATS, bool MIS>
-__global__ void __launch_bounds__(128) k_megakernel(RenderScene S, RenderParams P, float* __restrict__ film,
-                                                      float* __restrict__ film2, unsigned int* __restrict__ err) {
+__global__ void __launch_bounds__(MEGA_BLOCK) k_megakernel(RenderScene S, RenderParams P, float* __restrict__ film,
+                                                           float* __restrict__ film2) {
+    constexpr unsigned FULL = 0xffffffffu;
     extern __shared__ uint32_t s_stack[];
+    __shared__ uint8_t s_item[MEGA_BLOCK / 32][LEAF_ITEMS];
     uint32_t* stack = s_stack + threadIdx.x;
-    const int stride = blockDim.x;
+    uint8_t* item = s_item[threadIdx.x >> 5];
+    const int stride = MEGA_BLOCK;
     const uint32_t npix = S.cam.width * S.cam.height;
-    const uint32_t pixel = blockIdx.x * blockDim.x + threadIdx.x;
-    if (pixel >= npix) return;
+    const uint32_t pixel = blockIdx.x * MEGA_BLOCK + threadIdx.x;
     f3 acc = mk(0, 0, 0), acc2 = mk(0, 0, 0);
     const float pf = prune_factor(P.flags);
     const bool nee = (P.flags & WR_RENDER_NEE) != 0;
-    for (uint32_t s = P.s0; s < P.s1; s++) {
-        PathRng g;
-        g.init(P.seed, pixel, s);
-        PRay cur = camera_ray(S.cam, pixel, g);
-        InsideStack st;
-        st.reset(cur.inside);
-        f3 color = mk(1, 1, 1), result = mk(0, 0, 0), prev_d = mk(0, 0, 0), lit = mk(0, 0, 0);
-        uint32_t depth = 0;
-        bool filtered = false;  // the eye ray is traced without a condition (camera.cpp:52)
-        bool nee_here = false, has_lr = false;
-        float mis_pdf = 0.f;
+    uint32_t s = pixel < npix ? P.s0 : P.s1;  // the sample this lane is at
+    bool start = true;                        // it begins with this turn
+    PathRng g;
+    g.init(P.seed, pixel, s);
+    PRay cur = ray_default();
+    InsideStack st;
+    st.reset(-1);
+    f3 color = mk(1, 1, 1), result = mk(0, 0, 0), prev_d = mk(0, 0, 0), lit = mk(0, 0, 0);
+    uint32_t depth = 0;
+    float mis_pdf = 0.f;
+    while (__any_sync(FULL, s < P.s1)) {
+        const bool on = s < P.s1;
+        const bool filtered = !start;  // the eye ray is traced without a condition (camera.cpp:52)
+        if (on && start) {
+            g.init(P.seed, pixel, s);
+            cur = camera_ray(S.cam, pixel, g);
+            st.reset(cur.inside);
+            color = mk(1, 1, 1);
+            result = prev_d = lit = mk(0, 0, 0);
+            depth = 0;
+            mis_pdf = 0.f;
+            start = false;
+        }
+        const Hit h = search_warp(S.tree, on, cur.o, cur.d, pf, filtered, cur.inside, cur.contact, stack, stride,
+                                  P.stack_cap, item);
+        bool done = false, nee_here = false, has_lr = false;
         LightReq lr;
-        for (;;) {
-            RayQ q = make_rayq(cur.o, cur.d, S.tree.scene_mag);
-            q.pf = pf;
-            const Hit h = filtered ? trace_closest<true, true>(S.tree, q, cur.inside, cur.contact, stack, stride,
-                                                               P.stack_cap, err)
-                                   : trace_closest<false, true>(S.tree, q, -1, -1, stack, stride, P.stack_cap, err);
+        if (on) {
             if (h.slot < 0 && filtered) {  // a scattered ray that escapes ends with zero radiance
                 nee_here = nee;
-                break;
+                done = true;
+            } else {
+                set_hit(S, cur, h);
+                done = path_advance<MIS>(S, cur, color, prev_d, depth, st, g, P.max_path_len, P.flags, result,
+                                         nee_here, mis_pdf, lr, has_lr);
             }
-            set_hit(S, cur, h);
-            filtered = true;
-            const bool done = path_advance<MIS>(S, cur, color, prev_d, depth, st, g, P.max_path_len, P.flags,
-                                                result, nee_here, mis_pdf, lr, has_lr);
-            if (MIS && has_lr) {  // the light connection of WR_RENDER_NEE_MIS, traced inline
-                RayQ lq = make_rayq(lr.o, lr.d, S.tree.scene_mag);
-                lq.pf = pf;
-                const Hit lh =
-                    trace_closest<true, true>(S.tree, lq, lr.inside, lr.contact, stack, stride, P.stack_cap, err);
-                if (light_req_visible(S, lh, lr)) lit = lit + lr.contrib;
-            }
-            if (done) break;
         }
-        if (nee_here) {  // the connection of the NEE branch, traced inline
+        if (MIS && __any_sync(FULL, has_lr)) {  // the light connection of WR_RENDER_NEE_MIS
+            const Hit lh = search_warp(S.tree, has_lr, lr.o, lr.d, pf, true, lr.inside, lr.contact, stack, stride,
+                                       P.stack_cap, item);
+            if (has_lr && light_req_visible(S, lh, lr)) lit = lit + lr.contrib;
+        }
+        if (__any_sync(FULL, nee_here)) {  // the connection of the NEE branch
             ShadowReq sr;
-            if (nee_prepare(S, cur, prev_d, color, g, sr)) {
-                RayQ q = make_rayq(sr.o, sr.d, S.tree.scene_mag);
-                q.pf = pf;
-                const Hit h =
-                    trace_closest<true, true>(S.tree, q, sr.inside, sr.contact, stack, stride, P.stack_cap, err);
-                if (nee_visible(h, sr.dist)) result = sr.contrib;
-            }
+            const bool conn = nee_here && nee_prepare(S, cur, prev_d, color, g, sr);
+            const Hit sh = search_warp(S.tree, conn, sr.o, sr.d, pf, true, sr.inside, sr.contact, stack, stride,
+                                       P.stack_cap, item);
+            if (conn && nee_visible(sh, sr.dist)) result = sr.contrib;
         }
-        if (!legal(result)) result = mk(0, 0, 0);
-        result = result + lit;
-        const f3 c = fix_vignetting(S.cam, result, pixel);
-        acc = acc + c;
-        if (STATS) acc2 = acc2 + vmul(c, c);
+        if (done) {
+            if (!legal(result)) result = mk(0, 0, 0);
+            result = result + lit;
+            const f3 c = fix_vignetting(S.cam, result, pixel);
+            acc = acc + c;
+            if (STATS) acc2 = acc2 + vmul(c, c);
+            s++;
+            start = true;
+        }
     }
+    if (pixel >= npix) return;
     float* f = film + 3 * (size_t)pixel;
     f[0] += acc.x;
     f[1] += acc.y;
@@ -84,8 +101,8 @@ __global__ void __launch_bounds__(128) k_megakernel(RenderScene S, RenderParams 
 }
 
 cudaError_t launch_megakernel(const RenderScene& S, const RenderParams& P, float* film, float* film2,
-                              unsigned int* err, cudaStream_t stream) {
-    const int block = 128;
+                              cudaStream_t stream) {
+    const int block = MEGA_BLOCK;
     const size_t smem = (size_t)P.stack_cap * block * sizeof(uint32_t);
     const uint32_t npix = S.cam.width * S.cam.height;
     const int grid = (int)((npix + block - 1) / block);
@@ -96,7 +113,7 @@ cudaError_t launch_megakernel(const RenderScene& S, const RenderParams& P, float
         cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
         if (e != cudaSuccess) return e;
     }
-    kern<<<grid, block, smem, stream>>>(S, P, film, film2, err);
+    kern<<<grid, block, smem, stream>>>(S, P, film, film2);
     return cudaGetLastError();
 }
 

@@ -116,12 +116,12 @@ static int render_noalloc_body(wr_ctx* ctx, wr_scene_id id, const wr_render_desc
     P.seed = desc->seed;
     P.max_path_len = desc->max_path_len;
     P.flags = desc->flags;
-    P.stack_cap = (int)sc->tree.max_depth + 3;
+    P.stack_cap = quad_stack_cap(sc->tree);
     const uint64_t per_launch = std::max<uint64_t>(1, (16ull << 20) / std::max<uint64_t>(1, npix));
     for (uint64_t s0 = 0; s0 < desc->spp; s0 += per_launch) {
         P.s0 = (uint32_t)(desc->spp_offset + s0);
         P.s1 = (uint32_t)(desc->spp_offset + std::min<uint64_t>(desc->spp, s0 + per_launch));
-        WR_CUDA(ctx, launch_megakernel(S, P, film, nullptr, err, s));
+        WR_CUDA(ctx, launch_megakernel(S, P, film, nullptr, s));
     }
     const float inv = desc->spp ? 1.0f / (float)desc->spp : 0.f;
     k_film_mean<<<(unsigned)std::min<size_t>((n + 255) / 256, 4096), 256, 0, s>>>(film, d_rgb_out, n, inv);

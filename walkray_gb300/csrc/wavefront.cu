@@ -483,9 +483,8 @@ __global__ void __launch_bounds__(128, 4) k_wf_shade(const RenderScene* __restri
 // side by side instead.  Same paths, draws and film additions as the loop.
 __global__ void __launch_bounds__(128) k_wf_drain(const RenderScene* __restrict__ scenes,
                                                     const WfJob* __restrict__ jobs,
-                                                    WfJobCounters* __restrict__ counters, WfSide X, int stack_cap,
-                                                    unsigned int* __restrict__ err) {
-    extern __shared__ uint32_t s_stack[];
+                                                    WfJobCounters* __restrict__ counters, WfSide X, int stack_cap) {
+    extern __shared__ __align__(16) uint32_t s_stack[];
     uint32_t* stack = s_stack + threadIdx.x;
     const uint32_t n = X.counts[0] + X.counts[1];
     const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
@@ -503,11 +502,8 @@ __global__ void __launch_bounds__(128) k_wf_drain(const RenderScene* __restrict_
     f3 result = mk(0, 0, 0);
     LightReq lr;
     for (;;) {
-        RayQ q = make_rayq(p.cur.o, p.cur.d, S.tree.scene_mag);
-        q.pf = pf;
-        const Hit h = filtered ? trace_closest<true, true>(S.tree, q, p.cur.inside, p.cur.contact, stack,
-                                                           blockDim.x, stack_cap, err)
-                               : trace_closest<false, true>(S.tree, q, -1, -1, stack, blockDim.x, stack_cap, err);
+        const Hit h = search_closest(S.tree, p.cur.o, p.cur.d, pf, filtered, p.cur.inside, p.cur.contact, stack,
+                                     blockDim.x, stack_cap);
         if (h.slot < 0 && filtered) {  // a scattered ray that escapes ends with zero radiance
             nee_here = nee;
             break;
@@ -517,10 +513,8 @@ __global__ void __launch_bounds__(128) k_wf_drain(const RenderScene* __restrict_
         const bool done = path_advance<true>(S, p.cur, p.color, p.prev_d, p.depth, p.st, g, J.max_path_len,
                                              J.flags, result, nee_here, p.mis_pdf, lr, has_lr);
         if (has_lr) {
-            RayQ lq = make_rayq(lr.o, lr.d, S.tree.scene_mag);
-            lq.pf = pf;
-            const Hit lh = trace_closest<true, true>(S.tree, lq, lr.inside, lr.contact, stack, blockDim.x, stack_cap,
-                                                     err);
+            const Hit lh = search_closest(S.tree, lr.o, lr.d, pf, true, lr.inside, lr.contact, stack, blockDim.x,
+                                          stack_cap);
             if (light_req_visible(S, lh, lr)) p.acc = p.acc + lr.contrib;
         }
         if (done) break;
@@ -529,9 +523,8 @@ __global__ void __launch_bounds__(128) k_wf_drain(const RenderScene* __restrict_
         ShadowReq sr;
         result = mk(0, 0, 0);
         if (nee_prepare(S, p.cur, p.prev_d, p.color, g, sr)) {
-            RayQ q = make_rayq(sr.o, sr.d, S.tree.scene_mag);
-            q.pf = pf;
-            const Hit h = trace_closest<true, true>(S.tree, q, sr.inside, sr.contact, stack, blockDim.x, stack_cap, err);
+            const Hit h = search_closest(S.tree, sr.o, sr.d, pf, true, sr.inside, sr.contact, stack, blockDim.x,
+                                         stack_cap);
             if (nee_visible(h, sr.dist)) result = sr.contrib;
         }
     }
@@ -1162,12 +1155,12 @@ int wf_read_counters(wr_ctx* ctx, WfEngine* E, std::vector<WfJobCounters>& out, 
 int wf_drain(wr_ctx* ctx, WfEngine* E, int side, uint32_t n, cudaStream_t s) {
     if (n == 0) return WR_OK;
     const int block = 128;
-    const size_t smem = (size_t)E->stack_cap * block * sizeof(uint32_t);
+    const size_t smem = (size_t)E->quad_cap * block * sizeof(uint32_t);
     if (smem > 48 * 1024)
         WR_CUDA(ctx, cudaFuncSetAttribute(k_wf_drain, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
     k_wf_drain<<<(n + block - 1) / block, block, smem, s>>>(E->scenes.as<RenderScene>(), E->jobs.as<WfJob>(),
                                                            E->counters.as<WfJobCounters>(), E->side[side],
-                                                           E->stack_cap, E->err_word.as<unsigned int>());
+                                                           E->quad_cap);
     WR_CUDA(ctx, cudaGetLastError());
     ctx->kernel_launches++;
     return WR_OK;

@@ -211,4 +211,222 @@ static __device__ __noinline__ Hit reference_search(const DevTree& T, f3 o, f3 d
     }
 }
 
+// ---------------------------------------------------------------------------
+// one ray per lane
+// ---------------------------------------------------------------------------
+constexpr uint32_t NO_WORD = QUAD_HOLE;
+constexpr int SLOT_REFERENCE = -2;  // Hit::slot of a ray that is left to reference_search
+
+// stack entries a thread is given: what the deepest walk can need, but at most
+// 28.  (On the 1.3 M-triangle icosphere and the mixed-material scene no ray
+// holds more than 17 at once, where the bound from the tree is 39; a ray that
+// would need more is left to reference_search.)
+__host__ __device__ inline int quad_stack_cap(const DevTree& T) {
+    return (int)(T.quad_stack + 4 < 28 ? T.quad_stack + 4 : 28);
+}
+
+struct SearchLane {
+    const QuadNode* quads;
+    const TriRec* tris;
+    f3 o, d;
+    QuadRay r;
+    float M, lim;          // the pruning rule's margin (infinite: no pruning) and limit
+    Hit h;
+    uint32_t cur, pend;    // the node or leaf to visit; the postponed leaf
+    int sp;                // stack[0], stack[stride], ... below it are waiting
+    bool filt;
+    int inside, contact;   // NoSelfCondition object ids (used when filt)
+
+    __device__ __forceinline__ bool walking() const { return !(cur & QUAD_LEAF); }
+    __device__ __forceinline__ bool at_leaf() const { return pend != NO_WORD && (cur & QUAD_LEAF); }
+    __device__ __forceinline__ bool finished() const { return cur == NO_WORD && pend == NO_WORD; }
+    __device__ __forceinline__ void clear() {
+        quads = nullptr;
+        tris = nullptr;
+        o = d = mk(0, 0, 0);
+        r = QuadRay{mk(0, 0, 0), mk(0, 0, 0), mk(0, 0, 0)};
+        M = lim = 0.f;
+        h = Hit{0.f, -1};
+        cur = pend = NO_WORD;
+        sp = 0;
+        filt = false;
+        inside = contact = -1;
+    }
+    // starts at the root
+    __device__ __forceinline__ void begin(const DevTree& T, f3 ro, f3 rd, float pf, bool f, int in, int co) {
+        o = ro;
+        d = rd;
+        quads = T.quads;
+        tris = T.tris;
+        filt = f;
+        inside = in;
+        contact = co;
+        M = box_margin(o, T.scene_mag);
+        lim = INFINITY;
+        sp = 0;
+        pend = NO_WORD;
+        const bool ok = make_quad_ray(o, d, T.scene_mag, M, r) && quads;
+        if (!(pf < INFINITY)) M = INFINITY;
+        h = Hit{INFINITY, ok ? -1 : SLOT_REFERENCE};
+        cur = ok ? 0u : NO_WORD;
+    }
+    __device__ __forceinline__ void pop(const uint32_t* stack, int stride) {
+        cur = NO_WORD;
+        if (sp > 0) {
+            sp -= stride;
+            cur = stack[sp];
+        }
+    }
+    // visits the node `cur`; `top`: the last `sp` with room for four more
+    __device__ __forceinline__ void visit(uint32_t* stack, int stride, int top) {
+        float4 t;
+        uint4 w;
+        quad_children(quads + cur, r, lim, t, w);
+        if (t.w < INFINITY) {
+            stack[sp] = w.w;
+            sp += stride;
+        }
+        if (t.z < INFINITY) {
+            stack[sp] = w.z;
+            sp += stride;
+        }
+        if (t.y < INFINITY) {
+            stack[sp] = w.y;
+            sp += stride;
+        }
+        cur = w.x;
+        if (!(t.x < INFINITY)) {
+            pop(stack, stride);
+        } else if (sp > top) {  // deeper than the stack: the reference's own walk needs none
+            sp = 0;
+            cur = pend = NO_WORD;
+            h.slot = SLOT_REFERENCE;
+        }
+        if ((cur & QUAD_LEAF) && cur != NO_WORD && pend == NO_WORD) {  // postpone it and walk on
+            pend = cur;
+            pop(stack, stride);
+        }
+    }
+    // a triangle hit that NoSelfCondition allows
+    __device__ __forceinline__ void take(float t, int slot, float dd) {
+        if (!(t < h.t || (t == h.t && slot > h.slot))) return;
+        // a near-grazing hit turns pruning off for good (graze_check)
+        const bool off = fabsf(dd) < GRAZE_COS * length(d) || (h.slot >= 0 && !(lim < INFINITY));
+        lim = off ? INFINITY : t * 1.001f + M;
+        h = Hit{t, slot};
+    }
+    // the postponed leaf is done: the next one, if the walk stands at it
+    __device__ __forceinline__ void leaf_done(const uint32_t* stack, int stride) {
+        pend = NO_WORD;
+        if ((cur & QUAD_LEAF) && cur != NO_WORD) {
+            pend = cur;
+            pop(stack, stride);
+        }
+    }
+};
+
+// the winner checked against the reference's boxes
+__device__ __forceinline__ Hit settle(const DevTree& T, const Hit& h, f3 o, f3 d, float pf, bool filt, int inside,
+                                      int contact) {
+    if (h.slot == -1 || (h.slot >= 0 && reference_reaches(T, h.slot, o, d))) return h;
+    return reference_search(T, o, d, pf, filt, inside, contact);
+}
+
+// Closest hit of this thread's ray on its own (any subset of a warp may call
+// it).  Its stack: entries at stack[k * stride], k < cap.
+__device__ __forceinline__ Hit search_closest(const DevTree& T, f3 o, f3 d, float pf, bool filt, int inside,
+                                              int contact, uint32_t* stack, int stride, int cap) {
+    SearchLane L;
+    L.begin(T, o, d, pf, filt, inside, contact);
+    const int top = (cap - 4) * stride;
+    while (!L.finished()) {
+        while (L.walking()) L.visit(stack, stride, top);
+        if (L.pend == NO_WORD) break;
+        const uint32_t first = L.pend & ((1u << QUAD_COUNT_AT) - 1u), count = L.pend >> QUAD_COUNT_AT & 7u;
+        for (uint32_t k = 0; k < count; k++) {
+            const int slot = (int)(first + k);
+            float dd = 0.f;
+            const float t = tri_slot_test(L.tris, slot, o, d, &dd);
+            if (t >= 0.f && t <= L.h.t && (!filt || noself_slot(L.tris, slot, d, inside, contact))) L.take(t, slot, dd);
+        }
+        L.leaf_done(stack, stride);
+    }
+    return settle(T, L.h, o, d, pf, filt, inside, contact);
+}
+
+constexpr int LEAF_ITEMS = 32 * (int)QUAD_LEAF_MAX;  // a warp's triangles in one leaf phase
+
+// Tests the postponed leaves of a warp's lanes (`has`): their triangles are
+// dealt out over all 32 lanes, one each, so that leaves of different lengths do
+// not leave lanes idle (the test in each lane's own loop kept 7 to 14 lanes
+// busy, this 24 to 29; the batch of 2^24 rays 2.69 -> 2.31 ms).  Every lane of
+// the warp calls it.  `item`: LEAF_ITEMS bytes of shared memory of the warp;
+// tris_of(tris, l): the triangles of lane l's tree.  Returns this lane's count.
+template <class TrisOf>
+__device__ __forceinline__ uint32_t warp_leaves(SearchLane& L, bool has, uint8_t* item, const uint32_t* stack,
+                                                int stride, TrisOf tris_of) {
+    constexpr unsigned FULL = 0xffffffffu;
+    const unsigned lane = threadIdx.x & 31u;
+    const unsigned lt_mask = (1u << lane) - 1u;
+    const uint32_t first = has ? L.pend & ((1u << QUAD_COUNT_AT) - 1u) : 0u;
+    const uint32_t count = has ? L.pend >> QUAD_COUNT_AT & 7u : 0u;
+    const unsigned c0 = __ballot_sync(FULL, count & 1u), c1 = __ballot_sync(FULL, count & 2u),
+                   c2 = __ballot_sync(FULL, count & 4u);
+    const uint32_t before = __popc(c0 & lt_mask) + 2u * __popc(c1 & lt_mask) + 4u * __popc(c2 & lt_mask);
+    const uint32_t total = __popc(c0) + 2u * __popc(c1) + 4u * __popc(c2);
+    for (uint32_t k = 0; k < count; k++) item[before + k] = (uint8_t)(lane | k << 5);
+    __syncwarp();
+    for (uint32_t base = 0; base < total; base += 32u) {
+        const bool on = base + lane < total;
+        const uint32_t it = on ? item[base + lane] : lane;
+        const int own = (int)(it & 31u);
+        const f3 ro = mk(__shfl_sync(FULL, L.o.x, own), __shfl_sync(FULL, L.o.y, own), __shfl_sync(FULL, L.o.z, own));
+        const f3 rd = mk(__shfl_sync(FULL, L.d.x, own), __shfl_sync(FULL, L.d.y, own), __shfl_sync(FULL, L.d.z, own));
+        const int slot = (int)(__shfl_sync(FULL, first, own) + (it >> 5));
+        const float best = __shfl_sync(FULL, L.h.t, own);
+        const TriRec* rt = tris_of(L.tris, own);
+        float t = -1.f, dd = 0.f;
+        if (on) t = tri_slot_test(rt, slot, ro, rd, &dd);
+        bool cand = t >= 0.f && t <= best;
+        unsigned cm = __ballot_sync(FULL, cand);
+        if (cm) {
+            const bool rf = __shfl_sync(FULL, (int)L.filt, own) != 0;
+            const int ri = __shfl_sync(FULL, L.inside, own), rc = __shfl_sync(FULL, L.contact, own);
+            if (cand && rf) cand = noself_slot(rt, slot, rd, ri, rc);
+            // the candidates go back to their rays one by one
+            for (cm = __ballot_sync(FULL, cand); cm; cm &= cm - 1u) {
+                const int b = __ffs(cm) - 1;
+                const int bo = __shfl_sync(FULL, own, b), bs = __shfl_sync(FULL, slot, b);
+                const float bt = __shfl_sync(FULL, t, b), bd = __shfl_sync(FULL, dd, b);
+                if ((int)lane == bo) L.take(bt, bs, bd);
+            }
+        }
+    }
+    if (has) L.leaf_done(stack, stride);
+    __syncwarp();
+    return count;
+}
+
+// Closest hits of a warp's rays, one per lane with `on`; every lane of the
+// warp calls it.  All rays in one tree.
+__device__ __forceinline__ Hit search_warp(const DevTree& T, bool on, f3 o, f3 d, float pf, bool filt, int inside,
+                                           int contact, uint32_t* stack, int stride, int cap, uint8_t* item) {
+    constexpr unsigned FULL = 0xffffffffu;
+    SearchLane L;
+    L.clear();
+    if (on) L.begin(T, o, d, pf, filt, inside, contact);
+    const int top = (cap - 4) * stride;
+    for (;;) {
+        const bool walking = L.walking();
+        const unsigned wm = __ballot_sync(FULL, walking), lm = __ballot_sync(FULL, L.at_leaf());
+        if (!(wm | lm)) break;
+        if (lm && (wm == 0 || __popc(lm) >= 8)) {
+            warp_leaves(L, L.pend != NO_WORD, item, stack, stride, [&](const TriRec*, int) { return T.tris; });
+        } else if (walking) {
+            for (int k = 0; k < 6 && L.walking(); k++) L.visit(stack, stride, top);
+        }
+    }
+    return on ? settle(T, L.h, o, d, pf, filt, inside, contact) : Hit{INFINITY, -1};
+}
+
 }  // namespace wr

@@ -40,22 +40,12 @@ struct WarpQueues {
     uint32_t id[64];
     int slot[64];
     float t[64];
-    uint8_t item[224];  // the leaf phase's triangles: lane | index in its leaf << 5
+    uint8_t item[LEAF_ITEMS];  // the leaf phase's triangles: lane | index in its leaf << 5
 };
-constexpr int SLOT_REFERENCE = -2;
-
-constexpr uint32_t NO_WORD = QUAD_HOLE;
-
 // this thread's work counts (profiling launches)
 struct TraceWork {
     unsigned long long rays, boxes, tris;
 };
-
-// stack entries a thread is given: what the deepest walk can need, but at most
-// 28.  (Measured on the 1.3 M-triangle icosphere and the mixed-material scene:
-// no ray holds more than 17 at once, where the bound from the tree is 39; a ray
-// that would need more is left to reference_search.)
-inline int quad_stack_cap(const DevTree& T) { return (int)(T.quad_stack + 4 < 28 ? T.quad_stack + 4 : 28); }
 
 // dynamic shared memory of a CTA: the threads' stacks, then the warps' queues
 inline size_t quad_smem(int cap, int block) {
@@ -81,8 +71,7 @@ template <class Src>
 __device__ __forceinline__ void finish_ray(Src& src, uint32_t id, Hit h) {
     TraceRay r;
     src.fetch(id, r);
-    if (h.slot < 0 || !reference_reaches(*r.T, h.slot, r.o, r.d))
-        h = reference_search(*r.T, r.o, r.d, r.pf, r.filt, r.inside, r.contact);
+    h = settle(*r.T, h, r.o, r.d, r.pf, r.filt, r.inside, r.contact);
     src.put(id, r, h);
 }
 
@@ -109,17 +98,9 @@ __device__ __forceinline__ void quad_trace(Src& src, uint32_t n, unsigned int* c
     uint32_t nin = 0, nfin = 0;  // entries of the queues
 
     uint32_t id = 0;
-    const QuadNode* quads = nullptr;
-    const TriRec* tris = nullptr;
-    f3 o = mk(0, 0, 0), d = mk(0, 0, 0);
-    QuadRay r;
-    float M = 0.f, lim = 0.f;
-    bool filt = false, active = false;
-    int inside = -1, contact = -1, sp = 0;
-    uint32_t cur = NO_WORD, pend = NO_WORD;  // the node or leaf to visit; the postponed leaf
-    Hit h;
-    h.t = 0.f;
-    h.slot = -1;
+    bool active = false;
+    SearchLane L;
+    L.clear();
 
     for (;;) {
         const unsigned idle = __ballot_sync(FULL, !active);
@@ -161,133 +142,31 @@ __device__ __forceinline__ void quad_trace(Src& src, uint32_t n, unsigned int* c
                 id = Q.in[nin - 1u - k];
                 TraceRay a;
                 src.fetch(id, a);
-                o = a.o;
-                d = a.d;
-                quads = a.T->quads;
-                tris = a.T->tris;
-                filt = a.filt;
-                inside = a.inside;
-                contact = a.contact;
-                M = box_margin(o, a.T->scene_mag);
-                h.t = lim = INFINITY;
-                sp = 0;
-                pend = NO_WORD;
+                L.begin(*a.T, a.o, a.d, a.pf, a.filt, a.inside, a.contact);
                 active = true;
-                const bool ok = make_quad_ray(o, d, a.T->scene_mag, M, r) && quads;
-                if (!(a.pf < INFINITY)) M = INFINITY;  // no pruning: `lim` stays infinite
-                h.slot = ok ? -1 : SLOT_REFERENCE;
-                cur = ok ? 0u : NO_WORD;
             }
             nin -= min(want, nin);
             __syncwarp();
         }
-        const bool walking = active && !(cur & QUAD_LEAF);
-        const bool waiting = active && pend != NO_WORD && (cur & QUAD_LEAF);
-        const unsigned wm = __ballot_sync(FULL, walking), lm = __ballot_sync(FULL, waiting);
+        const bool walking = active && L.walking();
+        const unsigned wm = __ballot_sync(FULL, walking), lm = __ballot_sync(FULL, active && L.at_leaf());
         if (lm && (wm == 0 || __popc(lm) >= tune.leaf_min)) {
-            // every postponed leaf, those of lanes still walking too: their
-            // triangles are dealt out over all lanes, one each
-            const bool has = active && pend != NO_WORD;
-            const uint32_t first = has ? pend & ((1u << QUAD_COUNT_AT) - 1u) : 0u;
-            const uint32_t count = has ? pend >> QUAD_COUNT_AT & 7u : 0u;
-            if (STATS) work.tris += count;
-            const unsigned c0 = __ballot_sync(FULL, count & 1u), c1 = __ballot_sync(FULL, count & 2u),
-                           c2 = __ballot_sync(FULL, count & 4u);
-            const uint32_t before =
-                __popc(c0 & lt_mask) + 2u * __popc(c1 & lt_mask) + 4u * __popc(c2 & lt_mask);
-            const uint32_t total = __popc(c0) + 2u * __popc(c1) + 4u * __popc(c2);
-            for (uint32_t k = 0; k < count; k++) Q.item[before + k] = (uint8_t)(lane | k << 5);
-            __syncwarp();
-            for (uint32_t base = 0; base < total; base += 32u) {
-                const bool on = base + lane < total;
-                const uint32_t it = on ? Q.item[base + lane] : lane;
-                const int own = (int)(it & 31u);
-                const f3 ro = mk(__shfl_sync(FULL, o.x, own), __shfl_sync(FULL, o.y, own), __shfl_sync(FULL, o.z, own));
-                const f3 rd = mk(__shfl_sync(FULL, d.x, own), __shfl_sync(FULL, d.y, own), __shfl_sync(FULL, d.z, own));
-                const int slot = (int)(__shfl_sync(FULL, first, own) + (it >> 5));
-                const float best = __shfl_sync(FULL, h.t, own);
-                const TriRec* rt = src.tris_of(tris, own);
-                float t = -1.f, dd = 0.f;
-                if (on) t = tri_slot_test(rt, slot, ro, rd, &dd);
-                bool cand = t >= 0.f && t <= best;
-                unsigned cm = __ballot_sync(FULL, cand);
-                if (cm) {
-                    const bool rf = __shfl_sync(FULL, (int)filt, own) != 0;
-                    const int ri = __shfl_sync(FULL, inside, own), rc = __shfl_sync(FULL, contact, own);
-                    if (cand && rf) cand = noself_slot(rt, slot, rd, ri, rc);
-                    // the candidates go back to their rays one by one
-                    for (cm = __ballot_sync(FULL, cand); cm; cm &= cm - 1u) {
-                        const int b = __ffs(cm) - 1;
-                        const int bo = __shfl_sync(FULL, own, b), bs = __shfl_sync(FULL, slot, b);
-                        const float bt = __shfl_sync(FULL, t, b), bd = __shfl_sync(FULL, dd, b);
-                        if ((int)lane == bo && (bt < h.t || (bt == h.t && bs > h.slot))) {
-                            // a near-grazing hit turns pruning off for good (graze_check)
-                            const bool off = fabsf(bd) < GRAZE_COS * length(d) || (h.slot >= 0 && !(lim < INFINITY));
-                            lim = off ? INFINITY : bt * 1.001f + M;
-                            h.t = bt;
-                            h.slot = bs;
-                        }
-                    }
-                }
-            }
-            if (has) {
-                pend = NO_WORD;
-                if ((cur & QUAD_LEAF) && cur != NO_WORD) {
-                    pend = cur;
-                    cur = NO_WORD;
-                    if (sp > 0) {
-                        sp -= stride;
-                        cur = stack[sp];
-                    }
-                }
-            }
-            __syncwarp();
+            // every postponed leaf, those of lanes still walking too
+            const uint32_t tested =
+                warp_leaves(L, active && L.pend != NO_WORD, Q.item, stack, stride,
+                            [&](const TriRec* t, int from) { return src.tris_of(t, from); });
+            if (STATS) work.tris += tested;
         } else if (walking) {
-            for (int k = 0; k < tune.steps; k++) {
-                float4 t;
-                uint4 w;
-                quad_children(quads + cur, r, lim, t, w);
+            for (int k = 0; k < tune.steps && L.walking(); k++) {
+                L.visit(stack, stride, top);
                 if (STATS) work.boxes += 4;
-                if (t.w < INFINITY) {
-                    stack[sp] = w.w;
-                    sp += stride;
-                }
-                if (t.z < INFINITY) {
-                    stack[sp] = w.z;
-                    sp += stride;
-                }
-                if (t.y < INFINITY) {
-                    stack[sp] = w.y;
-                    sp += stride;
-                }
-                cur = w.x;
-                if (!(t.x < INFINITY)) {
-                    cur = NO_WORD;
-                    if (sp > 0) {
-                        sp -= stride;
-                        cur = stack[sp];
-                    }
-                } else if (sp > top) {  // deeper than the stack: the reference's own walk needs none
-                    sp = 0;
-                    cur = pend = NO_WORD;
-                    h.slot = SLOT_REFERENCE;
-                }
-                if ((cur & QUAD_LEAF) && cur != NO_WORD && pend == NO_WORD) {  // postpone it and walk on
-                    pend = cur;
-                    cur = NO_WORD;
-                    if (sp > 0) {
-                        sp -= stride;
-                        cur = stack[sp];
-                    }
-                }
-                if (cur & QUAD_LEAF) break;
             }
         }
         // finished rays: misses at once, hits through the queue
-        const bool done = active && cur == NO_WORD && pend == NO_WORD;
+        const bool done = active && L.finished();
         const unsigned dm = __ballot_sync(FULL, done);
         if (dm) {
-            const bool queue = done && h.slot != -1;
+            const bool queue = done && L.h.slot != -1;
             if (done && !queue) {
                 TraceRay a;
                 src.put(id, a, Hit{INFINITY, -1});
@@ -296,8 +175,8 @@ __device__ __forceinline__ void quad_trace(Src& src, uint32_t n, unsigned int* c
             if (queue) {
                 const uint32_t at = nfin + __popc(qm & lt_mask);
                 Q.id[at] = id;
-                Q.slot[at] = h.slot;
-                Q.t[at] = h.t;
+                Q.slot[at] = L.h.slot;
+                Q.t[at] = L.h.t;
             }
             nfin += __popc(qm);
             if (done) active = false;

@@ -19,7 +19,7 @@
 #pragma once
 
 #include "../../include/walkray.h"
-#include "wr_traverse.cuh"
+#include "wr_quad.cuh"
 
 namespace wr {
 

@@ -256,28 +256,7 @@ struct Hit {
 __device__ __forceinline__ float4 ldg4(const float4* p) { return __ldg(p); }
 __device__ __forceinline__ uint4 ldg4u(const uint4* p) { return __ldg(p); }
 
-template <bool FILTERED, bool PRUNE>
-__device__ __forceinline__ void leaf_test(const DevTree& T, uint32_t first, uint32_t count, RayQ& q, int inside,
-                                          int contact, Hit& h) {
-    for (uint32_t k = 0; k < count; k++) {
-        const int slot = (int)(first + k);
-        const TriRec* tr = T.tris + slot;
-        const float4 a = ldg4(&tr->v0), b = ldg4(&tr->v1), c = ldg4(&tr->v2);
-        const f3 v0 = xyz(a), v1 = xyz(b), v2 = xyz(c);
-        float dd;
-        const float t = tri_test(v0, v1, v2, q, &dd);
-        if (t >= 0.f && (t < h.t || (t == h.t && slot > h.slot))) {
-            if (FILTERED) {
-                if (!noself_legal(inside, contact, (int)__float_as_uint(b.w), q.d, face_normal(v0, v1, v2))) continue;
-            }
-            h.t = t;
-            h.slot = slot;
-            if (PRUNE) graze_check(q, dd);
-        }
-    }
-}
-
-// The same with the filter chosen per ray (eye rays are traced without one)
+// the triangles of a leaf; the filter is chosen per ray (eye rays are traced without one)
 template <bool PRUNE>
 __device__ __forceinline__ void leaf_test_dyn(const TriRec* tris, uint32_t first, uint32_t count, RayQ& q, bool filt,
                                               int inside, int contact, Hit& h) {
@@ -296,65 +275,6 @@ __device__ __forceinline__ void leaf_test_dyn(const TriRec* tris, uint32_t first
             if (PRUNE) graze_check(q, dd);
         }
     }
-}
-
-// Closest hit.  `stack` is this thread's stack: entries at stack[k * stride],
-// at most `cap` of them (cap >= tree depth + 2 always suffices; a traversal
-// that would exceed it stops and sets bit 0 of *err instead of writing past).
-template <bool FILTERED, bool PRUNE>
-__device__ __forceinline__ Hit trace_closest(const DevTree& T, const RayQ& q0, int inside, int contact,
-                                             uint32_t* stack, int stride, int cap, unsigned int* err) {
-    RayQ q = q0;
-    Hit h;
-    h.t = __int_as_float(0x7f800000);
-    h.slot = -1;
-    float tn;
-    if (!box_pred(root_box(T), q, &tn)) return h;
-    if (T.root_w1 & LEAF_FLAG) {
-        leaf_test<FILTERED, PRUNE>(T, T.root_w0, T.root_w1 & ~LEAF_FLAG, q, inside, contact, h);
-        return h;
-    }
-    int sp = 0;
-    stack[0] = T.root_w0;
-    sp = 1;
-    while (sp > 0) {
-        const uint32_t pi = stack[(--sp) * stride];
-        const NodePair* P = T.pairs + pi;
-        const float4 A = ldg4(&P->a), B = ldg4(&P->b), C = ldg4(&P->c);
-        const uint4 W = ldg4u(&P->t);
-        float tl, tr;
-        bool hl, hr;
-        pair_pred(Box{A.x, A.y, A.z, A.w, B.x, B.y}, Box{B.z, B.w, C.x, C.y, C.z, C.w}, q, &hl, &hr, &tl, &tr);
-        if (PRUNE) {
-            const float lim = h.t * q.pf + q.M;
-            hl = hl && !(tl > lim);
-            hr = hr && !(tr > lim);
-        }
-        // leaves first (they can tighten the bound), both through one code
-        // path; then push internal children far-first so the near one is
-        // popped next
-        const bool ll = hl && (W.y & LEAF_FLAG), lr = hr && (W.w & LEAF_FLAG);
-        for (int k = 0, nk = (int)ll + (int)lr; k < nk; k++) {
-            const bool right = k == 1 || !ll;
-            leaf_test<FILTERED, PRUNE>(T, right ? W.z : W.x, (right ? W.w : W.y) & ~LEAF_FLAG, q, inside, contact, h);
-        }
-        hl = hl && !ll;
-        hr = hr && !lr;
-        if (sp + 2 > cap) {
-            atomicOr(err, 1u);
-            break;
-        }
-        if (hl && hr) {
-            const bool lnear = tl <= tr;
-            stack[(sp++) * stride] = lnear ? W.z : W.x;
-            stack[(sp++) * stride] = lnear ? W.x : W.z;
-        } else if (hl) {
-            stack[(sp++) * stride] = W.x;
-        } else if (hr) {
-            stack[(sp++) * stride] = W.z;
-        }
-    }
-    return h;
 }
 
 // barycentric weights of v1, v2 at the hit point (mesh.h:67-73)
