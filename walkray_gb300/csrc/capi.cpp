@@ -191,16 +191,16 @@ int wr_scene_upload(wr_ctx* ctx, const wr_scene_desc* d, wr_scene_id* out) {
     if (!L.slots.empty())
         WR_CUDA(ctx, cudaMemcpy(sc->tris.p, L.slots.data(), sizeof(TriRec) * L.slots.size(), cudaMemcpyHostToDevice));
     const size_t qb = sizeof(QuadNode) * Q.quads.size();
-    const size_t ub = sizeof(uint32_t) * (Q.leaf_up.size() + Q.pair_up.size());
+    const size_t ub = sizeof(uint32_t) * Q.leaf_up.size() + sizeof(uint4) * Q.pair_up.size();
     WR_CUDA(ctx, sc->quads.reserve(qb ? qb : 1));
     WR_CUDA(ctx, sc->leaf_up.reserve(sizeof(uint32_t) * std::max<size_t>(1, Q.leaf_up.size())));
-    WR_CUDA(ctx, sc->pair_up.reserve(sizeof(uint32_t) * std::max<size_t>(1, Q.pair_up.size())));
+    WR_CUDA(ctx, sc->pair_up.reserve(sizeof(uint4) * std::max<size_t>(1, Q.pair_up.size())));
     if (qb) WR_CUDA(ctx, cudaMemcpy(sc->quads.p, Q.quads.data(), qb, cudaMemcpyHostToDevice));
     if (!Q.leaf_up.empty())
         WR_CUDA(ctx, cudaMemcpy(sc->leaf_up.p, Q.leaf_up.data(), sizeof(uint32_t) * Q.leaf_up.size(),
                                 cudaMemcpyHostToDevice));
     if (!Q.pair_up.empty())
-        WR_CUDA(ctx, cudaMemcpy(sc->pair_up.p, Q.pair_up.data(), sizeof(uint32_t) * Q.pair_up.size(),
+        WR_CUDA(ctx, cudaMemcpy(sc->pair_up.p, Q.pair_up.data(), sizeof(uint4) * Q.pair_up.size(),
                                 cudaMemcpyHostToDevice));
     DevTree& T = sc->tree;
     T.pairs = sc->pairs.as<NodePair>();
@@ -217,7 +217,7 @@ int wr_scene_upload(wr_ctx* ctx, const wr_scene_desc* d, wr_scene_id* out) {
     T.num_slots = (uint32_t)L.slots.size();
     T.quads = qb ? sc->quads.as<QuadNode>() : nullptr;
     T.leaf_up = sc->leaf_up.as<uint32_t>();
-    T.pair_up = sc->pair_up.as<uint32_t>();
+    T.pair_up = sc->pair_up.as<uint4>();
     T.quad_stack = Q.stack;
     sc->info.num_triangles = nt;
     sc->info.num_nodes = ht.num_nodes();

@@ -298,13 +298,21 @@ QuadLayout build_quads(const HostTree& t, int threads) {
     std::vector<Item> items;
     items.reserve(t.num_leaves);
     std::vector<uint32_t> node_item(N, 0u);  // first item at or after each node
-    const bool fits = t.leaf_tris.size() <= QUAD_MAX_SLOTS;
+    bool fits = t.leaf_tris.size() <= QUAD_MAX_SLOTS;
     for (uint32_t n = 0; n < N; n++) {
         node_item[n] = (uint32_t)items.size();
         if (t.left[n] >= 0) {
             up[t.left[n]] = np << 1;
             up[t.right[n]] = np << 1 | 1u;
-            L.pair_up.push_back(up[n]);
+            const uint32_t u = up[n];
+            uint4 a = make_uint4(u, UP_ROOT, UP_ROOT, UP_ROOT);
+            if (u != UP_ROOT) {  // parents come first
+                const uint4& p = L.pair_up[u >> 1];
+                a.y = p.x;
+                a.z = p.y;
+                a.w = p.z;
+            }
+            L.pair_up.push_back(a);
             np++;
             continue;
         }
@@ -312,6 +320,7 @@ QuadLayout build_quads(const HostTree& t, int threads) {
             Item it;
             std::memcpy(it.box.lo, &t.box[6 * (size_t)n], 12);
             std::memcpy(it.box.hi, &t.box[6 * (size_t)n + 3], 12);
+            for (int d = 0; d < 3; d++) fits &= std::isfinite(it.box.lo[d]) && std::isfinite(it.box.hi[d]);
             it.count = std::min(QUAD_LEAF_MAX, t.leaf_count[n] - k);
             it.word = QUAD_LEAF | it.count << QUAD_COUNT_AT | (uint32_t)(slot + k);
             items.push_back(it);

@@ -14,13 +14,14 @@ namespace wr {
 struct QuadLayout {
     std::vector<QuadNode> quads;     // [0] is the root
     std::vector<uint32_t> leaf_up;   // per triangle slot: (pair << 1 | side) of its leaf, UP_ROOT if the root is that leaf
-    std::vector<uint32_t> pair_up;   // per pair: (parent pair << 1 | side), UP_ROOT for the root's
+    std::vector<uint4> pair_up;      // per pair: (pair << 1 | side) of its parent and the three above, UP_ROOT past the root
     uint32_t stack = 0;              // entries that the deepest walk can need (a node's other children, all the way down)
 };
 
 // Four-wide tree over the reference tree's leaves (their own boxes, bit for
 // bit) by the surface-area heuristic, and the reference tree's parent links.
-// A scene of more than QUAD_MAX_SLOTS triangles gets an empty `quads`.
+// A scene of more than QUAD_MAX_SLOTS triangles, or with a vertex that is not
+// finite, gets an empty `quads` (reference_search alone).
 QuadLayout build_quads(const HostTree& t, int threads);
 
 }  // namespace wr

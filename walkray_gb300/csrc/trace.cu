@@ -6,10 +6,10 @@
 // in shared memory, column-major (entry k of thread t at k * blockDim.x + t) so
 // a warp's pushes hit 32 distinct banks.
 //
-// Bound by the latency of the tree's nodes in L2 and by issue (2^24 incoherent
-// rays on the 1,310,720-triangle icosphere: 3.38 ms walking the reference's
-// tree with both of its slab tests per box, 2.30 ms here; 93 -> 61 warp
-// instructions a ray).
+// Bound by the L1 cache's load pipe and the latency behind it: on 4.2 M
+// incoherent rays (1,310,720-triangle icosphere) the pipe is 64 % busy, issue
+// 46 %, 78 warp instructions a ray (174 when it walked the reference's tree with
+// two slab tests a box).  2^24 rays: 3.38 -> 2.23 ms.
 #include <cuda_runtime.h>
 
 #include <algorithm>
@@ -49,7 +49,7 @@ struct BatchSrc {
         }
         reinterpret_cast<uint4*>(hits)[id] = out;
     }
-    __device__ __forceinline__ const TriRec* tris_of(const TriRec*, int) const { return T.tris; }
+    __device__ __forceinline__ const TriRec* tris_of(const RayInShared&, int) const { return T.tris; }
     // the same for the walk that visits every box the reference visits (warp_trace)
     __device__ __forceinline__ void load(uint64_t id, TraceLane& L, uint32_t* stack, int stride) const {
         TraceRay a;
@@ -111,8 +111,8 @@ cudaError_t launch_trace_closest(const DevTree& T, const float* d_rays, uint64_t
     if (e != cudaSuccess) return e;
     // blocks per SM from the occupancy calculator for this stack size
     int per_sm = 1;
-    // 0: the 7-CTA variant (72 registers; 2^24 rays: 2.31 ms, 2.30 with 6, 2.38 with 5, 2.49 with 8)
-    const int variant = ctas_per_sm ? ctas_per_sm : 7;
+    // 0: the 6-CTA variant (80 registers; 2^24 rays: 2.23 ms, 2.38 with 7, 2.64 with 5, 2.69 with 8)
+    const int variant = ctas_per_sm ? ctas_per_sm : 6;
     void (*kern)(DevTree, const float*, uint64_t, const int32_t*, const int32_t*, wr_hit*, unsigned long long*, int,
                  TraceTune, unsigned int*) = !prune         ? k_trace_closest_exact
                                              : variant >= 8 ? k_trace_closest<8>
@@ -127,7 +127,8 @@ cudaError_t launch_trace_closest(const DevTree& T, const float* d_rays, uint64_t
     if (e != cudaSuccess) return e;
     if (ctas_per_sm > 0) per_sm = std::min(per_sm, ctas_per_sm);
     if (per_sm < 1) per_sm = 1;
-    uint64_t need_blocks = (n + block - 1) / block;
+    // few rays: a warp for each, as far as the grid goes
+    uint64_t need_blocks = prune ? (n + block / 32 - 1) / (block / 32) : (n + block - 1) / block;
     int grid = num_sms * per_sm;
     if ((uint64_t)grid > need_blocks) grid = (int)(need_blocks ? need_blocks : 1);
     if (launched_blocks) *launched_blocks = grid;

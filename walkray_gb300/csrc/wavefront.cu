@@ -254,8 +254,8 @@ struct ExtendSrc {
         hits[id] = make_int2(h.slot, __float_as_int(h.t));
     }
     // rays of several scenes share the queue
-    __device__ __forceinline__ const TriRec* tris_of(const TriRec* tris, int from) const {
-        return shfl_ptr(tris, from);
+    __device__ __forceinline__ const TriRec* tris_of(const RayInShared& rays, int from) const {
+        return rays.tris_of(from);
     }
     __device__ __forceinline__ void load(uint64_t id, TraceLane& L, uint32_t* stack, int stride) const {
         TraceRay a;
@@ -331,8 +331,8 @@ struct ShadowSrc {
         hits[id] = make_int2(h.slot, __float_as_int(h.t));
     }
     // rays of several scenes share the queue
-    __device__ __forceinline__ const TriRec* tris_of(const TriRec* tris, int from) const {
-        return shfl_ptr(tris, from);
+    __device__ __forceinline__ const TriRec* tris_of(const RayInShared& rays, int from) const {
+        return rays.tris_of(from);
     }
 };
 
@@ -354,7 +354,7 @@ using ShadowTraceKernel = void (*)(const RenderScene*, const WfJob*, WfShadow, i
 
 // the shadow traversal for a configuration: the extend stage's register cap
 static ShadowTraceKernel shadow_trace_kernel(int ctas_per_sm) {
-    if (ctas_per_sm == 0) ctas_per_sm = 7;
+    if (ctas_per_sm == 0) ctas_per_sm = 6;
     if (ctas_per_sm >= 8) return k_wf_shadow_trace<8>;
     if (ctas_per_sm >= 7) return k_wf_shadow_trace<7>;
     if (ctas_per_sm >= 6) return k_wf_shadow_trace<6>;
@@ -362,10 +362,10 @@ static ShadowTraceKernel shadow_trace_kernel(int ctas_per_sm) {
 }
 
 // the extend kernel for a configuration: register cap from ctas_per_sm
-// (0 = the 7-CTA variant: mixed-material scene 1024^2 x 32 spp 35.3 ms, 35.6 with 6, 37.4 with 8)
+// (0 = the 6-CTA variant: mixed-material scene 1024^2 x 32 spp 33.2 ms, 33.9 with 7, 36.3 with 8)
 static ExtendKernel extend_kernel(int ctas_per_sm, bool stats, bool exact) {
     if (exact) return stats ? k_wf_extend<true, true, 6> : k_wf_extend<false, true, 6>;
-    if (ctas_per_sm == 0) ctas_per_sm = 7;
+    if (ctas_per_sm == 0) ctas_per_sm = 6;
     if (ctas_per_sm >= 8) return stats ? k_wf_extend<true, false, 8> : k_wf_extend<false, false, 8>;
     if (ctas_per_sm >= 7) return stats ? k_wf_extend<true, false, 7> : k_wf_extend<false, false, 7>;
     if (ctas_per_sm >= 6) return stats ? k_wf_extend<true, false, 6> : k_wf_extend<false, false, 6>;

@@ -60,7 +60,7 @@ constexpr uint32_t QUAD_HOLE = 0xffffffffu;  // an unused child: its box meets n
 constexpr uint32_t QUAD_COUNT_AT = 28u;      // leaf words: first slot below this bit, triangle count above it
 constexpr uint32_t QUAD_LEAF_MAX = 7u;       // triangles of one leaf word
 constexpr uint32_t QUAD_MAX_SLOTS = (1u << QUAD_COUNT_AT) - 8u;
-constexpr uint32_t UP_ROOT = 0xffffffffu;    // leaf_up / pair_up of the root
+constexpr uint32_t UP_ROOT = 0xffffffffu;    // leaf_up / pair_up: the root and beyond
 
 struct DevTree {
     const NodePair* pairs;
@@ -70,11 +70,10 @@ struct DevTree {
     float scene_mag;            // max |coordinate| over all vertices
     uint32_t max_depth;
     uint32_t num_pairs, num_slots;
-    // the four-wide tree the search walks (nullptr: more than QUAD_MAX_SLOTS
-    // triangles) and the reference tree's parent links, (pair << 1 | side)
+    // the four-wide tree the search walks (nullptr: none, see build_quads) and the reference tree's parent links, (pair << 1 | side)
     const QuadNode* quads;
     const uint32_t* leaf_up;  // per triangle slot
-    const uint32_t* pair_up;  // per pair
+    const uint4* pair_up;     // per pair: its next four ancestors, nearest first
     uint32_t quad_stack;      // stack entries that the deepest walk of `quads` can need
 };
 

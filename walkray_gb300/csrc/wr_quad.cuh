@@ -62,8 +62,17 @@ __device__ __forceinline__ bool make_quad_ray(f3 o, f3 d, float scene_mag, float
     return on + scene_mag <= 1e9f && dn >= 1e-6f && dn <= 1e6f;  // false for a NaN
 }
 
-__device__ __forceinline__ float max3(float a, float b, float c) { return fmaxf(fmaxf(a, b), c); }
-__device__ __forceinline__ float min3(float a, float b, float c) { return fminf(fminf(a, b), c); }
+// of three at once (a NaN is dropped, as by fmaxf and fminf)
+__device__ __forceinline__ float max3(float a, float b, float c) {
+    float r;
+    asm("max.f32 %0, %1, %2, %3;" : "=f"(r) : "f"(a), "f"(b), "f"(c));
+    return r;
+}
+__device__ __forceinline__ float min3(float a, float b, float c) {
+    float r;
+    asm("min.f32 %0, %1, %2, %3;" : "=f"(r) : "f"(a), "f"(b), "f"(c));
+    return r;
+}
 
 // entry distance of one child, +inf when the ray misses it or enters it beyond `lim`
 __device__ __forceinline__ float quad_entry(const QuadRay& r, float nx, float ny, float nz, float fx, float fy,
@@ -86,7 +95,8 @@ __device__ __forceinline__ void quad_order(float& ta, uint32_t& a, float& tb, ui
     a = w;
 }
 
-// the four children of a node, nearest first; t = +inf: not to be visited
+// The four children of a node, the nearest first (ordering the others too saves
+// 1 % of the visits); t = +inf: not to be visited.
 __device__ __forceinline__ void quad_children(const QuadNode* q, const QuadRay& r, float lim, float4& t, uint4& w) {
     const char* p = reinterpret_cast<const char*>(q);
     // 48 bytes on where the near plane is the upper one (the hi rows)
@@ -104,10 +114,8 @@ __device__ __forceinline__ void quad_children(const QuadNode* q, const QuadRay& 
     t.z = quad_entry(r, nx.z, ny.z, nz.z, fx.z, fy.z, fz.z, lim);
     t.w = quad_entry(r, nx.w, ny.w, nz.w, fx.w, fy.w, fz.w, lim);
     quad_order(t.x, w.x, t.y, w.y);
-    quad_order(t.z, w.z, t.w, w.w);
     quad_order(t.x, w.x, t.z, w.z);
-    quad_order(t.y, w.y, t.w, w.w);
-    quad_order(t.y, w.y, t.z, w.z);
+    quad_order(t.x, w.x, t.w, w.w);
 }
 
 // the reference's triangle test on one record
@@ -118,6 +126,26 @@ __device__ __forceinline__ float tri_slot_test(const TriRec* tris, int slot, f3 
     q.o = o;
     q.d = d;
     return tri_test(xyz(a), xyz(b), xyz(c), q, dd);
+}
+
+// its first half: false where the ray passes outside an edge
+__device__ __forceinline__ bool tri_slot_inside(const TriRec* tris, int slot, f3 o, f3 d) {
+    const TriRec* tr = tris + slot;
+    const float4 a = ldg4(&tr->v0), b = ldg4(&tr->v1), c = ldg4(&tr->v2);
+    RayQ q;
+    q.o = o;
+    q.d = d;
+    return tri_inside(xyz(a), xyz(b), xyz(c), q);
+}
+
+// its second half
+__device__ __forceinline__ float tri_slot_distance(const TriRec* tris, int slot, f3 o, f3 d, float* dd) {
+    const TriRec* tr = tris + slot;
+    const float4 a = ldg4(&tr->v0), b = ldg4(&tr->v1), c = ldg4(&tr->v2);
+    RayQ q;
+    q.o = o;
+    q.d = d;
+    return tri_distance(xyz(a), xyz(b), xyz(c), q, dd);
 }
 
 // NoSelfCondition on one record
@@ -132,9 +160,10 @@ __device__ __forceinline__ bool noself_slot(const TriRec* tris, int slot, f3 d, 
 // ---------------------------------------------------------------------------
 // box and topology words of one child (at = pair << 1 | side)
 __device__ __forceinline__ Box child_box(const DevTree& T, uint32_t at) {
-    const float2* p = reinterpret_cast<const float2*>(T.pairs + (at >> 1)) + 3 * (at & 1u);
-    const float2 a = __ldg(p), b = __ldg(p + 1), c = __ldg(p + 2);
-    return Box{a.x, a.y, b.x, b.y, c.x, c.y};
+    const bool right = at & 1u;
+    const float4* p = &T.pairs[at >> 1].a + (right ? 1 : 0);
+    const float4 a = ldg4(p), b = ldg4(p + 1);  // two 16-byte pieces hold either box
+    return right ? Box{a.z, a.w, b.x, b.y, b.z, b.w} : Box{a.x, a.y, a.z, a.w, b.x, b.y};
 }
 
 // the reference's face tests on a box
@@ -142,38 +171,44 @@ static __device__ __noinline__ bool box_faces(Box b, f3 o, f3 d, float scene_mag
     return box_exact(b, make_rayq(o, d, scene_mag));
 }
 
-// Does the reference's predicate pass on a box?  Usually told by the exit face
-// alone: the ray passes the box shrunk by M (entry sn = near planes moved in,
-// exit U2) and leaves the grown box (U1) through one axis before it comes
-// within M of any other axis's far plane.  The reference's test of that exit
-// face then passes: its plane point is at least M inside the box on both other
-// axes, and in front of the origin.  Anything else (a box thinner than 2M, an
-// edge within M, a NaN) runs the face tests.  With QuadRay's constants the
-// planes moved in are fb for a near and nb for a far one.
+// Does the reference's predicate pass on a box?  Usually told by one far face:
+// with the distances to its plane moved in (s) and out (g) by M, the face's
+// plane point lies at least M inside the box on another axis when that axis's
+// near plane moved in comes before s and its far plane moved in after g.  If
+// so on both other axes, and s is in front of the origin, the reference's test
+// of this face passes.  (A flat box passes by the face of its thin axis.)
+// Anything else -- an edge within M, a NaN -- runs the face tests.  With
+// QuadRay's constants the planes moved in are fb for a near and nb for a far
+// one.
 __device__ __forceinline__ bool reference_passes(const Box& b, const QuadRay& r, f3 o, f3 d, float scene_mag) {
     const bool px = r.inv.x > 0.f, py = r.inv.y > 0.f, pz = r.inv.z > 0.f;
     const float fx = px ? b.hx : b.lx, fy = py ? b.hy : b.ly, fz = pz ? b.hz : b.lz;
+    const float nx = __fmaf_rn(px ? b.lx : b.hx, r.inv.x, r.fb.x), ny = __fmaf_rn(py ? b.ly : b.hy, r.inv.y, r.fb.y),
+                nz = __fmaf_rn(pz ? b.lz : b.hz, r.inv.z, r.fb.z);
     const float sx = __fmaf_rn(fx, r.inv.x, r.nb.x), sy = __fmaf_rn(fy, r.inv.y, r.nb.y),
                 sz = __fmaf_rn(fz, r.inv.z, r.nb.z);
-    const float U2 = min3(sx, sy, sz);
-    const float U1 = min3(__fmaf_rn(fx, r.inv.x, r.fb.x), __fmaf_rn(fy, r.inv.y, r.fb.y),
-                          __fmaf_rn(fz, r.inv.z, r.fb.z));
-    const bool in = (__fmaf_rn(px ? b.lx : b.hx, r.inv.x, r.fb.x) <= U2) &
-                    (__fmaf_rn(py ? b.ly : b.hy, r.inv.y, r.fb.y) <= U2) &
-                    (__fmaf_rn(pz ? b.lz : b.hz, r.inv.z, r.fb.z) <= U2) & (U2 >= 0.f);
-    const bool gx = sx >= U1, gy = sy >= U1, gz = sz >= U1;
-    if (in & ((gx & gy) | (gx & gz) | (gy & gz))) return true;
-    return box_faces(b, o, d, scene_mag);
+    const float gx = __fmaf_rn(fx, r.inv.x, r.fb.x), gy = __fmaf_rn(fy, r.inv.y, r.fb.y),
+                gz = __fmaf_rn(fz, r.inv.z, r.fb.z);
+    const bool by_x = (ny <= sx) & (nz <= sx) & (sy >= gx) & (sz >= gx) & (sx >= 0.f);
+    const bool by_y = (nx <= sy) & (nz <= sy) & (sx >= gy) & (sz >= gy) & (sy >= 0.f);
+    const bool by_z = (nx <= sz) & (ny <= sz) & (sx >= gz) & (sy >= gz) & (sz >= 0.f);
+    return (by_x | by_y | by_z) || box_faces(b, o, d, scene_mag);
 }
 
-// does the reference's predicate pass on every box above `slot`'s triangle?
-__device__ __forceinline__ bool reference_reaches(const DevTree& T, int slot, f3 o, f3 d) {
+// Does the reference's predicate pass on every box above `slot`'s triangle?
+// Each pair knows its next four ancestors, so the loads of a way of 22 boxes
+// are 6 deep instead of 22.  Out of line: inlined, its registers made the
+// search spill (mixed-material scene 1024^2 x 32 spp 34.7 ms, 34.0 this way).
+static __device__ __noinline__ bool reference_reaches(const DevTree& T, int slot, f3 o, f3 d) {
     QuadRay r;
     make_quad_ray(o, d, T.scene_mag, box_margin(o, T.scene_mag), r);
     for (uint32_t at = __ldg(T.leaf_up + slot); at != UP_ROOT;) {
-        const Box b = child_box(T, at);
-        at = __ldg(T.pair_up + (at >> 1));
-        if (!reference_passes(b, r, o, d, T.scene_mag)) return false;
+        const uint4 up = ldg4u(T.pair_up + (at >> 1));
+        const uint32_t a[4] = {at, up.x, up.y, up.z};
+        at = up.w;
+#pragma unroll
+        for (int k = 0; k < 4; k++)
+            if (a[k] != UP_ROOT && !reference_passes(child_box(T, a[k]), r, o, d, T.scene_mag)) return false;
     }
     return reference_passes(root_box(T), r, o, d, T.scene_mag);
 }
@@ -204,7 +239,7 @@ static __device__ __noinline__ Hit reference_search(const DevTree& T, f3 o, f3 d
             leaf_test_dyn<true>(T.tris, w.x, w.y & ~LEAF_FLAG, q, filt, inside, contact, h);
         }
         while (at & 1u) {
-            at = __ldg(T.pair_up + (at >> 1));
+            at = __ldg(&T.pair_up[at >> 1].x);
             if (at == UP_ROOT) return h;
         }
         at |= 1u;
@@ -214,59 +249,132 @@ static __device__ __noinline__ Hit reference_search(const DevTree& T, f3 o, f3 d
 // ---------------------------------------------------------------------------
 // one ray per lane
 // ---------------------------------------------------------------------------
-constexpr uint32_t NO_WORD = QUAD_HOLE;
+constexpr uint32_t NO_WORD = QUAD_HOLE;  // neither node nor leaf
 constexpr int SLOT_REFERENCE = -2;  // Hit::slot of a ray that is left to reference_search
 
-// stack entries a thread is given: what the deepest walk can need, but at most
-// 28.  (On the 1.3 M-triangle icosphere and the mixed-material scene no ray
+// Stack entries a thread is given: what the deepest walk can need, but at most
+// 20.  (On the 1.3 M-triangle icosphere and the mixed-material scene no ray
 // holds more than 17 at once, where the bound from the tree is 39; a ray that
-// would need more is left to reference_search.)
+// would need more is left to reference_search.  28 entries leave the L1 cache
+// 20 to 30 KB less: mixed-material scene 37.6 ms, with 20 37.0.)
 __host__ __device__ inline int quad_stack_cap(const DevTree& T) {
-    return (int)(T.quad_stack + 4 < 28 ? T.quad_stack + 4 : 28);
+    return (int)(T.quad_stack + 4 < 20 ? T.quad_stack + 4 : 20);
 }
 
+// What a search reads only at leaves: the ray, the pruning rule's margin
+// (infinite: no pruning) and NoSelfCondition's object ids (used when filt).
+// In registers:
+struct RayInRegs {
+    const TriRec* tt;
+    f3 ro, rd;
+    float rm;
+    bool f;
+    int in, co;
+    __device__ __forceinline__ void set(const DevTree* T, f3 o, f3 d, float M, bool filt, int inside, int contact) {
+        tt = T ? T->tris : nullptr;
+        ro = o;
+        rd = d;
+        rm = M;
+        f = filt;
+        in = inside;
+        co = contact;
+    }
+    __device__ __forceinline__ float margin() const { return rm; }
+    __device__ __forceinline__ float length_d() const { return length(rd); }
+    // lane l's (every lane of the warp calls these)
+    __device__ __forceinline__ void ray_of(int l, f3& o, f3& d) const {
+        constexpr unsigned FULL = 0xffffffffu;
+        o = mk(__shfl_sync(FULL, ro.x, l), __shfl_sync(FULL, ro.y, l), __shfl_sync(FULL, ro.z, l));
+        d = mk(__shfl_sync(FULL, rd.x, l), __shfl_sync(FULL, rd.y, l), __shfl_sync(FULL, rd.z, l));
+    }
+    __device__ __forceinline__ const TriRec* tris_of(int l) const {
+        return reinterpret_cast<const TriRec*>(__shfl_sync(0xffffffffu, reinterpret_cast<unsigned long long>(tt), l));
+    }
+    __device__ __forceinline__ void ids_of(int l, bool& filt, int& inside, int& contact) const {
+        constexpr unsigned FULL = 0xffffffffu;
+        filt = __shfl_sync(FULL, (int)f, l) != 0;
+        inside = __shfl_sync(FULL, in, l);
+        contact = __shfl_sync(FULL, co, l);
+    }
+};
+// or in shared memory, word k of thread t at p[k * stride] of its own p: in
+// registers the persistent loop spills at 6 CTAs (2^24 rays 2.30 ms, 2.16 this
+// way)
+constexpr int RAY_WORDS = 12;
+struct RayInShared {
+    float* p;
+    int stride;
+    __device__ __forceinline__ void put_ptr(int k, const void* v) const {
+        const unsigned long long x = reinterpret_cast<unsigned long long>(v);
+        p[k * stride] = __uint_as_float((uint32_t)x);
+        p[(k + 1) * stride] = __uint_as_float((uint32_t)(x >> 32));
+    }
+    __device__ __forceinline__ static unsigned long long get_ptr(const float* q, int k, int stride) {
+        return __float_as_uint(q[k * stride]) | (unsigned long long)__float_as_uint(q[(k + 1) * stride]) << 32;
+    }
+    __device__ __forceinline__ void set(const DevTree* T, f3 o, f3 d, float M, bool filt, int inside, int contact) {
+        put_ptr(10, T ? T->tris : nullptr);
+        p[0] = o.x;
+        p[stride] = o.y;
+        p[2 * stride] = o.z;
+        p[3 * stride] = d.x;
+        p[4 * stride] = d.y;
+        p[5 * stride] = d.z;
+        p[6 * stride] = M;
+        p[7 * stride] = __int_as_float((int)filt);
+        p[8 * stride] = __int_as_float(inside);
+        p[9 * stride] = __int_as_float(contact);
+    }
+    __device__ __forceinline__ const TriRec* tris_of(int l) const {
+        return reinterpret_cast<const TriRec*>(get_ptr(p + (l - (int)(threadIdx.x & 31u)), 10, stride));
+    }
+    __device__ __forceinline__ float margin() const { return p[6 * stride]; }
+    __device__ __forceinline__ float length_d() const { return length(mk(p[3 * stride], p[4 * stride], p[5 * stride])); }
+    __device__ __forceinline__ void ray_of(int l, f3& o, f3& d) const {
+        const float* q = p + (l - (int)(threadIdx.x & 31u));
+        o = mk(q[0], q[stride], q[2 * stride]);
+        d = mk(q[3 * stride], q[4 * stride], q[5 * stride]);
+    }
+    __device__ __forceinline__ void ids_of(int l, bool& filt, int& inside, int& contact) const {
+        const float* q = p + (l - (int)(threadIdx.x & 31u));
+        filt = __float_as_int(q[7 * stride]) != 0;
+        inside = __float_as_int(q[8 * stride]);
+        contact = __float_as_int(q[9 * stride]);
+    }
+};
+
+template <class Ray>
 struct SearchLane {
+    Ray ray;
     const QuadNode* quads;
-    const TriRec* tris;
-    f3 o, d;
     QuadRay r;
-    float M, lim;          // the pruning rule's margin (infinite: no pruning) and limit
+    float lim;             // boxes entered beyond it are skipped
     Hit h;
     uint32_t cur, pend;    // the node or leaf to visit; the postponed leaf
     int sp;                // stack[0], stack[stride], ... below it are waiting
-    bool filt;
-    int inside, contact;   // NoSelfCondition object ids (used when filt)
 
     __device__ __forceinline__ bool walking() const { return !(cur & QUAD_LEAF); }
     __device__ __forceinline__ bool at_leaf() const { return pend != NO_WORD && (cur & QUAD_LEAF); }
     __device__ __forceinline__ bool finished() const { return cur == NO_WORD && pend == NO_WORD; }
     __device__ __forceinline__ void clear() {
         quads = nullptr;
-        tris = nullptr;
-        o = d = mk(0, 0, 0);
+        ray.set(nullptr, mk(0, 0, 0), mk(0, 0, 0), 0.f, false, -1, -1);
         r = QuadRay{mk(0, 0, 0), mk(0, 0, 0), mk(0, 0, 0)};
-        M = lim = 0.f;
+        lim = 0.f;
         h = Hit{0.f, -1};
         cur = pend = NO_WORD;
         sp = 0;
-        filt = false;
-        inside = contact = -1;
     }
     // starts at the root
-    __device__ __forceinline__ void begin(const DevTree& T, f3 ro, f3 rd, float pf, bool f, int in, int co) {
-        o = ro;
-        d = rd;
+    __device__ __forceinline__ void begin(const DevTree& T, f3 o, f3 d, float pf, bool filt, int inside,
+                                          int contact) {
         quads = T.quads;
-        tris = T.tris;
-        filt = f;
-        inside = in;
-        contact = co;
-        M = box_margin(o, T.scene_mag);
         lim = INFINITY;
         sp = 0;
         pend = NO_WORD;
+        const float M = box_margin(o, T.scene_mag);
         const bool ok = make_quad_ray(o, d, T.scene_mag, M, r) && quads;
-        if (!(pf < INFINITY)) M = INFINITY;
+        ray.set(&T, o, d, pf < INFINITY ? M : INFINITY, filt, inside, contact);
         h = Hit{INFINITY, ok ? -1 : SLOT_REFERENCE};
         cur = ok ? 0u : NO_WORD;
     }
@@ -276,6 +384,11 @@ struct SearchLane {
             sp -= stride;
             cur = stack[sp];
         }
+    }
+    // the postponed leaf's triangles
+    __device__ __forceinline__ uint32_t leaf(uint32_t& first) const {
+        first = pend & ((1u << QUAD_COUNT_AT) - 1u);
+        return pend >> QUAD_COUNT_AT & 7u;
     }
     // visits the node `cur`; `top`: the last `sp` with room for four more
     __device__ __forceinline__ void visit(uint32_t* stack, int stride, int top) {
@@ -311,8 +424,8 @@ struct SearchLane {
     __device__ __forceinline__ void take(float t, int slot, float dd) {
         if (!(t < h.t || (t == h.t && slot > h.slot))) return;
         // a near-grazing hit turns pruning off for good (graze_check)
-        const bool off = fabsf(dd) < GRAZE_COS * length(d) || (h.slot >= 0 && !(lim < INFINITY));
-        lim = off ? INFINITY : t * 1.001f + M;
+        const bool off = fabsf(dd) < GRAZE_COS * ray.length_d() || (h.slot >= 0 && !(lim < INFINITY));
+        lim = off ? INFINITY : t * 1.001f + ray.margin();
         h = Hit{t, slot};
     }
     // the postponed leaf is done: the next one, if the walk stands at it
@@ -336,18 +449,19 @@ __device__ __forceinline__ Hit settle(const DevTree& T, const Hit& h, f3 o, f3 d
 // it).  Its stack: entries at stack[k * stride], k < cap.
 __device__ __forceinline__ Hit search_closest(const DevTree& T, f3 o, f3 d, float pf, bool filt, int inside,
                                               int contact, uint32_t* stack, int stride, int cap) {
-    SearchLane L;
+    SearchLane<RayInRegs> L;
     L.begin(T, o, d, pf, filt, inside, contact);
     const int top = (cap - 4) * stride;
     while (!L.finished()) {
         while (L.walking()) L.visit(stack, stride, top);
         if (L.pend == NO_WORD) break;
-        const uint32_t first = L.pend & ((1u << QUAD_COUNT_AT) - 1u), count = L.pend >> QUAD_COUNT_AT & 7u;
+        uint32_t first;
+        const uint32_t count = L.leaf(first);
         for (uint32_t k = 0; k < count; k++) {
             const int slot = (int)(first + k);
             float dd = 0.f;
-            const float t = tri_slot_test(L.tris, slot, o, d, &dd);
-            if (t >= 0.f && t <= L.h.t && (!filt || noself_slot(L.tris, slot, d, inside, contact))) L.take(t, slot, dd);
+            const float t = tri_slot_test(T.tris, slot, o, d, &dd);
+            if (t >= 0.f && t <= L.h.t && (!filt || noself_slot(T.tris, slot, d, inside, contact))) L.take(t, slot, dd);
         }
         L.leaf_done(stack, stride);
     }
@@ -359,39 +473,58 @@ constexpr int LEAF_ITEMS = 32 * (int)QUAD_LEAF_MAX;  // a warp's triangles in on
 // Tests the postponed leaves of a warp's lanes (`has`): their triangles are
 // dealt out over all 32 lanes, one each, so that leaves of different lengths do
 // not leave lanes idle (the test in each lane's own loop kept 7 to 14 lanes
-// busy, this 24 to 29; the batch of 2^24 rays 2.69 -> 2.31 ms).  Every lane of
-// the warp calls it.  `item`: LEAF_ITEMS bytes of shared memory of the warp;
+// busy, this 24 to 29; the batch of 2^24 rays 2.69 -> 2.31 ms).  The distance
+// half of the test runs once for the triangles whose edges the rays pass
+// inside, about one in ten.  Every lane of the warp calls it.  `item`: LEAF_ITEMS bytes of shared memory of the warp;
 // tris_of(tris, l): the triangles of lane l's tree.  Returns this lane's count.
-template <class TrisOf>
-__device__ __forceinline__ uint32_t warp_leaves(SearchLane& L, bool has, uint8_t* item, const uint32_t* stack,
+template <class Ray, class TrisOf>
+__device__ __forceinline__ uint32_t warp_leaves(SearchLane<Ray>& L, bool has, uint8_t* item, const uint32_t* stack,
                                                 int stride, TrisOf tris_of) {
     constexpr unsigned FULL = 0xffffffffu;
     const unsigned lane = threadIdx.x & 31u;
     const unsigned lt_mask = (1u << lane) - 1u;
-    const uint32_t first = has ? L.pend & ((1u << QUAD_COUNT_AT) - 1u) : 0u;
-    const uint32_t count = has ? L.pend >> QUAD_COUNT_AT & 7u : 0u;
+    uint32_t first = 0u, count = 0u;
+    if (has) count = L.leaf(first);
     const unsigned c0 = __ballot_sync(FULL, count & 1u), c1 = __ballot_sync(FULL, count & 2u),
                    c2 = __ballot_sync(FULL, count & 4u);
     const uint32_t before = __popc(c0 & lt_mask) + 2u * __popc(c1 & lt_mask) + 4u * __popc(c2 & lt_mask);
     const uint32_t total = __popc(c0) + 2u * __popc(c1) + 4u * __popc(c2);
     for (uint32_t k = 0; k < count; k++) item[before + k] = (uint8_t)(lane | k << 5);
     __syncwarp();
+    // the edge tests of all; those inside stay in the list
+    uint32_t left = 0;
     for (uint32_t base = 0; base < total; base += 32u) {
         const bool on = base + lane < total;
         const uint32_t it = on ? item[base + lane] : lane;
         const int own = (int)(it & 31u);
-        const f3 ro = mk(__shfl_sync(FULL, L.o.x, own), __shfl_sync(FULL, L.o.y, own), __shfl_sync(FULL, L.o.z, own));
-        const f3 rd = mk(__shfl_sync(FULL, L.d.x, own), __shfl_sync(FULL, L.d.y, own), __shfl_sync(FULL, L.d.z, own));
+        f3 ro, rd;
+        L.ray.ray_of(own, ro, rd);
+        const int slot = (int)(__shfl_sync(FULL, first, own) + (it >> 5));
+        const TriRec* rt = tris_of(own);
+        const bool in = on && tri_slot_inside(rt, slot, ro, rd);
+        const unsigned im = __ballot_sync(FULL, in);
+        if (in) item[left + __popc(im & lt_mask)] = (uint8_t)it;
+        left += __popc(im);
+        __syncwarp();
+    }
+    // the distances of the few that are left
+    for (uint32_t base = 0; base < left; base += 32u) {
+        const bool on = base + lane < left;
+        const uint32_t it = on ? item[base + lane] : lane;
+        const int own = (int)(it & 31u);
+        f3 ro, rd;
+        L.ray.ray_of(own, ro, rd);
         const int slot = (int)(__shfl_sync(FULL, first, own) + (it >> 5));
         const float best = __shfl_sync(FULL, L.h.t, own);
-        const TriRec* rt = tris_of(L.tris, own);
+        const TriRec* rt = tris_of(own);
         float t = -1.f, dd = 0.f;
-        if (on) t = tri_slot_test(rt, slot, ro, rd, &dd);
+        if (on) t = tri_slot_distance(rt, slot, ro, rd, &dd);
         bool cand = t >= 0.f && t <= best;
         unsigned cm = __ballot_sync(FULL, cand);
         if (cm) {
-            const bool rf = __shfl_sync(FULL, (int)L.filt, own) != 0;
-            const int ri = __shfl_sync(FULL, L.inside, own), rc = __shfl_sync(FULL, L.contact, own);
+            bool rf;
+            int ri, rc;
+            L.ray.ids_of(own, rf, ri, rc);
             if (cand && rf) cand = noself_slot(rt, slot, rd, ri, rc);
             // the candidates go back to their rays one by one
             for (cm = __ballot_sync(FULL, cand); cm; cm &= cm - 1u) {
@@ -412,7 +545,7 @@ __device__ __forceinline__ uint32_t warp_leaves(SearchLane& L, bool has, uint8_t
 __device__ __forceinline__ Hit search_warp(const DevTree& T, bool on, f3 o, f3 d, float pf, bool filt, int inside,
                                            int contact, uint32_t* stack, int stride, int cap, uint8_t* item) {
     constexpr unsigned FULL = 0xffffffffu;
-    SearchLane L;
+    SearchLane<RayInRegs> L;
     L.clear();
     if (on) L.begin(T, o, d, pf, filt, inside, contact);
     const int top = (cap - 4) * stride;
@@ -421,7 +554,7 @@ __device__ __forceinline__ Hit search_warp(const DevTree& T, bool on, f3 o, f3 d
         const unsigned wm = __ballot_sync(FULL, walking), lm = __ballot_sync(FULL, L.at_leaf());
         if (!(wm | lm)) break;
         if (lm && (wm == 0 || __popc(lm) >= 8)) {
-            warp_leaves(L, L.pend != NO_WORD, item, stack, stride, [&](const TriRec*, int) { return T.tris; });
+            warp_leaves(L, L.pend != NO_WORD, item, stack, stride, [&](int) { return T.tris; });
         } else if (walking) {
             for (int k = 0; k < 6 && L.walking(); k++) L.visit(stack, stride, top);
         }

@@ -16,8 +16,7 @@
 // A source class supplies the rays:
 //   fetch(id, ray)   fills a TraceRay
 //   put(id, ray, h)  writes the closest hit (h.slot < 0: none)
-//   tris_of(tris, l) triangles of lane l's ray (`tris`: of this lane's, which
-//                    may never have had one); every lane calls it
+//   tris_of(rays, l) triangles of lane l's ray (RayInShared)
 #pragma once
 
 #include "wr_quad.cuh"
@@ -40,6 +39,7 @@ struct WarpQueues {
     uint32_t id[64];
     int slot[64];
     float t[64];
+    float ray[RAY_WORDS * 32];  // the lanes' rays (RayInShared)
     uint8_t item[LEAF_ITEMS];  // the leaf phase's triangles: lane | index in its leaf << 5
 };
 // this thread's work counts (profiling launches)
@@ -75,10 +75,6 @@ __device__ __forceinline__ void finish_ray(Src& src, uint32_t id, Hit h) {
     src.put(id, r, h);
 }
 
-__device__ __forceinline__ const TriRec* shfl_ptr(const TriRec* p, int from) {
-    return reinterpret_cast<const TriRec*>(__shfl_sync(0xffffffffu, reinterpret_cast<unsigned long long>(p), from));
-}
-
 // Traces rays [0, n) of `src`, handing out ray ids from *counter (which
 // starts at 0).  Every lane of the warp must call it.  `stack`: this thread's
 // entries at stack[k * stride], k < cap; `Q`: the warp's queues.
@@ -89,9 +85,12 @@ __device__ __forceinline__ void quad_trace(Src& src, uint32_t n, unsigned int* c
     const unsigned lane = threadIdx.x & 31u;
     const unsigned lt_mask = (1u << lane) - 1u;
     // ids are drawn in runs: long enough that the counter is quiet, short
-    // enough that the warps end together
+    // enough that the warps end together.  Fewer rays than lanes are shared
+    // out evenly, a few to a warp: its leaf phases then end sooner.
     const uint32_t warps = gridDim.x * (blockDim.x >> 5);
-    const uint32_t run = min(256u, max(32u, n / (warps * 8u) & ~31u));
+    const uint32_t share = max(1u, n / warps + (n % warps != 0));
+    const uint32_t lanes = min(32u, share);
+    const uint32_t run = share >= 512u ? min(256u, share / 8u & ~31u) : lanes;
     uint32_t next = 0, end = 0;  // the warp's run
     bool dry = false;            // no more runs
     const int top = (cap - 4) * stride;
@@ -99,15 +98,17 @@ __device__ __forceinline__ void quad_trace(Src& src, uint32_t n, unsigned int* c
 
     uint32_t id = 0;
     bool active = false;
-    SearchLane L;
+    SearchLane<RayInShared> L;
+    L.ray = RayInShared{Q.ray + lane, 32};
     L.clear();
 
     for (;;) {
         const unsigned idle = __ballot_sync(FULL, !active);
-        if (idle == FULL || __popc(idle) >= tune.refill_min) {
+        if (idle == FULL || __popc(idle) >= (int)(32u - lanes) + tune.refill_min) {
             // intake: 32 rays at a time against the scene's box; those that
             // meet it are queued
-            const uint32_t want = (uint32_t)__popc(idle);
+            const uint32_t busy = 32u - (uint32_t)__popc(idle);
+            const uint32_t want = lanes > busy ? lanes - busy : 0u;
             while (nin < want && !dry) {
                 if (next == end) {
                     uint32_t b = 0;
@@ -138,7 +139,7 @@ __device__ __forceinline__ void quad_trace(Src& src, uint32_t n, unsigned int* c
                 __syncwarp();
             }
             const uint32_t k = (uint32_t)__popc(idle & lt_mask);
-            if (!active && k < nin) {
+            if (!active && k < want && k < nin) {
                 id = Q.in[nin - 1u - k];
                 TraceRay a;
                 src.fetch(id, a);
@@ -154,7 +155,7 @@ __device__ __forceinline__ void quad_trace(Src& src, uint32_t n, unsigned int* c
             // every postponed leaf, those of lanes still walking too
             const uint32_t tested =
                 warp_leaves(L, active && L.pend != NO_WORD, Q.item, stack, stride,
-                            [&](const TriRec* t, int from) { return src.tris_of(t, from); });
+                            [&](int from) { return src.tris_of(L.ray, from); });
             if (STATS) work.tris += tested;
         } else if (walking) {
             for (int k = 0; k < tune.steps && L.walking(); k++) {

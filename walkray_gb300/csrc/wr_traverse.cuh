@@ -204,10 +204,10 @@ __device__ __forceinline__ void pair_pred(const Box& L, const Box& R, const RayQ
     *hr = cr == BOX_HIT;
 }
 
-// KDTree::intersect(ray, tri) geometric part (kdtree.cpp:279-301); returns
-// the distance or -1.  The edge-mask rejection is taken before the plane
-// distance (same result, less work).
-__device__ __forceinline__ float tri_test(f3 v0, f3 v1, f3 v2, const RayQ& q, float* dd_out = nullptr) {
+// KDTree::intersect(ray, tri) geometric part (kdtree.cpp:279-301).  The
+// edge-mask rejection is taken before the plane distance (same result, less
+// work).
+__device__ __forceinline__ bool tri_inside(f3 v0, f3 v1, f3 v2, const RayQ& q) {
     const f3 l0 = sub3_x(v1, v0), l1 = sub3_x(v2, v1), l2 = sub3_x(v0, v2);
     const f3 r0 = sub3_x(v0, q.o), r1 = sub3_x(v1, q.o), r2 = sub3_x(v2, q.o);
     const float s0 = dot_x(q.d, cross_x(l0, r0));
@@ -215,7 +215,12 @@ __device__ __forceinline__ float tri_test(f3 v0, f3 v1, f3 v2, const RayQ& q, fl
     const float s2 = dot_x(q.d, cross_x(l2, r2));
     const bool pos = s0 >= 0.f && s1 >= 0.f && s2 >= 0.f;
     const bool neg = s0 <= 0.f && s1 <= 0.f && s2 <= 0.f;
-    if (!pos && !neg) return -1.f;
+    return pos || neg;
+}
+
+// the distance of a triangle whose edges the ray passes inside, or -1
+__device__ __forceinline__ float tri_distance(f3 v0, f3 v1, f3 v2, const RayQ& q, float* dd_out = nullptr) {
+    const f3 l0 = sub3_x(v1, v0), l1 = sub3_x(v2, v1), r2 = sub3_x(v2, q.o);
     const f3 n = normalize_x(cross_x(l0, l1));
     const float od = dot_x(n, r2);
     const float dd = dot_x(n, q.d);
@@ -224,6 +229,11 @@ __device__ __forceinline__ float tri_test(f3 v0, f3 v1, f3 v2, const RayQ& q, fl
     const float t = div_x(od, dd);
     if (t < 0.f) return -1.f;
     return t;
+}
+
+// both: the distance or -1
+__device__ __forceinline__ float tri_test(f3 v0, f3 v1, f3 v2, const RayQ& q, float* dd_out = nullptr) {
+    return tri_inside(v0, v1, v2, q) ? tri_distance(v0, v1, v2, q, dd_out) : -1.f;
 }
 
 // pruning stays on only while the closest hit is not a near-grazing one
