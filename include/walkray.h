@@ -323,7 +323,7 @@ typedef struct wr_render_profile {
     uint64_t box_tests;        /* AABB predicate evaluations (reference count) */
     uint64_t tri_tests;        /* ray-triangle tests */
     uint64_t paths;
-    double ms_drain;           /* the per-path finish of the last paths (k_wf_drain) */
+    double ms_drain;           /* the per-path finish of the last paths (k_wf_finish) */
     uint64_t drained_paths;    /* paths it finished */
     uint32_t iter_rays[32];    /* rays in the queue of bounce iteration i (first 32 iterations) */
     float iter_extend_ms[32];  /* extend stage time of iteration i */
@@ -424,7 +424,8 @@ typedef struct wr_wavefront_config {
     int32_t leaf_min;        /* traversal: lanes holding leaves that start a warp's leaf tests (1..32,
                                 0 = default); both also apply to wr_trace_closest */
     int32_t drain_paths;     /* wr_render: once every path is generated and at most this many remain,
-                                finish them in one per-path kernel (0 = never) */
+                                finish them in one per-path kernel (0 = never; a context that was given
+                                no configuration does so at 2^15, 2^13 with a density grid) */
     int32_t pixel_tile;      /* camera paths generated tile by tile, square tiles of this many pixels a
                                 side (0 = row by row); the image does not depend on it */
     int32_t steps_per_turn;  /* traversal: steps a searching lane takes per turn of a warp's loop (1..8,

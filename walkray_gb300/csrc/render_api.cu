@@ -372,6 +372,7 @@ int wr_render_progressive(wr_ctx* ctx, wr_scene_id id, const wr_render_desc* des
 namespace wr {
 
 const RenderScene& RenderDataView::scene(const RenderData* rd) { return rd->S; }
+bool RenderDataView::hetero(const RenderData* rd) { return rd->has_hetero; }
 const std::string& RenderDataView::unsupported(const RenderData* rd) { return rd->unsupported; }
 
 // the wavefront configuration: what wr_autotune picked for this context, else defaults
@@ -383,7 +384,7 @@ WfConfig wf_tuned_config(wr_ctx* ctx) {
     if (ctx->wf_ctas_per_sm) c.ctas_per_sm = ctx->wf_ctas_per_sm;
     if (ctx->wf_iters) c.iters_per_graph = ctx->wf_iters;
     c.trace = trace_tune_of(ctx);
-    c.drain_paths = ctx->wf_drain_paths;
+    if (ctx->wf_drain_paths >= 0) c.drain_paths = ctx->wf_drain_paths;
     c.pixel_tile = ctx->wf_pixel_tile;
     return c;
 }

@@ -14,6 +14,7 @@ namespace wr {
 
 constexpr uint32_t WF_MAX_JOBS = 256;
 constexpr uint32_t WF_MAX_SCENES = 64;
+constexpr int WF_FINISH_BLOCK = 128;
 
 uint32_t wf_max_jobs() { return WF_MAX_JOBS; }
 
@@ -38,10 +39,17 @@ __device__ __forceinline__ float4 as_f4(int4 v) {
     return make_float4(__int_as_float(v.x), __int_as_float(v.y), __int_as_float(v.z), __int_as_float(v.w));
 }
 
+// Field f of record i lies in the record's 16-byte chunk f ^ (i & 7): lanes that
+// read or write one field of neighbouring records then use all banks of the L1
+// cache instead of one group of four (a 128-byte stride takes 0.99 cycles a
+// piece on an SM, spread 0.34).
+__device__ __forceinline__ uint32_t wf_swizzle(uint64_t i) { return (uint32_t)i & 7u; }
+
 __device__ __forceinline__ void wf_load(const WfSide& X, uint32_t i, WfPath& p) {
     const float4* r = X.rec + (size_t)WF_REC * i;
-    const float4 a0 = r[WF_O], a1 = r[WF_D], a2 = r[WF_RAD], a3 = r[WF_COL];
-    const int4 ids = as_i4(r[WF_IDS]), misc = as_i4(r[WF_MISC]), stk = as_i4(r[WF_STK]);
+    const uint32_t x = wf_swizzle(i);
+    const float4 a0 = r[WF_O ^ x], a1 = r[WF_D ^ x], a2 = r[WF_RAD ^ x], a3 = r[WF_COL ^ x];
+    const int4 ids = as_i4(r[WF_IDS ^ x]), misc = as_i4(r[WF_MISC ^ x]), stk = as_i4(r[WF_STK ^ x]);
     p.cur = ray_default();
     p.cur.o = mk(a0.x, a0.y, a0.z);
     p.cur.oP = a0.w;
@@ -62,7 +70,7 @@ __device__ __forceinline__ void wf_load(const WfSide& X, uint32_t i, WfPath& p) 
     p.st.v1 = stk.y;
     p.st.v2 = stk.z;
     p.st.v3 = stk.w;
-    const float4 a4 = r[WF_PREV];
+    const float4 a4 = r[WF_PREV ^ x];
     p.prev_d = mk(a4.x, a4.y, a4.z);
     p.mis_pdf = a4.w;
     p.acc = mk(0, 0, 0);
@@ -73,27 +81,9 @@ __device__ __forceinline__ void wf_load_acc(const WfSide& X, uint32_t i, WfPath&
     p.acc = mk(a5.x, a5.y, a5.z);
 }
 
-__device__ __forceinline__ void wf_store(const WfSide& Y, uint32_t j, const WfPath& p) {
-    float4* r = Y.rec + (size_t)WF_REC * j;
-    r[WF_O] = make_float4(p.cur.o.x, p.cur.o.y, p.cur.o.z, p.cur.oP);
-    r[WF_D] = make_float4(p.cur.d.x, p.cur.d.y, p.cur.d.z, p.cur.dP);
-    r[WF_IDS] = as_f4(make_int4(p.cur.inside, p.cur.contact, p.job, (int)p.pixel));
-    r[WF_MISC] = as_f4(make_int4((int)p.sample, (int)p.dim, (int)(p.depth | ((uint32_t)p.st.n << 16)),
-                                 __float_as_int(p.cur.cnorm.z)));
-    r[WF_RAD] = make_float4(p.cur.rad.x, p.cur.rad.y, p.cur.rad.z, p.cur.cnorm.x);
-    r[WF_COL] = make_float4(p.color.x, p.color.y, p.color.z, p.cur.cnorm.y);
-    r[WF_STK] = as_f4(make_int4(p.st.v0, p.st.v1, p.st.v2, p.st.v3));
-    r[WF_PREV] = make_float4(p.prev_d.x, p.prev_d.y, p.prev_d.z, p.mis_pdf);
-}
-
-// The same record written into row `row` of a shared-memory tile of 128-byte
-// rows in the 128-byte swizzle of the tensor-memory-access unit (16-byte
-// chunk c of row r at chunk c ^ (r & 7)): eight consecutive rows' stores of
-// one field then fall on eight different bank groups, and the bulk tensor
-// store writes the rows to global memory unswizzled.
-__device__ __forceinline__ void wf_store_tile(float4* tile, uint32_t row, const WfPath& p) {
-    float4* r = tile + (size_t)WF_REC * row;
-    const uint32_t x = row & 7u;
+// a path as record number i (its swizzle), its chunks at r
+__device__ __forceinline__ void wf_store_at(float4* r, uint32_t i, const WfPath& p) {
+    const uint32_t x = wf_swizzle(i);
     r[WF_O ^ x] = make_float4(p.cur.o.x, p.cur.o.y, p.cur.o.z, p.cur.oP);
     r[WF_D ^ x] = make_float4(p.cur.d.x, p.cur.d.y, p.cur.d.z, p.cur.dP);
     r[WF_IDS ^ x] = as_f4(make_int4(p.cur.inside, p.cur.contact, p.job, (int)p.pixel));
@@ -103,6 +93,9 @@ __device__ __forceinline__ void wf_store_tile(float4* tile, uint32_t row, const 
     r[WF_COL ^ x] = make_float4(p.color.x, p.color.y, p.color.z, p.cur.cnorm.y);
     r[WF_STK ^ x] = as_f4(make_int4(p.st.v0, p.st.v1, p.st.v2, p.st.v3));
     r[WF_PREV ^ x] = make_float4(p.prev_d.x, p.prev_d.y, p.prev_d.z, p.mis_pdf);
+}
+__device__ __forceinline__ void wf_store(const WfSide& Y, uint32_t j, const WfPath& p) {
+    wf_store_at(Y.rec + (size_t)WF_REC * j, j, p);
 }
 
 __device__ __forceinline__ void wf_store_acc(const WfSide& Y, uint32_t j, const WfPath& p) {
@@ -148,7 +141,7 @@ __global__ void __launch_bounds__(256) k_wf_sort(const RenderScene* __restrict__
         if (valid) {
             const int slot = hits[i].x;
             if (slot >= 0) {
-                const int4 ids = as_i4(X.rec[(size_t)WF_REC * i + WF_IDS]);
+                const int4 ids = as_i4(X.rec[(size_t)WF_REC * i + (WF_IDS ^ wf_swizzle(i))]);
                 const RenderScene& S = scenes[jobs[ids.z].scene];
                 const int self = ids.x >= 0 ? ids.x : (int)__float_as_uint(__ldg(&S.tree.tris[slot].v1.w));
                 key = 1 + (int)obj_type(S, self);
@@ -239,8 +232,9 @@ struct ExtendSrc {
 
     __device__ __forceinline__ void fetch(uint64_t id, TraceRay& a) const {
         const float4* r = X.rec + (size_t)WF_REC * id;
-        const float4 a0 = r[WF_O], a1 = r[WF_D];
-        const int4 ids = as_i4(r[WF_IDS]);
+        const uint32_t x = wf_swizzle(id);
+        const float4 a0 = r[WF_O ^ x], a1 = r[WF_D ^ x];
+        const int4 ids = as_i4(r[WF_IDS ^ x]);
         const WfJob& J = jobs[ids.z];
         a.T = &scenes[J.scene].tree;
         a.o = mk(a0.x, a0.y, a0.z);
@@ -290,6 +284,7 @@ __global__ void WR_EXTEND_BOUNDS(MINB) k_wf_extend(const RenderScene* __restrict
                                                      unsigned long long* __restrict__ stats) {
     extern __shared__ __align__(16) uint32_t s_stack[];
     const uint64_t n = (uint64_t)X.counts[0] + X.counts[1];
+    if (n == 0) return;
     ExtendSrc src{scenes, jobs, X, hits, TraceWork{0ull, 0ull, 0ull}};
     if (EXACT)
         warp_trace<true, STATS>(src, n, work, tune, s_stack + threadIdx.x, blockDim.x, stack_cap, err);
@@ -343,6 +338,7 @@ __global__ void WR_EXTEND_BOUNDS(MINB)
                       unsigned int* __restrict__ err) {
     extern __shared__ __align__(16) uint32_t s_stack[];
     const uint64_t n = *Q.count;
+    if (n == 0) return;
     ShadowSrc src{scenes, jobs, Q, hits};
     TraceWork none;
     quad_trace<false>(src, (uint32_t)n, reinterpret_cast<unsigned int*>(work), tune, s_stack + threadIdx.x, blockDim.x, stack_cap,
@@ -476,64 +472,97 @@ __global__ void __launch_bounds__(128, 4) k_wf_shade(const RenderScene* __restri
     }
 }
 
-// drain: the last paths of a render, each finished by one thread (trace,
-// bounce, NEE connection) without returning to the bounce loop.  Once nothing
-// is left to generate, the loop's iterations each cost about the latency of
-// their slowest ray however few rays remain; here the remaining paths run
-// side by side instead.  Same paths, draws and film additions as the loop.
-__global__ void __launch_bounds__(128) k_wf_drain(const RenderScene* __restrict__ scenes,
-                                                    const WfJob* __restrict__ jobs,
-                                                    WfJobCounters* __restrict__ counters, WfSide X, int stack_cap) {
+// finish: the paths waiting in X run to their ends without returning to the
+// bounce loop, one path to a lane, the lanes of a warp together (search_warp).
+// Once nothing is left to generate, each iteration of the loop costs the
+// latency of its slowest ray and of seven launches however few paths remain;
+// here the paths go on side by side.  Same paths, draws and film additions as
+// the loop.  MIS: compiled with the WR_RENDER_NEE_MIS code.
+// Bound by latency: a warp's turn lasts as long as its slowest ray's search.
+// Few paths are therefore spread over all warps, a few lanes to each.
+template <bool MIS>
+__global__ void __launch_bounds__(WF_FINISH_BLOCK, MIS ? 3 : 4)
+    k_wf_finish(const RenderScene* __restrict__ scenes, const WfJob* __restrict__ jobs,
+                WfJobCounters* __restrict__ counters, WfSide X, unsigned int* __restrict__ next, int stack_cap) {
+    constexpr unsigned FULL = 0xffffffffu;
     extern __shared__ __align__(16) uint32_t s_stack[];
+    __shared__ uint8_t s_item[WF_FINISH_BLOCK / 32][LEAF_ITEMS];
     uint32_t* stack = s_stack + threadIdx.x;
+    uint8_t* item = s_item[threadIdx.x >> 5];
+    const unsigned lane = threadIdx.x & 31u;
     const uint32_t n = X.counts[0] + X.counts[1];
-    const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= n) return;
+    const uint32_t warps = gridDim.x * (WF_FINISH_BLOCK / 32);
+    const uint32_t lanes = min(32u, n / warps + (n % warps != 0));
+    bool active = false, dry = lane >= lanes;
     WfPath p;
-    wf_load(X, i, p);
-    const WfJob& J = jobs[p.job];
-    const RenderScene& S = scenes[J.scene];
-    if (J.flags & WR_RENDER_NEE_MIS) wf_load_acc(X, i, p);
+    p.cur = ray_default();
+    p.job = 0;
     PathRng g;
-    g.init(J.seed, p.pixel, p.sample, p.dim);
-    const bool nee = (J.flags & WR_RENDER_NEE) != 0;
-    const float pf = prune_factor(J.flags);
-    bool filtered = p.cur.contact != CAMERA_OBJ, nee_here = false, has_lr = false;
-    f3 result = mk(0, 0, 0);
-    LightReq lr;
+    g.init(0, 0, 0);
     for (;;) {
-        const Hit h = search_closest(S.tree, p.cur.o, p.cur.d, pf, filtered, p.cur.inside, p.cur.contact, stack,
-                                     blockDim.x, stack_cap);
-        if (h.slot < 0 && filtered) {  // a scattered ray that escapes ends with zero radiance
-            nee_here = nee;
-            break;
+        const unsigned need = __ballot_sync(FULL, !active && !dry);
+        if (need) {
+            const int leader = __ffs(need) - 1;
+            uint32_t base = 0;
+            if ((int)lane == leader) base = atomicAdd(next, (unsigned)__popc(need));
+            base = __shfl_sync(FULL, base, leader);
+            if (need >> lane & 1u) {
+                const uint32_t i = base + __popc(need & ((1u << lane) - 1u));
+                if (i < n) {
+                    wf_load(X, i, p);
+                    const WfJob& J = jobs[p.job];
+                    if (MIS && (J.flags & WR_RENDER_NEE_MIS)) wf_load_acc(X, i, p);
+                    g.init(J.seed, p.pixel, p.sample, p.dim);
+                    active = true;
+                } else {
+                    dry = true;
+                }
+            }
         }
-        set_hit(S, p.cur, h);
-        filtered = true;
-        const bool done = path_advance<true>(S, p.cur, p.color, p.prev_d, p.depth, p.st, g, J.max_path_len,
-                                             J.flags, result, nee_here, p.mis_pdf, lr, has_lr);
-        if (has_lr) {
-            const Hit lh = search_closest(S.tree, lr.o, lr.d, pf, true, lr.inside, lr.contact, stack, blockDim.x,
-                                          stack_cap);
-            if (light_req_visible(S, lh, lr)) p.acc = p.acc + lr.contrib;
+        if (!__any_sync(FULL, active)) break;
+        const WfJob& J = jobs[p.job];
+        const RenderScene& S = scenes[J.scene];
+        const float pf = prune_factor(J.flags);
+        const bool filtered = p.cur.contact != CAMERA_OBJ;
+        const Hit h = search_warp<false>(S.tree, active, p.cur.o, p.cur.d, pf, filtered, p.cur.inside, p.cur.contact,
+                                         stack, WF_FINISH_BLOCK, stack_cap, item);
+        bool done = false, nee_here = false, has_lr = false;
+        f3 result = mk(0, 0, 0);
+        LightReq lr;
+        if (active) {
+            if (h.slot < 0 && filtered) {  // a scattered ray that escapes ends with zero radiance
+                done = true;
+                nee_here = (J.flags & WR_RENDER_NEE) != 0;
+            } else {
+                set_hit(S, p.cur, h);
+                done = path_advance<MIS>(S, p.cur, p.color, p.prev_d, p.depth, p.st, g, J.max_path_len, J.flags,
+                                         result, nee_here, p.mis_pdf, lr, has_lr);
+            }
         }
-        if (done) break;
+        if (MIS && __any_sync(FULL, has_lr)) {  // the light connection of WR_RENDER_NEE_MIS
+            const Hit lh = search_warp<false>(S.tree, has_lr, lr.o, lr.d, pf, true, lr.inside, lr.contact, stack,
+                                              WF_FINISH_BLOCK, stack_cap, item);
+            if (has_lr && light_req_visible(S, lh, lr)) p.acc = p.acc + lr.contrib;
+        }
+        if (__any_sync(FULL, nee_here)) {  // the connection of the NEE branch
+            ShadowReq sr;
+            const bool conn = nee_here && nee_prepare(S, p.cur, p.prev_d, p.color, g, sr);
+            const Hit sh = search_warp<false>(S.tree, conn, sr.o, sr.d, pf, true, sr.inside, sr.contact, stack,
+                                              WF_FINISH_BLOCK, stack_cap, item);
+            if (nee_here) result = conn && nee_visible(sh, sr.dist) ? sr.contrib : mk(0, 0, 0);
+        }
+        if (done) {
+            if (!legal(result)) result = mk(0, 0, 0);
+            result = result + p.acc;
+            if (result.x != 0.f || result.y != 0.f || result.z != 0.f) film_add(J, p.pixel, result);
+            active = false;
+        }
+        const unsigned dm = __ballot_sync(FULL, done);
+        if (done) {
+            const unsigned same = __match_any_sync(dm, p.job);
+            if ((int)lane == __ffs(same) - 1) atomicAdd(&counters[p.job].finished, (unsigned long long)__popc(same));
+        }
     }
-    if (nee_here) {
-        ShadowReq sr;
-        result = mk(0, 0, 0);
-        if (nee_prepare(S, p.cur, p.prev_d, p.color, g, sr)) {
-            const Hit h = search_closest(S.tree, sr.o, sr.d, pf, true, sr.inside, sr.contact, stack, blockDim.x,
-                                         stack_cap);
-            if (nee_visible(h, sr.dist)) result = sr.contrib;
-        }
-    }
-    if (!legal(result)) result = mk(0, 0, 0);
-    result = result + p.acc;
-    if (result.x != 0.f || result.y != 0.f || result.z != 0.f) film_add(J, p.pixel, result);
-    const unsigned same = __match_any_sync(__activemask(), p.job);
-    if ((threadIdx.x & 31u) == (unsigned)(__ffs(same) - 1))
-        atomicAdd(&counters[p.job].finished, (unsigned long long)__popc(same));
 }
 
 // plan: how the free slots of Y are shared out among the jobs this turn.
@@ -566,7 +595,7 @@ __device__ __forceinline__ unsigned long long block_excl_scan(unsigned long long
 __global__ void __launch_bounds__(WF_MAX_JOBS) k_wf_plan(const WfJob* __restrict__ jobs, const int* __restrict__ order,
                                                           WfJobCounters* __restrict__ counters, WfSide Y,
                                                           uint32_t capacity, const uint32_t* __restrict__ live_cap,
-                                                          int equal_share, WfPlan P) {
+                                                          int equal_share, WfPlan P, volatile WfStatus* status) {
     __shared__ unsigned long long buf[WF_MAX_JOBS];
     __shared__ unsigned long long s_total_q;
     const int n = order[0];
@@ -601,12 +630,18 @@ __global__ void __launch_bounds__(WF_MAX_JOBS) k_wf_plan(const WfJob* __restrict
         P.first[k] = claimed;
         P.off[k] = (uint32_t)off;
         if (quota) counters[j].claimed = claimed + quota;
+        if (k == 0) {  // what the host waits for, written to its memory
+            status->claimed = claimed + quota;
+            status->finished = counters[j].finished;
+        }
     }
     if (k == n - 1 || (n == 0 && k == 0)) {
         const uint32_t total = n ? (uint32_t)(off + quota) : 0u;
         P.off[n] = total;
         *P.n = n;
         Y.counts[1] = total;
+        status->waiting = survivors + total;
+        __threadfence_system();
     }
 }
 
@@ -643,7 +678,7 @@ constexpr uint32_t WF_GEN_ROWS = 128;  // = the generate kernel's block size
 
 __global__ void __launch_bounds__(WF_GEN_ROWS) k_wf_generate(const WfJob* __restrict__ jobs, WfPlan P, WfSide Y,
                                                              const __grid_constant__ CUtensorMap tmap) {
-    __shared__ __align__(1024) float4 s_tile[WF_GEN_ROWS * WF_REC];  // 16 KiB, 128-byte swizzle
+    __shared__ __align__(1024) float4 s_tile[WF_GEN_ROWS * WF_REC];  // 16 KiB
     __shared__ uint32_t s_off[WF_MAX_JOBS + 1];
     __shared__ int s_slot[WF_MAX_JOBS];
     __shared__ unsigned long long s_first[WF_MAX_JOBS];
@@ -685,7 +720,7 @@ __global__ void __launch_bounds__(WF_GEN_ROWS) k_wf_generate(const WfJob* __rest
             p.st.reset(p.cur.inside);
             p.mis_pdf = 0.f;
             p.acc = mk(0, 0, 0);
-            wf_store_tile(s_tile, threadIdx.x, p);
+            wf_store_at(s_tile + WF_REC * threadIdx.x, survivors + t, p);
             if (J.flags & WR_RENDER_NEE_MIS) wf_store_acc(Y, survivors + t, p);
         }
         // the tile's generic-proxy writes before the tensor unit reads it
@@ -737,16 +772,22 @@ struct WfEngine {
     bool conn_any = true;  // a job in the table connects to lights (NEE or MIS): the shadow stage is in the loop
     int launches_per_iteration() const { return conn_any ? 8 : 6; }
     WfJobCounters* host_counters = nullptr;  // pinned
+    WfStatus* status = nullptr;              // pinned and mapped: written by k_wf_plan
+    cudaEvent_t turn[2] = {};                // the end of the last two graph replays of a render
+    int grid_finish[2] = {};                 // k_wf_finish without and with the light connections
     ~WfEngine() {
         if (graph) cudaGraphExecDestroy(graph);
         if (host_counters) cudaFreeHost(host_counters);
+        if (status) cudaFreeHost(status);
+        for (cudaEvent_t e : turn)
+            if (e) cudaEventDestroy(e);
     }
 };
 
 const WfConfig& wf_config(const WfEngine* E) { return E->cfg; }
 
 // side k's records as a tensor of 32 floats x capacity rows (128-byte rows),
-// written in WF_GEN_ROWS x 32 boxes from 128-byte-swizzled shared memory
+// written in WF_GEN_ROWS x 32 boxes from shared memory
 static PFN_cuTensorMapEncodeTiled_v12000 lookup_encode_tiled() {
     cudaDriverEntryPointQueryResult q{};
     void* fn = nullptr;
@@ -764,7 +805,7 @@ static int map_side(wr_ctx* ctx, WfEngine* E, int k) {
     const cuuint32_t box[2] = {4 * WF_REC, WF_GEN_ROWS};
     const cuuint32_t estr[2] = {1, 1};
     const CUresult r = encode(&E->rec_map[k], CU_TENSOR_MAP_DATA_TYPE_FLOAT32, 2, E->side[k].rec, dims, strides, box,
-                              estr, CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_128B,
+                              estr, CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_NONE,
                               CU_TENSOR_MAP_L2_PROMOTION_NONE, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
     if (r != CUDA_SUCCESS) return set_error(ctx, WR_ERR_INTERNAL, "cuTensorMapEncodeTiled failed for the path records");
     return WR_OK;
@@ -846,6 +887,9 @@ int wf_engine_get(wr_ctx* ctx, const WfConfig& cfg, WfEngine** out) {
     WR_CUDA(ctx, cudaMemset(E->err_word.p, 0, sizeof(unsigned int)));
     // the job counters, then one extra record for the queue counts of side 0
     WR_CUDA(ctx, cudaMallocHost(&E->host_counters, sizeof(WfJobCounters) * (WF_MAX_JOBS + 1)));
+    WR_CUDA(ctx, cudaHostAlloc(&E->status, sizeof(WfStatus), cudaHostAllocMapped));
+    *E->status = WfStatus{};
+    for (cudaEvent_t& e : E->turn) WR_CUDA(ctx, cudaEventCreateWithFlags(&e, cudaEventDisableTiming));
     E->job_tab.assign(WF_MAX_JOBS, WfJob{});
     E->order_host.assign(1, 0);
     // persistent grids from the occupancy calculator
@@ -967,7 +1011,7 @@ int wf_update_jobs(wr_ctx* ctx, WfEngine* E, const std::vector<WfSlotUpdate>& up
         E->mis_any = mis_any;
         E->conn_any = conn_any;
         if (E->graph) {
-            WR_CUDA(ctx, cudaStreamSynchronize(s));
+            WR_CUDA(ctx, cudaStreamSynchronize(s));  // a replay may still run
             cudaGraphExecDestroy(E->graph);
             E->graph = nullptr;
         }
@@ -976,8 +1020,7 @@ int wf_update_jobs(wr_ctx* ctx, WfEngine* E, const std::vector<WfSlotUpdate>& up
     E->order_host.insert(E->order_host.end(), order.begin(), order.end());
     WR_CUDA(ctx, cudaMemcpyAsync(E->order.p, E->order_host.data(), sizeof(int) * E->order_host.size(),
                                  cudaMemcpyHostToDevice, s));
-    // the host mirrors must stay alive until the copies ran
-    WR_CUDA(ctx, cudaStreamSynchronize(s));
+    // (copies from pageable memory: the calls have read the host mirrors when they return)
     return WR_OK;
 }
 
@@ -1009,9 +1052,18 @@ static void enqueue_iteration(WfEngine* E, int x, cudaStream_t s, cudaEvent_t* e
     if (ev) cudaEventRecord(ev[3], s);
     k_wf_plan<<<1, WF_MAX_JOBS, 0, s>>>(jobs, E->order.as<int>(), cnt, E->side[y], E->cfg.capacity,
                                         E->live_cap.as<uint32_t>(), E->equal_share,
-                                        E->plan);
+                                        E->plan, E->status);
     k_wf_generate<<<E->grid_gen, WF_GEN_ROWS, 0, s>>>(jobs, E->plan, E->side[y], E->rec_map[y]);
     if (ev) cudaEventRecord(ev[4], s);
+}
+
+// the first camera paths of a render into the empty side 0
+static void enqueue_first(WfEngine* E, cudaStream_t s) {
+    k_wf_reset<<<1, 1, 0, s>>>(E->side[0], E->work.as<unsigned long long>(), E->shadow.count, E->sort);
+    k_wf_plan<<<1, WF_MAX_JOBS, 0, s>>>(E->jobs.as<WfJob>(), E->order.as<int>(), E->counters.as<WfJobCounters>(),
+                                        E->side[0], E->cfg.capacity, E->live_cap.as<uint32_t>(), E->equal_share,
+                                        E->plan, E->status);
+    k_wf_generate<<<E->grid_gen, WF_GEN_ROWS, 0, s>>>(E->jobs.as<WfJob>(), E->plan, E->side[0], E->rec_map[0]);
 }
 
 // wr_profile_render: the render of render_wavefront with eager launches
@@ -1068,9 +1120,9 @@ int profile_wavefront(wr_ctx* ctx, RenderData& rd, const RenderParams& P, uint32
         if ((rc = wf_read_counters(ctx, E, c, s, &waiting, x)) != WR_OK) break;
         queued = waiting;
         if (c[0].finished >= total) break;
-        if (c[0].claimed >= total && waiting <= E->cfg.drain_threshold()) {
+        if (c[0].claimed >= total && waiting <= E->cfg.drain_threshold(RenderDataView::hetero(&rd))) {
             cudaEventRecord(ev[0], s);
-            if ((rc = wf_drain(ctx, E, x, waiting, s)) != WR_OK) break;
+            if ((rc = wf_finish(ctx, E, x, s)) != WR_OK) break;
             cudaEventRecord(ev[1], s);
             WR_CUDA(ctx, cudaEventSynchronize(ev[1]));
             float dm = 0;
@@ -1152,15 +1204,19 @@ int wf_read_counters(wr_ctx* ctx, WfEngine* E, std::vector<WfJobCounters>& out, 
     return WR_OK;
 }
 
-int wf_drain(wr_ctx* ctx, WfEngine* E, int side, uint32_t n, cudaStream_t s) {
-    if (n == 0) return WR_OK;
-    const int block = 128;
-    const size_t smem = (size_t)E->quad_cap * block * sizeof(uint32_t);
-    if (smem > 48 * 1024)
-        WR_CUDA(ctx, cudaFuncSetAttribute(k_wf_drain, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-    k_wf_drain<<<(n + block - 1) / block, block, smem, s>>>(E->scenes.as<RenderScene>(), E->jobs.as<WfJob>(),
-                                                           E->counters.as<WfJobCounters>(), E->side[side],
-                                                           E->quad_cap);
+int wf_finish(wr_ctx* ctx, WfEngine* E, int side, cudaStream_t s) {
+    const auto kern = E->mis_any ? k_wf_finish<true> : k_wf_finish<false>;
+    const size_t smem = (size_t)E->quad_cap * WF_FINISH_BLOCK * sizeof(uint32_t);
+    int& grid = E->grid_finish[E->mis_any];
+    if (!grid) {
+        int per_sm = 0;
+        WR_CUDA(ctx, cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kern, WF_FINISH_BLOCK, smem));
+        grid = ctx->num_sms * std::max(1, per_sm);
+    }
+    WR_CUDA(ctx, cudaMemsetAsync(E->work.p, 0, sizeof(unsigned long long), s));
+    kern<<<grid, WF_FINISH_BLOCK, smem, s>>>(E->scenes.as<RenderScene>(), E->jobs.as<WfJob>(),
+                                             E->counters.as<WfJobCounters>(), E->side[side],
+                                             E->work.as<unsigned int>(), E->quad_cap);
     WR_CUDA(ctx, cudaGetLastError());
     ctx->kernel_launches++;
     return WR_OK;
@@ -1235,33 +1291,53 @@ int render_wavefront(wr_ctx* ctx, RenderData& rd, const RenderParams& P, uint32_
     rc = wf_update_jobs(ctx, E, {u}, {0}, s);
     if (rc != WR_OK) return rc;
     if ((rc = wf_reset_queues(ctx, E, s)) != WR_OK) return rc;
-    // replay the captured bounce loop until every path of the job has reached the film
-    std::vector<WfJobCounters> c;
     const unsigned long long total = u.jh.job.total;
-    const uint64_t max_launches =
-        1 + (total / std::max<uint32_t>(1, E->cfg.capacity) + 4) * (uint64_t)(P.max_path_len + 4) * 4;
-    const uint32_t drain_at = E->cfg.drain_threshold();
-    for (uint64_t l = 0;; l++) {
-        if ((rc = wf_launch(ctx, E, s)) != WR_OK) return rc;
-        uint32_t waiting = 0;
-        if ((rc = wf_read_counters(ctx, E, c, s, &waiting)) != WR_OK) return rc;
-        if (c[0].finished >= total) break;
-        if (c[0].claimed >= total && waiting <= drain_at) {
-            // every path is generated and few remain: finish them one per thread
-            if ((rc = wf_drain(ctx, E, 0, waiting, s)) != WR_OK) return rc;
-            if ((rc = wf_read_counters(ctx, E, c, s)) != WR_OK) return rc;
-            if (c[0].finished < total) return set_error(ctx, WR_ERR_INTERNAL, "wavefront drain left paths");
-            break;
+    const uint32_t few = E->cfg.drain_threshold(RenderDataView::hetero(&rd));
+    volatile WfStatus* st = E->status;
+    st->claimed = st->finished = 0;
+    st->waiting = 0;
+    enqueue_first(E, s);
+    ctx->kernel_launches += 3;
+    bool finished = false;
+    if (total <= few && total <= E->cfg.capacity) {  // every path is in the queue
+        if ((rc = wf_finish(ctx, E, 0, s)) != WR_OK) return rc;
+    } else {
+        // Replay the captured bounce loop until every path of the job has
+        // reached the film, or few enough remain.  While camera paths are left
+        // to generate, or many wait, the next replay is queued before the last
+        // one's counts are read.
+        const uint64_t max_launches =
+            1 + (total / std::max<uint32_t>(1, E->cfg.capacity) + 4) * (uint64_t)(P.max_path_len + 4) * 4;
+        uint64_t queued = 0, seen = 0;
+        for (;;) {
+            while (queued == seen || (queued == seen + 1 && (st->claimed < total || st->waiting / 4 > few))) {
+                if ((rc = wf_launch(ctx, E, s)) != WR_OK) return rc;
+                WR_CUDA(ctx, cudaEventRecord(E->turn[queued & 1], s));
+                queued++;
+            }
+            WR_CUDA(ctx, cudaEventSynchronize(E->turn[seen & 1]));
+            seen++;
+            if (st->finished >= total) {
+                finished = true;
+                break;
+            }
+            if (queued == seen && st->claimed >= total && st->waiting <= few) {
+                if ((rc = wf_finish(ctx, E, 0, s)) != WR_OK) return rc;
+                break;
+            }
+            if (seen > max_launches) return set_error(ctx, WR_ERR_TIMEOUT, "wavefront did not drain");
         }
-        if (l > max_launches) return set_error(ctx, WR_ERR_TIMEOUT, "wavefront did not drain");
     }
-    // retire the job so a later render starts from an empty table
-    u.jh.job.active = 0;
-    u.reset_counters = false;
-    if ((rc = wf_update_jobs(ctx, E, {u}, {}, s)) != WR_OK) return rc;
-    unsigned int herr = 0;
-    if ((rc = wf_error_word(ctx, E, &herr, s)) != WR_OK) return rc;
-    if (herr) return set_error(ctx, WR_ERR_INTERNAL, "traversal stack overflow");
+    // the job's counters and the error word
+    unsigned int* herr = reinterpret_cast<unsigned int*>(E->host_counters + 1);
+    WR_CUDA(ctx, cudaMemcpyAsync(E->host_counters, E->counters.p, sizeof(WfJobCounters), cudaMemcpyDeviceToHost, s));
+    WR_CUDA(ctx, cudaMemcpyAsync(herr, E->err_word.p, sizeof(unsigned int), cudaMemcpyDeviceToHost, s));
+    WR_CUDA(ctx, cudaStreamSynchronize(s));
+    // retired on the host: nothing launches without a new job table
+    E->job_tab[0].active = 0;
+    if (!finished && E->host_counters[0].finished < total)
+        return set_error(ctx, WR_ERR_INTERNAL, "wavefront finish left paths");
+    if (*herr) return set_error(ctx, WR_ERR_INTERNAL, "traversal stack overflow");
     return WR_OK;
 }
 

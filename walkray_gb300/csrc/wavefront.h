@@ -37,6 +37,7 @@ namespace wr {
 struct RenderData;
 struct RenderDataView {  // what the engine needs from RenderData (render_api.cu)
     static const RenderScene& scene(const RenderData* rd);
+    static bool hetero(const RenderData* rd);  // a heterogeneous medium is among its objects
     static const std::string& unsupported(const RenderData* rd);  // non-empty: why the scene cannot render
 };
 
@@ -56,6 +57,13 @@ struct WfJob {
 struct WfJobCounters {
     unsigned long long claimed;   // paths handed to the queues
     unsigned long long finished;  // paths whose colour reached the film
+};
+
+// the first listed job's counters and the queue's length after the last plan
+// stage, in host memory
+struct WfStatus {
+    unsigned long long claimed, finished;
+    uint32_t waiting;
 };
 
 // path state, one ping-pong side: one 128-byte record (a cache line) per
@@ -109,13 +117,17 @@ struct WfConfig {
     int extend_block = 128;
     int shade_block = 128;
     int ctas_per_sm = 0;           // 0 = occupancy calculator
-    int iters_per_graph = 4;       // ping-pong pairs per graph launch
+    int iters_per_graph = 1;       // ping-pong pairs per graph launch
     TraceTune trace = default_trace_tune();  // warp traversal loop of the extend stage
-    int drain_paths = 0;           // per-path finish of a render's last paths at most this many (0 = never)
+    int drain_paths = -1;          // a render's last paths, at most this many, leave the bounce loop (0 = never; -1: by scene)
     int pixel_tile = 0;            // generate camera paths tile by tile, tiles of this side (0: by rows)
 
-    uint32_t drain_threshold() const {
-        return drain_paths > 0 ? (uint32_t)drain_paths : 0u;
+    // Below about 2^15 paths an iteration of the loop costs its launches and its
+    // slowest ray (one sample of a 160x120 Cornell box: 0.25 ms out of the
+    // loop, 0.46 in it).  With a density grid lanes that track through it hold
+    // their warp's others up (512^2 x 16 spp: 21.3 ms at 2^13, 22.1 at 2^17).
+    uint32_t drain_threshold(bool hetero) const {
+        return drain_paths >= 0 ? (uint32_t)drain_paths : hetero ? 1u << 13 : 1u << 15;
     }
 };
 
@@ -158,8 +170,8 @@ int wf_launch(wr_ctx* ctx, WfEngine* E, cudaStream_t s);  // one graph replay
 // queue side `side` (side 0 after a graph replay)
 int wf_read_counters(wr_ctx* ctx, WfEngine* E, std::vector<WfJobCounters>& out, cudaStream_t s,
                      uint32_t* waiting = nullptr, int side = 0);
-// finishes the n paths waiting in side `side`, one thread per path (k_wf_drain)
-int wf_drain(wr_ctx* ctx, WfEngine* E, int side, uint32_t n, cudaStream_t s);
+// finishes the paths waiting in side `side` without the bounce loop (k_wf_finish)
+int wf_finish(wr_ctx* ctx, WfEngine* E, int side, cudaStream_t s);
 int wf_error_word(wr_ctx* ctx, WfEngine* E, unsigned int* herr, cudaStream_t s);
 int wf_reset_queues(wr_ctx* ctx, WfEngine* E, cudaStream_t s);
 // free queue slots shared equally among the jobs with paths left (default)

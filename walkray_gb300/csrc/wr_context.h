@@ -89,7 +89,7 @@ struct wr_ctx {
     int wf_extend_block = 0, wf_shade_block = 0, wf_ctas_per_sm = 0, wf_iters = 0;
     int trace_refill_min = 0, trace_leaf_min = 0;  // warp traversal loop (0 = defaults)
     int trace_steps = 0;                            // traversal steps per turn of the warp loop (0 = default)
-    int wf_drain_paths = 0;                          // drain threshold of wr_render (0 = never)
+    int wf_drain_paths = -1;                         // drain threshold of wr_render (0 = never; -1 = default)
     int wf_pixel_tile = 0;                           // camera paths generated tile by tile (0 = by rows)
 };
 

@@ -541,7 +541,8 @@ __device__ __forceinline__ uint32_t warp_leaves(SearchLane<Ray>& L, bool has, ui
 }
 
 // Closest hits of a warp's rays, one per lane with `on`; every lane of the
-// warp calls it.  All rays in one tree.
+// warp calls it.  ONE_TREE: all rays in the tree T (else each lane's own T).
+template <bool ONE_TREE = true>
 __device__ __forceinline__ Hit search_warp(const DevTree& T, bool on, f3 o, f3 d, float pf, bool filt, int inside,
                                            int contact, uint32_t* stack, int stride, int cap, uint8_t* item) {
     constexpr unsigned FULL = 0xffffffffu;
@@ -554,7 +555,8 @@ __device__ __forceinline__ Hit search_warp(const DevTree& T, bool on, f3 o, f3 d
         const unsigned wm = __ballot_sync(FULL, walking), lm = __ballot_sync(FULL, L.at_leaf());
         if (!(wm | lm)) break;
         if (lm && (wm == 0 || __popc(lm) >= 8)) {
-            warp_leaves(L, L.pend != NO_WORD, item, stack, stride, [&](int) { return T.tris; });
+            warp_leaves(L, L.pend != NO_WORD, item, stack, stride,
+                        [&](int from) { return ONE_TREE ? T.tris : L.ray.tris_of(from); });
         } else if (walking) {
             for (int k = 0; k < 6 && L.walking(); k++) L.visit(stack, stride, top);
         }
