@@ -73,88 +73,96 @@ struct BinNode {
     uint8_t split4;      // the same when given 4 (a node of its own)
 };
 
-// binary SAH tree over items[0, n); nodes appended to `out`, the root's index returned
-int32_t build_binary(Item* items, size_t n, std::vector<BinNode>& out) {
+// the box of items a[0, n), and where the surface-area heuristic parts them:
+// they are partitioned, the left part's size is returned
+size_t split_items(Item* a, size_t n, QBox& box) {
+    QBox cen;
+    box.clear();
+    cen.clear();
+    for (size_t i = 0; i < n; i++) {
+        box.add(a[i].box);
+        for (int k = 0; k < 3; k++) {
+            const float c = a[i].box.lo[k] + a[i].box.hi[k];
+            cen.lo[k] = std::min(cen.lo[k], c);
+            cen.hi[k] = std::max(cen.hi[k], c);
+        }
+    }
+    if (n == 1) return 1;
+    float best = INFINITY;
+    int best_d = -1, best_s = 0;
+    // bins of all three axes in one pass (scale 0: the axis cannot be split)
+    QBox bb[3][BINS];
+    uint32_t bc[3][BINS] = {};
+    float scale[3];
+    for (int d = 0; d < 3; d++) {
+        const float w = cen.hi[d] - cen.lo[d];
+        scale[d] = w > 0.f && (float)BINS / w < INFINITY ? (float)BINS / w : 0.f;
+        for (QBox& x : bb[d]) x.clear();
+    }
+    for (size_t i = 0; i < n; i++)
+        for (int d = 0; d < 3; d++) {
+            const int k = bin_of(a[i].box.lo[d] + a[i].box.hi[d], cen.lo[d], scale[d]);
+            bb[d][k].add(a[i].box);
+            bc[d][k] += a[i].count;
+        }
+    for (int d = 0; d < 3; d++) {
+        if (scale[d] == 0.f) continue;
+        float ra[BINS];
+        uint32_t rc[BINS], c = 0;
+        QBox acc;
+        acc.clear();
+        for (int k = BINS - 1; k > 0; k--) {
+            acc.add(bb[d][k]);
+            c += bc[d][k];
+            ra[k] = acc.area();
+            rc[k] = c;
+        }
+        acc.clear();
+        c = 0;
+        for (int k = 0; k + 1 < BINS; k++) {
+            acc.add(bb[d][k]);
+            c += bc[d][k];
+            if (!c || !rc[k + 1]) continue;
+            const float cost = acc.area() * (float)c + ra[k + 1] * (float)rc[k + 1];
+            if (cost < best) {
+                best = cost;
+                best_d = d;
+                best_s = k;
+            }
+        }
+    }
+    size_t m = 0;
+    if (best_d >= 0) {
+        const float base = cen.lo[best_d], sc = scale[best_d];
+        m = (size_t)(std::partition(a, a + n, [&](const Item& it) {
+                         return bin_of(it.box.lo[best_d] + it.box.hi[best_d], base, sc) <= best_s;
+                     }) -
+                     a);
+    }
+    return m == 0 || m == n ? n / 2 : m;  // equal centres: halves, in the order they have
+}
+
+// binary SAH tree over a[0, n): out[0] is its root, children come after their
+// parents
+void build_binary(Item* items, size_t n, std::vector<BinNode>& out) {
     struct Job {
         Item* a;
         size_t n;
         int32_t at;
     };
-    const int32_t root = (int32_t)out.size();
+    out.clear();
     out.emplace_back();
-    std::vector<Job> jobs{{items, n, root}};
+    std::vector<Job> jobs{{items, n, 0}};
     while (!jobs.empty()) {
         const Job j = jobs.back();
         jobs.pop_back();
-        QBox box, cen;
-        box.clear();
-        cen.clear();
-        for (size_t i = 0; i < j.n; i++) {
-            box.add(j.a[i].box);
-            for (int k = 0; k < 3; k++) {
-                const float c = j.a[i].box.lo[k] + j.a[i].box.hi[k];
-                cen.lo[k] = std::min(cen.lo[k], c);
-                cen.hi[k] = std::max(cen.hi[k], c);
-            }
-        }
-        out[j.at].box = box;
+        const size_t m = split_items(j.a, j.n, out[j.at].box);
         if (j.n == 1) {
             out[j.at].word = j.a[0].word;
             out[j.at].l = out[j.at].r = -1;
             out[j.at].cost[0] = (float)j.a[0].count;  // times area and TRI_COST below
             continue;
         }
-        float best = INFINITY;
-        int best_d = -1, best_s = 0;
-        float best_scale = 0.f;
-        for (int d = 0; d < 3; d++) {
-            const float w = cen.hi[d] - cen.lo[d];
-            if (!(w > 0.f)) continue;
-            const float scale = (float)BINS / w;
-            if (!(scale < INFINITY)) continue;
-            QBox bb[BINS];
-            uint32_t bc[BINS] = {};
-            for (QBox& b : bb) b.clear();
-            for (size_t i = 0; i < j.n; i++) {
-                const Item& it = j.a[i];
-                const int k = bin_of(it.box.lo[d] + it.box.hi[d], cen.lo[d], scale);
-                bb[k].add(it.box);
-                bc[k] += it.count;
-            }
-            float ra[BINS];
-            uint32_t rc[BINS], c = 0;
-            QBox acc;
-            acc.clear();
-            for (int k = BINS - 1; k > 0; k--) {
-                acc.add(bb[k]);
-                c += bc[k];
-                ra[k] = acc.area();
-                rc[k] = c;
-            }
-            acc.clear();
-            c = 0;
-            for (int k = 0; k + 1 < BINS; k++) {
-                acc.add(bb[k]);
-                c += bc[k];
-                if (!c || !rc[k + 1]) continue;
-                const float cost = acc.area() * (float)c + ra[k + 1] * (float)rc[k + 1];
-                if (cost < best) {
-                    best = cost;
-                    best_d = d;
-                    best_s = k;
-                    best_scale = scale;
-                }
-            }
-        }
-        size_t m = 0;
-        if (best_d >= 0) {
-            const float base = cen.lo[best_d];
-            m = (size_t)(std::partition(j.a, j.a + j.n, [&](const Item& it) {
-                             return bin_of(it.box.lo[best_d] + it.box.hi[best_d], base, best_scale) <= best_s;
-                         }) -
-                         j.a);
-        }
-        if (m == 0 || m == j.n) m = j.n / 2;  // equal centres: halves, in the order they have
         const int32_t l = (int32_t)out.size();
         out.emplace_back();
         out.emplace_back();
@@ -163,7 +171,38 @@ int32_t build_binary(Item* items, size_t n, std::vector<BinNode>& out) {
         jobs.push_back({j.a, m, l});
         jobs.push_back({j.a + m, j.n - m, l + 1});
     }
-    return root;
+}
+
+// the same by tasks: the halves of a large range are built beside each other
+// and put together
+void build_binary_tasks(Item* a, size_t n, std::vector<BinNode>& out) {
+    if (n < 512) {
+        build_binary(a, n, out);
+        return;
+    }
+    BinNode root{};
+    const size_t m = split_items(a, n, root.box);
+    std::vector<BinNode> half[2];
+#pragma omp task default(shared)
+    build_binary_tasks(a, m, half[0]);
+#pragma omp task default(shared)
+    build_binary_tasks(a + m, n - m, half[1]);
+#pragma omp taskwait
+    root.l = 1;
+    root.r = 1 + (int32_t)half[0].size();
+    out.clear();
+    out.reserve(1 + half[0].size() + half[1].size());
+    out.push_back(root);
+    for (int k = 0; k < 2; k++) {
+        const int32_t by = k ? root.r : root.l;
+        for (BinNode b : half[k]) {
+            if (b.l >= 0) {
+                b.l += by;
+                b.r += by;
+            }
+            out.push_back(b);
+        }
+    }
 }
 
 // least costs of nodes [first, end) (children come after their parents).
@@ -290,43 +329,51 @@ QuadLayout build_quads(const HostTree& t, int threads) {
 #endif
     (void)threads;
     // parent links of the reference tree, in the device layout's numbering
-    // (pairs in pre-order, slots leaf by leaf)
-    std::vector<uint32_t> up(N, UP_ROOT), leaves_below(N, 0u);
-    L.leaf_up.resize(t.leaf_tris.size());
-    uint32_t np = 0;
-    size_t slot = 0;
-    std::vector<Item> items;
-    items.reserve(t.num_leaves);
+    // (pairs in pre-order, slots leaf by leaf), and the leaves as items; a leaf
+    // of more than QUAD_LEAF_MAX triangles is several items with one box
+    std::vector<uint32_t> pair_of(N, 0u), slot_of(N, 0u), parent(N, 0u);
     std::vector<uint32_t> node_item(N, 0u);  // first item at or after each node
-    bool fits = t.leaf_tris.size() <= QUAD_MAX_SLOTS;
+    uint32_t np = 0, slots = 0, ni = 0;
     for (uint32_t n = 0; n < N; n++) {
-        node_item[n] = (uint32_t)items.size();
+        node_item[n] = ni;
+        slot_of[n] = slots;
         if (t.left[n] >= 0) {
-            up[t.left[n]] = np << 1;
-            up[t.right[n]] = np << 1 | 1u;
-            const uint32_t u = up[n];
-            uint4 a = make_uint4(u, UP_ROOT, UP_ROOT, UP_ROOT);
-            if (u != UP_ROOT) {  // parents come first
-                const uint4& p = L.pair_up[u >> 1];
-                a.y = p.x;
-                a.z = p.y;
-                a.w = p.z;
+            pair_of[n] = np++;
+            parent[t.left[n]] = parent[t.right[n]] = n;
+        } else {
+            ni += (t.leaf_count[n] + QUAD_LEAF_MAX - 1) / QUAD_LEAF_MAX;
+            slots += t.leaf_count[n];
+        }
+    }
+    L.leaf_up.resize(slots);
+    L.pair_up.resize(np);
+    std::vector<Item> items(ni);
+    auto up = [&](uint32_t n) {
+        return n == 0 ? UP_ROOT : pair_of[parent[n]] << 1 | (uint32_t)(t.right[parent[n]] == (int32_t)n);
+    };
+    bool fits = slots <= QUAD_MAX_SLOTS;
+#ifdef _OPENMP
+#pragma omp parallel for num_threads(threads) schedule(static, 4096) reduction(&& : fits) if (N > 16384)
+#endif
+    for (uint32_t n = 0; n < N; n++) {
+        if (t.left[n] >= 0) {
+            uint32_t a[4], m = n;
+            for (uint32_t& u : a) {  // (past the root: UP_ROOT again)
+                u = up(m);
+                m = parent[m];
             }
-            L.pair_up.push_back(a);
-            np++;
+            L.pair_up[pair_of[n]] = make_uint4(a[0], a[1], a[2], a[3]);
             continue;
         }
-        for (uint32_t k = 0; k < t.leaf_count[n]; k += QUAD_LEAF_MAX) {  // a longer leaf: several items, one box
-            Item it;
+        for (uint32_t k = 0, i = node_item[n]; k < t.leaf_count[n]; k += QUAD_LEAF_MAX, i++) {
+            Item& it = items[i];
             std::memcpy(it.box.lo, &t.box[6 * (size_t)n], 12);
             std::memcpy(it.box.hi, &t.box[6 * (size_t)n + 3], 12);
-            for (int d = 0; d < 3; d++) fits &= std::isfinite(it.box.lo[d]) && std::isfinite(it.box.hi[d]);
+            for (int d = 0; d < 3; d++) fits = fits && std::isfinite(it.box.lo[d]) && std::isfinite(it.box.hi[d]);
             it.count = std::min(QUAD_LEAF_MAX, t.leaf_count[n] - k);
-            it.word = QUAD_LEAF | it.count << QUAD_COUNT_AT | (uint32_t)(slot + k);
-            items.push_back(it);
+            it.word = QUAD_LEAF | it.count << QUAD_COUNT_AT | (slot_of[n] + k);
         }
-        for (uint32_t k = 0; k < t.leaf_count[n]; k++) L.leaf_up[slot + k] = up[n];
-        slot += t.leaf_count[n];
+        for (uint32_t k = 0; k < t.leaf_count[n]; k++) L.leaf_up[slot_of[n] + k] = up(n);
     }
     if (!fits) return L;
     if (items.empty()) {  // no triangles: a root of holes
@@ -372,10 +419,9 @@ QuadLayout build_quads(const HostTree& t, int threads) {
     {
         std::vector<BinNode> bin;
 #ifdef _OPENMP
-#pragma omp for schedule(dynamic, 16)
+#pragma omp for schedule(dynamic, 4)
 #endif
         for (size_t c = 0; c < nc; c++) {
-            bin.clear();
             const uint32_t a = range[c].first, e = range[c].second;
             top[c].word = (uint32_t)c;
             top[c].count = 0;
@@ -393,7 +439,11 @@ QuadLayout build_quads(const HostTree& t, int threads) {
         return L;
     }
     std::vector<BinNode> bin;
-    build_binary(top.data(), nc, bin);
+#ifdef _OPENMP
+#pragma omp parallel num_threads(threads)
+#pragma omp single
+#endif
+    build_binary_tasks(top.data(), nc, bin);
     cut_costs(bin, 0, &sub_cost);
     // the upper tree, its clusters marked by the leaf bit for now; the
     // clusters' nodes follow it in the order it reaches them
