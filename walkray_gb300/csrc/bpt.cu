@@ -165,7 +165,8 @@ __device__ __forceinline__ void warp_append(bool ok, uint2 item, uint2* list, un
 // traces it at one call site (the first ray of a sub-path too: the camera
 // ray unfiltered (camera.cpp:52), which a filter with no inside and no
 // contact object is, the emitted ray with NoSelfCondition).
-template <bool HM>
+// MED: what scatter() is compiled for (wr_shade.cuh)
+template <int MED>
 __global__ void __launch_bounds__(128) k_bpt_subpaths(RenderScene S, BptParams P) {
     constexpr unsigned FULL = 0xffffffffu;
     __shared__ uint8_t s_item[BPT_BLOCK / 32][LEAF_ITEMS];
@@ -245,7 +246,7 @@ __global__ void __launch_bounds__(128) k_bpt_subpaths(RenderScene S, BptParams P
                 out.put(sid, n++, term);
                 done = true;
             } else {
-                next = scatter<HM>(S, self, prev, g, st);
+                next = scatter<MED>(S, self, prev, g, st);
                 if (length(next.d) < 0.5f) {
                     out.put(sid, n++, next);
                     done = true;
@@ -1391,10 +1392,10 @@ __global__ void __launch_bounds__(128) k_ppm_eye(RenderScene S, BptParams P) {
                 float ps = 1.f;
                 next = scatter_heterogeneous_ref(S, self, cur, g, st, &del, &ps, chk);
             } else {
-                next = scatter<HM>(S, self, cur, g, st);
+                next = scatter<HM ? MED_REF : MED_TRACK>(S, self, cur, g, st);
             }
         } else {
-            next = scatter(S, self, prev, g, st);
+            next = scatter<MED_NONE>(S, self, prev, g, st);
         }
         const bool ended = length(next.d) < 0.5f;
         if (!ended && depth + 1 > PPM_MERGE_LEN) break;  // cut: `next` is not a record
@@ -1602,7 +1603,7 @@ int render_bidirectional(wr_ctx* ctx, const RenderScene& S, const RenderParams& 
     P.ncand = reinterpret_cast<unsigned long long*>(st.counts.as<char>() + ((4ull * nsamp + 7) & ~7ull));
     // scenes with a heterogeneous medium take the kernels that march its
     // integrals in the weights; the others compile without those calls
-    const auto k_subpaths = hetero ? k_bpt_subpaths<true> : k_bpt_subpaths<false>;
+    const auto k_subpaths = hetero ? k_bpt_subpaths<MED_REF> : media ? k_bpt_subpaths<MED_TRACK> : k_bpt_subpaths<MED_NONE>;
     const auto k_connect = hetero ? k_bpt_connect<true, 1> : vcm ? k_bpt_connect<false, 4> : k_bpt_connect<false, 5>;
     const auto k_merge = hetero ? k_vcm_merge<true> : k_vcm_merge<false>;
     const auto k_eval = hetero ? k_vcm_eval<true> : k_vcm_eval<false>;

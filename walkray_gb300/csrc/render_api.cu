@@ -268,7 +268,7 @@ int wr_render_device(wr_ctx* ctx, wr_scene_id id, const wr_render_desc* desc, fl
         for (uint64_t s0 = 0; s0 < desc->spp; s0 += per_launch) {
             P.s0 = (uint32_t)(desc->spp_offset + s0);
             P.s1 = (uint32_t)(desc->spp_offset + std::min<uint64_t>(desc->spp, s0 + per_launch));
-            WR_CUDA(ctx, launch_megakernel(rd->S, P, d_sum, d_sumsq, s));
+            WR_CUDA(ctx, launch_megakernel(rd->S, P, d_sum, d_sumsq, rd->has_media, s));
             ctx->kernel_launches++;
         }
         return WR_OK;
@@ -372,6 +372,7 @@ int wr_render_progressive(wr_ctx* ctx, wr_scene_id id, const wr_render_desc* des
 namespace wr {
 
 const RenderScene& RenderDataView::scene(const RenderData* rd) { return rd->S; }
+bool RenderDataView::media(const RenderData* rd) { return rd->has_media; }
 bool RenderDataView::hetero(const RenderData* rd) { return rd->has_hetero; }
 const std::string& RenderDataView::unsupported(const RenderData* rd) { return rd->unsupported; }
 

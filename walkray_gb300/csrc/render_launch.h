@@ -38,9 +38,10 @@ struct RenderParams {
 };
 
 // plain megakernel: film[3*p+c] += sum over samples of the pixel colour
-// (film2 != NULL: also the sum of squares)
+// (film2 != NULL: also the sum of squares); `media`: the scene has a
+// participating medium
 cudaError_t launch_megakernel(const RenderScene& S, const RenderParams& P, float* film, float* film2,
-                              cudaStream_t stream);
+                              bool media, cudaStream_t stream);
 
 // WR_MODE_BIDIRECTIONAL, WR_MODE_VCM and WR_MODE_PHOTON_MAP (bpt.cu): adds
 // samples [spp_offset, spp_offset + spp) of every pixel to d_sum (and their

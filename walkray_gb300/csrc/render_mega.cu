@@ -3,6 +3,8 @@
 // pathTracer.cpp:21-70: camera ray, samplePath bounce loop, throughput,
 // isLegalColor, fixVignetting) for a range of samples and adds the results
 // to an FP32 film (sum and optional sum of squares per channel).
+#include <type_traits>
+
 #include "render_launch.h"
 #include "wr_shade.cuh"
 
@@ -14,7 +16,7 @@ constexpr int MEGA_BLOCK = 128;
 // turn (search_warp) and goes on to its pixel's next sample as soon as a path
 // ends, so that a warp waits for the lane with the most rays in all, not for
 // the longest path of every sample.
-template <bool STATS, bool MIS>
+template <bool STATS, bool MIS, int MED>
 __global__ void __launch_bounds__(MEGA_BLOCK) k_megakernel(RenderScene S, RenderParams P, float* __restrict__ film,
                                                            float* __restrict__ film2) {
     constexpr unsigned FULL = 0xffffffffu;
@@ -61,7 +63,7 @@ __global__ void __launch_bounds__(MEGA_BLOCK) k_megakernel(RenderScene S, Render
                 done = true;
             } else {
                 set_hit(S, cur, h);
-                done = path_advance<MIS>(S, cur, color, prev_d, depth, st, g, P.max_path_len, P.flags, result,
+                done = path_advance<MIS, MED>(S, cur, color, prev_d, depth, st, g, P.max_path_len, P.flags, result,
                                          nee_here, mis_pdf, lr, has_lr);
             }
         }
@@ -101,14 +103,18 @@ __global__ void __launch_bounds__(MEGA_BLOCK) k_megakernel(RenderScene S, Render
 }
 
 cudaError_t launch_megakernel(const RenderScene& S, const RenderParams& P, float* film, float* film2,
-                              cudaStream_t stream) {
+                              bool media, cudaStream_t stream) {
     const int block = MEGA_BLOCK;
     const size_t smem = (size_t)P.stack_cap * block * sizeof(uint32_t);
     const uint32_t npix = S.cam.width * S.cam.height;
     const int grid = (int)((npix + block - 1) / block);
     const bool mis = (P.flags & WR_RENDER_NEE_MIS) != 0;
-    auto kern = film2 ? (mis ? k_megakernel<true, true> : k_megakernel<true, false>)
-                      : (mis ? k_megakernel<false, true> : k_megakernel<false, false>);
+    auto pick = [&](auto med) {
+        constexpr int M = decltype(med)::value;
+        return film2 ? (mis ? k_megakernel<true, true, M> : k_megakernel<true, false, M>)
+                     : (mis ? k_megakernel<false, true, M> : k_megakernel<false, false, M>);
+    };
+    auto kern = media ? pick(std::integral_constant<int, MED_TRACK>{}) : pick(std::integral_constant<int, MED_NONE>{});
     if (smem > 48 * 1024) {
         cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
         if (e != cudaSuccess) return e;

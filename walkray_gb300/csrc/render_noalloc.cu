@@ -121,7 +121,7 @@ static int render_noalloc_body(wr_ctx* ctx, wr_scene_id id, const wr_render_desc
     for (uint64_t s0 = 0; s0 < desc->spp; s0 += per_launch) {
         P.s0 = (uint32_t)(desc->spp_offset + s0);
         P.s1 = (uint32_t)(desc->spp_offset + std::min<uint64_t>(desc->spp, s0 + per_launch));
-        WR_CUDA(ctx, launch_megakernel(S, P, film, nullptr, s));
+        WR_CUDA(ctx, launch_megakernel(S, P, film, nullptr, RenderDataView::media(rd), s));
     }
     const float inv = desc->spp ? 1.0f / (float)desc->spp : 0.f;
     k_film_mean<<<(unsigned)std::min<size_t>((n + 255) / 256, 4096), 256, 0, s>>>(film, d_rgb_out, n, inv);

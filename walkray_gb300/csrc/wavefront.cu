@@ -370,8 +370,9 @@ static ExtendKernel extend_kernel(int ctas_per_sm, bool stats, bool exact) {
 
 // shade: one bounce per path; survivors compacted into Y, finished paths to
 // the film.  MIS: compiled with the WR_RENDER_NEE_MIS code (launched while a
-// job with that flag is in the table).
-template <bool MIS>
+// job with that flag is in the table).  MED: MED_TRACK while a scene with
+// participating media is.
+template <bool MIS, int MED>
 __global__ void __launch_bounds__(128, 4) k_wf_shade(const RenderScene* __restrict__ scenes,
                                                     const WfJob* __restrict__ jobs,
                                                     WfJobCounters* __restrict__ counters, WfSide X,
@@ -423,7 +424,7 @@ __global__ void __launch_bounds__(128, 4) k_wf_shade(const RenderScene* __restri
                 nee_here = nee;
             } else {
                 set_hit(S, p.cur, h);
-                done = path_advance<MIS>(S, p.cur, p.color, p.prev_d, p.depth, p.st, g, J.max_path_len, J.flags,
+                done = path_advance<MIS, MED>(S, p.cur, p.color, p.prev_d, p.depth, p.st, g, J.max_path_len, J.flags,
                                          result, nee_here, p.mis_pdf, lr, has_lr);
             }
             if (nee_here) shadow = nee_prepare(S, p.cur, p.prev_d, p.color, g, sr);
@@ -472,6 +473,11 @@ __global__ void __launch_bounds__(128, 4) k_wf_shade(const RenderScene* __restri
     }
 }
 
+static auto shade_kernel(bool mis, bool media) {
+    if (media) return mis ? k_wf_shade<true, MED_TRACK> : k_wf_shade<false, MED_TRACK>;
+    return mis ? k_wf_shade<true, MED_NONE> : k_wf_shade<false, MED_NONE>;
+}
+
 // finish: the paths waiting in X run to their ends without returning to the
 // bounce loop, one path to a lane, the lanes of a warp together (search_warp).
 // Once nothing is left to generate, each iteration of the loop costs the
@@ -480,7 +486,7 @@ __global__ void __launch_bounds__(128, 4) k_wf_shade(const RenderScene* __restri
 // the loop.  MIS: compiled with the WR_RENDER_NEE_MIS code.
 // Bound by latency: a warp's turn lasts as long as its slowest ray's search.
 // Few paths are therefore spread over all warps, a few lanes to each.
-template <bool MIS>
+template <bool MIS, int MED>
 __global__ void __launch_bounds__(WF_FINISH_BLOCK, MIS ? 3 : 4)
     k_wf_finish(const RenderScene* __restrict__ scenes, const WfJob* __restrict__ jobs,
                 WfJobCounters* __restrict__ counters, WfSide X, unsigned int* __restrict__ next, int stack_cap) {
@@ -535,7 +541,7 @@ __global__ void __launch_bounds__(WF_FINISH_BLOCK, MIS ? 3 : 4)
                 nee_here = (J.flags & WR_RENDER_NEE) != 0;
             } else {
                 set_hit(S, p.cur, h);
-                done = path_advance<MIS>(S, p.cur, p.color, p.prev_d, p.depth, p.st, g, J.max_path_len, J.flags,
+                done = path_advance<MIS, MED>(S, p.cur, p.color, p.prev_d, p.depth, p.st, g, J.max_path_len, J.flags,
                                          result, nee_here, p.mis_pdf, lr, has_lr);
             }
         }
@@ -768,13 +774,14 @@ struct WfEngine {
     cudaGraphExec_t graph = nullptr;
     int graph_stack = -1;
     bool mis_any = false;  // a job in the table has WR_RENDER_NEE_MIS: the shade stage with that code
+    bool media_any = false;  // a job's scene has participating media: the shading kernels with that code
     bool exact_any = false;  // a job in the table has WR_RENDER_EXACT_TRAVERSAL: the extend stage of that walk
     bool conn_any = true;  // a job in the table connects to lights (NEE or MIS): the shadow stage is in the loop
     int launches_per_iteration() const { return conn_any ? 8 : 6; }
     WfJobCounters* host_counters = nullptr;  // pinned
     WfStatus* status = nullptr;              // pinned and mapped: written by k_wf_plan
     cudaEvent_t turn[2] = {};                // the end of the last two graph replays of a render
-    int grid_finish[2] = {};                 // k_wf_finish without and with the light connections
+    int grid_finish[4] = {};                 // k_wf_finish without and with the light connections, then with media
     ~WfEngine() {
         if (graph) cudaGraphExecDestroy(graph);
         if (host_counters) cudaFreeHost(host_counters);
@@ -894,7 +901,7 @@ int wf_engine_get(wr_ctx* ctx, const WfConfig& cfg, WfEngine** out) {
     E->order_host.assign(1, 0);
     // persistent grids from the occupancy calculator
     int per_sm = 0;
-    WR_CUDA(ctx, cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_wf_shade<false>, cfg.shade_block, 0));
+    WR_CUDA(ctx, cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, shade_kernel(false, true), cfg.shade_block, 0));
     if (cfg.ctas_per_sm > 0) per_sm = std::min(per_sm, cfg.ctas_per_sm);
     E->grid_shade = ctx->num_sms * std::max(1, per_sm);
     WR_CUDA(ctx, cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_wf_generate, WF_GEN_ROWS, 0));
@@ -999,15 +1006,18 @@ int wf_update_jobs(wr_ctx* ctx, WfEngine* E, const std::vector<WfSlotUpdate>& up
     }
     // the shade stage compiled with the light-connection code only while a job needs it
     // and the shadow stage only while a job can queue a connection
-    bool mis_any = false, conn_any = false, exact_any = false;
+    bool mis_any = false, conn_any = false, exact_any = false, media_any = false;
     for (int slot : order) {
         if (!E->job_tab[slot].active) continue;
         if (E->job_tab[slot].flags & WR_RENDER_NEE_MIS) mis_any = true;
         if (E->job_tab[slot].flags & WR_RENDER_EXACT_TRAVERSAL) exact_any = true;
+        if (const RenderData* rd = E->scene_of[E->job_tab[slot].scene]) media_any |= RenderDataView::media(rd);
         if (E->job_tab[slot].flags & (WR_RENDER_NEE | WR_RENDER_NEE_MIS)) conn_any = true;
     }
-    if (mis_any != E->mis_any || conn_any != E->conn_any || exact_any != E->exact_any) {
+    if (mis_any != E->mis_any || conn_any != E->conn_any || exact_any != E->exact_any ||
+        media_any != E->media_any) {
         E->exact_any = exact_any;
+        E->media_any = media_any;
         E->mis_any = mis_any;
         E->conn_any = conn_any;
         if (E->graph) {
@@ -1040,7 +1050,7 @@ static void enqueue_iteration(WfEngine* E, int x, cudaStream_t s, cudaEvent_t* e
             E->exact_any ? E->stack_cap : E->quad_cap, E->cfg.trace, E->err_word.as<unsigned int>(), stats);
     if (ev) cudaEventRecord(ev[1], s);
     k_wf_sort<<<E->grid_sort, 256, 0, s>>>(scenes, jobs, E->side[x], E->hits.as<int2>(), E->sort, E->cfg.capacity);
-    (E->mis_any ? k_wf_shade<true> : k_wf_shade<false>)<<<E->grid_shade, E->cfg.shade_block, 0, s>>>(scenes, jobs, cnt, E->side[x], E->hits.as<int2>(),
+    shade_kernel(E->mis_any, E->media_any)<<<E->grid_shade, E->cfg.shade_block, 0, s>>>(scenes, jobs, cnt, E->side[x], E->hits.as<int2>(),
                                                             E->side[y], E->shadow, E->sort, E->cfg.capacity);
     if (ev) cudaEventRecord(ev[2], s);
     if (E->conn_any) {  // the connections' closest hits go into E->hits, which shade has read
@@ -1205,9 +1215,10 @@ int wf_read_counters(wr_ctx* ctx, WfEngine* E, std::vector<WfJobCounters>& out, 
 }
 
 int wf_finish(wr_ctx* ctx, WfEngine* E, int side, cudaStream_t s) {
-    const auto kern = E->mis_any ? k_wf_finish<true> : k_wf_finish<false>;
+    const auto kern = E->media_any ? (E->mis_any ? k_wf_finish<true, MED_TRACK> : k_wf_finish<false, MED_TRACK>)
+                                   : (E->mis_any ? k_wf_finish<true, MED_NONE> : k_wf_finish<false, MED_NONE>);
     const size_t smem = (size_t)E->quad_cap * WF_FINISH_BLOCK * sizeof(uint32_t);
-    int& grid = E->grid_finish[E->mis_any];
+    int& grid = E->grid_finish[E->mis_any + 2 * E->media_any];
     if (!grid) {
         int per_sm = 0;
         WR_CUDA(ctx, cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kern, WF_FINISH_BLOCK, smem));

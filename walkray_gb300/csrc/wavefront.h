@@ -37,7 +37,8 @@ namespace wr {
 struct RenderData;
 struct RenderDataView {  // what the engine needs from RenderData (render_api.cu)
     static const RenderScene& scene(const RenderData* rd);
-    static bool hetero(const RenderData* rd);  // a heterogeneous medium is among its objects
+    static bool media(const RenderData* rd);   // a participating medium is among its objects
+    static bool hetero(const RenderData* rd);  // a heterogeneous one
     static const std::string& unsupported(const RenderData* rd);  // non-empty: why the scene cannot render
 };
 

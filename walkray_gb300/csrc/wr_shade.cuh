@@ -167,10 +167,21 @@ struct InsideStack {
     }
 };
 
+// What a kernel is compiled for.  A scene's participating media are most of the
+// shading code, and the kernels are bound by its size (with the density grid
+// the shade stage waited 12 cycles for instructions per instruction issued), so
+// scenes without media run kernels without it.
+enum : int {
+    MED_NONE = 0,   // no participating media
+    MED_TRACK = 1,  // heterogeneous media by delta tracking
+    MED_REF = 2     // heterogeneous media by the reference's own sampler
+};
+
 // Ray::cosineTerm (ray.cpp:52-58)
+template <int MED = MED_TRACK>
 __device__ __forceinline__ float cos_term(const RenderScene& S, const PRay& r) {
     float c = 1.f;
-    bool has_cos = r.contact == CAMERA_OBJ || (r.contact >= 0 && !is_volume(S, r.contact));
+    bool has_cos = r.contact == CAMERA_OBJ || (r.contact >= 0 && (MED == MED_NONE || !is_volume(S, r.contact)));
     if (r.contact != -1 && has_cos && length(r.d) > 0.5f) c = fabsf(dot(r.cnorm, r.d));
     return c > EPS_F ? c : EPS_F;
 }
@@ -396,7 +407,7 @@ struct Fresnel {
     float er;
 };
 // shared dielectric boundary step (refractiveObj.h:37-82)
-__device__ __forceinline__ Fresnel fresnel_split(f3 N, f3 d, float cn, float nn) {
+__device__ __forceinline__ Fresnel fresnel_here(f3 N, f3 d, float cn, float nn) {
     Fresnel f;
     f.refl = mirror_dir(N, d);
     f.refr = mk(0, 0, 0);
@@ -414,6 +425,11 @@ __device__ __forceinline__ Fresnel fresnel_split(f3 N, f3 d, float cn, float nn)
     const float a2 = fabsf(nn * ct - cn * cp) / (nn * ct + cn * cp);
     f.er = (a1 * a1 + a2 * a2) / 2.f;
     return f;
+}
+
+// with media there are five places that ask: one copy for all of them
+static __device__ __noinline__ Fresnel fresnel_split(f3 N, f3 d, float cn, float nn) {
+    return fresnel_here(N, d, cn, nn);
 }
 
 __device__ __forceinline__ void set_contact(const RenderScene& S, PRay& out, int obj, uint32_t tri, f3 n) {
@@ -473,6 +489,7 @@ __device__ __forceinline__ PRay scatter_emissive(const RenderScene& S, int self,
 // survival radiance color / cosineTerm, pdf p (a delta direction).  The
 // reference's MAX macro (macros.h:13) has no parentheses, so MAX_VEC_COMP
 // evaluates to x > y ? x : max(y, z), reproduced here.
+template <int MED>
 __device__ __forceinline__ PRay scatter_reflective(const RenderScene& S, int self, const PRay& in, PathRng& g) {
     PRay out = ray_default();
     const f3 N = in.inorm;
@@ -484,7 +501,7 @@ __device__ __forceinline__ PRay scatter_reflective(const RenderScene& S, int sel
     if (g.next() < p) {
         out.contact = self;
         out.cnorm = self == in.iobj ? N : obj_normal(S, self, in.itri);
-        out.rad = divs(c, cos_term(S, out));
+        out.rad = divs(c, cos_term<MED>(S, out));
         out.dP = p;
         out.delta = true;
     } else {
@@ -496,6 +513,7 @@ __device__ __forceinline__ PRay scatter_reflective(const RenderScene& S, int sel
 }
 
 // RefractiveObject::scatter (refractiveObj.h:27-88)
+template <int MED>
 __device__ __forceinline__ PRay scatter_refractive(const RenderScene& S, int self, const PRay& in, PathRng& g,
                                                    InsideStack& st, bool* delegate) {
     *delegate = in.iobj != self && in.inside == self;
@@ -509,7 +527,7 @@ __device__ __forceinline__ PRay scatter_refractive(const RenderScene& S, int sel
     const float cn = curIn >= 0 ? obj_ior(S, curIn) : 1.f, nn = curOut >= 0 ? obj_ior(S, curOut) : 1.f;
     out.contact = self;
     out.cnorm = self == in.iobj ? N : obj_normal(S, self, in.itri);
-    const Fresnel f = fresnel_split(N, in.d, cn, nn);
+    const Fresnel f = MED == MED_NONE ? fresnel_here(N, in.d, cn, nn) : fresnel_split(N, in.d, cn, nn);
     if (f.tir) {
         out.d = f.refl;
         out.inside = in.inside;
@@ -517,11 +535,11 @@ __device__ __forceinline__ PRay scatter_refractive(const RenderScene& S, int sel
         out.d = f.refr;
         if (g.next() < f.er) {
             out.d = f.refl;
-            out.rad = out.rad * (f.er / cos_term(S, out));
+            out.rad = out.rad * (f.er / cos_term<MED>(S, out));
             out.dP = f.er;
             out.inside = in.inside;
         } else {
-            out.rad = out.rad * ((1.f - f.er) / cos_term(S, out));
+            out.rad = out.rad * ((1.f - f.er) / cos_term<MED>(S, out));
             out.dP = 1.f - f.er;
             out.inside = curOut;
         }
@@ -882,8 +900,7 @@ static __device__ __noinline__ PRay scatter_heterogeneous_ref(const RenderScene&
 
 // one scatter() call, following delegations (RefractiveObject handing a hit
 // inside it to the hit object; media handing over to the surface hit).
-// RefMedia: heterogeneous media by the reference's own sampler.
-template <bool RefMedia = false>
+template <int MED = MED_TRACK>
 static __device__ __forceinline__ PRay scatter(const RenderScene& S, int self, const PRay& in, PathRng& g,
                                             InsideStack& st, bool mirror = false) {
     PRay cur = in;
@@ -899,21 +916,25 @@ static __device__ __forceinline__ PRay scatter(const RenderScene& S, int self, c
             case WR_MAT_GLOSSY:
             case WR_MAT_ANISO: out = scatter_surface(S, self, cur, g, mirror); break;
             case WR_MAT_EMISSIVE: out = scatter_emissive(S, self, cur); break;
-            case WR_MAT_REFLECTIVE: out = scatter_reflective(S, self, cur, g); break;
+            case WR_MAT_REFLECTIVE: out = scatter_reflective<MED>(S, self, cur, g); break;
             case WR_MAT_REFRACTIVE:
-                out = scatter_refractive(S, self, cur, g, st, &del);
+                out = scatter_refractive<MED>(S, self, cur, g, st, &del);
                 if (del) {  // `return inRay.intersectObj->scatter(inRay)`
                     self = cur.iobj;
                     continue;
                 }
                 break;
-            case WR_MAT_HOMOGENEOUS: out = scatter_homogeneous(S, self, cur, g, st, &del, &ps); break;
+            case WR_MAT_HOMOGENEOUS:
+                if constexpr (MED != MED_NONE) out = scatter_homogeneous(S, self, cur, g, st, &del, &ps);
+                else out = ray_default();
+                break;
             default:
-                if constexpr (RefMedia) out = scatter_heterogeneous_ref(S, self, cur, g, st, &del, &ps);
-                else out = scatter_heterogeneous(S, self, cur, g, st, &del, &ps);
+                if constexpr (MED == MED_REF) out = scatter_heterogeneous_ref(S, self, cur, g, st, &del, &ps);
+                else if constexpr (MED == MED_TRACK) out = scatter_heterogeneous(S, self, cur, g, st, &del, &ps);
+                else out = ray_default();
                 break;
         }
-        if (del) {  // medium hands over to the surface it hit: scatter there, oP *= P_surface
+        if (MED != MED_NONE && del) {  // medium hands over to the surface it hit: scatter there, oP *= P_surface
             oP_scale *= ps;
             self = cur.iobj;
             medium_hit = self;
@@ -931,6 +952,7 @@ static __device__ __forceinline__ PRay scatter(const RenderScene& S, int self, c
 
 // Ray::radianceDecay (ray.cpp:46-50): refractive decay^dist, homogeneous
 // exp(-sigma_t dist); heterogeneous media are already weighted by tracking
+template <int MED = MED_TRACK>
 __device__ __forceinline__ f3 radiance_decay(const RenderScene& S, const PRay& r, float dist) {
     if (r.inside < 0) return mk(1, 1, 1);
     const wr_object_desc* m = &S.objs[r.inside];
@@ -939,7 +961,7 @@ __device__ __forceinline__ f3 radiance_decay(const RenderScene& S, const PRay& r
         const f3 dc = ld3(m->decay);
         return mk(powf(dc.x, dist), powf(dc.y, dist), powf(dc.z, dist));
     }
-    if (t == WR_MAT_HOMOGENEOUS) {
+    if (MED != MED_NONE && t == WR_MAT_HOMOGENEOUS) {
         const f3 s = ld3(m->sigma_s) + ld3(m->sigma_a);
         return mk(expf(-s.x * dist), expf(-s.y * dist), expf(-s.z * dist));
     }
@@ -1288,7 +1310,8 @@ __device__ __forceinline__ bool mis_light_request(const RenderScene& S, int self
 // the scatter's density of the current ray (0: nothing to weigh).
 // MIS_CODE: compiled with the WR_RENDER_NEE_MIS code (kernels that never see
 // the flag leave it out, which keeps their register count down).
-template <bool MIS_CODE>
+// MED: as scatter's.
+template <bool MIS_CODE, int MED>
 __device__ __forceinline__ bool path_advance(const RenderScene& S, PRay& cur, f3& color, f3& prev_d,
                                              uint32_t& depth, InsideStack& st, PathRng& g, uint32_t max_path_len,
                                              uint32_t flags, f3& result, bool& nee_here, float& mis_pdf,
@@ -1308,10 +1331,10 @@ __device__ __forceinline__ bool path_advance(const RenderScene& S, PRay& cur, f3
     // the reference only has while its scattered ray may still be traced
     const bool mis_vertex = mis && cur.inside < 0 && mis_material(stype) && depth + 1 <= max_path_len;
     if (mis_vertex) {
-        const f3 T = vmul(color * cos_term(S, cur), weight(cur));
+        const f3 T = vmul(color * cos_term<MED>(S, cur), weight(cur));
         has_lr = mis_light_request(S, self, cur, T, g, mirror, lr);
     }
-    PRay next = scatter(S, self, cur, g, st, mirror);
+    PRay next = scatter<MED>(S, self, cur, g, st, mirror);
     if (length(next.d) < 0.5f) {
         const bool zero = next.rad.x == 0.f && next.rad.y == 0.f && next.rad.z == 0.f;
         if (nee && zero) {
@@ -1319,8 +1342,8 @@ __device__ __forceinline__ bool path_advance(const RenderScene& S, PRay& cur, f3
             nee_here = next.contact == -1 && next.inside == -1 && depth >= 1;
             return true;
         }
-        color = color * cos_term(S, cur);
-        color = vmul(color, radiance_decay(S, cur, length(next.o - cur.o)));
+        color = color * cos_term<MED>(S, cur);
+        color = vmul(color, radiance_decay<MED>(S, cur, length(next.o - cur.o)));
         color = vmul(color, weight(cur));
         result = vmul(color, weight(next));
         if (mis && mis_pdf > 0.f && stype == WR_MAT_EMISSIVE && cur.inside < 0 && !zero) {
@@ -1337,8 +1360,8 @@ __device__ __forceinline__ bool path_advance(const RenderScene& S, PRay& cur, f3
     }
     mis_pdf = mis_vertex ? bsdf_pdf(S, self, cur.d, cur.inorm, next.d, mirror) : 0.f;
     st.set_top(next.inside);
-    color = color * cos_term(S, cur);
-    color = vmul(color, radiance_decay(S, cur, length(next.o - cur.o)));
+    color = color * cos_term<MED>(S, cur);
+    color = vmul(color, radiance_decay<MED>(S, cur, length(next.o - cur.o)));
     color = vmul(color, weight(cur));
     prev_d = cur.d;
     cur = next;
