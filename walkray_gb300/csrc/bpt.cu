@@ -169,7 +169,7 @@ __device__ __forceinline__ void warp_append(bool ok, uint2 item, uint2* list, un
 template <int MED>
 __global__ void __launch_bounds__(128) k_bpt_subpaths(RenderScene S, BptParams P) {
     constexpr unsigned FULL = 0xffffffffu;
-    __shared__ uint8_t s_item[BPT_BLOCK / 32][LEAF_ITEMS];
+    __shared__ WarpLeaves s_leaves[BPT_BLOCK / 32];
     extern __shared__ uint32_t s_stack[];
     uint32_t* stack = s_stack + threadIdx.x;
     const int stride = blockDim.x;
@@ -266,7 +266,7 @@ __global__ void __launch_bounds__(128) k_bpt_subpaths(RenderScene S, BptParams P
         }
         // every ray of the turn at one call site
         const Hit h = search_warp(S.tree, has_ray, ray.o, ray.d, P.pf, !(fresh && !light), ray.inside, ray.contact,
-                                  stack, stride, P.stack_cap, s_item[threadIdx.x >> 5]);
+                                  stack, stride, P.stack_cap, s_leaves[threadIdx.x >> 5]);
         if (active && fresh) {  // the sub-path's first record, its hit set
             if (light) {
                 if (has_ray && h.slot >= 0 && h.t > 0.f) set_hit(S, ray, h);  // `if(dist > 0)`
@@ -736,7 +736,7 @@ __device__ __forceinline__ void bpt_connect_edge(const RenderScene& S, const Bpt
 // the eye vertex towards the light vertex; the visible ones join the list of
 // contributing connections.  Persistent: the grid strides over the list.
 __global__ void __launch_bounds__(128) k_bpt_visible(RenderScene S, BptParams P) {
-    __shared__ uint8_t s_item[BPT_BLOCK / 32][LEAF_ITEMS];
+    __shared__ WarpLeaves s_leaves[BPT_BLOCK / 32];
     extern __shared__ uint32_t s_stack[];
     uint32_t* stack = s_stack + threadIdx.x;
     const int stride = blockDim.x;
@@ -754,7 +754,7 @@ __global__ void __launch_bounds__(128) k_bpt_visible(RenderScene S, BptParams P)
             bpt_connect_edge(S, P, c.x, (int)(c.y & 0xffu), (int)(c.y >> 8), lc, ec);
         }
         const Hit h = search_warp(S.tree, i < total, ec.o, ec.d, P.pf, true, ec.inside, ec.contact, stack, stride,
-                                  P.stack_cap, s_item[threadIdx.x >> 5]);
+                                  P.stack_cap, s_leaves[threadIdx.x >> 5]);
         if (i < total) ok = h.slot < 0 || (double)(h.t - length(ec.o - lc.o)) >= -EPS_D;
         warp_append(ok, c, P.vis, P.ncand + 1);
     }

@@ -21,9 +21,9 @@ __global__ void __launch_bounds__(MEGA_BLOCK) k_megakernel(RenderScene S, Render
                                                            float* __restrict__ film2) {
     constexpr unsigned FULL = 0xffffffffu;
     extern __shared__ uint32_t s_stack[];
-    __shared__ uint8_t s_item[MEGA_BLOCK / 32][LEAF_ITEMS];
+    __shared__ WarpLeaves s_leaves[MEGA_BLOCK / 32];
     uint32_t* stack = s_stack + threadIdx.x;
-    uint8_t* item = s_item[threadIdx.x >> 5];
+    WarpLeaves& leaves = s_leaves[threadIdx.x >> 5];
     const int stride = MEGA_BLOCK;
     const uint32_t npix = S.cam.width * S.cam.height;
     const uint32_t pixel = blockIdx.x * MEGA_BLOCK + threadIdx.x;
@@ -54,7 +54,7 @@ __global__ void __launch_bounds__(MEGA_BLOCK) k_megakernel(RenderScene S, Render
             start = false;
         }
         const Hit h = search_warp(S.tree, on, cur.o, cur.d, pf, filtered, cur.inside, cur.contact, stack, stride,
-                                  P.stack_cap, item);
+                                  P.stack_cap, leaves);
         bool done = false, nee_here = false, has_lr = false;
         LightReq lr;
         if (on) {
@@ -69,14 +69,14 @@ __global__ void __launch_bounds__(MEGA_BLOCK) k_megakernel(RenderScene S, Render
         }
         if (MIS && __any_sync(FULL, has_lr)) {  // the light connection of WR_RENDER_NEE_MIS
             const Hit lh = search_warp(S.tree, has_lr, lr.o, lr.d, pf, true, lr.inside, lr.contact, stack, stride,
-                                       P.stack_cap, item);
+                                       P.stack_cap, leaves);
             if (has_lr && light_req_visible(S, lh, lr)) lit = lit + lr.contrib;
         }
         if (__any_sync(FULL, nee_here)) {  // the connection of the NEE branch
             ShadowReq sr;
             const bool conn = nee_here && nee_prepare(S, cur, prev_d, color, g, sr);
             const Hit sh = search_warp(S.tree, conn, sr.o, sr.d, pf, true, sr.inside, sr.contact, stack, stride,
-                                       P.stack_cap, item);
+                                       P.stack_cap, leaves);
             if (conn && nee_visible(sh, sr.dist)) result = sr.contrib;
         }
         if (done) {

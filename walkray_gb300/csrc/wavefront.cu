@@ -492,9 +492,9 @@ __global__ void __launch_bounds__(WF_FINISH_BLOCK, MIS ? 3 : 4)
                 WfJobCounters* __restrict__ counters, WfSide X, unsigned int* __restrict__ next, int stack_cap) {
     constexpr unsigned FULL = 0xffffffffu;
     extern __shared__ __align__(16) uint32_t s_stack[];
-    __shared__ uint8_t s_item[WF_FINISH_BLOCK / 32][LEAF_ITEMS];
+    __shared__ WarpLeaves s_leaves[WF_FINISH_BLOCK / 32];
     uint32_t* stack = s_stack + threadIdx.x;
-    uint8_t* item = s_item[threadIdx.x >> 5];
+    WarpLeaves& leaves = s_leaves[threadIdx.x >> 5];
     const unsigned lane = threadIdx.x & 31u;
     const uint32_t n = X.counts[0] + X.counts[1];
     const uint32_t warps = gridDim.x * (WF_FINISH_BLOCK / 32);
@@ -531,7 +531,7 @@ __global__ void __launch_bounds__(WF_FINISH_BLOCK, MIS ? 3 : 4)
         const float pf = prune_factor(J.flags);
         const bool filtered = p.cur.contact != CAMERA_OBJ;
         const Hit h = search_warp<false>(S.tree, active, p.cur.o, p.cur.d, pf, filtered, p.cur.inside, p.cur.contact,
-                                         stack, WF_FINISH_BLOCK, stack_cap, item);
+                                         stack, WF_FINISH_BLOCK, stack_cap, leaves);
         bool done = false, nee_here = false, has_lr = false;
         f3 result = mk(0, 0, 0);
         LightReq lr;
@@ -547,14 +547,14 @@ __global__ void __launch_bounds__(WF_FINISH_BLOCK, MIS ? 3 : 4)
         }
         if (MIS && __any_sync(FULL, has_lr)) {  // the light connection of WR_RENDER_NEE_MIS
             const Hit lh = search_warp<false>(S.tree, has_lr, lr.o, lr.d, pf, true, lr.inside, lr.contact, stack,
-                                              WF_FINISH_BLOCK, stack_cap, item);
+                                              WF_FINISH_BLOCK, stack_cap, leaves);
             if (has_lr && light_req_visible(S, lh, lr)) p.acc = p.acc + lr.contrib;
         }
         if (__any_sync(FULL, nee_here)) {  // the connection of the NEE branch
             ShadowReq sr;
             const bool conn = nee_here && nee_prepare(S, p.cur, p.prev_d, p.color, g, sr);
             const Hit sh = search_warp<false>(S.tree, conn, sr.o, sr.d, pf, true, sr.inside, sr.contact, stack,
-                                              WF_FINISH_BLOCK, stack_cap, item);
+                                              WF_FINISH_BLOCK, stack_cap, leaves);
             if (nee_here) result = conn && nee_visible(sh, sr.dist) ? sr.contrib : mk(0, 0, 0);
         }
         if (done) {

@@ -468,17 +468,26 @@ __device__ __forceinline__ Hit search_closest(const DevTree& T, f3 o, f3 d, floa
     return settle(T, L.h, o, d, pf, filt, inside, contact);
 }
 
-constexpr int LEAF_ITEMS = 32 * (int)QUAD_LEAF_MAX;  // a warp's triangles in one leaf phase
+// a warp's scratch of a leaf phase, in shared memory
+struct WarpLeaves {
+    float t[32], dd[32];
+    int slot[32];                       // a lane's closest candidate (-1: none)
+    uint8_t item[32 * QUAD_LEAF_MAX];   // triangles: lane | index in its leaf << 5
+};
 
 // Tests the postponed leaves of a warp's lanes (`has`): their triangles are
 // dealt out over all 32 lanes, one each, so that leaves of different lengths do
 // not leave lanes idle (the test in each lane's own loop kept 7 to 14 lanes
 // busy, this 24 to 29; the batch of 2^24 rays 2.69 -> 2.31 ms).  The distance
 // half of the test runs once for the triangles whose edges the rays pass
-// inside, about one in ten.  Every lane of the warp calls it.  `item`: LEAF_ITEMS bytes of shared memory of the warp;
+// inside, about one in ten.  Every lane of the warp calls it.
 // tris_of(tris, l): the triangles of lane l's tree.  Returns this lane's count.
-template <class Ray, class TrisOf>
-__device__ __forceinline__ uint32_t warp_leaves(SearchLane<Ray>& L, bool has, uint8_t* item, const uint32_t* stack,
+// FEW: a pass's candidates, up to so many, are handed back to their rays one by
+// one (25 instructions each), more by groups (60): 3 in the persistent loop
+// (Cornell box 3.95 -> 3.55 ms); where a warp waits for its own rays the groups'
+// longer chain costs more than it saves (megakernel 4.92 -> 5.11 ms).
+template <int FEW, class Ray, class TrisOf>
+__device__ __forceinline__ uint32_t warp_leaves(SearchLane<Ray>& L, bool has, WarpLeaves& W, const uint32_t* stack,
                                                 int stride, TrisOf tris_of) {
     constexpr unsigned FULL = 0xffffffffu;
     const unsigned lane = threadIdx.x & 31u;
@@ -489,13 +498,13 @@ __device__ __forceinline__ uint32_t warp_leaves(SearchLane<Ray>& L, bool has, ui
                    c2 = __ballot_sync(FULL, count & 4u);
     const uint32_t before = __popc(c0 & lt_mask) + 2u * __popc(c1 & lt_mask) + 4u * __popc(c2 & lt_mask);
     const uint32_t total = __popc(c0) + 2u * __popc(c1) + 4u * __popc(c2);
-    for (uint32_t k = 0; k < count; k++) item[before + k] = (uint8_t)(lane | k << 5);
+    for (uint32_t k = 0; k < count; k++) W.item[before + k] = (uint8_t)(lane | k << 5);
     __syncwarp();
     // the edge tests of all; those inside stay in the list
     uint32_t left = 0;
     for (uint32_t base = 0; base < total; base += 32u) {
         const bool on = base + lane < total;
-        const uint32_t it = on ? item[base + lane] : lane;
+        const uint32_t it = on ? W.item[base + lane] : lane;
         const int own = (int)(it & 31u);
         f3 ro, rd;
         L.ray.ray_of(own, ro, rd);
@@ -503,14 +512,14 @@ __device__ __forceinline__ uint32_t warp_leaves(SearchLane<Ray>& L, bool has, ui
         const TriRec* rt = tris_of(own);
         const bool in = on && tri_slot_inside(rt, slot, ro, rd);
         const unsigned im = __ballot_sync(FULL, in);
-        if (in) item[left + __popc(im & lt_mask)] = (uint8_t)it;
+        if (in) W.item[left + __popc(im & lt_mask)] = (uint8_t)it;
         left += __popc(im);
         __syncwarp();
     }
     // the distances of the few that are left
     for (uint32_t base = 0; base < left; base += 32u) {
         const bool on = base + lane < left;
-        const uint32_t it = on ? item[base + lane] : lane;
+        const uint32_t it = on ? W.item[base + lane] : lane;
         const int own = (int)(it & 31u);
         f3 ro, rd;
         L.ray.ray_of(own, ro, rd);
@@ -520,19 +529,48 @@ __device__ __forceinline__ uint32_t warp_leaves(SearchLane<Ray>& L, bool has, ui
         float t = -1.f, dd = 0.f;
         if (on) t = tri_slot_distance(rt, slot, ro, rd, &dd);
         bool cand = t >= 0.f && t <= best;
-        unsigned cm = __ballot_sync(FULL, cand);
-        if (cm) {
+        if (__any_sync(FULL, cand)) {
             bool rf;
             int ri, rc;
             L.ray.ids_of(own, rf, ri, rc);
             if (cand && rf) cand = noself_slot(rt, slot, rd, ri, rc);
-            // the candidates go back to their rays one by one
-            for (cm = __ballot_sync(FULL, cand); cm; cm &= cm - 1u) {
-                const int b = __ffs(cm) - 1;
-                const int bo = __shfl_sync(FULL, own, b), bs = __shfl_sync(FULL, slot, b);
-                const float bt = __shfl_sync(FULL, t, b), bd = __shfl_sync(FULL, dd, b);
-                if ((int)lane == bo) L.take(bt, bs, bd);
+            unsigned cm = __ballot_sync(FULL, cand);
+            if (__popc(cm) <= FEW) {
+                for (; cm; cm &= cm - 1u) {
+                    const int b = __ffs(cm) - 1;
+                    const int bo = __shfl_sync(FULL, own, b), bs = __shfl_sync(FULL, slot, b);
+                    const float bt = __shfl_sync(FULL, t, b), bd = __shfl_sync(FULL, dd, b);
+                    if ((int)lane == bo) L.take(bt, bs, bd);
+                }
+                continue;
             }
+            // A ray's candidates sit on consecutive lanes (at most 7): the
+            // closest is found among them, and the group's first lane hands
+            // it to the ray's own.
+            const int group = on ? own : 32 + (int)lane;
+            float bt = cand ? t : INFINITY, bd = dd;
+            int bs = slot;
+#pragma unroll
+            for (int k = 1; k < 8; k <<= 1) {
+                const float t2 = __shfl_down_sync(FULL, bt, k), d2 = __shfl_down_sync(FULL, bd, k);
+                const int s2 = __shfl_down_sync(FULL, bs, k), g2 = __shfl_down_sync(FULL, group, k);
+                if (lane + k < 32u && g2 == group && (t2 < bt || (t2 == bt && s2 > bs))) {
+                    bt = t2;
+                    bd = d2;
+                    bs = s2;
+                }
+            }
+            const int g0 = __shfl_up_sync(FULL, group, 1);
+            W.slot[lane] = -1;
+            __syncwarp();
+            if (on && (lane == 0 || g0 != group) && bt < INFINITY) {
+                W.t[own] = bt;
+                W.dd[own] = bd;
+                W.slot[own] = bs;
+            }
+            __syncwarp();
+            if (W.slot[lane] >= 0) L.take(W.t[lane], W.slot[lane], W.dd[lane]);
+            __syncwarp();
         }
     }
     if (has) L.leaf_done(stack, stride);
@@ -544,7 +582,7 @@ __device__ __forceinline__ uint32_t warp_leaves(SearchLane<Ray>& L, bool has, ui
 // warp calls it.  ONE_TREE: all rays in the tree T (else each lane's own T).
 template <bool ONE_TREE = true>
 __device__ __forceinline__ Hit search_warp(const DevTree& T, bool on, f3 o, f3 d, float pf, bool filt, int inside,
-                                           int contact, uint32_t* stack, int stride, int cap, uint8_t* item) {
+                                           int contact, uint32_t* stack, int stride, int cap, WarpLeaves& leaves) {
     constexpr unsigned FULL = 0xffffffffu;
     SearchLane<RayInRegs> L;
     L.clear();
@@ -555,7 +593,7 @@ __device__ __forceinline__ Hit search_warp(const DevTree& T, bool on, f3 o, f3 d
         const unsigned wm = __ballot_sync(FULL, walking), lm = __ballot_sync(FULL, L.at_leaf());
         if (!(wm | lm)) break;
         if (lm && (wm == 0 || __popc(lm) >= 8)) {
-            warp_leaves(L, L.pend != NO_WORD, item, stack, stride,
+            warp_leaves<32>(L, L.pend != NO_WORD, leaves, stack, stride,
                         [&](int from) { return ONE_TREE ? T.tris : L.ray.tris_of(from); });
         } else if (walking) {
             for (int k = 0; k < 6 && L.walking(); k++) L.visit(stack, stride, top);

@@ -40,7 +40,7 @@ struct WarpQueues {
     int slot[64];
     float t[64];
     float ray[RAY_WORDS * 32];  // the lanes' rays (RayInShared)
-    uint8_t item[LEAF_ITEMS];  // the leaf phase's triangles: lane | index in its leaf << 5
+    WarpLeaves leaves;
 };
 // this thread's work counts (profiling launches)
 struct TraceWork {
@@ -154,7 +154,7 @@ __device__ __forceinline__ void quad_trace(Src& src, uint32_t n, unsigned int* c
         if (lm && (wm == 0 || __popc(lm) >= tune.leaf_min)) {
             // every postponed leaf, those of lanes still walking too
             const uint32_t tested =
-                warp_leaves(L, active && L.pend != NO_WORD, Q.item, stack, stride,
+                warp_leaves<3>(L, active && L.pend != NO_WORD, Q.leaves, stack, stride,
                             [&](int from) { return src.tris_of(L.ray, from); });
             if (STATS) work.tris += tested;
         } else if (walking) {
