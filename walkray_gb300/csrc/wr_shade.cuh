@@ -906,7 +906,9 @@ static __device__ __forceinline__ PRay scatter(const RenderScene& S, int self, c
     PRay cur = in;
     float oP_scale = 1.f;
     int medium_hit = -1;  // the object a medium handed over to (photonType, homogeneousVolume.cpp:192-194)
-    for (int hop = 0; hop < 4; hop++) {
+    // (self < 0: handed over to a hit that is not there, a path that leaves an open or
+    // leaking object unseen; it ends)
+    for (int hop = 0; hop < 4 && self >= 0; hop++) {
         const uint32_t type = obj_type(S, self);
         bool del = false;
         float ps = 1.f;
