@@ -123,6 +123,7 @@ __global__ void k_wf_reset(WfSide Y, unsigned long long* work, unsigned int* sha
     Y.counts[1] = 0;
     work[0] = 0;  // the extend stage's ray counter
     work[1] = 0;  // the shadow stage's
+    work[2] = 0;  // the track stage's
     *shadow_count = 0;
     for (int k = 0; k < WF_SORT_KEYS; k++) B.counts[k] = 0;
 }
@@ -140,8 +141,8 @@ __global__ void __launch_bounds__(256) k_wf_sort(const RenderScene* __restrict__
         int key = 0;
         if (valid) {
             const int slot = hits[i].x;
-            if (slot >= 0) {
-                const int4 ids = as_i4(X.rec[(size_t)WF_REC * i + (WF_IDS ^ wf_swizzle(i))]);
+            const int4 ids = as_i4(X.rec[(size_t)WF_REC * i + (WF_IDS ^ wf_swizzle(i))]);
+            if (slot >= 0 || ids.x >= 0) {
                 const RenderScene& S = scenes[jobs[ids.z].scene];
                 const int self = ids.x >= 0 ? ids.x : (int)__float_as_uint(__ldg(&S.tree.tris[slot].v1.w));
                 key = 1 + (int)obj_type(S, self);
@@ -156,6 +157,94 @@ __global__ void __launch_bounds__(256) k_wf_sort(const RenderScene* __restrict__
             if ((int)lane == leader) b = atomicAdd(&B.counts[key], (unsigned)__popc(peers));
             b = __shfl_sync(peers, b, leader);
             B.idx[(size_t)key * capacity + b + __popc(peers & ((1u << lane) - 1u))] = i;
+        }
+    }
+}
+
+// track: the flights of the paths inside heterogeneous media (the bucket of
+// that material), delta tracking with lanes that take the next path when
+// theirs ends.  A step waits for eight grid reads and a logarithm; in the shade
+// stage the longest flight of 32 held the others up, at half of this kernel's
+// warps and behind an instruction cache full of materials (media scene
+// 18.8 ms, 17.4 this way).  Launched only while a scene has such a medium.
+// Refilled at 8 idle lanes, runs of at most 256 paths and a quarter of a warp's
+// share, so that the last warps end together.
+constexpr int WF_TRACK_BLOCK = 128;
+__global__ void __launch_bounds__(WF_TRACK_BLOCK, 7)
+    k_wf_track(const RenderScene* __restrict__ scenes, const WfJob* __restrict__ jobs, WfSide X,
+               const int2* __restrict__ hits, WfSort B, uint32_t capacity, Flight* __restrict__ flights,
+               unsigned int* __restrict__ counter) {
+    constexpr unsigned FULL = 0xffffffffu;
+    constexpr int KEY = 1 + WR_MAT_HETEROGENEOUS;
+    const unsigned lane = threadIdx.x & 31u;
+    const uint32_t n = B.counts[KEY];
+    const uint32_t warps = gridDim.x * (WF_TRACK_BLOCK / 32);
+    const uint32_t run = min(256u, max(1u, n / (warps * 4u)));
+    const uint32_t* __restrict__ idx = B.idx + (size_t)KEY * capacity;
+    uint32_t next = 0, end = 0;
+    bool dry = false, active = false;
+    uint32_t i = 0;
+    int steps = 0;
+    f3 o = mk(0, 0, 0), d = mk(0, 0, 0);
+    float far = 0.f, scale = 0.f, mu = 0.f, sgt = 0.f;
+    GridDev G{};
+    PathRng g;
+    g.init(0, 0, 0);
+    Flight f{0.f, 0.f, 0, 0u};
+    for (;;) {
+        unsigned idle = __ballot_sync(FULL, !active);
+        while (!dry && (idle == FULL || __popc(idle) >= 8)) {
+            if (next == end) {
+                uint32_t b = 0;
+                if (lane == 0) b = atomicAdd(counter, run);
+                next = __shfl_sync(FULL, b, 0);
+                if (next >= n) {
+                    dry = true;
+                    break;
+                }
+                end = min(next + run, n);
+            }
+            const uint32_t k = next + __popc(idle & ((1u << lane) - 1u));
+            if (!active && k < end) {
+                i = idx[k];
+                const float4* r = X.rec + (size_t)WF_REC * i;
+                const uint32_t x = wf_swizzle(i);
+                const int4 ids = as_i4(r[WF_IDS ^ x]);
+                if (ids.x >= 0) {  // inside the medium (else the path enters it)
+                    const float4 a0 = r[WF_O ^ x], a1 = r[WF_D ^ x];
+                    const int4 misc = as_i4(r[WF_MISC ^ x]);
+                    const WfJob& J = jobs[ids.z];
+                    const RenderScene& S = scenes[J.scene];
+                    const wr_object_desc* m = &S.objs[ids.x];
+                    G = S.grids[__ldg(&m->grid_index)];
+                    scale = __ldg(&m->density_scale);
+                    sgt = __ldg(&m->sigma_s[0]) + __ldg(&m->sigma_a[0]);
+                    mu = G.majorant * scale * sgt;
+                    o = mk(a0.x, a0.y, a0.z);
+                    d = mk(a1.x, a1.y, a1.z);
+                    const int2 hv = hits[i];
+                    far = hv.x < 0 ? -1.f : __int_as_float(hv.y);  // as set_hit has it
+                    g.init(J.seed, (uint32_t)ids.w, (uint32_t)misc.x, (uint32_t)misc.y);
+                    f = Flight{0.f, 0.f, 0, 0u};
+                    steps = mu > 0.f ? 0 : TRACK_STEPS;
+                    active = true;
+                }
+            }
+            next = min(next + (uint32_t)__popc(idle), end);
+            idle = __ballot_sync(FULL, !active);
+        }
+        if (idle == FULL) break;
+        if (active) {
+            bool done = steps >= TRACK_STEPS;
+            if (!done) {
+                done = track_step(G, scale, mu, sgt, o, d, far, g, f);
+                steps++;
+            }
+            if (done) {
+                f.dim = g.dim;
+                flights[i] = f;
+                active = false;
+            }
         }
     }
 }
@@ -370,14 +459,14 @@ static ExtendKernel extend_kernel(int ctas_per_sm, bool stats, bool exact) {
 
 // shade: one bounce per path; survivors compacted into Y, finished paths to
 // the film.  MIS: compiled with the WR_RENDER_NEE_MIS code (launched while a
-// job with that flag is in the table).  MED: MED_TRACK while a scene with
+// job with that flag is in the table).  MED: MED_FLIGHT while a scene with
 // participating media is.
 template <bool MIS, int MED>
 __global__ void __launch_bounds__(128, 4) k_wf_shade(const RenderScene* __restrict__ scenes,
                                                     const WfJob* __restrict__ jobs,
                                                     WfJobCounters* __restrict__ counters, WfSide X,
                                                     const int2* __restrict__ hits, WfSide Y, WfShadow Q, WfSort B,
-                                                    uint32_t capacity) {
+                                                    uint32_t capacity, const Flight* __restrict__ flights) {
     __shared__ uint32_t s_first[WF_SORT_KEYS + 1];  // first queue position of each bucket
     if (threadIdx.x == 0) {
         uint32_t a = 0;
@@ -425,7 +514,7 @@ __global__ void __launch_bounds__(128, 4) k_wf_shade(const RenderScene* __restri
             } else {
                 set_hit(S, p.cur, h);
                 done = path_advance<MIS, MED>(S, p.cur, p.color, p.prev_d, p.depth, p.st, g, J.max_path_len, J.flags,
-                                         result, nee_here, p.mis_pdf, lr, has_lr);
+                                              result, nee_here, p.mis_pdf, lr, has_lr, flights + i);
             }
             if (nee_here) shadow = nee_prepare(S, p.cur, p.prev_d, p.color, g, sr);
             p.dim = g.dim;
@@ -474,7 +563,7 @@ __global__ void __launch_bounds__(128, 4) k_wf_shade(const RenderScene* __restri
 }
 
 static auto shade_kernel(bool mis, bool media) {
-    if (media) return mis ? k_wf_shade<true, MED_TRACK> : k_wf_shade<false, MED_TRACK>;
+    if (media) return mis ? k_wf_shade<true, MED_FLIGHT> : k_wf_shade<false, MED_FLIGHT>;
     return mis ? k_wf_shade<true, MED_NONE> : k_wf_shade<false, MED_NONE>;
 }
 
@@ -752,7 +841,7 @@ __global__ void __launch_bounds__(WF_GEN_ROWS) k_wf_generate(const WfJob* __rest
 // ---------------------------------------------------------------------------
 struct WfEngine {
     WfConfig cfg;
-    DeviceBuffer side_mem[2], hits, scenes, jobs, order, counters, work, err_word, shadow_mem, sort_mem, plan_mem;
+    DeviceBuffer side_mem[2], hits, flights, scenes, jobs, order, counters, work, err_word, shadow_mem, sort_mem, plan_mem;
     WfSide side[2];
     CUtensorMap rec_map[2];  // each side's records as a 2-D tensor (k_wf_generate's bulk stores)
     WfPlan plan{};
@@ -761,7 +850,7 @@ struct WfEngine {
     uint32_t live_cap_host = 0;
     WfShadow shadow{};
     WfSort sort{};
-    int grid_sort = 0;
+    int grid_sort = 0, grid_track = 0;
     int grid_shadow = 0;
     std::vector<const RenderData*> scene_of;  // host mirror of the scene table
     std::vector<RenderScene> scene_tab;
@@ -774,10 +863,11 @@ struct WfEngine {
     cudaGraphExec_t graph = nullptr;
     int graph_stack = -1;
     bool mis_any = false;  // a job in the table has WR_RENDER_NEE_MIS: the shade stage with that code
+    bool hetero_any = false;  // a job's scene has a heterogeneous medium: the track stage
     bool media_any = false;  // a job's scene has participating media: the shading kernels with that code
     bool exact_any = false;  // a job in the table has WR_RENDER_EXACT_TRAVERSAL: the extend stage of that walk
     bool conn_any = true;  // a job in the table connects to lights (NEE or MIS): the shadow stage is in the loop
-    int launches_per_iteration() const { return conn_any ? 8 : 6; }
+    int launches_per_iteration() const { return (conn_any ? 8 : 6) + (hetero_any ? 1 : 0); }
     WfJobCounters* host_counters = nullptr;  // pinned
     WfStatus* status = nullptr;              // pinned and mapped: written by k_wf_plan
     cudaEvent_t turn[2] = {};                // the end of the last two graph replays of a render
@@ -856,11 +946,13 @@ int wf_engine_get(wr_ctx* ctx, const WfConfig& cfg, WfEngine** out) {
         if (rc != WR_OK) return rc;
     }
     WR_CUDA(ctx, E->hits.reserve(sizeof(int2) * (size_t)cfg.capacity));
+    WR_CUDA(ctx, E->flights.reserve(sizeof(Flight) * (size_t)cfg.capacity));
     WR_CUDA(ctx, E->sort_mem.reserve(sizeof(uint32_t) * ((size_t)WF_SORT_KEYS * cfg.capacity + 64)));
     E->sort.counts = E->sort_mem.as<unsigned int>();
     E->sort.idx = E->sort.counts + 64;
     WR_CUDA(ctx, cudaMemset(E->sort.counts, 0, sizeof(unsigned int) * WF_SORT_KEYS));
     E->grid_sort = ctx->num_sms * 4;
+    E->grid_track = ctx->num_sms * 7;
     {
         const size_t Q = cfg.capacity;
         WR_CUDA(ctx, E->shadow_mem.reserve(Q * (4 * sizeof(float4) + sizeof(int4)) + 256));
@@ -886,7 +978,7 @@ int wf_engine_get(wr_ctx* ctx, const WfConfig& cfg, WfEngine** out) {
     E->plan.n = reinterpret_cast<int*>(E->plan.off + WF_MAX_JOBS + 1);
     WR_CUDA(ctx, E->counters.reserve(sizeof(WfJobCounters) * WF_MAX_JOBS));
     WR_CUDA(ctx, cudaMemset(E->counters.p, 0, sizeof(WfJobCounters) * WF_MAX_JOBS));
-    WR_CUDA(ctx, E->work.reserve(2 * sizeof(unsigned long long)));
+    WR_CUDA(ctx, E->work.reserve(3 * sizeof(unsigned long long)));
     WR_CUDA(ctx, E->err_word.reserve(sizeof(unsigned int)));
     WR_CUDA(ctx, E->live_cap.reserve(sizeof(uint32_t)));
     E->live_cap_host = cfg.capacity;
@@ -1006,16 +1098,20 @@ int wf_update_jobs(wr_ctx* ctx, WfEngine* E, const std::vector<WfSlotUpdate>& up
     }
     // the shade stage compiled with the light-connection code only while a job needs it
     // and the shadow stage only while a job can queue a connection
-    bool mis_any = false, conn_any = false, exact_any = false, media_any = false;
+    bool mis_any = false, conn_any = false, exact_any = false, media_any = false, hetero_any = false;
     for (int slot : order) {
         if (!E->job_tab[slot].active) continue;
         if (E->job_tab[slot].flags & WR_RENDER_NEE_MIS) mis_any = true;
         if (E->job_tab[slot].flags & WR_RENDER_EXACT_TRAVERSAL) exact_any = true;
-        if (const RenderData* rd = E->scene_of[E->job_tab[slot].scene]) media_any |= RenderDataView::media(rd);
+        if (const RenderData* rd = E->scene_of[E->job_tab[slot].scene]) {
+            media_any |= RenderDataView::media(rd);
+            hetero_any |= RenderDataView::hetero(rd);
+        }
         if (E->job_tab[slot].flags & (WR_RENDER_NEE | WR_RENDER_NEE_MIS)) conn_any = true;
     }
     if (mis_any != E->mis_any || conn_any != E->conn_any || exact_any != E->exact_any ||
-        media_any != E->media_any) {
+        media_any != E->media_any || hetero_any != E->hetero_any) {
+        E->hetero_any = hetero_any;
         E->exact_any = exact_any;
         E->media_any = media_any;
         E->mis_any = mis_any;
@@ -1050,8 +1146,13 @@ static void enqueue_iteration(WfEngine* E, int x, cudaStream_t s, cudaEvent_t* e
             E->exact_any ? E->stack_cap : E->quad_cap, E->cfg.trace, E->err_word.as<unsigned int>(), stats);
     if (ev) cudaEventRecord(ev[1], s);
     k_wf_sort<<<E->grid_sort, 256, 0, s>>>(scenes, jobs, E->side[x], E->hits.as<int2>(), E->sort, E->cfg.capacity);
+    if (E->hetero_any)
+        k_wf_track<<<E->grid_track, WF_TRACK_BLOCK, 0, s>>>(scenes, jobs, E->side[x], E->hits.as<int2>(), E->sort,
+                                                            E->cfg.capacity, E->flights.as<Flight>(),
+                                                            E->work.as<unsigned int>() + 4);
     shade_kernel(E->mis_any, E->media_any)<<<E->grid_shade, E->cfg.shade_block, 0, s>>>(scenes, jobs, cnt, E->side[x], E->hits.as<int2>(),
-                                                            E->side[y], E->shadow, E->sort, E->cfg.capacity);
+                                                            E->side[y], E->shadow, E->sort, E->cfg.capacity,
+                                                            E->flights.as<Flight>());
     if (ev) cudaEventRecord(ev[2], s);
     if (E->conn_any) {  // the connections' closest hits go into E->hits, which shade has read
         shadow_trace_kernel(E->cfg.ctas_per_sm)<<<E->grid_extend, E->cfg.extend_block, E->smem_extend, s>>>(
@@ -1195,7 +1296,7 @@ int wf_launch(wr_ctx* ctx, WfEngine* E, cudaStream_t s) {
         E->graph_stack = caps;
     }
     WR_CUDA(ctx, cudaGraphLaunch(E->graph, s));
-    // reset, extend, sort, shade, [shadow trace, shadow,] plan, generate
+    // reset, extend, sort, [track,] shade, [shadow trace, shadow,] plan, generate
     ctx->kernel_launches += (uint64_t)E->launches_per_iteration() * 2 * E->cfg.iters_per_graph;
     return WR_OK;
 }

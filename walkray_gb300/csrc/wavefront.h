@@ -4,6 +4,8 @@
 //   extend    persistent warps trace every queued ray (closest hit, the same
 //             bit-exact traversal as k_trace_closest)
 //   sort      buckets the queue by the material each ray hit
+//   track     flights through heterogeneous media (only while a job's scene
+//             has one)
 //   shade     one bounce of the reference loop per path (scatter, throughput,
 //             termination) in bucket order; survivors are compacted into the
 //             other state buffer with warp-aggregated appends, finished
@@ -16,7 +18,7 @@
 //   generate  refills free queue slots with camera paths of the jobs as
 //             planned (continuous batching)
 //
-// The [reset, extend, sort, shade, shadow trace, shadow, plan, generate] x 2
+// The [reset, extend, sort, track, shade, shadow trace, shadow, plan, generate] x 2
 // sequence (one per ping-pong side; the two shadow kernels only while a job
 // in the table connects to lights) is captured once into a CUDA graph and
 // replayed until every job is done; kernel sizes never depend on host-side
@@ -89,7 +91,7 @@ struct WfSide {
 };
 
 // the extend stage's queue bucketed by the material that shades each path
-// (0 = no hit, 1 + WR_MAT_* of the inside or hit object), so that the shade
+// (1 + WR_MAT_* of the inside or hit object, 0 without either), so that the shade
 // stage runs one material's code per warp
 constexpr int WF_SORT_KEYS = 9;
 struct WfSort {

@@ -219,6 +219,11 @@ struct PathRng {
         dim = d0;
         cached_block = 0xffffffffu;
     }
+    // the next draw is number `d`
+    __host__ __device__ __forceinline__ void skip_to(uint32_t d) {
+        if (d >> 2 != cached_block) cached_block = 0xffffffffu;
+        dim = d;
+    }
     __host__ __device__ __forceinline__ float next() {
         uint32_t blk = dim >> 2;
         if (blk != cached_block) {

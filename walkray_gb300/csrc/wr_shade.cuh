@@ -174,7 +174,16 @@ struct InsideStack {
 enum : int {
     MED_NONE = 0,   // no participating media
     MED_TRACK = 1,  // heterogeneous media by delta tracking
-    MED_REF = 2     // heterogeneous media by the reference's own sampler
+    MED_REF = 2,    // heterogeneous media by the reference's own sampler
+    MED_FLIGHT = 3  // the flights through heterogeneous media are given (k_wf_track)
+};
+
+// a flight through a heterogeneous medium: the collision, or past `far` without
+// one, and the path's next draw
+struct Flight {
+    float t, dens;
+    int collided;
+    uint32_t dim;
 };
 
 // Ray::cosineTerm (ray.cpp:52-58)
@@ -673,13 +682,30 @@ __device__ __forceinline__ PRay scatter_homogeneous(const RenderScene& S, int se
     return ray_default();
 }
 
+// One step of delta tracking (Woodcock) against the grid's majorant mu: true
+// when the flight ends, by a collision (f.collided) or beyond `far`.
+__device__ __forceinline__ bool track_step(const GridDev& G, float scale, float mu, float sgt, f3 o, f3 d, float far,
+                                           PathRng& g, Flight& f) {
+    f.t += -logf(1.f - g.next()) / mu;
+    if (f.t >= far) return true;
+    f.dens = grid_density(G, o + d * f.t, scale);
+    if (g.next() * mu < sgt * f.dens) {
+        f.collided = 1;
+        return true;
+    }
+    return false;
+}
+constexpr int TRACK_STEPS = 1 << 16;  // bound of a flight; the expected count is mu * distance
+
 // HeterogeneousVolume::scatter (HeterogeneousVolume.cpp:449-641) with delta
-// tracking (Woodcock) against the grid's majorant in place of Simpson +
-// Newton inversion.  For a grey sigma_t the reference's throughput weights
-// reduce to 1 per free flight; this keeps the same product with
-// oP = sigma_t * density at a collision and 1 on passing.
+// tracking in place of Simpson + Newton inversion.  For a grey sigma_t the
+// reference's throughput weights reduce to 1 per free flight; this keeps the
+// same product with oP = sigma_t * density at a collision and 1 on passing.
+// MED_FLIGHT: the flight is `known` (a path inside the medium always has one).
+template <int MED>
 __device__ __forceinline__ PRay scatter_heterogeneous(const RenderScene& S, int self, const PRay& in, PathRng& g,
-                                                      InsideStack& st, bool* delegate, float* psurf) {
+                                                      InsideStack& st, bool* delegate, float* psurf,
+                                                      const Flight* known) {
     const wr_object_desc* m = &S.objs[self];
     *delegate = false;
     const bool go_in = in.iobj == self && in.inside != self;
@@ -687,23 +713,20 @@ __device__ __forceinline__ PRay scatter_heterogeneous(const RenderScene& S, int 
     if (go_in) return medium_enter(S, self, in, g);
     const f3 ss = ld3(m->sigma_s), st_ = ss + ld3(m->sigma_a);
     const float sgt = st_.x;  // grey extinction (checked at upload)
-    const GridDev G = S.grids[__ldg(&m->grid_index)];
-    const float scale = __ldg(&m->density_scale);
-    const float mu = G.majorant * scale * sgt;
-    float t = 0.f;
-    bool collided = false;
-    float dens = 0.f;
-    if (mu > 0.f) {
-        for (int it = 0; it < 1 << 16; it++) {  // bounded: the expected count is mu * distance
-            t += -logf(1.f - g.next()) / mu;
-            if (t >= in.idist) break;
-            dens = grid_density(G, in.o + in.d * t, scale);
-            if (g.next() * mu < sgt * dens) {
-                collided = true;
-                break;
-            }
-        }
+    Flight f{0.f, 0.f, 0, 0u};
+    if constexpr (MED == MED_FLIGHT) {
+        f = *known;
+        g.skip_to(f.dim);
+    } else {
+        const GridDev G = S.grids[__ldg(&m->grid_index)];
+        const float scale = __ldg(&m->density_scale);
+        const float mu = G.majorant * scale * sgt;
+        if (mu > 0.f)
+            for (int it = 0; it < TRACK_STEPS; it++)
+                if (track_step(G, scale, mu, sgt, in.o, in.d, in.idist, g, f)) break;
     }
+    const float t = f.t, dens = f.dens;
+    const bool collided = f.collided != 0;
     if (be_in && collided) {
         PRay out = ray_default();
         out.o = in.o + in.d * t;
@@ -902,7 +925,8 @@ static __device__ __noinline__ PRay scatter_heterogeneous_ref(const RenderScene&
 // inside it to the hit object; media handing over to the surface hit).
 template <int MED = MED_TRACK>
 static __device__ __forceinline__ PRay scatter(const RenderScene& S, int self, const PRay& in, PathRng& g,
-                                            InsideStack& st, bool mirror = false) {
+                                            InsideStack& st, bool mirror = false,
+                                            const Flight* flight = nullptr) {
     PRay cur = in;
     float oP_scale = 1.f;
     int medium_hit = -1;  // the object a medium handed over to (photonType, homogeneousVolume.cpp:192-194)
@@ -932,7 +956,8 @@ static __device__ __forceinline__ PRay scatter(const RenderScene& S, int self, c
                 break;
             default:
                 if constexpr (MED == MED_REF) out = scatter_heterogeneous_ref(S, self, cur, g, st, &del, &ps);
-                else if constexpr (MED == MED_TRACK) out = scatter_heterogeneous(S, self, cur, g, st, &del, &ps);
+                else if constexpr (MED != MED_NONE)
+                    out = scatter_heterogeneous<MED>(S, self, cur, g, st, &del, &ps, flight);
                 else out = ray_default();
                 break;
         }
@@ -1317,7 +1342,7 @@ template <bool MIS_CODE, int MED>
 __device__ __forceinline__ bool path_advance(const RenderScene& S, PRay& cur, f3& color, f3& prev_d,
                                              uint32_t& depth, InsideStack& st, PathRng& g, uint32_t max_path_len,
                                              uint32_t flags, f3& result, bool& nee_here, float& mis_pdf,
-                                             LightReq& lr, bool& has_lr) {
+                                             LightReq& lr, bool& has_lr, const Flight* flight = nullptr) {
     nee_here = false;
     has_lr = false;
     const bool nee = (flags & WR_RENDER_NEE) != 0;
@@ -1336,7 +1361,7 @@ __device__ __forceinline__ bool path_advance(const RenderScene& S, PRay& cur, f3
         const f3 T = vmul(color * cos_term<MED>(S, cur), weight(cur));
         has_lr = mis_light_request(S, self, cur, T, g, mirror, lr);
     }
-    PRay next = scatter<MED>(S, self, cur, g, st, mirror);
+    PRay next = scatter<MED>(S, self, cur, g, st, mirror, flight);
     if (length(next.d) < 0.5f) {
         const bool zero = next.rad.x == 0.f && next.rad.y == 0.f && next.rad.z == 0.f;
         if (nee && zero) {
