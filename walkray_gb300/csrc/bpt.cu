@@ -109,10 +109,12 @@ struct BptParams {
     VtxStore eye, light;
     uint32_t* counts;     // per sample: eye records | light records << 8 (bytes 0 and 1, little-endian)
     float* film;          // per sample slot of the batch: npix * 3 floats
-    uint2* cand;          // connection candidates with a light sub-path (l >= 1): {sample, l | e << 8}
-    uint2* vis;           // connections that contribute: visible candidates and whole eye paths
-    unsigned long long* ncand;  // [0]: entries of cand, [1]: entries of vis, [2]: light points, [3]: merges,
-                                // [4]: sub-paths handed out
+    // one list per (light length, eye length) pair, pair_of's p-th at p * nsamp: samples
+    uint32_t* cand;       // connection candidates with a light sub-path (l >= 1)
+    uint32_t* vis;        // connections that contribute: visible candidates and whole eye paths
+    uint32_t npairs;
+    uint32_t* npair;      // entries of each cand list, then of each vis list, PAIR_WORDS apart
+    unsigned long long* ncand;  // [2]: light points, [3]: merges, [4]: sub-paths handed out
     // vertex merging (WR_MODE_VCM); per sample slot s of the batch, the hash grid of hashgrid.hxx
     bool vcm;
     const float* radii;   // merge radius of each slot's iteration
@@ -144,16 +146,66 @@ __device__ __forceinline__ MisKind mis_kind(const BptParams& P, uint32_t sid, bo
 
 // appends `item` for the lanes with `ok` at consecutive places of list[*count++]
 // (one atomic per warp); every lane of the warp must call it
-__device__ __forceinline__ void warp_append(bool ok, uint2 item, uint2* list, unsigned long long* count) {
+template <class Item, class Count>
+__device__ __forceinline__ void warp_append(bool ok, Item item, Item* list, Count* count) {
     constexpr unsigned FULL = 0xffffffffu;
     const unsigned lane = threadIdx.x & 31u;
     const unsigned want = __ballot_sync(FULL, ok);
     if (!want) return;
     const int leader = __ffs(want) - 1;
-    unsigned long long base = 0;
-    if ((int)lane == leader) base = atomicAdd(count, (unsigned long long)__popc(want));
+    Count base = 0;
+    if ((int)lane == leader) base = atomicAdd(count, (Count)__popc(want));
     base = __shfl_sync(FULL, base, leader);
     if (ok) list[base + __popc(want & ((1u << lane) - 1u))] = item;
+}
+
+// Connections are listed by pair of light length l and eye length e, so that a
+// warp works on 32 paths of one shape: the same loop lengths, the same vertex
+// of the same sub-path, neighbouring samples' records (k_bpt_connect).  The
+// counters are 32 bytes apart: the warps that added to one counter queued up
+// for it (k_bpt_enum 0.31 -> 0.16 ms a batch).
+constexpr int BPT_MAX_PAIRS = BPT_MAX_RECORDS * (BPT_MAX_RECORDS + 1);
+constexpr uint32_t PAIR_WORDS = 8;
+__device__ __forceinline__ uint32_t pair_at(const BptParams& P, int l, int e) {
+    return (uint32_t)(e - 1) * (P.max_path_len + 3u) + (uint32_t)l;
+}
+__device__ __forceinline__ void pair_of(const BptParams& P, uint32_t p, int& l, int& e) {
+    e = (int)(p / (P.max_path_len + 3u)) + 1;
+    l = (int)(p % (P.max_path_len + 3u));
+}
+// first[p]: a list's first run of 32 in the order of all lists' runs; returns
+// the number of runs.  The whole block calls it.
+__device__ __forceinline__ uint32_t pair_runs(const uint32_t* counts, uint32_t npairs, uint32_t* first) {
+    constexpr unsigned FULL = 0xffffffffu;
+    if (threadIdx.x < 32) {
+        const uint32_t lane = threadIdx.x;
+        uint32_t before = 0;
+        for (uint32_t base = 0; base < npairs; base += 32) {
+            const uint32_t n = base + lane < npairs ? counts[(base + lane) * PAIR_WORDS] : 0u;
+            const uint32_t runs = n / 32u + (n % 32u != 0u);
+            uint32_t sum = runs;
+#pragma unroll
+            for (uint32_t k = 1; k < 32; k <<= 1) {
+                const uint32_t x = __shfl_up_sync(FULL, sum, k);
+                if (lane >= k) sum += x;
+            }
+            if (base + lane < npairs) first[base + lane] = before + sum - runs;
+            before += __shfl_sync(FULL, sum, 31);
+        }
+        if (lane == 0) first[npairs] = before;
+    }
+    __syncthreads();
+    return first[npairs];
+}
+// the list that run r is of
+__device__ __forceinline__ uint32_t pair_of_run(const uint32_t* first, uint32_t npairs, uint32_t r) {
+    uint32_t a = 0, b = npairs;  // first[a] <= r < first[b]
+    while (b - a > 1) {
+        const uint32_t m = (a + b) / 2;
+        if (first[m] <= r) a = m;
+        else b = m;
+    }
+    return a;
 }
 
 // Persistent: each lane takes sub-paths from a counter (eye sub-paths of
@@ -165,9 +217,11 @@ __device__ __forceinline__ void warp_append(bool ok, uint2 item, uint2* list, un
 // traces it at one call site (the first ray of a sub-path too: the camera
 // ray unfiltered (camera.cpp:52), which a filter with no inside and no
 // contact object is, the emitted ray with NoSelfCondition).
-// MED: what scatter() is compiled for (wr_shade.cuh)
+// MED: what scatter() is compiled for (wr_shade.cuh).  Four blocks per SM (128
+// registers) where it has no media code: bidirectional Cornell box 9.15 -> 9.00
+// ms, 9.33 with five.
 template <int MED>
-__global__ void __launch_bounds__(128) k_bpt_subpaths(RenderScene S, BptParams P) {
+__global__ void __launch_bounds__(128, MED == MED_NONE ? 4 : 1) k_bpt_subpaths(RenderScene S, BptParams P) {
     constexpr unsigned FULL = 0xffffffffu;
     __shared__ WarpLeaves s_leaves[BPT_BLOCK / 32];
     extern __shared__ uint32_t s_stack[];
@@ -299,10 +353,35 @@ __global__ void __launch_bounds__(128) k_bpt_subpaths(RenderScene S, BptParams P
 // ---------------------------------------------------------------------------
 // the connection step
 // ---------------------------------------------------------------------------
+// The reference mixes floats and doubles here.  The FP64 unit does some two
+// operations per SM and clock, conversions and comparisons included, so what
+// has one result either way is done without it: a / b, a + b, a - b of floats
+// rounded to double and then to float is the float operation (53 >= 2 * 24 + 2
+// bits), and 1e-5f is the largest float below 1e-5.  The sums and products
+// that the reference keeps in double stay so.
+__device__ __forceinline__ float max_eps(float a) { return a > EPS_F ? a : EPS_F; }
+// x / pi of a double product rounded to float: the constant in two floats (the
+// same result for every 24-bit significand)
+constexpr float OVER_PI_HI = (float)INV_PI_D, OVER_PI_LO = (float)(INV_PI_D - (double)OVER_PI_HI);
+__device__ __forceinline__ float over_pi(float x) {
+    const float p = __fmul_rn(x, OVER_PI_HI);
+    return __fadd_rn(p, __fmaf_rn(x, OVER_PI_LO, __fmaf_rn(x, OVER_PI_HI, -p)));
+}
+// (power + 1) * c / (2 pi), to some 46 bits before the last rounding
+__device__ __forceinline__ float lobe_density(float power, float c) {
+    const float a = __fadd_rn(power, 1.f), b = __fsub_rn(a, power);
+    const float al = __fadd_rn(__fsub_rn(power, __fsub_rn(a, b)), __fsub_rn(1.f, b));  // a + al = power + 1
+    const float p = __fmul_rn(a, c), pl = __fmaf_rn(al, c, __fmaf_rn(a, c, -p));
+    const float h = 0.5f * OVER_PI_HI, l = 0.5f * OVER_PI_LO;
+    const float q = __fmul_rn(p, h);
+    return __fadd_rn(q, __fadd_rn(__fmaf_rn(p, h, -q), __fmaf_rn(p, l, __fmul_rn(pl, h))));
+}
+
 // Camera::getPixelSolidAngle (camera.cpp:125-131)
 __device__ __forceinline__ float pixel_solid_angle(const CamParams& C, uint32_t pid) {
     const uint32_t x = pid % C.width, y = pid / C.width;
-    const float xc = (float)((double)x + 0.5 - (C.width / 2.0)), yc = (float)((C.height / 2.0) - 0.5 - (double)y);
+    // x + 0.5 - width / 2 and height / 2 - 0.5 - y, whole multiples of a half
+    const float xc = (float)(int)(2u * x + 1u - C.width) * 0.5f, yc = (float)(int)(C.height - 1u - 2u * y) * 0.5f;
     const float dist = sqrtf(xc * xc + yc * yc + C.ipd * C.ipd);
     return C.ipd / powf(dist, 3.f);
 }
@@ -310,7 +389,7 @@ __device__ __forceinline__ float pixel_solid_angle(const CamParams& C, uint32_t 
 // Ray::evalDirectionProbability (ray.cpp:32-38) with the objects' overrides;
 // `same` is the reference's `&inRay == &outRay` (an emitted ray)
 __device__ float bpt_dir_prob(const RenderScene& S, f3 in_d, const PRay& out, bool same, uint32_t cam_pixel) {
-    if (out.contact == CAMERA_OBJ) return (float)(1.0 / (double)pixel_solid_angle(S.cam, cam_pixel));
+    if (out.contact == CAMERA_OBJ) return 1.f / pixel_solid_angle(S.cam, cam_pixel);
     const int o = out.contact >= 0 ? out.contact : out.inside;
     if (o < 0) return 0.f;
     const wr_object_desc* m = &S.objs[o];
@@ -322,10 +401,10 @@ __device__ float bpt_dir_prob(const RenderScene& S, f3 in_d, const PRay& out, bo
         if (al.y > p) p = al.y;
         if (al.z > p) p = al.z;
         const float dn = dot(out.cnorm, out.d);
-        if (t == WR_MAT_DIFFUSE) return p * (dn > 0.f ? (float)((double)dn * INV_PI_D) : 0.f);
-        const float ct = (double)dn > EPS_D ? dn : (float)EPS_D;
+        if (t == WR_MAT_DIFFUSE) return p * (dn > 0.f ? over_pi(dn) : 0.f);
+        const float ct = max_eps(dn);
         const float power = __ldg(&m->power);
-        return p * (float)(((double)power + 1.0) * (double)powf(ct, power) * (INV_PI_D * 0.5));
+        return p * lobe_density(power, powf(ct, power));
     }
     if (t == WR_MAT_ANISO) {  // anisotropicGlossyObj.h:47-52, anisotropicPhong.h:19-33
         if (out.contact < 0) return 0.f;
@@ -433,7 +512,7 @@ __device__ __noinline__ float hv_origin_prob(const RenderScene& S, const PRay& i
                                             const HvCtx& hc) {
     const wr_object_desc* m = &S.objs[in.inside];
     const float d0 = length(in.o - out_o);
-    const float dist = (double)d0 > EPS_D ? d0 : (float)EPS_D;
+    const float dist = max_eps(d0);
     const float tau = hv_integrate(S, in, dist, hc);
     if (out_contact != -1) return expf(-tau);
     const f3 st = ld3(m->sigma_s) + ld3(m->sigma_a);
@@ -457,7 +536,7 @@ __device__ __forceinline__ float bpt_origin_prob(const RenderScene& S, const PRa
     const wr_object_desc* m = &S.objs[in.inside];
     const f3 st = ld3(m->sigma_s) + ld3(m->sigma_a);
     const float d0 = length(in.o - out_o);
-    const float dist = (double)d0 > 1e-5 ? d0 : (float)1e-5;
+    const float dist = max_eps(d0);
     const f3 e = mk(expf(-st.x * dist), expf(-st.y * dist), expf(-st.z * dist));
     return out_contact != -1 ? luminance(e) : luminance(vmul(st, e));
 }
@@ -474,8 +553,6 @@ __device__ __forceinline__ f3 bpt_decay(const RenderScene& S, const PRay& r, flo
 __device__ __forceinline__ bool emissive(const RenderScene& S, int o) {
     return o >= 0 && obj_type(S, o) == WR_MAT_EMISSIVE;
 }
-
-__device__ __forceinline__ float max_eps(float a) { return (double)a > EPS_D ? a : (float)EPS_D; }
 
 // PdfWtoA (util.h:100-106) with aPdfW = 1
 __device__ __forceinline__ float pdf_w_to_a(float dist, float cos_there) { return fabsf(cos_there) / (dist * dist); }
@@ -594,8 +671,8 @@ __device__ float bpt_mis_weight(const RenderScene& S, const Conn& C, uint32_t pi
     }
     if (!can_connect) all += rev[0];
     if (K.merge) self *= K.nvm;
-    const double w = self / all;
-    return (float)(w > 0.0 ? w : 0.0);  // also VCMTracer's `!(w >= 0) -> 0`
+    const float w = (float)(self / all);
+    return w > 0.f ? w : 0.f;  // also VCMTracer's `!(w >= 0) -> 0`
 }
 
 // BidirectionalPathTracer::connectingColorProb (bidirPathTracer.cpp:267-290),
@@ -666,11 +743,9 @@ __device__ __forceinline__ void film_add(float* f, uint32_t pid, f3 c) {
 // per record: the connected path must start at an emitter; a whole eye path
 // (l = 0) counts only if no two neighbours are both non-delta; no emitter
 // may sit at a connection vertex; connectEdge needs both connection vertices
-// non-delta.  Passing pairs with a light sub-path go to the candidate list
-// (their visibility is tested next), whole eye paths straight to the list of
-// contributing connections; e outer and l inner with the same loop bounds in
-// every lane, so that each warp appends runs of one (l, e) pair and the later
-// kernels' warps get uniform work.
+// non-delta.  Passing samples with a light sub-path go to the pair's candidates
+// (their visibility is tested next), whole eye paths straight to its
+// contributing connections.
 __global__ void __launch_bounds__(128) k_bpt_enum(RenderScene S, BptParams P) {
     constexpr unsigned FULL = 0xffffffffu;
     const uint32_t sid = blockIdx.x * blockDim.x + threadIdx.x;
@@ -704,9 +779,9 @@ __global__ void __launch_bounds__(128) k_bpt_enum(RenderScene S, BptParams P) {
                          !((dL >> (l - 1)) & 1u) && !((dE >> (e - 1)) & 1u);
                 }
             }
-            const uint2 item = make_uint2(sid, (uint32_t)l | ((uint32_t)e << 8));
-            if (l == 0) warp_append(ok, item, P.vis, P.ncand + 1);
-            else warp_append(ok, item, P.cand, P.ncand);
+            const uint32_t p = pair_at(P, l, e);
+            if (l == 0) warp_append(ok, sid, P.vis + (size_t)p * P.nsamp, P.npair + (P.npairs + p) * PAIR_WORDS);
+            else warp_append(ok, sid, P.cand + (size_t)p * P.nsamp, P.npair + p * PAIR_WORDS);
         }
     }
 }
@@ -734,29 +809,33 @@ __device__ __forceinline__ void bpt_connect_edge(const RenderScene& S, const Bpt
 
 // MCRenderer::visibilityTest (mcRenderer.cpp:59-65) of every candidate, from
 // the eye vertex towards the light vertex; the visible ones join the list of
-// contributing connections.  Persistent: the grid strides over the list.
-__global__ void __launch_bounds__(128) k_bpt_visible(RenderScene S, BptParams P) {
+// contributing connections.  Persistent: the warps stride over the runs of 32, six
+// blocks per SM (bidirectional Cornell box 9.15 -> 9.00 ms, 9.12 with seven).
+__global__ void __launch_bounds__(128, 6) k_bpt_visible(RenderScene S, BptParams P) {
     __shared__ WarpLeaves s_leaves[BPT_BLOCK / 32];
     extern __shared__ uint32_t s_stack[];
     uint32_t* stack = s_stack + threadIdx.x;
     const int stride = blockDim.x;
-    const unsigned long long total = P.ncand[0];
-    const unsigned long long step = (unsigned long long)gridDim.x * blockDim.x;
-    // every lane runs the same number of turns (warp_append needs the whole warp)
-    const unsigned long long turns = (total + step - 1) / step;
-    for (unsigned long long t = 0; t < turns; t++) {
-        const unsigned long long i = t * step + (unsigned long long)blockIdx.x * blockDim.x + threadIdx.x;
+    __shared__ uint32_t s_first[BPT_MAX_PAIRS + 1];
+    const uint32_t runs = pair_runs(P.npair, P.npairs, s_first);
+    const uint32_t warps = gridDim.x * (blockDim.x >> 5);
+    for (uint32_t r = blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5); r < runs; r += warps) {
+        const uint32_t p = pair_of_run(s_first, P.npairs, r);
+        const uint32_t i = (r - s_first[p]) * 32u + (threadIdx.x & 31u);
+        const bool on = i < P.npair[p * PAIR_WORDS];
         bool ok = false;
-        uint2 c = make_uint2(0, 0);
+        uint32_t sid = 0;
         PRay lc = ray_default(), ec = ray_default();
-        if (i < total) {
-            c = P.cand[i];
-            bpt_connect_edge(S, P, c.x, (int)(c.y & 0xffu), (int)(c.y >> 8), lc, ec);
+        if (on) {
+            int l, e;
+            pair_of(P, p, l, e);
+            sid = P.cand[(size_t)p * P.nsamp + i];
+            bpt_connect_edge(S, P, sid, l, e, lc, ec);
         }
-        const Hit h = search_warp(S.tree, i < total, ec.o, ec.d, P.pf, true, ec.inside, ec.contact, stack, stride,
+        const Hit h = search_warp(S.tree, on, ec.o, ec.d, P.pf, true, ec.inside, ec.contact, stack, stride,
                                   P.stack_cap, s_leaves[threadIdx.x >> 5]);
-        if (i < total) ok = h.slot < 0 || (double)(h.t - length(ec.o - lc.o)) >= -EPS_D;
-        warp_append(ok, c, P.vis, P.ncand + 1);
+        if (on) ok = h.slot < 0 || h.t - length(ec.o - lc.o) >= -EPS_F;
+        warp_append(ok, sid, P.vis + (size_t)p * P.nsamp, P.npair + (P.npairs + p) * PAIR_WORDS);
     }
 }
 
@@ -807,23 +886,29 @@ __device__ void bpt_connect_one(const RenderScene& S, const BptParams& P, uint32
     } else {
         sa = pixel_solid_angle(S.cam, pid);
     }
-    const float f = (float)(1.0 / (double)sa);
+    const float f = 1.f / sa;
     contrib = contrib * (f / (float)P.npix);
     film_add(film, pid, contrib);
 }
 
-// persistent: the grid strides over the contributing connections, 32
-// consecutive ones (mostly one (l, e) pair) per warp
-// MINB: resident blocks per SM the registers are fitted to (5 for the
-// bidirectional weights: 96 registers, +5 % over 4 blocks; VCM's weights
-// spill at that size and take 4; the marching instantiation 1)
-template <bool HM, int MINB>
-__global__ void __launch_bounds__(128, MINB) k_bpt_connect(RenderScene S, BptParams P) {
-    const unsigned long long total = P.ncand[1];
-    for (unsigned long long i = (unsigned long long)blockIdx.x * blockDim.x + threadIdx.x; i < total;
-         i += (unsigned long long)gridDim.x * blockDim.x) {
-        const uint2 c = P.vis[i];
-        bpt_connect_one<HM>(S, P, c.x, (int)(c.y & 0xffu), (int)(c.y >> 8));
+// persistent: the warps stride over the runs of 32 connections of one (l, e)
+// pair.  What is left is instruction fetch and the FP64 sums (a fifth of the
+// unit's rate).  Four blocks per SM (120 registers; five spill), the marching
+// instantiation one.  Batch of the bidirectional Cornell box: 1.30 ms over one
+// mixed list with 15.8 lanes at work, 0.58 with 30.9.
+template <bool HM>
+__global__ void __launch_bounds__(128, HM ? 1 : 4) k_bpt_connect(RenderScene S, BptParams P) {
+    __shared__ uint32_t s_first[BPT_MAX_PAIRS + 1];
+    const uint32_t* count = P.npair + P.npairs * PAIR_WORDS;
+    const uint32_t runs = pair_runs(count, P.npairs, s_first);
+    const uint32_t warps = gridDim.x * (blockDim.x >> 5);
+    for (uint32_t r = blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5); r < runs; r += warps) {
+        const uint32_t p = pair_of_run(s_first, P.npairs, r);
+        const uint32_t i = (r - s_first[p]) * 32u + (threadIdx.x & 31u);
+        if (i >= count[p * PAIR_WORDS]) continue;
+        int l, e;
+        pair_of(P, p, l, e);
+        bpt_connect_one<HM>(S, P, P.vis[(size_t)p * P.nsamp + i], l, e);
     }
 }
 
@@ -1551,10 +1636,11 @@ int render_bidirectional(wr_ctx* ctx, const RenderScene& S, const RenderParams& 
                              std::to_string((uint64_t)per_sample * nsamp) + " bytes) exceeds the device-memory budget");
     if (!ppm) WR_CUDA(ctx, st.eye.reserve(64ull * nrec * nsamp));
     WR_CUDA(ctx, st.light.reserve(64ull * nrec * nsamp));
-    WR_CUDA(ctx, st.counts.reserve(4ull * nsamp + 48));
+    const uint32_t npairs = ppm ? 0u : nrec * (nrec + 1);
+    WR_CUDA(ctx, st.counts.reserve(4ull * nsamp + 48 + 8ull * PAIR_WORDS * npairs));
     if (!ppm) {
-        WR_CUDA(ctx, st.cand.reserve(8ull * nrec * (nrec + 1) * nsamp));
-        WR_CUDA(ctx, st.vis.reserve(8ull * nrec * (nrec + 1) * nsamp));
+        WR_CUDA(ctx, st.cand.reserve(4ull * npairs * nsamp));
+        WR_CUDA(ctx, st.vis.reserve(4ull * npairs * nsamp));
     }
     const size_t film_bytes = 12ull * nsamp;
     if (st.film.bytes < film_bytes) {
@@ -1571,8 +1657,9 @@ int render_bidirectional(wr_ctx* ctx, const RenderScene& S, const RenderParams& 
     P.light.base = st.light.as<float4>();
     P.counts = st.counts.as<uint32_t>();
     P.film = st.film.as<float>();
-    P.cand = st.cand.as<uint2>();
-    P.vis = st.vis.as<uint2>();
+    P.cand = st.cand.as<uint32_t>();
+    P.vis = st.vis.as<uint32_t>();
+    P.npairs = npairs;
     P.vcm = vcm;
     P.light_only = ppm;
     P.vol_grid = vol_grid;
@@ -1599,12 +1686,13 @@ int render_bidirectional(wr_ctx* ctx, const RenderScene& S, const RenderParams& 
         WR_CUDA(ctx, st.tput.reserve(16ull * nrec * nsamp));
         P.tput = st.tput.as<float4>();
     }
-    // the five counters live after the per-sample counts (8-byte aligned)
+    // the counters live after the per-sample counts (8-byte aligned)
     P.ncand = reinterpret_cast<unsigned long long*>(st.counts.as<char>() + ((4ull * nsamp + 7) & ~7ull));
+    P.npair = reinterpret_cast<uint32_t*>(P.ncand + 5);
     // scenes with a heterogeneous medium take the kernels that march its
     // integrals in the weights; the others compile without those calls
     const auto k_subpaths = hetero ? k_bpt_subpaths<MED_REF> : media ? k_bpt_subpaths<MED_TRACK> : k_bpt_subpaths<MED_NONE>;
-    const auto k_connect = hetero ? k_bpt_connect<true, 1> : vcm ? k_bpt_connect<false, 4> : k_bpt_connect<false, 5>;
+    const auto k_connect = hetero ? k_bpt_connect<true> : k_bpt_connect<false>;
     const auto k_merge = hetero ? k_vcm_merge<true> : k_vcm_merge<false>;
     const auto k_eval = hetero ? k_vcm_eval<true> : k_vcm_eval<false>;
     const auto k_tput = hetero ? k_ppm_tput<true> : k_ppm_tput<false>;
@@ -1631,7 +1719,7 @@ int render_bidirectional(wr_ctx* ctx, const RenderScene& S, const RenderParams& 
         P.nsamp = npix * b;
         P.eye.nsamp = P.light.nsamp = P.nsamp;
         const int grid = (int)((P.nsamp + block - 1) / block);
-        WR_CUDA(ctx, cudaMemsetAsync(P.ncand, 0, 5 * sizeof(unsigned long long), stream));
+        WR_CUDA(ctx, cudaMemsetAsync(P.ncand, 0, 5 * sizeof(unsigned long long) + 8ull * PAIR_WORDS * npairs, stream));
         k_subpaths<<<subpath_grid, block, smem, stream>>>(S, P);
         WR_CUDA(ctx, cudaGetLastError());
         if (grid_on) {  // the batch's hash grids: one per slot (iteration), a second one for volume photons
