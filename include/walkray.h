@@ -142,9 +142,10 @@ typedef struct wr_ctx_desc {
     uint32_t pad;
 } wr_ctx_desc;
 
-/* wr_trace_closest visits every box the reference visits (KDTree::intersect,
- * kdtree.cpp:308-347, which never prunes by distance).  Without this flag it
- * skips a box entered beyond 1.001 x the closest hit found so far (plus the
+/* wr_trace_closest walks the reference's tree and visits every box the
+ * reference visits (KDTree::intersect, kdtree.cpp:308-347, which never prunes
+ * by distance).  Without this flag it searches a tree of its own over the same
+ * leaves, checks the winner with the reference's boxes, and skips a box entered beyond 1.001 x the closest hit found so far (plus the
  * box margin), except for a ray whose closest hit so far grazes its
  * triangle's plane (|n.d| < |d| / 32), which keeps every box: a triangle's
  * hit lies in its box up to the triangle test's rounding, which only a
@@ -227,12 +228,14 @@ int wr_trace_closest_device(wr_ctx* ctx, wr_scene_id scene, const float* d_rays,
                                     (photonMap.cpp:306-367); max_path_len <= 30 */
 
 #define WR_RENDER_NEE 1u      /* PathTracer's next-event-estimation branch (pathTracer.cpp:39-66) */
-/* Rendering traverses front to back and skips a box whose entry distance is
- * beyond the closest hit found so far (with a 0.1 % relative margin).  That
- * gives the reference's closest hit except for a ray that grazes a triangle
- * so nearly in its plane that the triangle test's rounding moves the hit
- * outside the triangle's box.  This flag visits every box the reference
- * visits (KDTree::intersect, kdtree.cpp:308-347), as wr_trace_closest does. */
+/* Rendering skips a box whose entry distance is beyond the closest hit found so
+ * far (with a 0.1 % relative margin).  That gives the reference's closest hit
+ * except for a ray that grazes a triangle so nearly in its plane that the
+ * triangle test's rounding moves the hit outside the triangle's box.  With this
+ * flag nothing is skipped for its distance; the wavefront's extend stage walks
+ * the reference's own tree (KDTree::intersect, kdtree.cpp:308-347), the other
+ * kernels search theirs, which tests every triangle the reference tests.  A
+ * connection to a light still ends at the first hit that hides it. */
 #define WR_RENDER_EXACT_TRAVERSAL 2u
 /* Low-variance estimators (no reference counterpart; the reference's
  * expectation is kept, only the variance changes).  Path tracing modes

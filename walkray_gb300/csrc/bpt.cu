@@ -832,9 +832,10 @@ __global__ void __launch_bounds__(128, 6) k_bpt_visible(RenderScene S, BptParams
             sid = P.cand[(size_t)p * P.nsamp + i];
             bpt_connect_edge(S, P, sid, l, e, lc, ec);
         }
+        const float dist = length(ec.o - lc.o);
         const Hit h = search_warp(S.tree, on, ec.o, ec.d, P.pf, true, ec.inside, ec.contact, stack, stride,
-                                  P.stack_cap, s_leaves[threadIdx.x >> 5]);
-        if (on) ok = h.slot < 0 || h.t - length(ec.o - lc.o) >= -EPS_F;
+                                  P.stack_cap, s_leaves[threadIdx.x >> 5], enough_before(dist));
+        if (on) ok = nee_visible(h, dist);
         warp_append(ok, sid, P.vis + (size_t)p * P.nsamp, P.npair + (P.npairs + p) * PAIR_WORDS);
     }
 }

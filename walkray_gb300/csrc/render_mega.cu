@@ -69,14 +69,14 @@ __global__ void __launch_bounds__(MEGA_BLOCK) k_megakernel(RenderScene S, Render
         }
         if (MIS && __any_sync(FULL, has_lr)) {  // the light connection of WR_RENDER_NEE_MIS
             const Hit lh = search_warp(S.tree, has_lr, lr.o, lr.d, pf, true, lr.inside, lr.contact, stack, stride,
-                                       P.stack_cap, leaves);
+                                       P.stack_cap, leaves, enough_before(lr.dist));
             if (has_lr && light_req_visible(S, lh, lr)) lit = lit + lr.contrib;
         }
         if (__any_sync(FULL, nee_here)) {  // the connection of the NEE branch
             ShadowReq sr;
             const bool conn = nee_here && nee_prepare(S, cur, prev_d, color, g, sr);
             const Hit sh = search_warp(S.tree, conn, sr.o, sr.d, pf, true, sr.inside, sr.contact, stack, stride,
-                                       P.stack_cap, leaves);
+                                       P.stack_cap, leaves, enough_before(sr.dist));
             if (conn && nee_visible(sh, sr.dist)) result = sr.contrib;
         }
         if (done) {

@@ -410,6 +410,7 @@ struct ShadowSrc {
         a.filt = true;
         a.inside = ids.x;
         a.contact = ids.y;
+        a.enough = enough_before(o.w);
     }
     __device__ __forceinline__ void put(uint64_t id, const TraceRay&, const Hit& h) const {
         hits[id] = make_int2(h.slot, __float_as_int(h.t));
@@ -636,14 +637,14 @@ __global__ void __launch_bounds__(WF_FINISH_BLOCK, MIS ? 3 : 4)
         }
         if (MIS && __any_sync(FULL, has_lr)) {  // the light connection of WR_RENDER_NEE_MIS
             const Hit lh = search_warp<false>(S.tree, has_lr, lr.o, lr.d, pf, true, lr.inside, lr.contact, stack,
-                                              WF_FINISH_BLOCK, stack_cap, leaves);
+                                              WF_FINISH_BLOCK, stack_cap, leaves, enough_before(lr.dist));
             if (has_lr && light_req_visible(S, lh, lr)) p.acc = p.acc + lr.contrib;
         }
         if (__any_sync(FULL, nee_here)) {  // the connection of the NEE branch
             ShadowReq sr;
             const bool conn = nee_here && nee_prepare(S, p.cur, p.prev_d, p.color, g, sr);
             const Hit sh = search_warp<false>(S.tree, conn, sr.o, sr.d, pf, true, sr.inside, sr.contact, stack,
-                                              WF_FINISH_BLOCK, stack_cap, leaves);
+                                              WF_FINISH_BLOCK, stack_cap, leaves, enough_before(sr.dist));
             if (nee_here) result = conn && nee_visible(sh, sr.dist) ? sr.contrib : mk(0, 0, 0);
         }
         if (done) {

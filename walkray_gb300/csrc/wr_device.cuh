@@ -13,9 +13,10 @@
 //                        to the largest slot" reproduces the reference's
 //                        tie rule (kdtree.cpp:319, 331-334).
 //
-// Arithmetic: all kernels are compiled with -fmad=false and IEEE div/sqrt, and
-// the vector helpers keep nvVector.h's operation order, so that the traversal
-// predicates are bit-identical to the reference's FP32 code.
+// Arithmetic: IEEE div/sqrt, and vector helpers in nvVector.h's operation order.
+// The reference's predicates (face test, triangle test, face normal,
+// NoSelfCondition) spell their products and sums as unfused intrinsics, so they
+// are bit-identical to its FP32 code in translation units with contraction too.
 #pragma once
 
 #include <cmath>

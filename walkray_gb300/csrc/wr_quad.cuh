@@ -261,25 +261,37 @@ __host__ __device__ inline int quad_stack_cap(const DevTree& T) {
     return (int)(T.quad_stack + 4 < 20 ? T.quad_stack + 4 : 20);
 }
 
+// A connection's ray asks whether something is hit before `dist` (nee_visible,
+// light_req_visible: up to max(1e-5, 1e-4 dist) short of it counts as reached).
+// One such hit answers it: the closest is no farther.  Below this distance its
+// search ends with the first hit that the reference reaches (low-variance
+// 641x479 x 16 spp 8.70 -> 8.40 ms, bidirectional Cornell box 8.85 -> 8.70).
+__device__ __forceinline__ float enough_before(float dist) { return dist - 2.f * fmaxf(1e-5f, 1e-4f * dist); }
+
 // What a search reads only at leaves: the ray, the pruning rule's margin
-// (infinite: no pruning) and NoSelfCondition's object ids (used when filt).
+// (infinite: no pruning), NoSelfCondition's object ids (used when filt) and the
+// distance below which any hit ends it (filtered rays only; at most 0: none).
+// That distance and filt share a word: 0 is no filter.
+__device__ __forceinline__ float filter_word(bool filt, float enough) { return !filt ? 0.f : enough == 0.f ? -1.f : enough; }
 // In registers:
 struct RayInRegs {
     const TriRec* tt;
     f3 ro, rd;
     float rm;
-    bool f;
+    float fw;
     int in, co;
-    __device__ __forceinline__ void set(const DevTree* T, f3 o, f3 d, float M, bool filt, int inside, int contact) {
+    __device__ __forceinline__ void set(const DevTree* T, f3 o, f3 d, float M, bool filt, int inside, int contact,
+                                        float enough) {
         tt = T ? T->tris : nullptr;
         ro = o;
         rd = d;
         rm = M;
-        f = filt;
+        fw = filter_word(filt, enough);
         in = inside;
         co = contact;
     }
     __device__ __forceinline__ float margin() const { return rm; }
+    __device__ __forceinline__ float enough() const { return fw; }
     __device__ __forceinline__ float length_d() const { return length(rd); }
     // lane l's (every lane of the warp calls these)
     __device__ __forceinline__ void ray_of(int l, f3& o, f3& d) const {
@@ -292,7 +304,7 @@ struct RayInRegs {
     }
     __device__ __forceinline__ void ids_of(int l, bool& filt, int& inside, int& contact) const {
         constexpr unsigned FULL = 0xffffffffu;
-        filt = __shfl_sync(FULL, (int)f, l) != 0;
+        filt = __shfl_sync(FULL, fw, l) != 0.f;
         inside = __shfl_sync(FULL, in, l);
         contact = __shfl_sync(FULL, co, l);
     }
@@ -312,7 +324,8 @@ struct RayInShared {
     __device__ __forceinline__ static unsigned long long get_ptr(const float* q, int k, int stride) {
         return __float_as_uint(q[k * stride]) | (unsigned long long)__float_as_uint(q[(k + 1) * stride]) << 32;
     }
-    __device__ __forceinline__ void set(const DevTree* T, f3 o, f3 d, float M, bool filt, int inside, int contact) {
+    __device__ __forceinline__ void set(const DevTree* T, f3 o, f3 d, float M, bool filt, int inside, int contact,
+                                        float enough) {
         put_ptr(10, T ? T->tris : nullptr);
         p[0] = o.x;
         p[stride] = o.y;
@@ -321,7 +334,7 @@ struct RayInShared {
         p[4 * stride] = d.y;
         p[5 * stride] = d.z;
         p[6 * stride] = M;
-        p[7 * stride] = __int_as_float((int)filt);
+        p[7 * stride] = filter_word(filt, enough);
         p[8 * stride] = __int_as_float(inside);
         p[9 * stride] = __int_as_float(contact);
     }
@@ -329,6 +342,7 @@ struct RayInShared {
         return reinterpret_cast<const TriRec*>(get_ptr(p + (l - (int)(threadIdx.x & 31u)), 10, stride));
     }
     __device__ __forceinline__ float margin() const { return p[6 * stride]; }
+    __device__ __forceinline__ float enough() const { return p[7 * stride]; }
     __device__ __forceinline__ float length_d() const { return length(mk(p[3 * stride], p[4 * stride], p[5 * stride])); }
     __device__ __forceinline__ void ray_of(int l, f3& o, f3& d) const {
         const float* q = p + (l - (int)(threadIdx.x & 31u));
@@ -337,7 +351,7 @@ struct RayInShared {
     }
     __device__ __forceinline__ void ids_of(int l, bool& filt, int& inside, int& contact) const {
         const float* q = p + (l - (int)(threadIdx.x & 31u));
-        filt = __float_as_int(q[7 * stride]) != 0;
+        filt = q[7 * stride] != 0.f;
         inside = __float_as_int(q[8 * stride]);
         contact = __float_as_int(q[9 * stride]);
     }
@@ -358,7 +372,7 @@ struct SearchLane {
     __device__ __forceinline__ bool finished() const { return cur == NO_WORD && pend == NO_WORD; }
     __device__ __forceinline__ void clear() {
         quads = nullptr;
-        ray.set(nullptr, mk(0, 0, 0), mk(0, 0, 0), 0.f, false, -1, -1);
+        ray.set(nullptr, mk(0, 0, 0), mk(0, 0, 0), 0.f, false, -1, -1, -1.f);
         r = QuadRay{mk(0, 0, 0), mk(0, 0, 0), mk(0, 0, 0)};
         lim = 0.f;
         h = Hit{0.f, -1};
@@ -367,14 +381,14 @@ struct SearchLane {
     }
     // starts at the root
     __device__ __forceinline__ void begin(const DevTree& T, f3 o, f3 d, float pf, bool filt, int inside,
-                                          int contact) {
+                                          int contact, float enough = -1.f) {
         quads = T.quads;
         lim = INFINITY;
         sp = 0;
         pend = NO_WORD;
         const float M = box_margin(o, T.scene_mag);
         const bool ok = make_quad_ray(o, d, T.scene_mag, M, r) && quads;
-        ray.set(&T, o, d, pf < INFINITY ? M : INFINITY, filt, inside, contact);
+        ray.set(&T, o, d, pf < INFINITY ? M : INFINITY, filt, inside, contact, enough);
         h = Hit{INFINITY, ok ? -1 : SLOT_REFERENCE};
         cur = ok ? 0u : NO_WORD;
     }
@@ -427,6 +441,7 @@ struct SearchLane {
         const bool off = fabsf(dd) < GRAZE_COS * ray.length_d() || (h.slot >= 0 && !(lim < INFINITY));
         lim = off ? INFINITY : t * 1.001f + ray.margin();
         h = Hit{t, slot};
+        if (t < ray.enough()) cur = pend = NO_WORD;
     }
     // the postponed leaf is done: the next one, if the walk stands at it
     __device__ __forceinline__ void leaf_done(const uint32_t* stack, int stride) {
@@ -582,11 +597,12 @@ __device__ __forceinline__ uint32_t warp_leaves(SearchLane<Ray>& L, bool has, Wa
 // warp calls it.  ONE_TREE: all rays in the tree T (else each lane's own T).
 template <bool ONE_TREE = true>
 __device__ __forceinline__ Hit search_warp(const DevTree& T, bool on, f3 o, f3 d, float pf, bool filt, int inside,
-                                           int contact, uint32_t* stack, int stride, int cap, WarpLeaves& leaves) {
+                                           int contact, uint32_t* stack, int stride, int cap, WarpLeaves& leaves,
+                                           float enough = -1.f) {
     constexpr unsigned FULL = 0xffffffffu;
     SearchLane<RayInRegs> L;
     L.clear();
-    if (on) L.begin(T, o, d, pf, filt, inside, contact);
+    if (on) L.begin(T, o, d, pf, filt, inside, contact, enough);
     const int top = (cap - 4) * stride;
     for (;;) {
         const bool walking = L.walking();

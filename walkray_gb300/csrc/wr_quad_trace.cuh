@@ -29,6 +29,7 @@ struct TraceRay {
     float pf;  // pruning factor
     bool filt;
     int inside, contact;  // NoSelfCondition object ids (used when filt)
+    float enough = -1.f;  // a hit below this distance ends the search (enough_before; used when filt)
 };
 
 // A warp's queues: rays that meet the scene's box and wait for a lane, and
@@ -143,7 +144,7 @@ __device__ __forceinline__ void quad_trace(Src& src, uint32_t n, unsigned int* c
                 id = Q.in[nin - 1u - k];
                 TraceRay a;
                 src.fetch(id, a);
-                L.begin(*a.T, a.o, a.d, a.pf, a.filt, a.inside, a.contact);
+                L.begin(*a.T, a.o, a.d, a.pf, a.filt, a.inside, a.contact, a.enough);
                 active = true;
             }
             nin -= min(want, nin);

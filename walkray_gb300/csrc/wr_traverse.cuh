@@ -38,7 +38,7 @@
 //    a zero (or subnormal) direction component has a non-finite 2M|inv|; its
 //    q.sm is NaN, so its shrunk test never passes and every box it grazes is
 //    decided by the face test.
-//  * Optional pruning (PRUNE, used by the renderers and wr_trace_closest): a
+//  * Pruning (reference_search in wr_quad.cuh; the exact walk does without): a
 //    child whose grown-box entry distance exceeds q.pf times the best hit
 //    (plus M) is skipped.  A triangle lies inside its box (boxes are the
 //    bounds of their triangles' vertices), so its hit distance is at least
