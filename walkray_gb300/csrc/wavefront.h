@@ -94,8 +94,10 @@ struct WfSide {
 // (1 + WR_MAT_* of the inside or hit object, 0 without either), so that the shade
 // stage runs one material's code per warp
 constexpr int WF_SORT_KEYS = 9;
+// and the paths of the heterogeneous media's bucket by how their flight ended
+enum : int { WF_FLIGHT_COLLIDED = 0, WF_FLIGHT_BOUNDARY, WF_FLIGHT_DIFFUSE, WF_FLIGHT_OTHER, WF_FLIGHT_KEYS };
 struct WfSort {
-    unsigned int* counts;  // [WF_SORT_KEYS]
+    unsigned int* counts;  // [WF_SORT_KEYS + WF_FLIGHT_KEYS]
     uint32_t* idx;         // bucket k at idx + k * capacity
 };
 
