@@ -26,3 +26,18 @@ def test_stages_equal_the_megakernel(ctx, width, height, nee, drain):
         ctx.set_wavefront_config(capacity=1 << 24)
     ctx.release(sid)
     assert np.allclose(a, b, rtol=1e-4, atol=1e-5), np.abs(a - b).max()
+
+
+@pytest.mark.parametrize("width,height", [(1023, 1), (32, 32), (41, 25), (64, 48)])
+def test_sorted_paths_equal_the_megakernel(ctx, width, height):
+    """Path counts at and around the sort stage's tile of 1024, materials mixed."""
+    s = S.mixed_spheres(width, height, seed=7, level=2)
+    sid = ctx.upload(s)
+    a = ctx.render(sid, 1, 16, seed=3, mode="megakernel")
+    try:
+        ctx.set_wavefront_config(capacity=1 << 14, drain_paths=0)
+        b = ctx.render(sid, 1, 16, seed=3, mode="wavefront")
+    finally:
+        ctx.set_wavefront_config(capacity=1 << 24)
+    ctx.release(sid)
+    assert np.allclose(a, b, rtol=1e-4, atol=1e-5), np.abs(a - b).max()

@@ -128,36 +128,57 @@ __global__ void k_wf_reset(WfSide Y, unsigned long long* work, unsigned int* sha
     for (int k = 0; k < WF_SORT_KEYS + WF_FLIGHT_KEYS; k++) B.counts[k] = 0;
 }
 
-// sort: bucket the queue by shading material (warp-aggregated appends)
-__global__ void __launch_bounds__(256) k_wf_sort(const RenderScene* __restrict__ scenes,
+// sort: bucket the queue by shading material.  A block counts a tile of
+// WF_SORT_TILE paths in shared memory and adds to the buckets' counters once for
+// it: with an addition per warp and key they queued up for the counters' sector
+// (mixed-material 1024^2 x 32 spp 30.85 ms,
+// 28.85 this way; twice the blocks or tiles of 512 and 2048: within 1 %).
+constexpr int WF_SORT_BLOCK = 256, WF_SORT_EACH = 4, WF_SORT_TILE = WF_SORT_BLOCK * WF_SORT_EACH;
+__global__ void __launch_bounds__(WF_SORT_BLOCK) k_wf_sort(const RenderScene* __restrict__ scenes,
                                                    const WfJob* __restrict__ jobs, WfSide X,
                                                    const int2* __restrict__ hits, WfSort B, uint32_t capacity) {
+    constexpr unsigned FULL = 0xffffffffu;
+    __shared__ uint32_t s_count[WF_SORT_KEYS], s_base[WF_SORT_KEYS];
     const uint32_t n = X.counts[0] + X.counts[1];
-    const uint32_t step = gridDim.x * blockDim.x;
+    const uint32_t tiles = n / WF_SORT_TILE + (n % WF_SORT_TILE != 0);
     const unsigned lane = threadIdx.x & 31u;
-    for (uint32_t base = blockIdx.x * blockDim.x; base < n; base += step) {  // warp-uniform trip count
-        const uint32_t i = base + threadIdx.x;
-        const bool valid = i < n;
-        int key = 0;
-        if (valid) {
-            const int slot = hits[i].x;
-            const int4 ids = as_i4(X.rec[(size_t)WF_REC * i + (WF_IDS ^ wf_swizzle(i))]);
-            if (slot >= 0 || ids.x >= 0) {
-                const RenderScene& S = scenes[jobs[ids.z].scene];
-                const int self = ids.x >= 0 ? ids.x : (int)__float_as_uint(__ldg(&S.tree.tris[slot].v1.w));
-                key = 1 + (int)obj_type(S, self);
-                key = key < WF_SORT_KEYS ? key : WF_SORT_KEYS - 1;
+    for (uint32_t tile = blockIdx.x; tile < tiles; tile += gridDim.x) {
+        if (threadIdx.x < WF_SORT_KEYS) s_count[threadIdx.x] = 0;
+        __syncthreads();
+        int key[WF_SORT_EACH];
+        uint32_t rank[WF_SORT_EACH];
+#pragma unroll
+        for (int t = 0; t < WF_SORT_EACH; t++) {
+            const uint32_t i = tile * WF_SORT_TILE + t * WF_SORT_BLOCK + threadIdx.x;
+            key[t] = -1;
+            if (i < n) {
+                key[t] = 0;
+                const int slot = hits[i].x;
+                const int4 ids = as_i4(X.rec[(size_t)WF_REC * i + (WF_IDS ^ wf_swizzle(i))]);
+                if (slot >= 0 || ids.x >= 0) {
+                    const RenderScene& S = scenes[jobs[ids.z].scene];
+                    const int self = ids.x >= 0 ? ids.x : (int)__float_as_uint(__ldg(&S.tree.tris[slot].v1.w));
+                    key[t] = min(1 + (int)obj_type(S, self), WF_SORT_KEYS - 1);
+                }
             }
         }
-        const unsigned vm = __ballot_sync(0xffffffffu, valid);
-        if (valid) {
-            const unsigned peers = __match_any_sync(vm, key);
+#pragma unroll
+        for (int t = 0; t < WF_SORT_EACH; t++) {
+            const unsigned peers = __match_any_sync(FULL, key[t]);
             const int leader = __ffs(peers) - 1;
-            unsigned int b = 0;
-            if ((int)lane == leader) b = atomicAdd(&B.counts[key], (unsigned)__popc(peers));
-            b = __shfl_sync(peers, b, leader);
-            B.idx[(size_t)key * capacity + b + __popc(peers & ((1u << lane) - 1u))] = i;
+            uint32_t at = 0;
+            if (key[t] >= 0 && (int)lane == leader) at = atomicAdd(&s_count[key[t]], (uint32_t)__popc(peers));
+            rank[t] = __shfl_sync(FULL, at, leader) + __popc(peers & ((1u << lane) - 1u));
         }
+        __syncthreads();
+        if (threadIdx.x < WF_SORT_KEYS && s_count[threadIdx.x])
+            s_base[threadIdx.x] = atomicAdd(&B.counts[threadIdx.x], s_count[threadIdx.x]);
+        __syncthreads();
+#pragma unroll
+        for (int t = 0; t < WF_SORT_EACH; t++)
+            if (key[t] >= 0)
+                B.idx[(size_t)key[t] * capacity + s_base[key[t]] + rank[t]] =
+                    tile * WF_SORT_TILE + t * WF_SORT_BLOCK + threadIdx.x;
     }
 }
 
@@ -1202,7 +1223,7 @@ static void enqueue_iteration(WfEngine* E, int x, cudaStream_t s, cudaEvent_t* e
             scenes, jobs, E->side[x], E->hits.as<int2>(), E->work.as<unsigned long long>(),
             E->exact_any ? E->stack_cap : E->quad_cap, E->cfg.trace, E->err_word.as<unsigned int>(), stats);
     if (ev) cudaEventRecord(ev[1], s);
-    k_wf_sort<<<E->grid_sort, 256, 0, s>>>(scenes, jobs, E->side[x], E->hits.as<int2>(), E->sort, E->cfg.capacity);
+    k_wf_sort<<<E->grid_sort, WF_SORT_BLOCK, 0, s>>>(scenes, jobs, E->side[x], E->hits.as<int2>(), E->sort, E->cfg.capacity);
     if (E->hetero_any)
         k_wf_track<<<E->grid_track, WF_TRACK_BLOCK, 0, s>>>(scenes, jobs, E->side[x], E->hits.as<int2>(), E->sort,
                                                             E->cfg.capacity, E->flights.as<Flight>(),
