@@ -13,12 +13,13 @@
 //                   samples are contiguous);
 //   k_bpt_enum      one thread per (pixel, sample): the (light length, eye
 //                   length) pairs that pass throughputByConnecting's path-shape
-//                   tests, appended to a candidate list in runs of one pair;
-//   k_bpt_visible   persistent, one candidate per thread and step: connectEdge
-//                   and the visibility ray (MCRenderer::visibilityTest); the
-//                   visible ones are appended to the contributing list;
-//   k_bpt_connect   persistent, one contributing connection per thread and
-//                   step: connectEdge again, connectingColorProb
+//                   tests, the sample appended to each pair's candidates;
+//   k_bpt_visible   persistent, runs of 32 candidates of one pair per warp:
+//                   connectEdge and the visibility ray
+//                   (MCRenderer::visibilityTest); the visible ones are appended
+//                   to the pair's contributing list;
+//   k_bpt_connect   persistent, runs of 32 contributing connections of one pair
+//                   per warp: connectEdge again, connectingColorProb
 //                   and the balance-heuristic weight of connectingMisWeight
 //                   (FP64 products, as the reference) — adding to the sample's
 //                   image: its own pixel, or, for one-vertex eye sub-paths, the

@@ -3,9 +3,9 @@
 //
 //   extend    persistent warps trace every queued ray (closest hit, the same
 //             bit-exact traversal as k_trace_closest)
-//   sort      buckets the queue by the material each ray hit
-//   track     flights through heterogeneous media (only while a job's scene
-//             has one)
+//   sort      buckets the queue by the material each ray hit or is inside
+//   track     flights through heterogeneous media, bucketed by how they end
+//             (only while a job's scene has one)
 //   shade     one bounce of the reference loop per path (scatter, throughput,
 //             termination) in bucket order; survivors are compacted into the
 //             other state buffer with warp-aggregated appends, finished
