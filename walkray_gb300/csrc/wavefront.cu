@@ -533,8 +533,9 @@ static ExtendKernel extend_kernel(int ctas_per_sm, bool stats, bool exact) {
 
 // shade: one bounce per path; survivors compacted into Y, finished paths to
 // the film.  MIS: compiled with the WR_RENDER_NEE_MIS code (launched while a
-// job with that flag is in the table).  MED: MED_FLIGHT while a scene with
-// participating media is.
+// job with that flag is in the table).  MED: MED_FLIGHT behind k_wf_track, else
+// MED_TRACK while a scene with participating media is (paths of a cancelled job
+// may still be inside a heterogeneous medium then), else MED_NONE.
 template <bool MIS, int MED>
 __global__ void __launch_bounds__(128, 4) k_wf_shade(const RenderScene* __restrict__ scenes,
                                                     const WfJob* __restrict__ jobs,
@@ -640,8 +641,9 @@ __global__ void __launch_bounds__(128, 4) k_wf_shade(const RenderScene* __restri
     }
 }
 
-static auto shade_kernel(bool mis, bool media) {
-    if (media) return mis ? k_wf_shade<true, MED_FLIGHT> : k_wf_shade<false, MED_FLIGHT>;
+static auto shade_kernel(bool mis, bool media, bool hetero) {
+    if (hetero) return mis ? k_wf_shade<true, MED_FLIGHT> : k_wf_shade<false, MED_FLIGHT>;
+    if (media) return mis ? k_wf_shade<true, MED_TRACK> : k_wf_shade<false, MED_TRACK>;
     return mis ? k_wf_shade<true, MED_NONE> : k_wf_shade<false, MED_NONE>;
 }
 
@@ -1071,7 +1073,7 @@ int wf_engine_get(wr_ctx* ctx, const WfConfig& cfg, WfEngine** out) {
     E->order_host.assign(1, 0);
     // persistent grids from the occupancy calculator
     int per_sm = 0;
-    WR_CUDA(ctx, cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, shade_kernel(false, true), cfg.shade_block, 0));
+    WR_CUDA(ctx, cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, shade_kernel(false, true, true), cfg.shade_block, 0));
     if (cfg.ctas_per_sm > 0) per_sm = std::min(per_sm, cfg.ctas_per_sm);
     E->grid_shade = ctx->num_sms * std::max(1, per_sm);
     WR_CUDA(ctx, cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_wf_generate, WF_GEN_ROWS, 0));
@@ -1228,7 +1230,7 @@ static void enqueue_iteration(WfEngine* E, int x, cudaStream_t s, cudaEvent_t* e
         k_wf_track<<<E->grid_track, WF_TRACK_BLOCK, 0, s>>>(scenes, jobs, E->side[x], E->hits.as<int2>(), E->sort,
                                                             E->cfg.capacity, E->flights.as<Flight>(),
                                                             E->work.as<unsigned int>() + 4);
-    shade_kernel(E->mis_any, E->media_any)<<<E->grid_shade, E->cfg.shade_block, 0, s>>>(scenes, jobs, cnt, E->side[x], E->hits.as<int2>(),
+    shade_kernel(E->mis_any, E->media_any, E->hetero_any)<<<E->grid_shade, E->cfg.shade_block, 0, s>>>(scenes, jobs, cnt, E->side[x], E->hits.as<int2>(),
                                                             E->side[y], E->shadow, E->sort, E->cfg.capacity,
                                                             E->flights.as<Flight>());
     if (ev) cudaEventRecord(ev[2], s);
