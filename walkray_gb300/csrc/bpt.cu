@@ -39,6 +39,7 @@
 #include <algorithm>
 #include <memory>
 
+#include "bpt_density.h"
 #include "render_launch.h"
 #include "wr_context.h"
 #include "wr_shade.cuh"
@@ -48,7 +49,6 @@ namespace wr {
 constexpr int BPT_BLOCK = 128;  // threads per CTA of the kernels that trace rays
 constexpr uint32_t BPT_LIGHT_DIM0 = 0x40000000u;
 constexpr int BPT_MAX_RECORDS = 32;  // records per sub-path: max_path_len + 2
-constexpr double INV_PI_D = 0.31830988618379067153776752674503;
 constexpr double PI_D = 3.1415926535897932384626433832795;
 constexpr double EPS_D = 1e-5;
 
@@ -361,22 +361,6 @@ __global__ void __launch_bounds__(128, MED == MED_NONE ? 4 : 1) k_bpt_subpaths(R
 // bits), and 1e-5f is the largest float below 1e-5.  The sums and products
 // that the reference keeps in double stay so.
 __device__ __forceinline__ float max_eps(float a) { return a > EPS_F ? a : EPS_F; }
-// x / pi of a double product rounded to float: the constant in two floats (the
-// same result for every 24-bit significand)
-constexpr float OVER_PI_HI = (float)INV_PI_D, OVER_PI_LO = (float)(INV_PI_D - (double)OVER_PI_HI);
-__device__ __forceinline__ float over_pi(float x) {
-    const float p = __fmul_rn(x, OVER_PI_HI);
-    return __fadd_rn(p, __fmaf_rn(x, OVER_PI_LO, __fmaf_rn(x, OVER_PI_HI, -p)));
-}
-// (power + 1) * c / (2 pi), to some 46 bits before the last rounding
-__device__ __forceinline__ float lobe_density(float power, float c) {
-    const float a = __fadd_rn(power, 1.f), b = __fsub_rn(a, power);
-    const float al = __fadd_rn(__fsub_rn(power, __fsub_rn(a, b)), __fsub_rn(1.f, b));  // a + al = power + 1
-    const float p = __fmul_rn(a, c), pl = __fmaf_rn(al, c, __fmaf_rn(a, c, -p));
-    const float h = 0.5f * OVER_PI_HI, l = 0.5f * OVER_PI_LO;
-    const float q = __fmul_rn(p, h);
-    return __fadd_rn(q, __fadd_rn(__fmaf_rn(p, h, -q), __fmaf_rn(p, l, __fmul_rn(pl, h))));
-}
 
 // Camera::getPixelSolidAngle (camera.cpp:125-131)
 __device__ __forceinline__ float pixel_solid_angle(const CamParams& C, uint32_t pid) {
