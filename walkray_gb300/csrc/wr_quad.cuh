@@ -24,10 +24,17 @@
 //
 // Pruning by distance is the rule of wr_traverse.cuh (q.pf, graze_check).
 //
-// Rays whose slab arithmetic could overflow or whose coordinates are not
-// finite take reference_search() alone.  A direction component below 1e-18 of
-// the direction's length is taken as that small: over the scene's extent the
-// ray moves by less than M along that axis either way.
+// Directions need not be of unit length: distances are in units of |d|, the
+// pruning rule's margin too (direction_unit).  Rays that are left to
+// reference_search() alone: |d| outside [1e-15, 1e15], where squares of d leave
+// the float range and the reference's distances may be subnormal (half an ulp
+// of one is 7e-46, times |d| below the 1e-30 in M); coordinates beyond 1e18 or
+// 1e19 |d|, where the slabs' products would overflow, and M below 1e-36 |d|,
+// where they would be subnormal; values that are not finite.  A direction
+// component below 1e-18 of the direction's length is taken as that small: over
+// the scene's extent the ray moves by less than M along that axis either way.
+// (With bounds of 1e-6 and 1e6 on |d| and 1e9 on coordinates 2^20 rays of length
+// 1e7 took 2.97 ms, of unit length 0.18.)
 //
 // On the mixed-material scene a bounce ray tests 70 boxes in 17 nodes here,
 // 104 in 52 node pairs on the reference's tree.
@@ -41,6 +48,11 @@ struct QuadRay {
     f3 inv;              // 1/d
     f3 nb, fb;           // plane * inv + nb (fb): distance to a near (far) plane moved out by M
 };
+
+// 1 / |d|, within a factor of two, as a power of two (1 for a unit vector)
+__device__ __forceinline__ float direction_unit(f3 d) {
+    return __int_as_float(0x7f000000 - (__float_as_int(fabsf(d.x) + fabsf(d.y) + fabsf(d.z)) & 0x7f800000));
+}
 
 // the margin M (wr_traverse.cuh)
 __device__ __forceinline__ float box_margin(f3 o, float scene_mag) {
@@ -59,7 +71,8 @@ __device__ __forceinline__ bool make_quad_ray(f3 o, f3 d, float scene_mag, float
               __fmaf_rn(-o.z, r.inv.z, -M * fabsf(r.inv.z)));
     r.fb = mk(__fmaf_rn(-o.x, r.inv.x, M * fabsf(r.inv.x)), __fmaf_rn(-o.y, r.inv.y, M * fabsf(r.inv.y)),
               __fmaf_rn(-o.z, r.inv.z, M * fabsf(r.inv.z)));
-    return on + scene_mag <= 1e9f && dn >= 1e-6f && dn <= 1e6f;  // false for a NaN
+    const float ext = on + scene_mag;
+    return ext <= 1e18f && ext <= 1e19f * dn && dn >= 1e-15f && dn <= 1e15f && M >= 1e-36f * dn;  // false for a NaN
 }
 
 // of three at once (a NaN is dropped, as by fmaxf and fminf)
@@ -268,8 +281,8 @@ __host__ __device__ inline int quad_stack_cap(const DevTree& T) {
 // 641x479 x 16 spp 8.70 -> 8.40 ms, bidirectional Cornell box 8.85 -> 8.70).
 __device__ __forceinline__ float enough_before(float dist) { return dist - 2.f * fmaxf(1e-5f, 1e-4f * dist); }
 
-// What a search reads only at leaves: the ray, the pruning rule's margin
-// (infinite: no pruning), NoSelfCondition's object ids (used when filt) and the
+// What a search reads only at leaves: the ray, the pruning rule's margin in
+// units of |d| (infinite: no pruning), NoSelfCondition's object ids (used when filt) and the
 // distance below which any hit ends it (filtered rays only; at most 0: none).
 // That distance and filt share a word: 0 is no filter.
 __device__ __forceinline__ float filter_word(bool filt, float enough) { return !filt ? 0.f : enough == 0.f ? -1.f : enough; }
@@ -388,7 +401,7 @@ struct SearchLane {
         pend = NO_WORD;
         const float M = box_margin(o, T.scene_mag);
         const bool ok = make_quad_ray(o, d, T.scene_mag, M, r) && quads;
-        ray.set(&T, o, d, pf < INFINITY ? M : INFINITY, filt, inside, contact, enough);
+        ray.set(&T, o, d, pf < INFINITY ? M * direction_unit(d) : INFINITY, filt, inside, contact, enough);
         h = Hit{INFINITY, ok ? -1 : SLOT_REFERENCE};
         cur = ok ? 0u : NO_WORD;
     }
@@ -564,7 +577,7 @@ __device__ __forceinline__ uint32_t warp_leaves(SearchLane<Ray>& L, bool has, Wa
             // it to the ray's own.
             const int group = on ? own : 32 + (int)lane;
             float bt = cand ? t : INFINITY, bd = dd;
-            int bs = slot;
+            int bs = cand ? slot : -1;  // (a candidate's distance may be infinite)
 #pragma unroll
             for (int k = 1; k < 8; k <<= 1) {
                 const float t2 = __shfl_down_sync(FULL, bt, k), d2 = __shfl_down_sync(FULL, bd, k);
@@ -578,7 +591,7 @@ __device__ __forceinline__ uint32_t warp_leaves(SearchLane<Ray>& L, bool has, Wa
             const int g0 = __shfl_up_sync(FULL, group, 1);
             W.slot[lane] = -1;
             __syncwarp();
-            if (on && (lane == 0 || g0 != group) && bt < INFINITY) {
+            if (on && (lane == 0 || g0 != group) && bs >= 0) {
                 W.t[own] = bt;
                 W.dd[own] = bd;
                 W.slot[own] = bs;
