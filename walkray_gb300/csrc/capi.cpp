@@ -212,6 +212,7 @@ int wr_scene_upload(wr_ctx* ctx, const wr_scene_desc* d, wr_scene_id* out) {
     T.root_w0 = L.root_w0;
     T.root_w1 = L.root_w1;
     T.scene_mag = L.scene_mag;
+    T.finite_mag = L.finite_mag;
     T.max_depth = ht.max_depth;
     T.num_pairs = (uint32_t)L.pairs.size();
     T.num_slots = (uint32_t)L.slots.size();

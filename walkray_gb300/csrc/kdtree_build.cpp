@@ -233,9 +233,14 @@ HostTree build_reference_tree(const float* verts, uint32_t nv, const uint32_t* t
 DeviceLayout layout_for_device(const HostTree& t, const float* verts, uint32_t nv, const uint32_t* tris,
                                const int32_t* tri_obj, const uint32_t* tri_local) {
     DeviceLayout L;
-    float mag = 0.f;
-    for (size_t i = 0; i < 3 * (size_t)nv; i++) mag = std::max(mag, std::fabs(verts[i]));
+    float mag = 0.f, finite = 0.f;
+    for (size_t i = 0; i < 3 * (size_t)nv; i++) {
+        const float a = std::fabs(verts[i]);
+        mag = std::max(mag, a);
+        finite = a < INFINITY ? std::max(finite, a) : finite;
+    }
     L.scene_mag = mag;
+    L.finite_mag = finite;
     const uint32_t N = t.num_nodes();
     if (N == 0) {
         for (int d = 0; d < 3; d++) L.root_lo[d] = L.root_hi[d] = 0.f;

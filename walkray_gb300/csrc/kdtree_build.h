@@ -37,7 +37,8 @@ struct DeviceLayout {
     std::vector<uint32_t> slot_of;  // global triangle id -> slot
     float root_lo[3], root_hi[3];
     uint32_t root_w0 = 0, root_w1 = LEAF_FLAG;
-    float scene_mag = 0.f;
+    float scene_mag = 0.f;   // largest |coordinate|
+    float finite_mag = 0.f;  // of the finite ones
 };
 
 // Flattens the tree: one NodePair per internal node (its two children), in

@@ -51,6 +51,11 @@ struct QBox {
             hi[k] = std::max(hi[k], b.hi[k]);
         }
     }
+    bool finite() const {
+        bool f = true;
+        for (int k = 0; k < 3; k++) f = f && std::isfinite(lo[k]) && std::isfinite(hi[k]);
+        return f;
+    }
     float area() const {
         const float x = hi[0] - lo[0], y = hi[1] - lo[1], z = hi[2] - lo[2];
         return x < 0.f ? 0.f : x * y + y * z + z * x;
@@ -321,65 +326,15 @@ static uint32_t stack_need(const std::vector<QuadNode>& q) {
     return most;
 }
 
-QuadLayout build_quads(const HostTree& t, int threads) {
-    QuadLayout L;
-    const uint32_t N = t.num_nodes();
-#ifdef _OPENMP
-    if (threads <= 0) threads = omp_get_max_threads();
-#endif
+// the tree over `items`, the leaves with finite boxes; node_item[n]: the first
+// of them at or after node n
+static void build_finite(const HostTree& t, const std::vector<uint32_t>& node_item, std::vector<Item>& items,
+                         int threads, QuadLayout& L) {
     (void)threads;
-    // parent links of the reference tree, in the device layout's numbering
-    // (pairs in pre-order, slots leaf by leaf), and the leaves as items; a leaf
-    // of more than QUAD_LEAF_MAX triangles is several items with one box
-    std::vector<uint32_t> pair_of(N, 0u), slot_of(N, 0u), parent(N, 0u);
-    std::vector<uint32_t> node_item(N, 0u);  // first item at or after each node
-    uint32_t np = 0, slots = 0, ni = 0;
-    for (uint32_t n = 0; n < N; n++) {
-        node_item[n] = ni;
-        slot_of[n] = slots;
-        if (t.left[n] >= 0) {
-            pair_of[n] = np++;
-            parent[t.left[n]] = parent[t.right[n]] = n;
-        } else {
-            ni += (t.leaf_count[n] + QUAD_LEAF_MAX - 1) / QUAD_LEAF_MAX;
-            slots += t.leaf_count[n];
-        }
-    }
-    L.leaf_up.resize(slots);
-    L.pair_up.resize(np);
-    std::vector<Item> items(ni);
-    auto up = [&](uint32_t n) {
-        return n == 0 ? UP_ROOT : pair_of[parent[n]] << 1 | (uint32_t)(t.right[parent[n]] == (int32_t)n);
-    };
-    bool fits = slots <= QUAD_MAX_SLOTS;
-#ifdef _OPENMP
-#pragma omp parallel for num_threads(threads) schedule(static, 4096) reduction(&& : fits) if (N > 16384)
-#endif
-    for (uint32_t n = 0; n < N; n++) {
-        if (t.left[n] >= 0) {
-            uint32_t a[4], m = n;
-            for (uint32_t& u : a) {  // (past the root: UP_ROOT again)
-                u = up(m);
-                m = parent[m];
-            }
-            L.pair_up[pair_of[n]] = make_uint4(a[0], a[1], a[2], a[3]);
-            continue;
-        }
-        for (uint32_t k = 0, i = node_item[n]; k < t.leaf_count[n]; k += QUAD_LEAF_MAX, i++) {
-            Item& it = items[i];
-            std::memcpy(it.box.lo, &t.box[6 * (size_t)n], 12);
-            std::memcpy(it.box.hi, &t.box[6 * (size_t)n + 3], 12);
-            for (int d = 0; d < 3; d++) fits = fits && std::isfinite(it.box.lo[d]) && std::isfinite(it.box.hi[d]);
-            it.count = std::min(QUAD_LEAF_MAX, t.leaf_count[n] - k);
-            it.word = QUAD_LEAF | it.count << QUAD_COUNT_AT | (slot_of[n] + k);
-        }
-        for (uint32_t k = 0; k < t.leaf_count[n]; k++) L.leaf_up[slot_of[n] + k] = up(n);
-    }
-    if (!fits) return L;
     if (items.empty()) {  // no triangles: a root of holes
         L.quads.emplace_back();
         for (int k = 0; k < 4; k++) set_child(L.quads[0], k, nullptr, QUAD_HOLE);
-        return L;
+        return;
     }
     // clusters: the reference's largest subtrees of at most CLUSTER items
     // (a subtree's leaves are consecutive in pre-order)
@@ -435,8 +390,7 @@ QuadLayout build_quads(const HostTree& t, int threads) {
     }
     if (nc == 1) {
         L.quads.swap(sub[0]);
-        L.stack = stack_need(L.quads);
-        return L;
+        return;
     }
     std::vector<BinNode> bin;
 #ifdef _OPENMP
@@ -480,6 +434,110 @@ QuadLayout build_quads(const HostTree& t, int threads) {
             }
             L.quads[base[c] + k] = q;
         }
+}
+
+// Leaves whose box has an infinite or NaN plane, above the root: their boxes say
+// nothing to the search, so every ray tests their triangles (the check of the
+// winner runs the reference's tests on their boxes).  The last slot of a node
+// leads on, so that its word lies below the leaves on a walk's stack.  A scene
+// of more than ODD_MAX such leaf words gets no tree: 24 cost a ray about what
+// the walk without one does (two visits and a leaf phase for each three).
+constexpr size_t ODD_MAX = 24;
+static void put_above(const std::vector<uint32_t>& odd, QuadLayout& L) {
+    const uint32_t add = (uint32_t)(odd.size() + 2) / 3;
+    std::vector<QuadNode> q(add);
+    const QBox all{{-1e30f, -1e30f, -1e30f}, {1e30f, 1e30f, 1e30f}};  // met by every ray of the search
+    for (uint32_t i = 0; i < add; i++) {
+        for (uint32_t k = 0; k < 3; k++) {
+            const size_t at = 3 * (size_t)i + k;
+            set_child(q[i], k, at < odd.size() ? &all : nullptr, at < odd.size() ? odd[at] : QUAD_HOLE);
+        }
+        set_child(q[i], 3, &all, i + 1);
+    }
+    for (QuadNode b : L.quads) {
+        for (int k = 0; k < 4; k++) {
+            uint32_t& w = (&b.child.x)[k];
+            if (!(w & QUAD_LEAF)) w += add;
+        }
+        q.push_back(b);
+    }
+    L.quads.swap(q);
+}
+
+QuadLayout build_quads(const HostTree& t, int threads) {
+    QuadLayout L;
+    const uint32_t N = t.num_nodes();
+#ifdef _OPENMP
+    if (threads <= 0) threads = omp_get_max_threads();
+#endif
+    (void)threads;
+    // parent links of the reference tree, in the device layout's numbering
+    // (pairs in pre-order, slots leaf by leaf), and the leaves as items; a leaf
+    // of more than QUAD_LEAF_MAX triangles is several items with one box
+    std::vector<uint32_t> pair_of(N, 0u), slot_of(N, 0u), parent(N, 0u);
+    std::vector<uint32_t> node_item(N, 0u);  // first item at or after each node
+    uint32_t np = 0, slots = 0, ni = 0;
+    for (uint32_t n = 0; n < N; n++) {
+        node_item[n] = ni;
+        slot_of[n] = slots;
+        if (t.left[n] >= 0) {
+            pair_of[n] = np++;
+            parent[t.left[n]] = parent[t.right[n]] = n;
+        } else {
+            ni += (t.leaf_count[n] + QUAD_LEAF_MAX - 1) / QUAD_LEAF_MAX;
+            slots += t.leaf_count[n];
+        }
+    }
+    L.leaf_up.resize(slots);
+    L.pair_up.resize(np);
+    std::vector<Item> items(ni);
+    auto up = [&](uint32_t n) {
+        return n == 0 ? UP_ROOT : pair_of[parent[n]] << 1 | (uint32_t)(t.right[parent[n]] == (int32_t)n);
+    };
+    bool finite = true;
+#ifdef _OPENMP
+#pragma omp parallel for num_threads(threads) schedule(static, 4096) reduction(&& : finite) if (N > 16384)
+#endif
+    for (uint32_t n = 0; n < N; n++) {
+        if (t.left[n] >= 0) {
+            uint32_t a[4], m = n;
+            for (uint32_t& u : a) {  // (past the root: UP_ROOT again)
+                u = up(m);
+                m = parent[m];
+            }
+            L.pair_up[pair_of[n]] = make_uint4(a[0], a[1], a[2], a[3]);
+            continue;
+        }
+        for (uint32_t k = 0, i = node_item[n]; k < t.leaf_count[n]; k += QUAD_LEAF_MAX, i++) {
+            Item& it = items[i];
+            std::memcpy(it.box.lo, &t.box[6 * (size_t)n], 12);
+            std::memcpy(it.box.hi, &t.box[6 * (size_t)n + 3], 12);
+            finite = finite && it.box.finite();
+            it.count = std::min(QUAD_LEAF_MAX, t.leaf_count[n] - k);
+            it.word = QUAD_LEAF | it.count << QUAD_COUNT_AT | (slot_of[n] + k);
+        }
+        for (uint32_t k = 0; k < t.leaf_count[n]; k++) L.leaf_up[slot_of[n] + k] = up(n);
+    }
+    if (slots > QUAD_MAX_SLOTS) return L;
+    // leaves with an infinite or NaN bound go above the tree of the others
+    std::vector<uint32_t> odd;
+    if (!finite) {
+        std::vector<Item> rest;
+        rest.reserve(ni);
+        for (uint32_t n = 0, i = 0; n < N; n++) {
+            const uint32_t first = i;
+            node_item[n] = (uint32_t)rest.size();
+            if (t.left[n] < 0) i += (t.leaf_count[n] + QUAD_LEAF_MAX - 1) / QUAD_LEAF_MAX;
+            for (uint32_t k = first; k < i; k++) {
+                if (items[k].box.finite()) rest.push_back(items[k]);
+                else odd.push_back(items[k].word);
+            }
+        }
+        items.swap(rest);
+        if (odd.size() > ODD_MAX) return L;
+    }
+    build_finite(t, node_item, items, threads, L);
+    if (!odd.empty()) put_above(odd, L);
     L.stack = stack_need(L.quads);
     return L;
 }

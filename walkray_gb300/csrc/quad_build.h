@@ -20,8 +20,9 @@ struct QuadLayout {
 
 // Four-wide tree over the reference tree's leaves (their own boxes, bit for
 // bit) by the surface-area heuristic, and the reference tree's parent links.
-// A scene of more than QUAD_MAX_SLOTS triangles, or with a vertex that is not
-// finite, gets an empty `quads` (reference_search alone).
+// The few leaves with a vertex that is not finite lie above it, for every ray.
+// A scene of more than QUAD_MAX_SLOTS triangles, or with many such leaves, gets
+// an empty `quads` (reference_search alone).
 QuadLayout build_quads(const HostTree& t, int threads);
 
 }  // namespace wr

@@ -69,6 +69,7 @@ struct DevTree {
     float root_lo[3], root_hi[3];
     uint32_t root_w0, root_w1;  // topology word of the root
     float scene_mag;            // max |coordinate| over all vertices
+    float finite_mag;           // over those that are finite: the search's (wr_quad.cuh)
     uint32_t max_depth;
     uint32_t num_pairs, num_slots;
     // the four-wide tree the search walks (nullptr: none, see build_quads) and the reference tree's parent links, (pair << 1 | side)

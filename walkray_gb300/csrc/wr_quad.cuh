@@ -30,7 +30,9 @@
 // the float range and the reference's distances may be subnormal (half an ulp
 // of one is 7e-46, times |d| below the 1e-30 in M); coordinates beyond 1e18 or
 // 1e19 |d|, where the slabs' products would overflow, and M below 1e-36 |d|,
-// where they would be subnormal; values that are not finite.  A direction
+// where they would be subnormal; values that are not finite.  (B leaves out a
+// scene's coordinates that are not finite: boxes with such a plane are always
+// visited, see build_quads.)  A direction
 // component below 1e-18 of the direction's length is taken as that small: over
 // the scene's extent the ray moves by less than M along that axis either way.
 // (With bounds of 1e-6 and 1e6 on |d| and 1e9 on coordinates 2^20 rays of length
@@ -193,7 +195,10 @@ static __device__ __noinline__ bool box_faces(Box b, f3 o, f3 d, float scene_mag
 // Anything else -- an edge within M, a NaN -- runs the face tests.  With
 // QuadRay's constants the planes moved in are fb for a near and nb for a far
 // one.
-__device__ __forceinline__ bool reference_passes(const Box& b, const QuadRay& r, f3 o, f3 d, float scene_mag) {
+// `quick`: the boxes are finite (else the face tests decide: on an infinite
+// plane the reference's point is infinite or a NaN).
+__device__ __forceinline__ bool reference_passes(const Box& b, const QuadRay& r, f3 o, f3 d, float scene_mag,
+                                                 bool quick) {
     const bool px = r.inv.x > 0.f, py = r.inv.y > 0.f, pz = r.inv.z > 0.f;
     const float fx = px ? b.hx : b.lx, fy = py ? b.hy : b.ly, fz = pz ? b.hz : b.lz;
     const float nx = __fmaf_rn(px ? b.lx : b.hx, r.inv.x, r.fb.x), ny = __fmaf_rn(py ? b.ly : b.hy, r.inv.y, r.fb.y),
@@ -205,7 +210,7 @@ __device__ __forceinline__ bool reference_passes(const Box& b, const QuadRay& r,
     const bool by_x = (ny <= sx) & (nz <= sx) & (sy >= gx) & (sz >= gx) & (sx >= 0.f);
     const bool by_y = (nx <= sy) & (nz <= sy) & (sx >= gy) & (sz >= gy) & (sy >= 0.f);
     const bool by_z = (nx <= sz) & (ny <= sz) & (sx >= gz) & (sy >= gz) & (sz >= 0.f);
-    return (by_x | by_y | by_z) || box_faces(b, o, d, scene_mag);
+    return (quick & (by_x | by_y | by_z)) || box_faces(b, o, d, scene_mag);
 }
 
 // Does the reference's predicate pass on every box above `slot`'s triangle?
@@ -214,16 +219,17 @@ __device__ __forceinline__ bool reference_passes(const Box& b, const QuadRay& r,
 // search spill (mixed-material scene 1024^2 x 32 spp 34.7 ms, 34.0 this way).
 static __device__ __noinline__ bool reference_reaches(const DevTree& T, int slot, f3 o, f3 d) {
     QuadRay r;
-    make_quad_ray(o, d, T.scene_mag, box_margin(o, T.scene_mag), r);
+    make_quad_ray(o, d, T.finite_mag, box_margin(o, T.finite_mag), r);
+    const bool quick = T.scene_mag < INFINITY;
     for (uint32_t at = __ldg(T.leaf_up + slot); at != UP_ROOT;) {
         const uint4 up = ldg4u(T.pair_up + (at >> 1));
         const uint32_t a[4] = {at, up.x, up.y, up.z};
         at = up.w;
 #pragma unroll
         for (int k = 0; k < 4; k++)
-            if (a[k] != UP_ROOT && !reference_passes(child_box(T, a[k]), r, o, d, T.scene_mag)) return false;
+            if (a[k] != UP_ROOT && !reference_passes(child_box(T, a[k]), r, o, d, T.scene_mag, quick)) return false;
     }
-    return reference_passes(root_box(T), r, o, d, T.scene_mag);
+    return reference_passes(root_box(T), r, o, d, T.scene_mag, quick);
 }
 
 // Closest hit where the reference's predicate decides every descent, without
@@ -399,8 +405,8 @@ struct SearchLane {
         lim = INFINITY;
         sp = 0;
         pend = NO_WORD;
-        const float M = box_margin(o, T.scene_mag);
-        const bool ok = make_quad_ray(o, d, T.scene_mag, M, r) && quads;
+        const float M = box_margin(o, T.finite_mag);
+        const bool ok = make_quad_ray(o, d, T.finite_mag, M, r) && quads;
         ray.set(&T, o, d, pf < INFINITY ? M * direction_unit(d) : INFINITY, filt, inside, contact, enough);
         h = Hit{INFINITY, ok ? -1 : SLOT_REFERENCE};
         cur = ok ? 0u : NO_WORD;

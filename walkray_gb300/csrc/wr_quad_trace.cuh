@@ -60,7 +60,7 @@ __device__ __forceinline__ WarpQueues& warp_queues(uint32_t* smem, int cap) {
 __device__ __forceinline__ bool meets_scene(const TraceRay& a) {
     const DevTree& T = *a.T;
     QuadRay r;
-    if (!make_quad_ray(a.o, a.d, T.scene_mag, box_margin(a.o, T.scene_mag), r)) return true;
+    if (!make_quad_ray(a.o, a.d, T.finite_mag, box_margin(a.o, T.finite_mag), r)) return true;
     const bool px = r.inv.x > 0.f, py = r.inv.y > 0.f, pz = r.inv.z > 0.f;
     return quad_entry(r, px ? T.root_lo[0] : T.root_hi[0], py ? T.root_lo[1] : T.root_hi[1],
                       pz ? T.root_lo[2] : T.root_hi[2], px ? T.root_hi[0] : T.root_lo[0],
