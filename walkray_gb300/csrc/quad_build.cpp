@@ -439,10 +439,10 @@ static void build_finite(const HostTree& t, const std::vector<uint32_t>& node_it
 // Leaves whose box has an infinite or NaN plane, above the root: their boxes say
 // nothing to the search, so every ray tests their triangles (the check of the
 // winner runs the reference's tests on their boxes).  The last slot of a node
-// leads on, so that its word lies below the leaves on a walk's stack.  A scene
-// of more than ODD_MAX such leaf words gets no tree: 24 cost a ray about what
-// the walk without one does (two visits and a leaf phase for each three).
-constexpr size_t ODD_MAX = 24;
+// leads on, so that its word lies below the leaves on a walk's stack.  Faster
+// than the walk of the reference's tree, which such a plane turns into face
+// tests throughout, for any number of them (2^18 rays with 80 such words 0.42
+// against 2.65 ms, with 5,115 30.5 against 155).
 static void put_above(const std::vector<uint32_t>& odd, QuadLayout& L) {
     const uint32_t add = (uint32_t)(odd.size() + 2) / 3;
     std::vector<QuadNode> q(add);
@@ -534,7 +534,6 @@ QuadLayout build_quads(const HostTree& t, int threads) {
             }
         }
         items.swap(rest);
-        if (odd.size() > ODD_MAX) return L;
     }
     build_finite(t, node_item, items, threads, L);
     if (!odd.empty()) put_above(odd, L);

@@ -20,9 +20,9 @@ struct QuadLayout {
 
 // Four-wide tree over the reference tree's leaves (their own boxes, bit for
 // bit) by the surface-area heuristic, and the reference tree's parent links.
-// The few leaves with a vertex that is not finite lie above it, for every ray.
-// A scene of more than QUAD_MAX_SLOTS triangles, or with many such leaves, gets
-// an empty `quads` (reference_search alone).
+// Leaves with a vertex that is not finite lie above it, for every ray.  A scene
+// of more than QUAD_MAX_SLOTS triangles gets an empty `quads` (reference_search
+// alone).
 QuadLayout build_quads(const HostTree& t, int threads);
 
 }  // namespace wr
