@@ -7,6 +7,7 @@ import pytest
 
 from test_search_gpu import directions, pair, rays_of, same_hits, soup  # noqa: F401  (pair: a fixture)
 from walkray_gb300 import scenes as S
+from walkray_gb300.api import LOW_VARIANCE
 
 pytestmark = pytest.mark.gpu
 INF, NAN = np.inf, np.nan
@@ -46,6 +47,25 @@ def test_a_scene_of_such_triangles_alone(pair, values):  # noqa: F811
     s.add(S.MAT_DIFFUSE, np.array([values, (1, 0, 0), (0, 1, 0)], np.float32), [(0, 1, 2)])
     rng = np.random.default_rng(2)
     same_hits(pair, s, np.concatenate([rng.random((3000, 3)), directions(3000, rng)], 1).astype(np.float32))
+
+
+@pytest.mark.parametrize("options", [{}, {"nee": True}, {"flags": LOW_VARIANCE}], ids=["plain", "nee", "low_variance"])
+@pytest.mark.parametrize("width,height", [(1, 1), (33, 1), (67, 61)])
+def test_images_of_such_a_scene(ctx, width, height, options):
+    """Wavefront against megakernel at one sample per pixel, so that each pixel is
+    one path: the kernels' own rounding alone may differ (3e-5, as in the
+    wavefront's stage tests)."""
+    s = S.mixed_spheres(width, height, seed=7, level=2)
+    rng = np.random.default_rng(1)
+    for k in range(100):
+        v = rng.random((3, 3)).astype(np.float32)
+        v[k % 3, k // 3 % 3] = INF
+        s.add(S.MAT_DIFFUSE, v, [(0, 1, 2)])
+    sid = ctx.upload(s)
+    a = ctx.render(sid, 1, 16, seed=5, mode="megakernel", **options)
+    b = ctx.render(sid, 1, 16, seed=5, mode="wavefront", **options)
+    ctx.release(sid)
+    assert np.allclose(a, b, rtol=1e-4, atol=1e-5), np.abs(a - b).max()
 
 
 def test_one_infinite_vertex_does_not_slow_the_search(pair):  # noqa: F811

@@ -21,8 +21,9 @@ struct QuadLayout {
 // Four-wide tree over the reference tree's leaves (their own boxes, bit for
 // bit) by the surface-area heuristic, and the reference tree's parent links.
 // Leaves with a vertex that is not finite lie above it, for every ray.  A scene
-// of more than QUAD_MAX_SLOTS triangles gets an empty `quads` (reference_search
-// alone).
+// of more than QUAD_MAX_SLOTS triangles gets an empty `quads` (the batch kernel
+// and the wavefront walk the reference's tree, the other renderers' rays take
+// reference_search one by one).
 QuadLayout build_quads(const HostTree& t, int threads);
 
 }  // namespace wr

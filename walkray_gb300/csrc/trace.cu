@@ -78,15 +78,19 @@ __global__ void __launch_bounds__(128, MINB > 0 ? MINB : 1)
                       warp_queues(s_stack, stack_cap), work);
 }
 
-// WR_CTX_EXACT_TRAVERSAL: every box the reference visits, without pruning by distance
+// The walk of the reference's own tree: without pruning by distance
+// (WR_CTX_EXACT_TRAVERSAL), or with it where a scene has no four-wide tree
+// (more than QUAD_MAX_SLOTS triangles: ray by ray through reference_search a
+// batch takes some four times the walk's time).
+template <bool PRUNE>
 __global__ void __launch_bounds__(128, 7)
-    k_trace_closest_exact(const __grid_constant__ DevTree T, const float* __restrict__ rays, uint64_t n,
+    k_trace_closest_walk(const __grid_constant__ DevTree T, const float* __restrict__ rays, uint64_t n,
                           const int32_t* __restrict__ inside, const int32_t* __restrict__ contact,
                           wr_hit* __restrict__ hits, unsigned long long* __restrict__ counter, int stack_cap,
                           TraceTune tune, unsigned int* __restrict__ err) {
     extern __shared__ __align__(16) uint32_t s_stack[];
     BatchSrc src{T, rays, inside, contact, hits, inside != nullptr};
-    warp_trace<false, false>(src, n, counter, tune, s_stack + threadIdx.x, blockDim.x, stack_cap, err);
+    warp_trace<PRUNE, false>(src, n, counter, tune, s_stack + threadIdx.x, blockDim.x, stack_cap, err);
 }
 
 cudaError_t launch_trace_closest(const DevTree& T, const float* d_rays, uint64_t n, const int32_t* d_inside,
@@ -105,8 +109,9 @@ cudaError_t launch_trace_closest(const DevTree& T, const float* d_rays, uint64_t
     const int block = 128;
     const int ref_cap = (int)T.max_depth + 3;  // stack of the reference's own walk
     if ((size_t)ref_cap * block * sizeof(uint32_t) > 200 * 1024) return cudaErrorInvalidValue;
-    const int stack_cap = prune ? quad_stack_cap(T) : ref_cap;
-    const size_t smem = prune ? quad_smem(stack_cap, block) : (size_t)stack_cap * block * sizeof(uint32_t);
+    const bool search = prune && T.quads;
+    const int stack_cap = search ? quad_stack_cap(T) : ref_cap;
+    const size_t smem = search ? quad_smem(stack_cap, block) : (size_t)stack_cap * block * sizeof(uint32_t);
     cudaError_t e = cudaMemsetAsync(d_counter, 0, sizeof(unsigned long long), stream);
     if (e != cudaSuccess) return e;
     // blocks per SM from the occupancy calculator for this stack size
@@ -114,7 +119,7 @@ cudaError_t launch_trace_closest(const DevTree& T, const float* d_rays, uint64_t
     // 0: the 6-CTA variant (80 registers; 2^24 rays: 2.23 ms, 2.38 with 7, 2.64 with 5, 2.69 with 8)
     const int variant = ctas_per_sm ? ctas_per_sm : 6;
     void (*kern)(DevTree, const float*, uint64_t, const int32_t*, const int32_t*, wr_hit*, unsigned long long*, int,
-                 TraceTune, unsigned int*) = !prune         ? k_trace_closest_exact
+                 TraceTune, unsigned int*) = !search        ? (prune ? k_trace_closest_walk<true> : k_trace_closest_walk<false>)
                                              : variant >= 8 ? k_trace_closest<8>
                                              : variant >= 7 ? k_trace_closest<7>
                                              : variant >= 6 ? k_trace_closest<6>
@@ -128,7 +133,7 @@ cudaError_t launch_trace_closest(const DevTree& T, const float* d_rays, uint64_t
     if (ctas_per_sm > 0) per_sm = std::min(per_sm, ctas_per_sm);
     if (per_sm < 1) per_sm = 1;
     // few rays: a warp for each, as far as the grid goes
-    uint64_t need_blocks = prune ? (n + block / 32 - 1) / (block / 32) : (n + block - 1) / block;
+    uint64_t need_blocks = search ? (n + block / 32 - 1) / (block / 32) : (n + block - 1) / block;
     int grid = num_sms * per_sm;
     if ((uint64_t)grid > need_blocks) grid = (int)(need_blocks ? need_blocks : 1);
     if (launched_blocks) *launched_blocks = grid;

@@ -436,9 +436,10 @@ __device__ __forceinline__ void warp_add(unsigned long long* dst, unsigned long 
 // (a register cap), chosen by the configuration's ctas_per_sm
 #define WR_EXTEND_BOUNDS(MINB) __launch_bounds__(128, (MINB) > 0 ? (MINB) : 1)
 
-// EXACT: every box the reference visits (launched while a job with
-// WR_RENDER_EXACT_TRAVERSAL is in the table; its counts are the reference's)
-template <bool STATS, bool EXACT, int MINB>
+// WALK: the reference's own tree (launched while a job with
+// WR_RENDER_EXACT_TRAVERSAL, whose counts are the reference's, or a scene
+// without a four-wide tree is in the table)
+template <bool STATS, bool WALK, int MINB>
 __global__ void WR_EXTEND_BOUNDS(MINB) k_wf_extend(const RenderScene* __restrict__ scenes,
                                                      const WfJob* __restrict__ jobs, WfSide X, int2* __restrict__ hits,
                                                      unsigned long long* __restrict__ work, int stack_cap,
@@ -448,7 +449,7 @@ __global__ void WR_EXTEND_BOUNDS(MINB) k_wf_extend(const RenderScene* __restrict
     const uint64_t n = (uint64_t)X.counts[0] + X.counts[1];
     if (n == 0) return;
     ExtendSrc src{scenes, jobs, X, hits, TraceWork{0ull, 0ull, 0ull}};
-    if (EXACT)
+    if (WALK)
         warp_trace<true, STATS>(src, n, work, tune, s_stack + threadIdx.x, blockDim.x, stack_cap, err);
     else
         quad_trace<STATS>(src, (uint32_t)n, reinterpret_cast<unsigned int*>(work), tune, s_stack + threadIdx.x, blockDim.x, stack_cap,
@@ -492,9 +493,17 @@ struct ShadowSrc {
     __device__ __forceinline__ const TriRec* tris_of(const RayInShared& rays, int from) const {
         return rays.tris_of(from);
     }
+    __device__ __forceinline__ void load(uint64_t id, TraceLane& L, uint32_t* stack, int stride) const {
+        TraceRay a;
+        fetch(id, a);
+        load_lane(a, L, stack, stride);
+    }
+    __device__ __forceinline__ void store(uint64_t id, const TraceLane& L) const {
+        hits[id] = make_int2(L.h.slot, __float_as_int(L.h.t));
+    }
 };
 
-template <int MINB>
+template <bool WALK, int MINB>
 __global__ void WR_EXTEND_BOUNDS(MINB)
     k_wf_shadow_trace(const RenderScene* __restrict__ scenes, const WfJob* __restrict__ jobs, WfShadow Q,
                       int2* __restrict__ hits, unsigned long long* __restrict__ work, int stack_cap, TraceTune tune,
@@ -504,26 +513,30 @@ __global__ void WR_EXTEND_BOUNDS(MINB)
     if (n == 0) return;
     ShadowSrc src{scenes, jobs, Q, hits};
     TraceWork none;
-    quad_trace<false>(src, (uint32_t)n, reinterpret_cast<unsigned int*>(work), tune, s_stack + threadIdx.x, blockDim.x, stack_cap,
-                      warp_queues(s_stack, stack_cap), none);
+    if (WALK)
+        warp_trace<true, false>(src, n, work, tune, s_stack + threadIdx.x, blockDim.x, stack_cap, err);
+    else
+        quad_trace<false>(src, (uint32_t)n, reinterpret_cast<unsigned int*>(work), tune, s_stack + threadIdx.x, blockDim.x, stack_cap,
+                          warp_queues(s_stack, stack_cap), none);
 }
 
 using ShadowTraceKernel = void (*)(const RenderScene*, const WfJob*, WfShadow, int2*, unsigned long long*, int,
                                    TraceTune, unsigned int*);
 
 // the shadow traversal for a configuration: the extend stage's register cap
-static ShadowTraceKernel shadow_trace_kernel(int ctas_per_sm) {
+static ShadowTraceKernel shadow_trace_kernel(int ctas_per_sm, bool walk) {
+    if (walk) return k_wf_shadow_trace<true, 6>;
     if (ctas_per_sm == 0) ctas_per_sm = 6;
-    if (ctas_per_sm >= 8) return k_wf_shadow_trace<8>;
-    if (ctas_per_sm >= 7) return k_wf_shadow_trace<7>;
-    if (ctas_per_sm >= 6) return k_wf_shadow_trace<6>;
-    return k_wf_shadow_trace<0>;
+    if (ctas_per_sm >= 8) return k_wf_shadow_trace<false, 8>;
+    if (ctas_per_sm >= 7) return k_wf_shadow_trace<false, 7>;
+    if (ctas_per_sm >= 6) return k_wf_shadow_trace<false, 6>;
+    return k_wf_shadow_trace<false, 0>;
 }
 
 // the extend kernel for a configuration: register cap from ctas_per_sm
 // (0 = the 6-CTA variant: mixed-material scene 1024^2 x 32 spp 33.2 ms, 33.9 with 7, 36.3 with 8)
-static ExtendKernel extend_kernel(int ctas_per_sm, bool stats, bool exact) {
-    if (exact) return stats ? k_wf_extend<true, true, 6> : k_wf_extend<false, true, 6>;
+static ExtendKernel extend_kernel(int ctas_per_sm, bool stats, bool walk) {
+    if (walk) return stats ? k_wf_extend<true, true, 6> : k_wf_extend<false, true, 6>;
     if (ctas_per_sm == 0) ctas_per_sm = 6;
     if (ctas_per_sm >= 8) return stats ? k_wf_extend<true, false, 8> : k_wf_extend<false, false, 8>;
     if (ctas_per_sm >= 7) return stats ? k_wf_extend<true, false, 7> : k_wf_extend<false, false, 7>;
@@ -938,14 +951,15 @@ struct WfEngine {
     std::vector<int> order_host;               // [n, slot...]
     int stack_cap = 0;       // the reference walk's stack (tree depth + 3)
     int quad_cap = 0;        // the search's stack
-    int grid_extend = 0, grid_exact = 0, grid_shade = 0, grid_gen = 0;
-    size_t smem_extend = 0, smem_exact = 0;
+    int grid_extend = 0, grid_walk = 0, grid_shade = 0, grid_gen = 0;
+    size_t smem_extend = 0, smem_walk = 0;
     cudaGraphExec_t graph = nullptr;
     int graph_stack = -1;
     bool mis_any = false;  // a job in the table has WR_RENDER_NEE_MIS: the shade stage with that code
     bool hetero_any = false;  // a job's scene has a heterogeneous medium: the track stage
     bool media_any = false;  // a job's scene has participating media: the shading kernels with that code
-    bool exact_any = false;  // a job in the table has WR_RENDER_EXACT_TRAVERSAL: the extend stage of that walk
+    bool bare_any = false;   // a job's scene has no four-wide tree: the walk of the reference's in both stages
+    bool walk_any = false;   // or a job has WR_RENDER_EXACT_TRAVERSAL: in the extend stage
     bool conn_any = true;  // a job in the table connects to lights (NEE or MIS): the shadow stage is in the loop
     int launches_per_iteration() const { return (conn_any ? 8 : 6) + (hetero_any ? 1 : 0); }
     WfJobCounters* host_counters = nullptr;  // pinned
@@ -1155,44 +1169,49 @@ int wf_update_jobs(wr_ctx* ctx, WfEngine* E, const std::vector<WfSlotUpdate>& up
             const int block = E->cfg.extend_block;
             E->stack_cap = std::max(cap, E->stack_cap);
             E->quad_cap = std::max(quad_cap, E->quad_cap);
-            E->smem_exact = (size_t)E->stack_cap * block * sizeof(uint32_t);
+            E->smem_walk = (size_t)E->stack_cap * block * sizeof(uint32_t);
             E->smem_extend = quad_smem(E->quad_cap, block);
-            if (E->smem_exact > 200 * 1024) return set_error(ctx, WR_ERR_UNSUPPORTED, "tree too deep for the stack");
-            if (E->smem_exact > 48 * 1024)
+            if (E->smem_walk > 200 * 1024) return set_error(ctx, WR_ERR_UNSUPPORTED, "tree too deep for the stack");
+            if (E->smem_walk > 48 * 1024) {
+                WR_CUDA(ctx, cudaFuncSetAttribute(shadow_trace_kernel(E->cfg.ctas_per_sm, true),
+                                                  cudaFuncAttributeMaxDynamicSharedMemorySize, (int)E->smem_walk));
                 for (bool st : {false, true})
                     WR_CUDA(ctx, cudaFuncSetAttribute(extend_kernel(E->cfg.ctas_per_sm, st, true),
                                                       cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                                      (int)E->smem_exact));
+                                                      (int)E->smem_walk));
+            }
             int per_sm = 0;
             WR_CUDA(ctx, cudaOccupancyMaxActiveBlocksPerMultiprocessor(
                              &per_sm, extend_kernel(E->cfg.ctas_per_sm, false, false), block, E->smem_extend));
             if (E->cfg.ctas_per_sm > 0) per_sm = std::min(per_sm, E->cfg.ctas_per_sm);
             E->grid_extend = ctx->num_sms * std::max(1, per_sm);
             WR_CUDA(ctx, cudaOccupancyMaxActiveBlocksPerMultiprocessor(
-                             &per_sm, extend_kernel(E->cfg.ctas_per_sm, false, true), block, E->smem_exact));
+                             &per_sm, extend_kernel(E->cfg.ctas_per_sm, false, true), block, E->smem_walk));
             if (E->cfg.ctas_per_sm > 0) per_sm = std::min(per_sm, E->cfg.ctas_per_sm);
-            E->grid_exact = ctx->num_sms * std::max(1, per_sm);
+            E->grid_walk = ctx->num_sms * std::max(1, per_sm);
             WR_CUDA(ctx, cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_wf_shadow, 128, 0));
             E->grid_shadow = ctx->num_sms * std::max(1, per_sm);
         }
     }
     // the shade stage compiled with the light-connection code only while a job needs it
     // and the shadow stage only while a job can queue a connection
-    bool mis_any = false, conn_any = false, exact_any = false, media_any = false, hetero_any = false;
+    bool mis_any = false, conn_any = false, walk_any = false, bare_any = false, media_any = false, hetero_any = false;
     for (int slot : order) {
         if (!E->job_tab[slot].active) continue;
         if (E->job_tab[slot].flags & WR_RENDER_NEE_MIS) mis_any = true;
-        if (E->job_tab[slot].flags & WR_RENDER_EXACT_TRAVERSAL) exact_any = true;
+        if (E->job_tab[slot].flags & WR_RENDER_EXACT_TRAVERSAL) walk_any = true;
         if (const RenderData* rd = E->scene_of[E->job_tab[slot].scene]) {
+            if (!RenderDataView::scene(rd).tree.quads) walk_any = bare_any = true;
             media_any |= RenderDataView::media(rd);
             hetero_any |= RenderDataView::hetero(rd);
         }
         if (E->job_tab[slot].flags & (WR_RENDER_NEE | WR_RENDER_NEE_MIS)) conn_any = true;
     }
-    if (mis_any != E->mis_any || conn_any != E->conn_any || exact_any != E->exact_any ||
-        media_any != E->media_any || hetero_any != E->hetero_any) {
+    if (mis_any != E->mis_any || conn_any != E->conn_any || walk_any != E->walk_any ||
+        bare_any != E->bare_any || media_any != E->media_any || hetero_any != E->hetero_any) {
         E->hetero_any = hetero_any;
-        E->exact_any = exact_any;
+        E->walk_any = walk_any;
+        E->bare_any = bare_any;
         E->media_any = media_any;
         E->mis_any = mis_any;
         E->conn_any = conn_any;
@@ -1219,11 +1238,11 @@ static void enqueue_iteration(WfEngine* E, int x, cudaStream_t s, cudaEvent_t* e
     WfJobCounters* cnt = E->counters.as<WfJobCounters>();
     k_wf_reset<<<1, 1, 0, s>>>(E->side[y], E->work.as<unsigned long long>(), E->shadow.count, E->sort);
     if (ev) cudaEventRecord(ev[0], s);
-    extend_kernel(E->cfg.ctas_per_sm, stats != nullptr, E->exact_any)
-        <<<E->exact_any ? E->grid_exact : E->grid_extend, E->cfg.extend_block,
-           E->exact_any ? E->smem_exact : E->smem_extend, s>>>(
+    extend_kernel(E->cfg.ctas_per_sm, stats != nullptr, E->walk_any)
+        <<<E->walk_any ? E->grid_walk : E->grid_extend, E->cfg.extend_block,
+           E->walk_any ? E->smem_walk : E->smem_extend, s>>>(
             scenes, jobs, E->side[x], E->hits.as<int2>(), E->work.as<unsigned long long>(),
-            E->exact_any ? E->stack_cap : E->quad_cap, E->cfg.trace, E->err_word.as<unsigned int>(), stats);
+            E->walk_any ? E->stack_cap : E->quad_cap, E->cfg.trace, E->err_word.as<unsigned int>(), stats);
     if (ev) cudaEventRecord(ev[1], s);
     k_wf_sort<<<E->grid_sort, WF_SORT_BLOCK, 0, s>>>(scenes, jobs, E->side[x], E->hits.as<int2>(), E->sort, E->cfg.capacity);
     if (E->hetero_any)
@@ -1235,9 +1254,11 @@ static void enqueue_iteration(WfEngine* E, int x, cudaStream_t s, cudaEvent_t* e
                                                             E->flights.as<Flight>());
     if (ev) cudaEventRecord(ev[2], s);
     if (E->conn_any) {  // the connections' closest hits go into E->hits, which shade has read
-        shadow_trace_kernel(E->cfg.ctas_per_sm)<<<E->grid_extend, E->cfg.extend_block, E->smem_extend, s>>>(
-            scenes, jobs, E->shadow, E->hits.as<int2>(), E->work.as<unsigned long long>() + 1, E->quad_cap,
-            E->cfg.trace, E->err_word.as<unsigned int>());
+        shadow_trace_kernel(E->cfg.ctas_per_sm, E->bare_any)
+            <<<E->bare_any ? E->grid_walk : E->grid_extend, E->cfg.extend_block,
+               E->bare_any ? E->smem_walk : E->smem_extend, s>>>(
+                scenes, jobs, E->shadow, E->hits.as<int2>(), E->work.as<unsigned long long>() + 1,
+                E->bare_any ? E->stack_cap : E->quad_cap, E->cfg.trace, E->err_word.as<unsigned int>());
         k_wf_shadow<<<E->grid_shadow, 128, 0, s>>>(scenes, jobs, E->shadow, E->hits.as<int2>(), E->side[y]);
     }
     if (ev) cudaEventRecord(ev[3], s);
