@@ -427,8 +427,9 @@ typedef struct wr_wavefront_config {
     int32_t leaf_min;        /* traversal: lanes holding leaves that start a warp's leaf tests (1..32,
                                 0 = default); both also apply to wr_trace_closest */
     int32_t drain_paths;     /* wr_render: once every path is generated and at most this many remain,
-                                finish them in one per-path kernel (0 = never; a context that was given
-                                no configuration does so at 2^15, 2^13 with a density grid) */
+                                finish them in one per-path kernel (0 = never; -1, the default of a
+                                context that was given no configuration: 2^15, 2^13 with a density
+                                grid) */
     int32_t pixel_tile;      /* camera paths generated tile by tile, square tiles of this many pixels a
                                 side (0 = row by row); the image does not depend on it */
     int32_t steps_per_turn;  /* traversal: steps a searching lane takes per turn of a warp's loop (1..8,

@@ -189,13 +189,16 @@ class Context:
                 for k, _ in L.wr_render_profile._fields_}
 
     def set_wavefront_config(self, capacity: int, extend_block: int = 128, shade_block: int = 128,
-                             ctas_per_sm: int = 0, iters_per_graph: int = 4, refill_min: int = 0,
-                             leaf_min: int = 0, drain_paths: int = 0, pixel_tile: int = 0,
+                             ctas_per_sm: int = 0, iters_per_graph: int = 1, refill_min: int = 0,
+                             leaf_min: int = 0, drain_paths: int = -1, pixel_tile: int = 0,
                              steps_per_turn: int = 0) -> None:
         """Queue sizes and block shapes of the wavefront renderer; refill_min,
         leaf_min and steps_per_turn (0 = defaults) tune the warp traversal
         loop of both the extend stage and trace_closest; pixel_tile orders
-        camera paths by square pixel tiles (0 = rows)."""
+        camera paths by square pixel tiles (0 = rows); drain_paths: a render's
+        last paths, at most so many, leave the bounce loop (0 = never, -1 = by
+        scene).  What is left out has the value of a context that was given no
+        configuration."""
         c = L.wr_wavefront_config(capacity, extend_block, shade_block, ctas_per_sm, iters_per_graph, refill_min,
                                   leaf_min, drain_paths, pixel_tile, steps_per_turn, 0.0)
         self._check(self.lib.wr_set_wavefront_config(self.h, C.byref(c)))

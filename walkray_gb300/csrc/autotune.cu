@@ -3,7 +3,7 @@
 // for later wavefront renders.  The search is coordinate descent from the
 // shipped defaults (2^24 paths in flight, the 6-CTA extend variant, refill
 // and leaf thresholds 8, six traversal steps per turn, rows, one iteration
-// pair per graph launch): each dimension in turn tries its candidate values
+// pair per graph launch, the last paths finished as the scene asks): each dimension in turn tries its candidate values
 // with the others held at the best so far, and keeps a value only if it
 // renders faster.
 #include <cuda_runtime.h>
@@ -22,7 +22,7 @@ int wr_set_wavefront_config(wr_ctx* ctx, const wr_wavefront_config* cfg) {
     if (cfg->capacity < 1024 || cfg->capacity > (1u << 25) || (cfg->extend_block % 32) || (cfg->shade_block % 32) ||
         cfg->extend_block <= 0 || cfg->extend_block > 128 || cfg->shade_block <= 0 || cfg->shade_block > 128 ||
         cfg->iters_per_graph <= 0 || cfg->iters_per_graph > 64 || cfg->ctas_per_sm < 0 || cfg->refill_min < 0 ||
-        cfg->refill_min > 32 || cfg->leaf_min < 0 || cfg->leaf_min > 32 || cfg->drain_paths < 0 ||
+        cfg->refill_min > 32 || cfg->leaf_min < 0 || cfg->leaf_min > 32 || cfg->drain_paths < -1 ||
         cfg->pixel_tile < 0 || cfg->pixel_tile > 1024 || cfg->steps_per_turn < 0 || cfg->steps_per_turn > 8)
         return set_error(ctx, WR_ERR_INVALID_ARGUMENT, "wavefront configuration out of range");
     ctx->wf_capacity = cfg->capacity;
@@ -70,7 +70,7 @@ int wr_autotune(wr_ctx* ctx, wr_scene_id scene, uint32_t spp_per_trial, uint32_t
         return (double)n / 3 * spp_per_trial / (ms * 1e-3) / 1e6;
     };
     // the shipped defaults, then one dimension at a time
-    wr_wavefront_config top{1u << 24, 128, 128, 6, 1, 8, 8, 1 << 13, 0, 6, 0.0};
+    wr_wavefront_config top{1u << 24, 128, 128, 6, 1, 8, 8, -1, 0, 6, 0.0};
     double top_rate = trial(top);
     enum { CAP, CTAS, REFILL, LEAF, STEPS, TILE, ITERS, NDIM };
     const std::vector<int> values[NDIM] = {
