@@ -280,6 +280,7 @@ int wr_serve_start(wr_ctx* ctx, const wr_serve_desc* desc) {
             return set_error(ctx, WR_ERR_INVALID_ARGUMENT, "paths_in_flight must be 1024 .. 2^25, reserved 0");
         int rc = wf_engine_get(ctx, wf_tuned_config(ctx), &S->E);
         if (rc != WR_OK) return rc;
+        if ((rc = wf_reserve_flights(ctx, S->E)) != WR_OK) return rc;  // no allocation while it serves
         S->short_queue = std::min(pif, wf_config(S->E).capacity);
         if ((rc = wf_set_live_cap(ctx, S->E, S->short_queue, S->stream)) != WR_OK) return rc;
         if ((rc = wf_set_equal_share(ctx, S->E, !(desc && (desc->flags & WR_SERVE_FIFO)))) != WR_OK) return rc;

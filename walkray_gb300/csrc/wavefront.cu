@@ -1052,7 +1052,6 @@ int wf_engine_get(wr_ctx* ctx, const WfConfig& cfg, WfEngine** out) {
         if (rc != WR_OK) return rc;
     }
     WR_CUDA(ctx, E->hits.reserve(sizeof(int2) * (size_t)cfg.capacity));
-    WR_CUDA(ctx, E->flights.reserve(sizeof(Flight) * (size_t)cfg.capacity));
     WR_CUDA(ctx, E->sort_mem.reserve(sizeof(uint32_t) * ((size_t)WF_SORT_KEYS * cfg.capacity + 64)));
     E->sort.counts = E->sort_mem.as<unsigned int>();
     E->sort.idx = E->sort.counts + 64;
@@ -1106,6 +1105,11 @@ int wf_engine_get(wr_ctx* ctx, const WfConfig& cfg, WfEngine** out) {
     E->grid_gen = ctx->num_sms * std::max(1, per_sm);
     *out = E.get();
     ctx->wavefront = E;
+    return WR_OK;
+}
+
+int wf_reserve_flights(wr_ctx* ctx, WfEngine* E) {
+    WR_CUDA(ctx, E->flights.reserve(sizeof(Flight) * (size_t)E->cfg.capacity));
     return WR_OK;
 }
 
@@ -1218,6 +1222,10 @@ int wf_update_jobs(wr_ctx* ctx, WfEngine* E, const std::vector<WfSlotUpdate>& up
             hetero_any |= RenderDataView::hetero(rd);
         }
         if (E->job_tab[slot].flags & (WR_RENDER_NEE | WR_RENDER_NEE_MIS)) conn_any = true;
+    }
+    if (hetero_any) {  // before the loop with the track stage is captured
+        const int rc = wf_reserve_flights(ctx, E);
+        if (rc != WR_OK) return rc;
     }
     E->hetero_any = hetero_any;
     E->walk_any = walk_any;

@@ -177,6 +177,9 @@ int wf_read_counters(wr_ctx* ctx, WfEngine* E, std::vector<WfJobCounters>& out, 
                      uint32_t* waiting = nullptr, int side = 0);
 // finishes the paths waiting in side `side` without the bounce loop (k_wf_finish)
 int wf_finish(wr_ctx* ctx, WfEngine* E, int side, cudaStream_t s);
+// the flights' memory (16 B per path of the queue), which a job of a scene with a
+// density grid needs; done by wf_update_jobs for such a job if it was not before
+int wf_reserve_flights(wr_ctx* ctx, WfEngine* E);
 int wf_error_word(wr_ctx* ctx, WfEngine* E, unsigned int* herr, cudaStream_t s);
 int wf_reset_queues(wr_ctx* ctx, WfEngine* E, cudaStream_t s);
 // free queue slots shared equally among the jobs with paths left (default)
