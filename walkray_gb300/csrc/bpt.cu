@@ -1608,7 +1608,7 @@ int render_bidirectional(wr_ctx* ctx, const RenderScene& S, const RenderParams& 
     // (64 B each), the counts, the lists and the batch's images in about 1 GiB
     const bool vol_grid = ppm && media;  // photon mapping's second grid, for the volume photons
     const uint32_t ngrid = vol_grid ? 2u : 1u;
-    const size_t per_sample = (ppm ? 1ull : 2ull) * nrec * 64 + 4 + 12 + (ppm ? 0 : 16ull * nrec * (nrec + 1)) +
+    const size_t per_sample = (ppm ? 1ull : 2ull) * nrec * 64 + 4 + 12 + (ppm ? 0 : 8ull * nrec * (nrec + 1)) +
                               (grid_on ? 12ull * nrec + 4ull * ngrid : 0) + (vcm ? 128 : 0) + (ppm ? 16ull * nrec : 0);
     const uint64_t max_samples = std::max<uint64_t>(npix, (1ull << 30) / per_sample);
     const uint32_t per_batch = (uint32_t)std::min<uint64_t>(spp, std::max<uint64_t>(1, max_samples / npix));
