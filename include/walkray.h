@@ -307,12 +307,11 @@ int wr_render_device(wr_ctx* ctx, wr_scene_id scene, const wr_render_desc* desc,
  * overlaps on the GPU race and must be serialised. */
 #define WR_NOALLOC_MAX_PIXELS 1048576u
 int wr_render_noalloc(wr_ctx* ctx, wr_scene_id scene, const wr_render_desc* desc, float* d_rgb_out, void* stream);
-/* Traversal status of the most recent wr_render_noalloc on this context's
- * device, read without allocating: waits for `stream` (NULL = the context's
- * stream) and stores the error word in *out_err: 0 when every traversal
- * finished, nonzero when a traversal stack would have overflowed (the image
- * of that call is then incomplete; wr_render reports the same case as
- * WR_ERR_INTERNAL).  Companion of wr_render_noalloc; no reference counterpart. */
+/* Status of the wr_render_noalloc calls on `stream` (NULL = the context's
+ * stream), without allocating: waits for the stream and stores 0 in *out_err
+ * (the renderer's search cannot run out of stack; an error of the stream's work
+ * is the return value).  Companion of wr_render_noalloc; no reference
+ * counterpart. */
 int wr_render_noalloc_status(wr_ctx* ctx, void* stream, unsigned int* out_err);
 
 /* Per-stage profile of one wavefront render (no reference counterpart: the

@@ -268,7 +268,7 @@ int wr_trace_closest_device(wr_ctx* ctx, wr_scene_id id, const float* d_rays, ui
     WR_CUDA(ctx, cudaSetDevice(ctx->device));
     unsigned long long* counter = ctx->scratch_words.as<unsigned long long>();
     unsigned int* err = reinterpret_cast<unsigned int*>(counter + 1);
-    WR_CUDA(ctx, cudaMemsetAsync(err, 0, sizeof(unsigned int), s));
+    if (trace_walks(sc->tree, ctx->trace_prune)) WR_CUDA(ctx, cudaMemsetAsync(err, 0, sizeof(unsigned int), s));
     const TraceTune tt = trace_tune_of(ctx);
     WR_CUDA(ctx, launch_trace_closest(sc->tree, d_rays, n, d_inside, d_contact, d_hits, counter, err, ctx->num_sms,
                                       ctx->trace_prune, s, &ctx->last_trace_blocks, &tt, ctx->wf_ctas_per_sm));
@@ -277,7 +277,7 @@ int wr_trace_closest_device(wr_ctx* ctx, wr_scene_id id, const float* d_rays, ui
 }
 
 // wr_trace_closest's copies and launches: rays in on `sin`, chunks traced on
-// the context's stream, hits (and, last, the error word into *herr) out on
+// the context's stream, hits (and, last, the walk's error word into *herr) out on
 // `sout`; the caller synchronises all three
 static cudaError_t enqueue_trace(wr_ctx* ctx, SceneGPU* sc, const float* rays, uint64_t n,
                                  const wr_trace_filter* filter, wr_hit* hits, int K, cudaStream_t sin,
@@ -286,7 +286,8 @@ static cudaError_t enqueue_trace(wr_ctx* ctx, SceneGPU* sc, const float* rays, u
     unsigned long long* counter = ctx->scratch_words.as<unsigned long long>();
     unsigned int* err = reinterpret_cast<unsigned int*>(counter + 1);
     const TraceTune tt = trace_tune_of(ctx);
-    cudaError_t e = cudaMemsetAsync(err, 0, sizeof(unsigned int), s);
+    const bool walks = trace_walks(sc->tree, ctx->trace_prune);
+    cudaError_t e = walks ? cudaMemsetAsync(err, 0, sizeof(unsigned int), s) : cudaSuccess;
 #define WR_TRY(call)                     \
     do {                                 \
         if (e == cudaSuccess) e = (call); \
@@ -325,8 +326,8 @@ static cudaError_t enqueue_trace(wr_ctx* ctx, SceneGPU* sc, const float* rays, u
         WR_TRY(cudaMemcpyAsync(hits + a, ctx->hits.as<wr_hit>() + a, m * sizeof(wr_hit), cudaMemcpyDeviceToHost,
                                sout));
     }
-    // the error word after the last kernel (sout waited for it)
-    WR_TRY(cudaMemcpyAsync(herr, err, sizeof *herr, cudaMemcpyDeviceToHost, sout));
+    // the walk's error word after the last kernel (sout waited for it)
+    if (walks) WR_TRY(cudaMemcpyAsync(herr, err, sizeof *herr, cudaMemcpyDeviceToHost, sout));
 #undef WR_TRY
     return e;
 }

@@ -295,8 +295,6 @@ int wr_render(wr_ctx* ctx, wr_scene_id id, const wr_render_desc* desc, float* rg
         DeviceBuffer& film = ctx->film;
         WR_CUDA(ctx, film.reserve(sizeof(float) * std::max<size_t>(n, 1)));
         cudaStream_t s = ctx->stream;
-        unsigned int* err = reinterpret_cast<unsigned int*>(ctx->scratch_words.as<unsigned long long>() + 1);
-        WR_CUDA(ctx, cudaMemsetAsync(err, 0, sizeof(unsigned int), s));
         WR_CUDA(ctx, cudaMemsetAsync(film.p, 0, sizeof(float) * n, s));
         int rc = wr_render_device(ctx, id, desc, film.as<float>(), nullptr, s);
         if (rc != WR_OK) return rc;
@@ -305,10 +303,7 @@ int wr_render(wr_ctx* ctx, wr_scene_id id, const wr_render_desc* desc, float* rg
         WR_CUDA(ctx, cudaGetLastError());
         ctx->kernel_launches++;
         WR_CUDA(ctx, cudaMemcpyAsync(rgb_out, film.p, sizeof(float) * n, cudaMemcpyDeviceToHost, s));
-        unsigned int herr = 0;
-        WR_CUDA(ctx, cudaMemcpyAsync(&herr, err, sizeof herr, cudaMemcpyDeviceToHost, s));
         WR_CUDA(ctx, cudaStreamSynchronize(s));
-        if (herr) return set_error(ctx, WR_ERR_INTERNAL, "traversal stack overflow");
         return WR_OK;
     } catch (const std::exception& ex) {
         return set_error(ctx, WR_ERR_INTERNAL, ex.what());
@@ -338,8 +333,6 @@ int wr_render_progressive(wr_ctx* ctx, wr_scene_id id, const wr_render_desc* des
         float* sum = film.as<float>();
         float* mean = sum + n;
         cudaStream_t s = ctx->stream;
-        unsigned int* err = reinterpret_cast<unsigned int*>(ctx->scratch_words.as<unsigned long long>() + 1);
-        WR_CUDA(ctx, cudaMemsetAsync(err, 0, sizeof(unsigned int), s));
         WR_CUDA(ctx, cudaMemsetAsync(sum, 0, sizeof(float) * n, s));
         uint32_t done = 0;
         while (done < desc->spp) {
@@ -354,10 +347,7 @@ int wr_render_progressive(wr_ctx* ctx, wr_scene_id id, const wr_render_desc* des
             WR_CUDA(ctx, cudaGetLastError());
             ctx->kernel_launches++;
             WR_CUDA(ctx, cudaMemcpyAsync(rgb_out, mean, sizeof(float) * n, cudaMemcpyDeviceToHost, s));
-            unsigned int herr = 0;
-            WR_CUDA(ctx, cudaMemcpyAsync(&herr, err, sizeof herr, cudaMemcpyDeviceToHost, s));
             WR_CUDA(ctx, cudaStreamSynchronize(s));
-            if (herr) return set_error(ctx, WR_ERR_INTERNAL, "traversal stack overflow");
             if (spp_done) *spp_done = done;
             if (progress && progress(user, rgb_out, done) != 0) break;
         }

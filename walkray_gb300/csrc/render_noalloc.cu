@@ -11,7 +11,7 @@
 // instead.
 //
 // The scratch: `g_film` below, a file-scope device array of
-// WR_NOALLOC_MAX_PIXELS * 3 floats (12 MiB) plus an error word.  Every GPU
+// WR_NOALLOC_MAX_PIXELS * 3 floats (12 MiB).  Every GPU
 // that loads the library holds it until the process exits.  All calls on a
 // device share it, and it keeps the previous call's contents; each call clears
 // the part it uses first.  Two calls whose work overlaps on the GPU (for
@@ -24,9 +24,9 @@
 // context (the one the CUDA runtime uses); calls must be made with that
 // context current.
 //
-// The traversal error word (a per-thread stack that would overflow) is
-// cleared by each call and set by its kernels; wr_render_noalloc_status reads
-// it back, also without allocating.
+// The megakernel's search has no traversal error to report (a ray that would
+// outgrow its stack takes a walk without one), so wr_render_noalloc_status
+// waits for the stream and answers 0.
 #include <cuda_runtime.h>
 
 #include <algorithm>
@@ -40,32 +40,25 @@
 namespace wr {
 
 static __device__ __align__(256) float g_film[3 * WR_NOALLOC_MAX_PIXELS];
-static __device__ __align__(256) unsigned int g_err_word[64];
 
 namespace {
 
 constexpr int MAX_DEVICES = 64;
 std::mutex g_mu;
 float* g_film_addr[MAX_DEVICES] = {};
-unsigned int* g_err_addr[MAX_DEVICES] = {};
 
-// device addresses of the scratch arrays on `dev` (set-up on first use)
-int scratch_for(wr_ctx* ctx, float** film, unsigned int** err) {
+// device address of the film on the context's device (set-up on first use)
+int scratch_for(wr_ctx* ctx, float** film) {
     const int dev = ctx->device;
     if (dev < 0 || dev >= MAX_DEVICES) return set_error(ctx, WR_ERR_UNSUPPORTED, "device ordinal too large");
     std::lock_guard<std::mutex> lk(g_mu);
     if (!g_film_addr[dev]) {
         void* f = nullptr;
-        void* e = nullptr;
         cudaError_t rc = cudaGetSymbolAddress(&f, g_film);
         if (rc != cudaSuccess) return cuda_error(ctx, rc, "cudaGetSymbolAddress(film)");
-        rc = cudaGetSymbolAddress(&e, g_err_word);
-        if (rc != cudaSuccess) return cuda_error(ctx, rc, "cudaGetSymbolAddress(error word)");
         g_film_addr[dev] = static_cast<float*>(f);
-        g_err_addr[dev] = static_cast<unsigned int*>(e);
     }
     *film = g_film_addr[dev];
-    *err = g_err_addr[dev];
     return WR_OK;
 }
 
@@ -105,13 +98,11 @@ static int render_noalloc_body(wr_ctx* ctx, wr_scene_id id, const wr_render_desc
     const RenderScene& S = RenderDataView::scene(rd);
     WR_CUDA(ctx, cudaSetDevice(ctx->device));
     float* film = nullptr;
-    unsigned int* err = nullptr;
-    int rc = scratch_for(ctx, &film, &err);
+    int rc = scratch_for(ctx, &film);
     if (rc != WR_OK) return rc;
     cudaStream_t s = stream ? static_cast<cudaStream_t>(stream) : ctx->stream;
     const size_t n = 3 * (size_t)npix;
     WR_CUDA(ctx, cudaMemsetAsync(film, 0, sizeof(float) * n, s));
-    WR_CUDA(ctx, cudaMemsetAsync(err, 0, sizeof(unsigned int), s));
     RenderParams P{};
     P.seed = desc->seed;
     P.max_path_len = desc->max_path_len;
@@ -143,15 +134,9 @@ extern "C" int wr_render_noalloc_status(wr_ctx* ctx, void* stream, unsigned int*
     if (!ctx || !out_err) return set_error(ctx, WR_ERR_INVALID_ARGUMENT, "null argument");
     try {
         WR_CUDA(ctx, cudaSetDevice(ctx->device));
-        float* film = nullptr;
-        unsigned int* err = nullptr;
-        int rc = scratch_for(ctx, &film, &err);
-        if (rc != WR_OK) return rc;
         cudaStream_t s = stream ? static_cast<cudaStream_t>(stream) : ctx->stream;
-        unsigned int word = 0;
-        WR_CUDA(ctx, cudaMemcpyAsync(&word, err, sizeof word, cudaMemcpyDeviceToHost, s));
         WR_CUDA(ctx, cudaStreamSynchronize(s));
-        *out_err = word;
+        *out_err = 0;
         return WR_OK;
     } catch (const std::exception& ex) {
         return set_error(ctx, WR_ERR_INTERNAL, ex.what());

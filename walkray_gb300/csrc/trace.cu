@@ -69,8 +69,8 @@ template <int MINB>
 __global__ void __launch_bounds__(128, MINB > 0 ? MINB : 1)
     k_trace_closest(const __grid_constant__ DevTree T, const float* __restrict__ rays, uint64_t n,
                     const int32_t* __restrict__ inside, const int32_t* __restrict__ contact,
-                    wr_hit* __restrict__ hits, unsigned long long* __restrict__ counter, int stack_cap, TraceTune tune,
-                    unsigned int* __restrict__ err) {
+                    wr_hit* __restrict__ hits, unsigned long long* __restrict__ counter, int stack_cap,
+                    TraceTune tune) {
     extern __shared__ __align__(16) uint32_t s_stack[];
     BatchSrc src{T, rays, inside, contact, hits, inside != nullptr};
     TraceWork work;
@@ -109,7 +109,7 @@ cudaError_t launch_trace_closest(const DevTree& T, const float* d_rays, uint64_t
     const int block = 128;
     const int ref_cap = (int)T.max_depth + 3;  // stack of the reference's own walk
     if ((size_t)ref_cap * block * sizeof(uint32_t) > 200 * 1024) return cudaErrorInvalidValue;
-    const bool search = prune && T.quads;
+    const bool search = !trace_walks(T, prune);
     const int stack_cap = search ? quad_stack_cap(T) : ref_cap;
     const size_t smem = search ? quad_smem(stack_cap, block) : (size_t)stack_cap * block * sizeof(uint32_t);
     cudaError_t e = cudaMemsetAsync(d_counter, 0, sizeof(unsigned long long), stream);
@@ -118,17 +118,17 @@ cudaError_t launch_trace_closest(const DevTree& T, const float* d_rays, uint64_t
     int per_sm = 1;
     // 0: the 6-CTA variant (80 registers; 2^24 rays: 2.23 ms, 2.38 with 7, 2.64 with 5, 2.69 with 8)
     const int variant = ctas_per_sm ? ctas_per_sm : 6;
-    void (*kern)(DevTree, const float*, uint64_t, const int32_t*, const int32_t*, wr_hit*, unsigned long long*, int,
-                 TraceTune, unsigned int*) = !search        ? (prune ? k_trace_closest_walk<true> : k_trace_closest_walk<false>)
-                                             : variant >= 8 ? k_trace_closest<8>
-                                             : variant >= 7 ? k_trace_closest<7>
-                                             : variant >= 6 ? k_trace_closest<6>
-                                                            : k_trace_closest<0>;
+    const auto kern = variant >= 8   ? k_trace_closest<8>
+                      : variant >= 7 ? k_trace_closest<7>
+                      : variant >= 6 ? k_trace_closest<6>
+                                     : k_trace_closest<0>;
+    const auto walk = prune ? k_trace_closest_walk<true> : k_trace_closest_walk<false>;
+    const void* fn = search ? reinterpret_cast<const void*>(kern) : reinterpret_cast<const void*>(walk);
     if (smem > 48 * 1024) {
-        e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+        e = cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
         if (e != cudaSuccess) return e;
     }
-    e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kern, block, smem);
+    e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, fn, block, smem);
     if (e != cudaSuccess) return e;
     if (ctas_per_sm > 0) per_sm = std::min(per_sm, ctas_per_sm);
     if (per_sm < 1) per_sm = 1;
@@ -138,7 +138,10 @@ cudaError_t launch_trace_closest(const DevTree& T, const float* d_rays, uint64_t
     if ((uint64_t)grid > need_blocks) grid = (int)(need_blocks ? need_blocks : 1);
     if (launched_blocks) *launched_blocks = grid;
     const TraceTune tt = tune ? *tune : default_trace_tune();
-    kern<<<grid, block, smem, stream>>>(T, d_rays, n, d_inside, d_contact, d_hits, d_counter, stack_cap, tt, d_err);
+    if (search)
+        kern<<<grid, block, smem, stream>>>(T, d_rays, n, d_inside, d_contact, d_hits, d_counter, stack_cap, tt);
+    else
+        walk<<<grid, block, smem, stream>>>(T, d_rays, n, d_inside, d_contact, d_hits, d_counter, stack_cap, tt, d_err);
     return cudaGetLastError();
 }
 
