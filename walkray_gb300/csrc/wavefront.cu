@@ -1532,23 +1532,27 @@ int render_wavefront(wr_ctx* ctx, RenderData& rd, const RenderParams& P, uint32_
         const uint64_t max_launches =
             1 + (total / std::max<uint32_t>(1, E->cfg.capacity) + 4) * (uint64_t)(P.max_path_len + 4) * 4;
         uint64_t queued = 0, seen = 0;
-        for (;;) {
-            while (queued == seen || (queued == seen + 1 && (st->claimed < total || st->waiting / 4 > few))) {
-                if ((rc = wf_launch(ctx, E, s)) != WR_OK) return rc;
-                WR_CUDA(ctx, cudaEventRecord(E->turn[queued & 1], s));
-                queued++;
+        const auto loop = [&]() -> int {
+            for (;;) {
+                while (queued == seen || (queued == seen + 1 && (st->claimed < total || st->waiting / 4 > few))) {
+                    const int r = wf_launch(ctx, E, s);
+                    if (r != WR_OK) return r;
+                    WR_CUDA(ctx, cudaEventRecord(E->turn[queued & 1], s));
+                    queued++;
+                }
+                WR_CUDA(ctx, cudaEventSynchronize(E->turn[seen & 1]));
+                seen++;
+                if (st->finished >= total) {
+                    finished = true;
+                    return WR_OK;
+                }
+                if (queued == seen && st->claimed >= total && st->waiting <= few) return wf_finish(ctx, E, 0, s);
+                if (seen > max_launches) return set_error(ctx, WR_ERR_TIMEOUT, "wavefront did not drain");
             }
-            WR_CUDA(ctx, cudaEventSynchronize(E->turn[seen & 1]));
-            seen++;
-            if (st->finished >= total) {
-                finished = true;
-                break;
-            }
-            if (queued == seen && st->claimed >= total && st->waiting <= few) {
-                if ((rc = wf_finish(ctx, E, 0, s)) != WR_OK) return rc;
-                break;
-            }
-            if (seen > max_launches) return set_error(ctx, WR_ERR_TIMEOUT, "wavefront did not drain");
+        };
+        if ((rc = loop()) != WR_OK) {
+            cudaStreamSynchronize(s);  // a queued replay may still write the caller's film
+            return rc;
         }
     }
     // the job's counters and the error word
