@@ -195,10 +195,7 @@ static __device__ __noinline__ bool box_faces(Box b, f3 o, f3 d, float scene_mag
 // Anything else -- an edge within M, a NaN -- runs the face tests.  With
 // QuadRay's constants the planes moved in are fb for a near and nb for a far
 // one.
-// `quick`: the boxes are finite (else the face tests decide: on an infinite
-// plane the reference's point is infinite or a NaN).
-__device__ __forceinline__ bool reference_passes(const Box& b, const QuadRay& r, f3 o, f3 d, float scene_mag,
-                                                 bool quick) {
+__device__ __forceinline__ bool reference_passes(const Box& b, const QuadRay& r, f3 o, f3 d, float scene_mag) {
     const bool px = r.inv.x > 0.f, py = r.inv.y > 0.f, pz = r.inv.z > 0.f;
     const float fx = px ? b.hx : b.lx, fy = py ? b.hy : b.ly, fz = pz ? b.hz : b.lz;
     const float nx = __fmaf_rn(px ? b.lx : b.hx, r.inv.x, r.fb.x), ny = __fmaf_rn(py ? b.ly : b.hy, r.inv.y, r.fb.y),
@@ -210,7 +207,7 @@ __device__ __forceinline__ bool reference_passes(const Box& b, const QuadRay& r,
     const bool by_x = (ny <= sx) & (nz <= sx) & (sy >= gx) & (sz >= gx) & (sx >= 0.f);
     const bool by_y = (nx <= sy) & (nz <= sy) & (sx >= gy) & (sz >= gy) & (sy >= 0.f);
     const bool by_z = (nx <= sz) & (ny <= sz) & (sx >= gz) & (sy >= gz) & (sz >= 0.f);
-    return (quick & (by_x | by_y | by_z)) || box_faces(b, o, d, scene_mag);
+    return (by_x | by_y | by_z) || box_faces(b, o, d, scene_mag);
 }
 
 // Does the reference's predicate pass on every box above `slot`'s triangle?
@@ -220,16 +217,18 @@ __device__ __forceinline__ bool reference_passes(const Box& b, const QuadRay& r,
 static __device__ __noinline__ bool reference_reaches(const DevTree& T, int slot, f3 o, f3 d) {
     QuadRay r;
     make_quad_ray(o, d, T.finite_mag, box_margin(o, T.finite_mag), r);
-    const bool quick = T.scene_mag < INFINITY;
+    // boxes with an infinite plane: the face tests decide (there the reference's
+    // point is infinite or a NaN)
+    if (!(T.scene_mag < INFINITY)) r.nb = mk(NAN, NAN, NAN);
     for (uint32_t at = __ldg(T.leaf_up + slot); at != UP_ROOT;) {
         const uint4 up = ldg4u(T.pair_up + (at >> 1));
         const uint32_t a[4] = {at, up.x, up.y, up.z};
         at = up.w;
 #pragma unroll
         for (int k = 0; k < 4; k++)
-            if (a[k] != UP_ROOT && !reference_passes(child_box(T, a[k]), r, o, d, T.scene_mag, quick)) return false;
+            if (a[k] != UP_ROOT && !reference_passes(child_box(T, a[k]), r, o, d, T.scene_mag)) return false;
     }
-    return reference_passes(root_box(T), r, o, d, T.scene_mag, quick);
+    return reference_passes(root_box(T), r, o, d, T.scene_mag);
 }
 
 // Closest hit where the reference's predicate decides every descent, without
