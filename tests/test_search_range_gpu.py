@@ -1,5 +1,5 @@
 """The four-wide search over the whole range of directions and coordinates that
-it takes (wr_quad.cuh: |d| from 1e-15 to 1e15, coordinates to 1e18) against the
+it takes (wr_quad.cuh: |d| from 1e-15 to 1e14, coordinates to 1e15 |d|) against the
 walk that visits every box the reference visits: the same triangle ids and the
 same t bit for bit on both sides of the range's ends, and rays of any length at
 the speed of unit ones."""

@@ -25,16 +25,15 @@
 // Pruning by distance is the rule of wr_traverse.cuh (q.pf, graze_check).
 //
 // Directions need not be of unit length: distances are in units of |d|, the
-// pruning rule's margin too (direction_unit).  Rays that are left to
-// reference_search() alone: |d| outside [1e-15, 1e15], where squares of d leave
-// the float range and the reference's distances may be subnormal (half an ulp
-// of one is 7e-46, times |d| below the 1e-30 in M); coordinates beyond 1e18 or
-// 1e19 |d|, where the slabs' products would overflow, and M below 1e-36 |d|,
-// where they would be subnormal; values that are not finite.  (B leaves out a
-// scene's coordinates that are not finite: boxes with such a plane are always
-// visited, see build_quads.)  A direction
-// component below 1e-18 of the direction's length is taken as that small: over
-// the scene's extent the ray moves by less than M along that axis either way.
+// pruning rule's margin too.  Rays that are left to reference_search() alone:
+// |d| outside [1e-15, 1e14], where squares of d leave the float range or
+// distances may be subnormal (half an ulp of one is 7e-46, times |d| far below
+// the 1e-30 in M); coordinates beyond 1e15 |d|, where the slabs' products could
+// overflow; values that are not finite.  (B leaves out a scene's coordinates
+// that are not finite: boxes with such a plane are always visited, see
+// build_quads.)  A direction component below 1e-18 of the direction's length is
+// taken as that small: over the scene's extent the ray moves by less than M
+// along that axis either way.
 // (With bounds of 1e-6 and 1e6 on |d| and 1e9 on coordinates 2^20 rays of length
 // 1e7 took 2.97 ms, of unit length 0.18.)
 //
@@ -50,11 +49,6 @@ struct QuadRay {
     f3 inv;              // 1/d
     f3 nb, fb;           // plane * inv + nb (fb): distance to a near (far) plane moved out by M
 };
-
-// 1 / |d|, within a factor of two, as a power of two (1 for a unit vector)
-__device__ __forceinline__ float direction_unit(f3 d) {
-    return __int_as_float(0x7f000000 - (__float_as_int(fabsf(d.x) + fabsf(d.y) + fabsf(d.z)) & 0x7f800000));
-}
 
 // the margin M (wr_traverse.cuh)
 __device__ __forceinline__ float box_margin(f3 o, float scene_mag) {
@@ -73,8 +67,7 @@ __device__ __forceinline__ bool make_quad_ray(f3 o, f3 d, float scene_mag, float
               __fmaf_rn(-o.z, r.inv.z, -M * fabsf(r.inv.z)));
     r.fb = mk(__fmaf_rn(-o.x, r.inv.x, M * fabsf(r.inv.x)), __fmaf_rn(-o.y, r.inv.y, M * fabsf(r.inv.y)),
               __fmaf_rn(-o.z, r.inv.z, M * fabsf(r.inv.z)));
-    const float ext = on + scene_mag;
-    return ext <= 1e18f && ext <= 1e19f * dn && dn >= 1e-15f && dn <= 1e15f && M >= 1e-36f * dn;  // false for a NaN
+    return on + scene_mag <= 1e15f * dn && dn >= 1e-15f && dn <= 1e14f;  // false for a NaN
 }
 
 // of three at once (a NaN is dropped, as by fmaxf and fminf)
@@ -216,10 +209,10 @@ __device__ __forceinline__ bool reference_passes(const Box& b, const QuadRay& r,
 // search spill (mixed-material scene 1024^2 x 32 spp 34.7 ms, 34.0 this way).
 static __device__ __noinline__ bool reference_reaches(const DevTree& T, int slot, f3 o, f3 d) {
     QuadRay r;
-    make_quad_ray(o, d, T.finite_mag, box_margin(o, T.finite_mag), r);
-    // boxes with an infinite plane: the face tests decide (there the reference's
-    // point is infinite or a NaN)
-    if (!(T.scene_mag < INFINITY)) r.nb = mk(NAN, NAN, NAN);
+    // (in a scene with an infinite coordinate M is infinite here and no box is
+    // told by its planes: on an infinite plane the reference's point is infinite
+    // or a NaN, so the face tests decide)
+    make_quad_ray(o, d, T.scene_mag, box_margin(o, T.scene_mag), r);
     for (uint32_t at = __ldg(T.leaf_up + slot); at != UP_ROOT;) {
         const uint4 up = ldg4u(T.pair_up + (at >> 1));
         const uint32_t a[4] = {at, up.x, up.y, up.z};
@@ -406,7 +399,8 @@ struct SearchLane {
         pend = NO_WORD;
         const float M = box_margin(o, T.finite_mag);
         const bool ok = make_quad_ray(o, d, T.finite_mag, M, r) && quads;
-        ray.set(&T, o, d, pf < INFINITY ? M * direction_unit(d) : INFINITY, filt, inside, contact, enough);
+        const float unit = min3(fabsf(r.inv.x), fabsf(r.inv.y), fabsf(r.inv.z));  // 1 / |d| to 1.7 / |d|
+        ray.set(&T, o, d, pf < INFINITY ? M * unit : INFINITY, filt, inside, contact, enough);
         h = Hit{INFINITY, ok ? -1 : SLOT_REFERENCE};
         cur = ok ? 0u : NO_WORD;
     }
