@@ -223,6 +223,20 @@ def cpu_baseline_pt(scene, rows: int, threads: int):
                       f"WalkRay's PathTracer restated in C (oracle), {threads} OpenMP threads, tree build excluded"}
 
 
+def dram_roofline(kernel, profile, rays_per_s, rays_per_launch, peak, peak_kind):
+    """A search kernel against the HBM roofline: the DRAM bytes per ray of its
+    captured launch (profiles/<profile>; without it the ray's own input and
+    output) at the measured rate.  Neither search is bound there: the L1
+    cache's load pipe and the latency behind it are (profiles/*.md)."""
+    path = os.path.join(ROOT, "profiles", profile)
+    captured = json.load(open(path)).get("dram_bytes_per_ray") if os.path.exists(path) else None
+    per_ray = captured or RAY_IO_BYTES
+    achieved = per_ray * rays_per_s / 1e9
+    return {"bound": "hbm", "kernel": kernel, "achieved": round(achieved, 1), "peak": peak, "unit": "GB/s",
+            "frac": round(achieved / peak, 4), "traffic": round(captured * rays_per_launch, 0) if captured else None,
+            "peak_source": peak_kind, "dram_bytes_per_ray": per_ray, "limiter": "L1 load pipe and latency"}
+
+
 def time_to_relmse(ctx, sid, flags, ms_per_spp):
     """Time to relMSE 1e-3 of one estimator: per-pixel variance from 64 spp
     (sum and sum of squares) against R, an independent 256-spp image of the
@@ -311,25 +325,21 @@ def run_pt(args, world, rank, local):
                                               "renders of this scene")
     if rank == 0 and not args.quick:
         # roofline of the dominant kernel (the extend / traversal stage), from a
-        # profiled render of one step.  Algorithmic bytes count the reference's
-        # traversal work (every box and triangle KDTree::intersect visits: the
-        # same render with WR_RENDER_EXACT_TRAVERSAL); the time is that of the
-        # default (pruned) extend stage.
+        # profiled render of one step: the DRAM bytes of the captured launch per
+        # ray over the stage's time.  Beside it the work of the reference's own
+        # traversal on the same rays (every box and triangle KDTree::intersect
+        # visits: the same render with WR_RENDER_EXACT_TRAVERSAL), which the
+        # search does not do and which is therefore no roofline.
         prof = ctx.profile_render(sid, PT_SPP, PT_DEPTH, film.data_ptr(), seed=seed + 2)
         refw = ctx.profile_render(sid, PT_SPP, PT_DEPTH, film.data_ptr(), seed=seed + 2, exact=True)
         peak, peak_kind = peaks()
         alg = refw["rays"] * RAY_IO_BYTES + refw["box_tests"] * BOX_BYTES + refw["tri_tests"] * TRI_BYTES
-        achieved = alg / (prof["ms_extend"] / 1e3) / 1e9
-        traffic = None
-        pf = os.path.join(ROOT, "profiles", "wf_extend_pt.json")
-        if os.path.exists(pf):
-            per_ray = json.load(open(pf)).get("dram_bytes_per_ray")
-            traffic = round(per_ray * prof["rays"] / max(1, prof["iterations"]), 0) if per_ray else None
         nr = max(1, refw["rays"])
-        line["roofline"] = {
-            "bound": "hbm", "kernel": "k_wf_extend", "achieved": round(achieved, 1), "peak": peak, "unit": "GB/s",
-            "frac": round(achieved / peak, 4), "traffic": traffic, "peak_source": peak_kind,
-            "algorithmic_bytes_per_ray": round(alg / nr, 1),
+        extend_s = prof["ms_extend"] / 1e3
+        line["roofline"] = dram_roofline("k_wf_extend", "wf_extend_pt.json", prof["rays"] / extend_s,
+                                         prof["rays"] / max(1, prof["iterations"]), peak, peak_kind) | {
+            "reference_walk_bytes_per_ray": round(alg / nr, 1),
+            "reference_walk_gbs": round(alg / extend_s / 1e9, 1),
             "reference_box_tests_per_ray": round(refw["box_tests"] / nr, 3),
             "reference_tri_tests_per_ray": round(refw["tri_tests"] / nr, 3),
             "executed_box_tests_per_ray": round(prof["box_tests"] / max(1, prof["rays"]), 3),
@@ -845,12 +855,6 @@ def run_kd(args, world, rank, local):
     e2e = allreduce(world, float(n * args.steps), "sum") / e2e_s / 1e6
 
     peak, peak_kind = peaks()
-    achieved = KD_BYTES_PER_RAY * n / avg_launch_s / 1e9
-    traffic = None
-    prof = os.path.join(ROOT, "profiles", "trace_closest_kd.json")
-    if os.path.exists(prof):
-        per_ray = json.load(open(prof)).get("dram_bytes_per_ray")
-        traffic = round(per_ray * n, 0) if per_ray else None
     line = {
         "metric": "Mrays/s (closest hit, bit-exact vs reference)", "value": round(value, 2), "unit": "Mrays/s",
         "n_gpus": world, "steps": args.steps, "warmup": args.warmup,
@@ -859,9 +863,9 @@ def run_kd(args, world, rank, local):
         "config": {"workload": KD_WORKLOAD, "rays_per_step": n, "l2": "flushed (512 MiB write) before every step",
                    "parallelism": f"replicas x{world}"},
         "e2e": {"value": round(e2e, 2), "unit": "Mrays/s", "h2d_bytes_per_step": n * 24, "d2h_bytes_per_step": n * 16},
-        "roofline": {"bound": "hbm", "kernel": "k_trace_closest", "achieved": round(achieved, 1), "peak": peak,
-                     "unit": "GB/s", "frac": round(achieved / peak, 4), "traffic": traffic, "peak_source": peak_kind,
-                     "algorithmic_bytes_per_ray": round(KD_BYTES_PER_RAY, 1)},
+        "roofline": dram_roofline("k_trace_closest", "trace_closest_kd.json", n / avg_launch_s, n, peak, peak_kind) | {
+            "reference_walk_bytes_per_ray": round(KD_BYTES_PER_RAY, 1),
+            "reference_walk_gbs": round(KD_BYTES_PER_RAY * n / avg_launch_s / 1e9, 1)},
         "gpu_launches": int(n_launch), "clocks": clk.summary(),
     }
     if rank == 0 and world == 1 and not args.no_cpu:

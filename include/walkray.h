@@ -322,7 +322,8 @@ typedef struct wr_render_profile {
     double ms_extend, ms_shade, ms_shadow, ms_generate, ms_total;
     uint64_t iterations;       /* bounce iterations run */
     uint64_t rays;             /* rays traced by the extend stage */
-    uint64_t box_tests;        /* AABB predicate evaluations (reference count) */
+    uint64_t box_tests;        /* boxes tested: the four-wide search's children (4 a node, holes
+                                  among them); with WR_RENDER_EXACT_TRAVERSAL the reference's count */
     uint64_t tri_tests;        /* ray-triangle tests */
     uint64_t paths;
     double ms_drain;           /* the per-path finish of the last paths (k_wf_finish) */

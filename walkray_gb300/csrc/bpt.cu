@@ -32,10 +32,9 @@
 // the two connection vertices, which connectEdge changes and which live in
 // registers.  Draws: the eye sub-path takes the Philox stream of (pixel,
 // sample) from draw 0, the light sub-path the same stream from draw 2^30;
-// the connections draw nothing.  Homogeneous media take part (their
-// free-flight densities are origin densities of the MIS weights);
-// heterogeneous ones do not (their densities need an integration along every
-// link) and scenes with one are refused by the caller.
+// the connections draw nothing.  Media take part: their free-flight densities
+// are origin densities of the MIS weights, a heterogeneous medium's integrated
+// along every link (kernels of their own).
 #include <algorithm>
 #include <memory>
 
@@ -878,8 +877,8 @@ __device__ void bpt_connect_one(const RenderScene& S, const BptParams& P, uint32
 }
 
 // persistent: the warps stride over the runs of 32 connections of one (l, e)
-// pair.  What is left is instruction fetch and the FP64 sums (a fifth of the
-// unit's rate).  Four blocks per SM (120 registers; five spill), the marching
+// pair.  What is left is instruction fetch and the FP64 products and sums (the
+// unit is 44 % busy).  Four blocks per SM (120 registers; five spill), the marching
 // instantiation one.  Batch of the bidirectional Cornell box: 1.30 ms over one
 // mixed list with 15.8 lanes at work, 0.58 with 30.9.
 template <bool HM>

@@ -7,9 +7,9 @@
 // a warp's pushes hit 32 distinct banks.
 //
 // Bound by the L1 cache's load pipe and the latency behind it: on 4.2 M
-// incoherent rays (1,310,720-triangle icosphere) the pipe is 64 % busy, issue
-// 46 %, 78 warp instructions a ray (174 when it walked the reference's tree with
-// two slab tests a box).  2^24 rays: 3.38 -> 2.23 ms.
+// incoherent rays (1,310,720-triangle icosphere) the pipe is 56 % busy, issue
+// 46 %, 75 warp instructions a ray (174 when it walked the reference's tree with
+// two slab tests a box).  2^24 rays: 3.38 -> 2.05 to 2.2 ms.
 #include <cuda_runtime.h>
 
 #include <algorithm>

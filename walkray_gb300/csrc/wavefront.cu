@@ -466,7 +466,8 @@ using ExtendKernel = void (*)(const RenderScene*, const WfJob*, WfSide, int2*, u
 
 // shadow stage, first half: the closest hit of every connection in the
 // shadow queue, through the same warp-persistent loop as extend (filtered by
-// the connection's inside / contact objects, as trace_closest<true, true>)
+// the connection's inside / contact objects).  WALK: the reference's own tree
+// (launched while a scene without a four-wide tree is in the table)
 struct ShadowSrc {
     const RenderScene* __restrict__ scenes;
     const WfJob* __restrict__ jobs;

@@ -79,14 +79,16 @@ struct DevTree {
     uint32_t quad_stack;      // stack entries that the deepest walk of `quads` can need
 };
 
-// Knobs of the warp-persistent traversal loop (wr_warp_trace.cuh)
+// Knobs of the warp-persistent loops (wr_quad_trace.cuh, wr_warp_trace.cuh)
 struct TraceTune {
     int refill_min;  // refill idle lanes once at least this many are idle (or none is busy)
     int leaf_min;    // lanes holding postponed leaves that start the warp's leaf phase
-    int steps;       // traversal steps a searching lane takes per turn of the warp loop (1..8)
+    int steps;       // nodes (four-wide or pairs) a searching lane visits per turn of the warp loop (1..8)
 };
-// fastest of sweeps on GB300, kd workload: 4349 Mrays/s with one step per
-// turn, 4568 with four, 4699 with six, 4673 with eight
+// Fastest of sweeps on the four-wide search, 2^24 rays and a 1024^2 x 16-spp
+// mixed-material film: six steps 2.21 ms and 15.4 (one 2.33 and 16.3, two 2.31 and
+// 15.7, four 2.25 and 15.4, eight 2.29 and 15.7); leaf_min 4 and refill_min 4 the
+// same within 1.5 %, 16 two to four percent slower.
 inline TraceTune default_trace_tune() { return TraceTune{8, 8, 6}; }
 
 struct f3 {

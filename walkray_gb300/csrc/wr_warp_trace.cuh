@@ -1,13 +1,14 @@
 // wr_warp_trace.cuh — the warp-persistent walk of the reference's own tree: the
 // exact forms of the batch kernel and of the wavefront's extend stage
 // (WR_CTX_EXACT_TRAVERSAL, WR_RENDER_EXACT_TRAVERSAL), which visit every box
-// the reference visits and count them.  wr_quad_trace.cuh is the search that
-// everything else runs.
+// the reference visits and count them, and what these and the shadow stage run
+// where a scene has no four-wide tree (build_quads).  wr_quad_trace.cuh is the
+// search that everything else runs.
 //
-// Same result as trace_closest() (wr_traverse.cuh): the same box predicate
-// decides every descent and the winner is order-free ("smallest t, then
-// largest slot"), so visiting order and the moment a leaf is tested do not
-// change it.  What changes is how a warp's 32 lanes are kept busy:
+// The reference's box predicate (wr_traverse.cuh) decides every descent and the
+// winner is order-free ("smallest t, then largest slot"), so that visiting order
+// and the moment a leaf is tested do not change it.  How a warp's 32 lanes are
+// kept busy:
 //
 //  * postponed leaves: a lane that reaches leaves parks them and waits; once
 //    `leaf_min` lanes hold leaves (or no lane is left searching) the warp
