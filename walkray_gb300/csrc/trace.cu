@@ -116,7 +116,7 @@ cudaError_t launch_trace_closest(const DevTree& T, const float* d_rays, uint64_t
     if (e != cudaSuccess) return e;
     // blocks per SM from the occupancy calculator for this stack size
     int per_sm = 1;
-    // 0: the 6-CTA variant (80 registers; 2^24 rays: 2.23 ms, 2.38 with 7, 2.64 with 5, 2.69 with 8)
+    // 0: the 6-CTA variant (80 registers; 2^24 rays: 2.22 ms, 2.36 with 7, 2.50 with 8, 2.52 with 5)
     const int variant = ctas_per_sm ? ctas_per_sm : 6;
     const auto kern = variant >= 8   ? k_trace_closest<8>
                       : variant >= 7 ? k_trace_closest<7>

@@ -535,7 +535,7 @@ static ShadowTraceKernel shadow_trace_kernel(int ctas_per_sm, bool walk) {
 }
 
 // the extend kernel for a configuration: register cap from ctas_per_sm
-// (0 = the 6-CTA variant: mixed-material scene 1024^2 x 32 spp 33.2 ms, 33.9 with 7, 36.3 with 8)
+// (0 = the 6-CTA variant: mixed-material scene 1024^2 x 16 spp 15.3 ms, 16.2 with 7, 16.9 with 5, 17.1 with 8)
 static ExtendKernel extend_kernel(int ctas_per_sm, bool stats, bool walk) {
     if (walk) return stats ? k_wf_extend<true, true, 6> : k_wf_extend<false, true, 6>;
     if (ctas_per_sm == 0) ctas_per_sm = 6;
